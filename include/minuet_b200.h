@@ -89,7 +89,7 @@ typedef struct {
 /* Version of this interface; mn_version() returns the value the library was
  * built with.  A binding should refuse a library whose version differs from the
  * header it was written against: argument lists change between versions. */
-#define MN_ABI_VERSION 14
+#define MN_ABI_VERSION 15
 
 const char *mn_last_error(void);
 int mn_version(void);

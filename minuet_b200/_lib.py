@@ -15,7 +15,7 @@ MN_F32, MN_F16, MN_BF16 = 0, 1, 2
 MN_MAX_NDIM = 4
 MN_MAX_OFFSETS = 128
 MN_CTRL_WORDS = 1024
-ABI_VERSION = 14         # must equal MN_ABI_VERSION of the header the library was built from
+ABI_VERSION = 15         # must equal MN_ABI_VERSION of the header the library was built from
 
 c_i32p = ctypes.c_void_p
 c_ptr = ctypes.c_void_p

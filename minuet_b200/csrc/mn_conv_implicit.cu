@@ -6,20 +6,28 @@
 // crosses HBM four times.  Here one persistent kernel owns 128 consecutive TARGET
 // rows at a time and accumulates ALL kernel offsets of that tile in one TMEM
 // accumulator:
-//   warps 0..7  producers: warp w fetches, for every active offset and k-block, the
-//               128-byte slices of the source rows that feed target rows 16w..16w+15
-//               (cp.async straight into the 128-byte-swizzled A tile, eight lanes per
-//               row, zeros where the kernel map has no entry); thread 0 also starts
-//               the TMA load of the offset's transposed weight tile
-//   warp 8      allocates TMEM and issues tcgen05.mma over (offset, k-block)
-//   warps 9..12 epilogue: TMEM -> registers -> optional per-channel scale/shift
-//               (folded BatchNorm or bias), residual add, ReLU -> swizzled shared
-//               tile -> TMA store of the output rows
+//   warps 0..7   producers: warp w fetches, for every active offset and k-block, the
+//                128-byte slices of the source rows that feed target rows 16w..16w+15
+//                (cp.async straight into the 128-byte-swizzled A tile, zeros where the
+//                kernel map has no entry)
+//   warp 8       allocates TMEM and issues tcgen05.mma over (offset, k-block)
+//   warp 9       starts the copy of every step's index block and the TMA load of every
+//                stage's transposed weight tile
+//   warps 10..13 epilogue: TMEM -> registers -> optional per-channel scale/shift
+//                (folded BatchNorm or bias), residual add, ReLU -> the output rows
 // so that features are read once per pair (mostly from L2), outputs are written
 // once, and no pair-row buffer exists.  Offsets with no pair inside a tile are
 // skipped through a per-tile bit mask.  The neighbour table [O, T] (source row
 // of target t under mask row p, or -1) is derived once per kernel map from the
 // masks by mn_build_neighbor_table.  Every barrier wait is bounded (status bit 2).
+//
+// What bounds it: the control code between two stages.  A 128 x 64 stage is 256 cycles
+// of tensor time at 128 output columns and about 280 of L2 time, but a warp needs five
+// cycles per dependent instruction, so every role's loop is kept short: the issuing
+// warps stay converged and elect one lane only around the instruction itself (issued
+// from a divergent lane-0 branch every MMA took about 150 cycles of register moves), a
+// lane reads the indices of all its rows with one load, two offsets ahead, and the next
+// stage's barrier is probed before the current stage is worked on.
 #include "mn_tc.cuh"
 
 #include <algorithm>
@@ -32,18 +40,22 @@ using namespace tc;
 
 constexpr int kProdWarps = 8;          // producer warps: warp w owns 128 / kProdWarps rows of a sub-tile
 constexpr int kProdRows = 128 / kProdWarps;
-constexpr int kMmaWarp = kProdWarps;   // then the MMA issuer, then four epilogue warps
-constexpr int kImThreads = (kProdWarps + 5) * 32;
-constexpr int kImCtas = kProdWarps > 4 ? 2 : 3;   // CTAs per SM the register file allows
+constexpr int kMmaWarp = kProdWarps;
+constexpr int kTmaWarp = kProdWarps + 1;
+constexpr int kEpiWarp = kProdWarps + 2;   // the first of four
+constexpr int kImThreads = (kProdWarps + 6) * 32;
+constexpr int kImCtas = 2;             // CTAs per SM the register file allows
 constexpr int kBM = 128;
 constexpr int kBK = 64;
 constexpr int kUmmaK = 16;
-constexpr int kMaxStages = 10;
-constexpr int kMaxSub = 4;             // 128-row sub-tiles per CTA tile
+constexpr int kMaxStages = 8;
+constexpr int kMaxN = 256;
+constexpr int kIdxSlots = 8;           // steps the index blocks run ahead
+constexpr int kMaxSub = 2;             // 128-row sub-tiles per CTA tile
 
 struct ImArgs {
   const uint8_t *in;          // [S, K] 16-bit
-  const int32_t *nbr;         // [O, T]
+  const int32_t *nbr;         // [O, pitch]
   const uint32_t *tile_bits;  // [tiles]
   const int32_t *order;       // [O] or NULL
   const float *scale;         // [N] or NULL
@@ -51,8 +63,9 @@ struct ImArgs {
   const uint8_t *residual;    // [T, N] 16-bit or NULL
   int32_t *status;
   int64_t T;
+  int64_t pitch;              // of the neighbour table: T rounded up to 128
   int32_t K, N, n_pad, k_blocks, stages, a_bytes, stage_bytes, elem_is_bf16, num_tiles, relu;
-  int32_t sub;         // 128-row sub-tiles per CTA tile (1..4): they share every weight tile
+  int32_t wide;        // rows of the output and the residual start on 32-byte boundaries
   int32_t acc_bufs;    // accumulator sets in TMEM (2 when 2 * sub * n_pad <= 512, else 1)
   int32_t n_tiles128;  // entries of tile_bits
   int32_t num_offsets; // O
@@ -60,12 +73,11 @@ struct ImArgs {
   // pair mode (step 1 of the pair-list forward): the rows are PRODUCT rows, row r reads
   // source row nbr[r], every tile has exactly one "offset" whose weight matrix follows from
   // the mask row that owns the tile, and the fp32 accumulators are stored as they are
-  int32_t pair_mode;
   int32_t pair_rows;                            // mask rows in pair_tile_prefix
   int32_t pair_tile_prefix[MN_MAX_PAIR_ROWS + 1];
   float *out_f32;                               // [T, N]
   const int32_t *perm;   // [T] or NULL: tile row r is target row perm[r] (nbr is in tile-row order)
-  uint8_t *out16;        // [T, N] 16-bit output, addressed row by row when perm is given
+  uint8_t *out16;        // [T, N] 16-bit output
 };
 
 // mask row that owns 128-row tile `tile` of the product buffer
@@ -85,25 +97,86 @@ __device__ __forceinline__ void cp_async_16(uint32_t dst, const void *src, uint3
                : "memory");
 }
 
+// One 32-byte sector of global memory per lane.
+__device__ __forceinline__ void ld_global_32(const void *src, uint32_t *r) {
+  asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+                 "=r"(r[7])
+               : "l"(src));
+}
+
+__device__ __forceinline__ void ld_global_16(const void *src, uint32_t *r) {
+  const uint4 v = *reinterpret_cast<const uint4 *>(src);
+  r[0] = v.x; r[1] = v.y; r[2] = v.z; r[3] = v.w;
+}
+
+__device__ __forceinline__ void st_global_32(void *dst, const uint32_t *r) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(r[0]),
+               "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+               : "memory");
+}
+
 template <bool kBf16>
 __device__ __forceinline__ float elem_to_f32(uint16_t v) {
   if (kBf16) return __uint_as_float((uint32_t)v << 16);
   return __half2float(__ushort_as_half(v));
 }
 
+// Loads that are issued where they stand: an ordinary read-only load may be moved down to its
+// first use, a step or a tile later, where its whole latency would be waited for.
+__device__ __forceinline__ int32_t load_ahead_1(const void *src) {
+  int32_t v;
+  asm volatile("ld.global.nc.b32 %0, [%1];" : "=r"(v) : "l"(src));
+  return v;
+}
+
+// 16-byte aligned block of global memory -> shared memory
+__device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {
+  asm volatile(
+      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+          smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar))
+      : "memory");
+}
+
+// Offset bits of the sub-tiles of a CTA tile (pair mode: one offset each).
+template <int kSub, bool kPairs>
+__device__ __forceinline__ void load_tile_bits(const ImArgs &args, int tile, uint32_t (&hb)[kSub]) {
+#pragma unroll
+  for (int h = 0; h < kSub; h++) {
+    hb[h] = 0u;
+    if (tile < args.num_tiles && tile * kSub + h < args.n_tiles128)
+      hb[h] = kPairs ? 1u : (uint32_t)load_ahead_1(args.tile_bits + tile * kSub + h);
+  }
+}
+
+template <int kSub>
+__device__ __forceinline__ uint32_t union_of(const uint32_t (&hb)[kSub]) {
+  uint32_t u = 0u;
+#pragma unroll
+  for (int h = 0; h < kSub; h++) u |= hb[h];
+  return u;
+}
+
+// kSub: sub-tiles per CTA tile (they share every weight tile); kLpr: lanes that copy one
+// 128-byte slice (4 where a source row has at most 64 bytes: half the copies, twice the rows
+// per copy); kPairs: pair mode.
+template <int kSub, int kLpr, bool kPairs>
 __global__ void __launch_bounds__(kImThreads, kImCtas)
 conv_implicit_kernel(const __grid_constant__ ImArgs args,
-                     const __grid_constant__ CUtensorMap map_b,     // weights^T [O, N, K]
-                     const __grid_constant__ CUtensorMap map_out) { // output    [T, N]
+                     const __grid_constant__ CUtensorMap map_b) {   // weights^T [O, N, K]
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   __shared__ uint64_t bar_full[kMaxStages], bar_empty[kMaxStages];
   __shared__ uint64_t bar_acc_full[2], bar_acc_empty[2];
+  __shared__ uint64_t bar_idx_full[kIdxSlots], bar_idx_empty[kIdxSlots];
+  __shared__ uint32_t s_idx_has[kIdxSlots];
   __shared__ uint32_t s_tmem_base;
   __shared__ int s_abort;
+  __shared__ __align__(16) float s_scale[kMaxN], s_shift[kMaxN];
 
   uint8_t *stage_base = reinterpret_cast<uint8_t *>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  int32_t *idx_ring = reinterpret_cast<int32_t *>(stage_base + (size_t)args.stages * args.stage_bytes);
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int stages = args.stages;
   const uint32_t tmem_cols = (uint32_t)args.tmem_cols;
 
@@ -113,8 +186,15 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
       mbar_init(&bar_empty[s], 1);
     }
     for (int a = 0; a < 2; a++) { mbar_init(&bar_acc_full[a], 1); mbar_init(&bar_acc_empty[a], 4); }
+    for (int i = 0; i < kIdxSlots; i++) { mbar_init(&bar_idx_full[i], 1); mbar_init(&bar_idx_empty[i], kProdWarps); }
     s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (!kPairs && (args.scale != nullptr || args.shift != nullptr)) {
+    for (int c = threadIdx.x; c < args.n_pad; c += kImThreads) {
+      s_scale[c] = args.scale != nullptr && c < args.N ? __ldg(args.scale + c) : 1.f;
+      s_shift[c] = args.shift != nullptr && c < args.N ? __ldg(args.shift + c) : 0.f;
+    }
   }
   if (warp == kMmaWarp) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
@@ -130,311 +210,331 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
 
   if (warp < kProdWarps) {
     // ------------------------------ producers ---------------------------------
-    // Eight warps feed the ring; warp w owns rows 16w .. 16w+15 of every 128-row sub-tile
-    // and lane l holds the source row of row 16w + (l & 15) (one coalesced load from the
-    // neighbour table per offset, the next offset's requested before the current one is
-    // copied).  Per stage eight lanes copy one row: a warp-wide cp.async reads four whole
-    // 128-byte lines (16 bytes of 32 different lines would cost a tag lookup per lane),
-    // zero fill where the kernel map has no source.  Each lane's arrival on the stage
-    // barrier fires when its copies have landed.  All sub-tiles of a CTA tile share every
-    // weight tile.  A stage is a serial chain per CTA (about 120 cycles per cp.async a
-    // thread issues): four producer warps with eight copies each were 5-18 % slower, a
-    // single producer warp 2.5x slower.
-    const int sub = args.sub;
-    const uint32_t b_bytes = (uint32_t)(args.stage_bytes - args.a_bytes);
-    const int chunk = lane & 7;
-    int stage = 0;
-    uint32_t phase = 0;
+    // Lane l of warp w copies 16-byte piece l % kLpr of rows r0 .. r0 + kRpl - 1 of every
+    // sub-tile, r0 = 16 w + kRpl (l / kLpr): the lane's indices are consecutive in the index
+    // block (one 8- or 16-byte shared-memory load per offset and sub-tile), and a warp-wide
+    // copy reads whole 128-byte lines.  Each lane's arrival on the stage barrier fires when its
+    // copies have landed.
+    constexpr int kRpl = kProdRows * kLpr / 32;   // rows per lane and sub-tile
+    const int chunk = lane % kLpr;
+    const int r0 = warp * kProdRows + (lane / kLpr) * kRpl;
+    const uint32_t ring = smem_u32(stage_base);
+    const uint32_t row_bytes = (uint32_t)args.K * 2u;
+    uint32_t dst0[kRpl];                           // place of the lane's pieces inside a sub-tile
+#pragma unroll
+    for (int i = 0; i < kRpl; i++)
+      dst0[i] = (uint32_t)(r0 + i) * 128u + (uint32_t)((chunk ^ ((r0 + i) & 7)) << 4);
+    int stage = 0, slot = 0;
+    uint32_t phase = 0, slot_phase = 0;
     bool alive = true;
-    for (int tile = blockIdx.x; alive && tile < args.num_tiles; tile += gridDim.x) {
-      uint32_t rest = 0u, hb[kMaxSub];   // offsets of the CTA tile and of each sub-tile
+    bool ready = mbar_test(&bar_empty[0], 1u);
+    while (alive) {
+      if (!mbar_wait(&bar_idx_full[slot], slot_phase, abort_flag, args.status)) break;
+      const uint32_t has = s_idx_has[slot];        // sub-tiles that have this offset; 0: no more steps
+      if (has == 0u) break;
+      int32_t q[kSub][kRpl];
 #pragma unroll
-      for (int h = 0; h < kMaxSub; h++) {
-        hb[h] = 0u;
-        if (h < sub && tile * sub + h < args.n_tiles128)
-          hb[h] = args.pair_mode ? 1u : __ldg(args.tile_bits + tile * sub + h);
-        rest |= hb[h];
+      for (int h = 0; h < kSub; h++) {
+        const int32_t *at = idx_ring + (slot * kSub + h) * kBM + r0;
+        if (kRpl == 4) {
+          const int4 v = *reinterpret_cast<const int4 *>(at);
+          q[h][0] = v.x; q[h][1] = v.y; q[h][kRpl - 2] = v.z; q[h][kRpl - 1] = v.w;
+        } else {
+          const int2 v = *reinterpret_cast<const int2 *>(at);
+          q[h][0] = v.x; q[h][1] = v.y;
+        }
       }
-      const int pair_row = args.pair_mode ? pair_row_of_tile(args, tile) : 0;
-      int p = rest != 0u ? __ffs(rest) - 1 : -1;
-      int src[kMaxSub], src_next[kMaxSub];
-      auto fetch = [&](int pp, int (&dst)[kMaxSub]) {
-#pragma unroll
-        for (int h = 0; h < kMaxSub; h++) {
-          const int64_t t = ((int64_t)tile * sub + h) * kBM + warp * kProdRows + (lane & (kProdRows - 1));
-          // a sub-tile without offset pp has no table block: its rows are zero rows
-          dst[h] = (pp >= 0 && ((hb[h] >> pp) & 1u) && t < args.T) ? __ldg(args.nbr + (int64_t)pp * args.T + t) : -1;
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bar_idx_empty[slot]);
+      if (++slot == kIdxSlots) { slot = 0; slot_phase ^= 1u; }
+      for (int kb = 0; kb < args.k_blocks; kb++) {
+        if (!ready && !mbar_wait(&bar_empty[stage], phase ^ 1u, abort_flag, args.status)) {
+          alive = false;
+          break;
         }
-      };
-      fetch(p, src);
-      while (alive && p >= 0) {
-        rest &= rest - 1u;
-        const int p_next = rest != 0u ? __ffs(rest) - 1 : -1;
-        fetch(p_next, src_next);
-        for (int kb = 0; kb < args.k_blocks; kb++) {
-          int ok = 1;   // one lane polls the barrier, the warp follows
-          if (lane == 0) ok = mbar_wait(&bar_empty[stage], phase ^ 1u, abort_flag, args.status) ? 1 : 0;
-          ok = __shfl_sync(0xffffffffu, ok, 0);
-          if (!ok) { alive = false; break; }
-          uint8_t *sa = stage_base + (size_t)stage * args.stage_bytes;
-          if (threadIdx.x == 0) {
-            const int wrow = args.pair_mode ? pair_row : p;
-            const int widx = args.order != nullptr ? __ldg(args.order + wrow) : wrow;
-            mbar_expect_tx(&bar_full[stage], b_bytes);
-            tma_load_3d(sa + args.a_bytes, &map_b, kb * kBK, 0, widx, &bar_full[stage]);
-          }
-          const int kcol = kb * kBK + chunk * 8;
+        const uint32_t sa = ring + (uint32_t)(stage * args.stage_bytes);
+        const int kcol = kb * kBK + chunk * 8;
+        const uint8_t *src = args.in + kcol * 2;
+        const bool inside = kcol < args.K;
+        uint64_t *full = &bar_full[stage];
+        if (++stage == stages) { stage = 0; phase ^= 1u; }
+        ready = mbar_test(&bar_empty[stage], phase ^ 1u);   // of the next stage
 #pragma unroll
-          for (int h = 0; h < kMaxSub; h++) {
-            if (h < sub) {
+        for (int h = 0; h < kSub; h++) {
+          // a sub-tile without this offset has no index block: its rows are zero rows
+          const bool use = inside && (kSub == 1 || ((has >> h) & 1u) != 0u);
 #pragma unroll
-              for (int i = 0; i < kProdRows / 4; i++) {
-                const int owner = 4 * i + (lane >> 3);           // lane that holds this row's index
-                const int s_idx = __shfl_sync(0xffffffffu, src[h], owner);
-                const int rr = warp * kProdRows + owner;           // row inside the sub-tile
-                const uint32_t dst = smem_u32(sa) + (uint32_t)(h * kBM + rr) * 128u +
-                                     (uint32_t)((chunk ^ (rr & 7)) << 4);
-                const bool valid = s_idx >= 0 && kcol < args.K;
-                cp_async_16(dst, valid ? args.in + ((int64_t)s_idx * args.K + kcol) * 2 : args.in,
-                            valid ? 16u : 0u);
-              }
-            }
+          for (int i = 0; i < kRpl; i++) {
+            const bool valid = q[h][i] >= 0 && use;
+            cp_async_16(sa + (uint32_t)(h * kBM * 128) + dst0[i],
+                        valid ? src + (uint64_t)(uint32_t)q[h][i] * row_bytes : args.in, valid ? 16u : 0u);
           }
-          // this lane's arrival fires when its copies above have landed: no stall here
-          asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(
-                           smem_u32(&bar_full[stage]))
-                       : "memory");
-          if (++stage == stages) { stage = 0; phase ^= 1u; }
         }
-        p = p_next;
-#pragma unroll
-        for (int h = 0; h < kMaxSub; h++) src[h] = src_next[h];
+        // this lane's arrival fires when its copies above have landed: no stall here
+        asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(full))
+                     : "memory");
       }
     }
     asm volatile("cp.async.wait_all;" ::: "memory");   // nothing of this lane is in flight at exit
   } else if (warp == kMmaWarp) {
     // ------------------------------ MMA issuer --------------------------------
-    if (lane == 0) {
-      const uint32_t fmt = args.elem_is_bf16 ? 1u : 0u;
-      const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) |
-                             ((uint32_t)(args.n_pad >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
-      int stage = 0, acc = 0;
-      uint32_t phase = 0, acc_phase = 0;
-      bool alive = true;
-      for (int tile = blockIdx.x; alive && tile < args.num_tiles; tile += gridDim.x) {
-        if (!mbar_wait(&bar_acc_empty[acc], acc_phase ^ 1u, abort_flag, args.status)) break;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t tmem_d = tmem_base + (uint32_t)(acc * args.sub * args.n_pad);
-        uint32_t tb = 0u;
-        for (int h = 0; h < args.sub; h++)
-          if (tile * args.sub + h < args.n_tiles128)
-            tb |= args.pair_mode ? 1u : __ldg(args.tile_bits + tile * args.sub + h);
-        const int n_stage = __popc(tb) * args.k_blocks;
-        uint32_t accumulate = 0u;
-        for (int it = 0; it < n_stage; it++) {
-          const int kb = it % args.k_blocks;
-          if (!mbar_wait(&bar_full[stage], phase, abort_flag, args.status)) { alive = false; break; }
+    const uint32_t fmt = args.elem_is_bf16 ? 1u : 0u;
+    const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) |
+                           ((uint32_t)(args.n_pad >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
+    const uint64_t desc0 = umma_desc(smem_u32(stage_base));
+    const uint32_t desc_hi = (uint32_t)(desc0 >> 32), desc_lo = (uint32_t)desc0;
+    const uint32_t stage_step = (uint32_t)args.stage_bytes >> 4, b_step = (uint32_t)args.a_bytes >> 4;
+    const int last_nk = (args.K - (args.k_blocks - 1) * kBK + kUmmaK - 1) / kUmmaK;
+    int stage = 0, acc = 0;
+    uint32_t phase = 0, acc_phase = 0;
+    bool alive = true;
+    uint32_t hb_next[kSub];
+    load_tile_bits<kSub, kPairs>(args, (int)blockIdx.x, hb_next);
+    bool ready = mbar_test(&bar_full[0], 0u);
+    for (int tile = blockIdx.x; alive && tile < args.num_tiles; tile += gridDim.x) {
+      const int n_offsets = __popc(union_of<kSub>(hb_next));
+      load_tile_bits<kSub, kPairs>(args, tile + (int)gridDim.x, hb_next);
+      if (!mbar_wait_warp(false, &bar_acc_empty[acc], acc_phase ^ 1u, abort_flag, args.status)) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint32_t tmem_d = tmem_base + (uint32_t)(acc * kSub * args.n_pad);
+      uint32_t accumulate = 0u;
+      for (int o = 0; alive && o < n_offsets; o++) {
+        for (int kb = 0; kb < args.k_blocks; kb++) {
+          if (!mbar_wait_warp(ready, &bar_full[stage], phase, abort_flag, args.status)) { alive = false; break; }
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t sa = smem_u32(stage_base + (size_t)stage * args.stage_bytes);
-          const uint32_t sb = sa + (uint32_t)args.a_bytes;
-          const int nk = min(kBK / kUmmaK, (args.K - kb * kBK + kUmmaK - 1) / kUmmaK);
-          for (int k = 0; k < nk; k++) {
-            const uint64_t db = umma_desc(sb + k * kUmmaK * 2);   // one weight tile, all sub-tiles
-            for (int h = 0; h < args.sub; h++)
-              umma_f16(tmem_d + (uint32_t)(h * args.n_pad),
-                       umma_desc(sa + h * (kBM * kBK * 2) + k * kUmmaK * 2), db, idesc, accumulate);
-            accumulate = 1u;
-          }
-          umma_commit(&bar_empty[stage]);
+          const uint32_t lo = desc_lo + (uint32_t)stage * stage_step;
+          const int nk = kb + 1 < args.k_blocks ? kBK / kUmmaK : last_nk;
+          uint64_t *empty = &bar_empty[stage];
           if (++stage == stages) { stage = 0; phase ^= 1u; }
+          ready = mbar_test(&bar_full[stage], phase);      // of the next stage
+          if (elect_one()) {
+#pragma unroll
+            for (int k = 0; k < kBK / kUmmaK; k++) {
+              if (k < nk) {
+                const uint64_t db = umma_desc_at(desc_hi, lo + b_step + k * (kUmmaK * 2 / 16));
+#pragma unroll
+                for (int h = 0; h < kSub; h++)                 // one weight tile, all sub-tiles
+                  umma_f16(tmem_d + (uint32_t)(h * args.n_pad),
+                           umma_desc_at(desc_hi, lo + h * (kBM * 128 / 16) + k * (kUmmaK * 2 / 16)), db,
+                           idesc, k == 0 ? accumulate : 1u);
+              }
+            }
+            umma_commit(empty);
+          }
+          accumulate = 1u;
         }
-        if (!alive) break;
-        umma_commit(&bar_acc_full[acc]);
-        if (++acc == args.acc_bufs) { acc = 0; acc_phase ^= 1u; }
+      }
+      if (!alive) break;
+      if (elect_one()) umma_commit(&bar_acc_full[acc]);
+      if (++acc == args.acc_bufs) { acc = 0; acc_phase ^= 1u; }
+    }
+  } else if (warp == kTmaWarp) {
+    // ------------------- index blocks and weight tiles --------------------------
+    // Two cursors over the same stream of (tile, offset) steps: the index blocks (128 entries
+    // of the neighbour table per sub-tile, one bulk copy each) run kIdxSlots steps ahead of
+    // the weight tiles, so that the producers never wait for an index from memory (loaded by
+    // the producers themselves, even two steps ahead, they cost a quarter of the time).
+    const uint32_t b_bytes = (uint32_t)(args.stage_bytes - args.a_bytes);
+    const int my_order = lane < args.num_offsets && args.order != nullptr ? __ldg(args.order + lane) : lane;
+    bool alive = true;
+    int itile = (int)blockIdx.x - (int)gridDim.x, slot = 0;
+    uint32_t irest = 0u, slot_phase = 0, ihb[kSub], ihb_next[kSub];
+    load_tile_bits<kSub, kPairs>(args, (int)blockIdx.x, ihb_next);
+    bool more = true;          // false once the end mark is out
+    auto send_indices = [&]() {
+      while (irest == 0u && itile < args.num_tiles) {
+        itile += (int)gridDim.x;
+#pragma unroll
+        for (int h = 0; h < kSub; h++) ihb[h] = ihb_next[h];
+        irest = union_of<kSub>(ihb);
+        load_tile_bits<kSub, kPairs>(args, itile + (int)gridDim.x, ihb_next);
+      }
+      if (!mbar_wait_warp(false, &bar_idx_empty[slot], slot_phase ^ 1u, abort_flag, args.status)) {
+        alive = false;
+        return;
+      }
+      uint32_t has = 0u;
+      int p = 0;
+      if (irest != 0u) {
+        p = __ffs(irest) - 1;
+        irest &= irest - 1u;
+#pragma unroll
+        for (int h = 0; h < kSub; h++) has |= ((ihb[h] >> p) & 1u) << h;
+      } else {
+        more = false;
+      }
+      if (elect_one()) {
+        s_idx_has[slot] = has;
+        if (has == 0u) {
+          mbar_arrive(&bar_idx_full[slot]);
+        } else {
+          mbar_expect_tx(&bar_idx_full[slot], (uint32_t)__popc(has) * (kBM * 4u));
+          const int32_t *src = args.nbr + (int64_t)p * args.pitch + (int64_t)itile * (kSub * kBM);
+#pragma unroll
+          for (int h = 0; h < kSub; h++)
+            if ((has >> h) & 1u)
+              bulk_load(idx_ring + (slot * kSub + h) * kBM, src + h * kBM, kBM * 4u, &bar_idx_full[slot]);
+        }
+      }
+      __syncwarp();
+      if (++slot == kIdxSlots) { slot = 0; slot_phase ^= 1u; }
+    };
+    for (int i = 0; i < kIdxSlots && alive && more; i++) send_indices();
+
+    int stage = 0;
+    uint32_t phase = 0;
+    uint32_t hb_next[kSub];
+    load_tile_bits<kSub, kPairs>(args, (int)blockIdx.x, hb_next);
+    bool ready = mbar_test(&bar_empty[0], 1u);
+    for (int tile = blockIdx.x; alive && tile < args.num_tiles; tile += gridDim.x) {
+      uint32_t rest = union_of<kSub>(hb_next);
+      load_tile_bits<kSub, kPairs>(args, tile + (int)gridDim.x, hb_next);
+      const int pair_row = kPairs ? pair_row_of_tile(args, tile) : 0;
+      while (alive && rest != 0u) {
+        const int p = kPairs ? pair_row : __ffs(rest) - 1;
+        rest &= rest - 1u;
+        const int widx = __shfl_sync(0xffffffffu, my_order, p);
+        for (int kb = 0; kb < args.k_blocks; kb++) {
+          if (!mbar_wait_warp(ready, &bar_empty[stage], phase ^ 1u, abort_flag, args.status)) { alive = false; break; }
+          uint8_t *sb = stage_base + (size_t)stage * args.stage_bytes + args.a_bytes;
+          uint64_t *full = &bar_full[stage];
+          if (++stage == stages) { stage = 0; phase ^= 1u; }
+          ready = mbar_test(&bar_empty[stage], phase ^ 1u);
+          if (elect_one()) {
+            mbar_expect_tx(full, b_bytes);
+            tma_load_3d(sb, &map_b, kb * kBK, 0, widx, full);
+          }
+          __syncwarp();
+        }
+        if (alive && more) send_indices();
       }
     }
   } else {
     // ------------------------------ epilogue ----------------------------------
+    // A lane owns one accumulator row and takes it 16 columns at a time: one 32-byte store
+    // (a whole sector of the output row, wherever perm puts it) and, with a residual, one
+    // 32-byte load requested a piece ahead; the TMEM read of the next piece is in flight while
+    // one is worked on.  No shared-memory staging: its barriers and index shuffles cost more
+    // than the wider stores gave (a tile of 32 columns took 3400 cycles of SM time, most of it
+    // here), and the 32 KB are worth more as ring stages.
     const int quarter = warp & 3;
-    uint8_t *cbuf = stage_base + (size_t)stages * args.stage_bytes + (size_t)(warp - kMmaWarp - 1) * 8192;
-    int acc = 0, chunk = 0;   // chunk: 64-column chunks so far (parity = staging buffer)
+    const int n = args.N, pieces = args.n_pad / 16;
+    const bool affine = args.scale != nullptr || args.shift != nullptr;
+    int acc = 0;
     uint32_t acc_phase = 0;
-    const int n = args.N;
-    const int cps = (args.n_pad + 63) / 64;   // 64-column chunks per sub-tile
-    // The residual rows of a chunk are copied into the chunk's staging buffer (eight lanes
-    // per row, whole 128-byte lines, asynchronously and one chunk ahead); the lanes then add
-    // them from shared memory and overwrite them with the output.  Per-lane loads of 16
-    // bytes from 32 different rows cost the residual layers 15-35 % of their time.
-    const bool staged_res = args.residual != nullptr && args.out_f32 == nullptr;
-    auto stage_residual = [&](uint8_t *dst, int out_row, int64_t grow, int c0) {
-      const int piece = lane & 7;
-      const int col = c0 + piece * 8;
+    uint32_t hb_next[kSub];
+    load_tile_bits<kSub, kPairs>(args, (int)blockIdx.x, hb_next);
+    // row of the output (and of the residual) that this lane's accumulator row belongs to, per
+    // sub-tile (-1: none), requested a tile ahead
+    int32_t grow_next[kSub];
+    auto load_rows = [&](int tile) {
 #pragma unroll
-      for (int i = 0; i < 8; i++) {
-        const int rl = 4 * i + (lane >> 3);
-        const int64_t drow = __shfl_sync(0xffffffffu, grow, rl);
-        const bool valid = (int64_t)out_row + rl < args.T && col < n;
-        cp_async_16(smem_u32(dst + rl * 128 + ((piece ^ (rl & 7)) << 4)),
-                    valid ? args.residual + (drow * n + col) * 2 : args.residual, valid ? 16u : 0u);
+      for (int h = 0; h < kSub; h++) {
+        const int64_t row = ((int64_t)tile * kSub + h) * kBM + quarter * 32 + lane;
+        grow_next[h] = -1;
+        if (tile < args.num_tiles && row < args.T)
+          grow_next[h] = !kPairs && args.perm != nullptr ? load_ahead_1(args.perm + row) : (int32_t)row;
       }
-      asm volatile("cp.async.commit_group;" ::: "memory");
     };
+    load_rows((int)blockIdx.x);
     for (int tile = blockIdx.x; tile < args.num_tiles; tile += gridDim.x) {
-      // row of the output (and of the residual) this lane's accumulator row belongs to, per
-      // sub-tile; nsub = sub-tiles of this CTA tile that have rows for this warp
-      int64_t grow[kMaxSub];
-      int nsub = 0;
+      const bool empty_tile = union_of<kSub>(hb_next) == 0u;   // no MMA ran: the rows are zero
+      load_tile_bits<kSub, kPairs>(args, tile + (int)gridDim.x, hb_next);
+      int32_t grow[kSub];
 #pragma unroll
-      for (int h = 0; h < kMaxSub; h++) {
-        const int64_t row = (int64_t)(tile * args.sub + h) * kBM + quarter * 32 + lane;
-        grow[h] = row;
-        if (h < args.sub && row - lane < args.T) {
-          nsub = h + 1;
-          if (args.perm != nullptr && row < args.T) grow[h] = (int64_t)__ldg(args.perm + row);
+      for (int h = 0; h < kSub; h++) grow[h] = grow_next[h];
+      load_rows(tile + (int)gridDim.x);
+      uint32_t res[2][8];
+      auto load_residual = [&](uint32_t (&r)[8], int h, int c) {
+#pragma unroll
+        for (int i = 0; i < 8; i++) r[i] = 0u;
+        if (args.residual == nullptr || grow[h] < 0) return;
+        const uint8_t *src = args.residual + ((int64_t)grow[h] * n + c) * 2;
+        if (args.wide && c + 16 <= n) {
+          ld_global_32(src, r);
+        } else {
+          if (c < n) ld_global_16(src, r);
+          if (c + 8 < n) ld_global_16(src + 16, r + 4);
         }
-      }
-      auto grow_of = [&](int h) {
-        int64_t g = grow[0];
-#pragma unroll
-        for (int k = 1; k < kMaxSub; k++) g = h == k ? grow[k] : g;
-        return g;
       };
-      const int total = nsub * cps;
-      if (staged_res && total > 0) {
-        // the first chunk's residual rows travel while the MMAs run
-        if (args.perm == nullptr && lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-        __syncwarp();
-        stage_residual(cbuf + (chunk & 1) * 4096, tile * args.sub * kBM + quarter * 32, grow[0], 0);
-      }
-      int ok = 1;
-      if (lane == 0) ok = mbar_wait(&bar_acc_full[acc], acc_phase, abort_flag, args.status) ? 1 : 0;
-      ok = __shfl_sync(0xffffffffu, ok, 0);
-      if (!ok) break;
+      if (!kPairs) load_residual(res[0], 0, 0);
+      if (!mbar_wait_warp(false, &bar_acc_full[acc], acc_phase, abort_flag, args.status)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      uint32_t tb = 0u;
-      for (int h = 0; h < args.sub; h++)
-        if (tile * args.sub + h < args.n_tiles128)
-          tb |= args.pair_mode ? 1u : __ldg(args.tile_bits + tile * args.sub + h);
-      const bool empty_tile = tb == 0u;   // no pair in the whole tile: no MMA ran, the rows are zero
-      for (int q = 0; q < total; q++, chunk++) {
-        const int h = q / cps;
-        const int c0 = (q - h * cps) * 64;
-        const int out_row = (tile * args.sub + h) * kBM + quarter * 32;
-        const int64_t row = (int64_t)out_row + lane;
-        const int64_t grow_h = grow_of(h);
+      uint32_t v[2][16];
+#pragma unroll
+      for (int h = 0; h < kSub; h++) {
         const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) +
-                               (uint32_t)((acc * args.sub + h) * args.n_pad);
-        uint8_t *buf = cbuf + (chunk & 1) * 4096;
-        if (args.out_f32 == nullptr) {
-          // this chunk's buffer (and, with a staged residual, the next chunk's) must have
-          // been read by the bulk stores that used them
-          if (args.perm == nullptr && lane == 0) {
-            if (staged_res) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-            else asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-          }
+                               (uint32_t)((acc * kSub + h) * args.n_pad);
+        auto piece = [&](uint32_t (&cur)[16], uint32_t (&cur_res)[8], uint32_t (&nxt)[16],
+                         uint32_t (&nxt_res)[8], int q) {
           __syncwarp();
-        }
-        if (staged_res) {
-          if (q + 1 < total) {
-            const int h2 = (q + 1) / cps;
-            stage_residual(cbuf + ((chunk + 1) & 1) * 4096, (tile * args.sub + h2) * kBM + quarter * 32,
-                           grow_of(h2), (q + 1 - h2 * cps) * 64);
-            asm volatile("cp.async.wait_group 1;" ::: "memory");   // this chunk's rows have landed
-          } else {
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
-          }
-          __syncwarp();
-        }
-        // 32 columns at a time: the two halves fill one 64-column staging tile
-        for (int half = 0; half < 2; half++) {
-          const int cb = c0 + 32 * half;
-          if (cb >= args.n_pad) break;
-          uint32_t rr[32];
-          tmem_ld_32x32(taddr + (uint32_t)cb, rr);
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-          if (args.out_f32 != nullptr) {
+          const bool more = q + 1 < pieces;
+          if (more) tmem_ld_32x16(taddr + (uint32_t)(q + 1) * 16, nxt);
+          if (!kPairs) {
+            if (more) load_residual(nxt_res, h, (q + 1) * 16);
+            else if (h + 1 < kSub) load_residual(nxt_res, h + 1, 0);
+          }
+          const int c = q * 16;
+          if (grow[h] < 0) return;
+          if (kPairs) {
             // pair mode: the fp32 accumulators of this row go out as they are
-            if (row < args.T) {
-              float4 *dst = reinterpret_cast<float4 *>(args.out_f32 + row * n + cb);
+            float *dst = args.out_f32 + (int64_t)grow[h] * n + c;
 #pragma unroll
-              for (int v = 0; v < 8; v++)
-                if (cb + 4 * v < n)
-                  dst[v] = make_float4(__uint_as_float(rr[4 * v]), __uint_as_float(rr[4 * v + 1]),
-                                       __uint_as_float(rr[4 * v + 2]), __uint_as_float(rr[4 * v + 3]));
-            }
-            continue;
+            for (int i = 0; i < 4; i++)
+              if (c + 4 * i < n)
+                *reinterpret_cast<float4 *>(dst + 4 * i) =
+                    make_float4(__uint_as_float(cur[4 * i]), __uint_as_float(cur[4 * i + 1]),
+                                __uint_as_float(cur[4 * i + 2]), __uint_as_float(cur[4 * i + 3]));
+            return;
           }
-#pragma unroll
-          for (int v = 0; v < 4; v++) {
-            float f[8];
-#pragma unroll
-            for (int i = 0; i < 8; i++) f[i] = empty_tile ? 0.f : __uint_as_float(rr[v * 8 + i]);
-            const int c = cb + v * 8;
-            const int piece = half * 4 + v;
-            uint4 *slot = reinterpret_cast<uint4 *>(buf + lane * 128 + ((piece ^ (lane & 7)) << 4));
-            if (c < n) {
-              if (args.scale != nullptr) {   // n is a multiple of 8 here
-                const float4 s0 = __ldg(reinterpret_cast<const float4 *>(args.scale + c));
-                const float4 s1 = __ldg(reinterpret_cast<const float4 *>(args.scale + c) + 1);
-                f[0] *= s0.x; f[1] *= s0.y; f[2] *= s0.z; f[3] *= s0.w;
-                f[4] *= s1.x; f[5] *= s1.y; f[6] *= s1.z; f[7] *= s1.w;
-              }
-              if (args.shift != nullptr) {
-                const float4 s0 = __ldg(reinterpret_cast<const float4 *>(args.shift + c));
-                const float4 s1 = __ldg(reinterpret_cast<const float4 *>(args.shift + c) + 1);
-                f[0] += s0.x; f[1] += s0.y; f[2] += s0.z; f[3] += s0.w;
-                f[4] += s1.x; f[5] += s1.y; f[6] += s1.z; f[7] += s1.w;
-              }
-              if (staged_res) {
-                const uint4 rv = *slot;      // this row's residual piece (zeros past the last row)
-                const uint16_t *r16 = reinterpret_cast<const uint16_t *>(&rv);
-#pragma unroll
-                for (int i = 0; i < 8; i++)
-                  f[i] += args.elem_is_bf16 ? elem_to_f32<true>(r16[i]) : elem_to_f32<false>(r16[i]);
-              }
-              if (args.relu) {
-#pragma unroll
-                for (int i = 0; i < 8; i++) f[i] = fmaxf(f[i], 0.f);
-              }
-            }
-            uint4 out;
-            uint32_t *o32 = reinterpret_cast<uint32_t *>(&out);
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-              if (args.elem_is_bf16) {
-                __nv_bfloat162 pk = __floats2bfloat162_rn(f[2 * k], f[2 * k + 1]);
-                o32[k] = *reinterpret_cast<uint32_t *>(&pk);
-              } else {
-                __half2 pk = __floats2half2_rn(f[2 * k], f[2 * k + 1]);
-                o32[k] = *reinterpret_cast<uint32_t *>(&pk);
-              }
-            }
-            *slot = out;
-          }
-        }
-        if (args.out_f32 != nullptr) continue;
-        if (args.perm != nullptr) {
-          // permuted rows: eight lanes store one row's 128 bytes of this chunk, four rows
-          // per instruction, each row at its own place in the output
-          __syncwarp();
-          const int piece = lane & 7;
-          const int col = c0 + piece * 8;
+          uint32_t out[8];
 #pragma unroll
           for (int i = 0; i < 8; i++) {
-            const int rl = 4 * i + (lane >> 3);
-            const int64_t drow = __shfl_sync(0xffffffffu, grow_h, rl);
-            const uint4 v = *reinterpret_cast<const uint4 *>(buf + rl * 128 + ((piece ^ (rl & 7)) << 4));
-            if ((int64_t)out_row + rl < args.T && col < n)
-              *reinterpret_cast<uint4 *>(args.out16 + (drow * n + col) * 2) = v;
+            float lo = empty_tile ? 0.f : __uint_as_float(cur[2 * i]);
+            float hi = empty_tile ? 0.f : __uint_as_float(cur[2 * i + 1]);
+            if (affine) {
+              const float2 sc = *reinterpret_cast<const float2 *>(s_scale + c + 2 * i);
+              const float2 sh = *reinterpret_cast<const float2 *>(s_shift + c + 2 * i);
+              lo = lo * sc.x + sh.x;
+              hi = hi * sc.y + sh.y;
+            }
+            if (args.residual != nullptr) {
+              const uint32_t w = cur_res[i];
+              const uint16_t a = (uint16_t)(w & 0xffffu), b = (uint16_t)(w >> 16);
+              lo += args.elem_is_bf16 ? elem_to_f32<true>(a) : elem_to_f32<false>(a);
+              hi += args.elem_is_bf16 ? elem_to_f32<true>(b) : elem_to_f32<false>(b);
+            }
+            if (args.relu) { lo = fmaxf(lo, 0.f); hi = fmaxf(hi, 0.f); }
+            if (args.elem_is_bf16) {
+              __nv_bfloat162 pk = __floats2bfloat162_rn(lo, hi);
+              out[i] = *reinterpret_cast<uint32_t *>(&pk);
+            } else {
+              __half2 pk = __floats2half2_rn(lo, hi);
+              out[i] = *reinterpret_cast<uint32_t *>(&pk);
+            }
           }
-          __syncwarp();
-          continue;
-        }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          uint8_t *dst = args.out16 + ((int64_t)grow[h] * n + c) * 2;
+          if (args.wide && c + 16 <= n) {
+            st_global_32(dst, out);
+          } else {
+            if (c < n) *reinterpret_cast<uint4 *>(dst) = make_uint4(out[0], out[1], out[2], out[3]);
+            if (c + 8 < n) *reinterpret_cast<uint4 *>(dst + 16) = make_uint4(out[4], out[5], out[6], out[7]);
+          }
+        };
         __syncwarp();
-        if (lane == 0) {
-          tma_store_2d(&map_out, c0, out_row, buf);
-          asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        tmem_ld_32x16(taddr, v[0]);
+        int q = 0;
+        for (; q + 1 < pieces; q += 2) {
+          piece(v[0], res[0], v[1], res[1], q);
+          piece(v[1], res[1], v[0], res[0], q + 1);
+        }
+        if (q < pieces) {
+          piece(v[0], res[0], v[1], res[1], q);
+          if (h + 1 < kSub) {   // the next sub-tile's first residual piece landed in the other set
+#pragma unroll
+            for (int i = 0; i < 8; i++) res[0][i] = res[1][i];
+          }
         }
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -442,8 +542,6 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
       if (lane == 0) mbar_arrive(&bar_acc_empty[acc]);
       if (++acc == args.acc_bufs) { acc = 0; acc_phase ^= 1u; }
     }
-    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
-    __syncwarp();
   }
 
   // ------------------------------ teardown ------------------------------------
@@ -498,9 +596,11 @@ rank_to_source_bits_kernel(const int32_t *__restrict__ source_masks,
 // (or -1); bit p of tile_bits[r / 128] is set when any row of that 128-row tile has such a
 // source.  With the targets' hit words (`bits`) only the (tile, p) blocks whose bit is set
 // are written, and a row looks its source up only for the offsets of its own word: the rest
-// of the table is never read by the forward pass, which checks tile_bits first.
+// of the table is never read by the forward pass, which checks tile_bits first.  The rows of
+// the table are `pitch` (T rounded up to 128) entries apart and -1 past T, so that the forward
+// pass reads whole tiles with vector loads.
 __global__ void __launch_bounds__(128)
-neighbor_table_kernel(const int32_t *__restrict__ target_masks, int64_t T, int O,
+neighbor_table_kernel(const int32_t *__restrict__ target_masks, int64_t T, int64_t pitch, int O,
                       const __grid_constant__ CumSizes cs,
                       const int32_t *__restrict__ src_of_rank, const int32_t *__restrict__ perm,
                       const uint32_t *__restrict__ bits, int32_t *__restrict__ nbr,
@@ -517,13 +617,12 @@ neighbor_table_kernel(const int32_t *__restrict__ target_masks, int64_t T, int O
     __syncthreads();
     const uint32_t tile = s_bits;
     if (threadIdx.x == 0) tile_bits[blockIdx.x] = tile;
-    if (r >= T) return;
     for (uint32_t rest = tile; rest != 0u; rest &= rest - 1u) {
       const int p = __ffs(rest) - 1;
       int v = -1;
       if ((mine >> p) & 1u)
         v = __ldg(src_of_rank + cs.cum[p] + __ldg(target_masks + (int64_t)p * T + t));
-      nbr[(int64_t)p * T + r] = v;
+      nbr[(int64_t)p * pitch + r] = v;
     }
     return;
   }
@@ -533,8 +632,8 @@ neighbor_table_kernel(const int32_t *__restrict__ target_masks, int64_t T, int O
     if (r < T) {
       const int m = __ldg(target_masks + (int64_t)p * T + t);
       if (m >= 0) v = __ldg(src_of_rank + cs.cum[p] + m);
-      nbr[(int64_t)p * T + r] = v;
     }
+    nbr[(int64_t)p * pitch + r] = v;
     mine |= (v >= 0 ? 1u : 0u) << p;
   }
   mine = __reduce_or_sync(0xffffffffu, mine);
@@ -563,6 +662,21 @@ __global__ void hit_word_keys_kernel(const uint32_t *__restrict__ bits, int64_t 
 
 }  // namespace
 
+namespace {
+
+template <int kSub, int kLpr, bool kPairs>
+mn_status launch_implicit(const ImArgs &a, const TcSizing &sizing, const CUtensorMap &map_b,
+                          cudaStream_t st) {
+  auto kernel = conv_implicit_kernel<kSub, kLpr, kPairs>;
+  MN_RETURN_IF(allow_max_shared_memory(reinterpret_cast<const void *>(kernel)));
+  const int grid = std::min(a.num_tiles, kNumSMs * sizing.ctas_per_sm);
+  MN_LAUNCH(kPairs ? "conv_implicit_kernel<pairs>" : "conv_implicit_kernel", st,
+            kernel<<<grid, kImThreads, sizing.smem_bytes, st>>>(a, map_b));
+  return MN_OK;
+}
+
+}  // namespace
+
 mn_status launch_pair_products(const PairPlan &plan, int64_t S, int64_t c_in, int64_t c_out, bool bf16,
                                const void *sources, const void *weights_t, int O,
                                const int32_t *pair_src, const int32_t *order, float *products,
@@ -571,7 +685,7 @@ mn_status launch_pair_products(const PairPlan &plan, int64_t S, int64_t c_in, in
   MN_CHECK_ARG(plan.total_rows > 0 && plan.total_rows % kBM == 0 && plan.total_rows < (1ll << 31),
                "pair products: bad product row count");
   MN_CHECK_ARG(((reinterpret_cast<uintptr_t>(sources) | reinterpret_cast<uintptr_t>(products) |
-                 reinterpret_cast<uintptr_t>(weights_t)) & 15) == 0,
+                 reinterpret_cast<uintptr_t>(weights_t) | reinterpret_cast<uintptr_t>(pair_src)) & 15) == 0,
                "pair products: arrays must be 16-byte aligned");
   ImArgs a{};
   a.in = static_cast<const uint8_t *>(sources);
@@ -585,30 +699,23 @@ mn_status launch_pair_products(const PairPlan &plan, int64_t S, int64_t c_in, in
   a.n_pad = (int)align_up((size_t)c_out, 16);
   a.k_blocks = (int)div_up(c_in, kBK);
   a.n_tiles128 = (int)(plan.total_rows / kBM);
-  a.sub = 1;
+  a.pitch = plan.total_rows;
   a.acc_bufs = 2;
   a.a_bytes = kBM * kBK * 2;
   a.stage_bytes = a.a_bytes + a.n_pad * kBK * 2;
-  const TcSizing sizing = size_tc_kernel(a.stage_bytes, a.acc_bufs * a.sub * a.n_pad, kMaxStages, kImCtas);
+  const TcSizing sizing = size_tc_kernel(a.stage_bytes, a.acc_bufs * a.n_pad, kMaxStages, kImCtas, kIdxSlots * kMaxSub * kBM * 4, kMaxStages);
   a.stages = sizing.stages;
   a.tmem_cols = sizing.tmem_cols;
-  a.num_offsets = 1;
+  a.num_offsets = O;
   a.elem_is_bf16 = bf16 ? 1 : 0;
   a.num_tiles = a.n_tiles128;
-  a.pair_mode = 1;
   a.pair_rows = plan.num_rows;
   for (int p = 0; p <= MN_MAX_PAIR_ROWS; p++) a.pair_tile_prefix[p] = plan.tile_prefix[p];
   a.out_f32 = products;
   CUtensorMap map_b;
   MN_RETURN_IF(make_kmajor_map(&map_b, weights_t, bf16, c_in, c_out, O, a.n_pad));
-  const size_t smem = sizing.smem_bytes;
-  MN_CHECK_CUDA(cudaFuncSetAttribute(conv_implicit_kernel,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const int grid = std::min(a.num_tiles, kNumSMs * sizing.ctas_per_sm);
-  // the output map is not used in pair mode; any valid map will do
-  MN_LAUNCH("conv_implicit_kernel<pairs>", st,
-            conv_implicit_kernel<<<grid, kImThreads, smem, st>>>(a, map_b, map_b));
-  return MN_OK;
+  return c_in <= 32 ? launch_implicit<1, 4, true>(a, sizing, map_b, st)
+                    : launch_implicit<1, 8, true>(a, sizing, map_b, st);
 }
 
 }  // namespace mn
@@ -682,7 +789,8 @@ extern "C" mn_status mn_build_neighbor_table(const int32_t *source_masks,
   }
   MN_LAUNCH("neighbor_table_kernel", st,
             neighbor_table_kernel<<<(unsigned)div_up(T, 128), 128, 0, st>>>(
-                target_masks, T, (int)O, cs, src_of_rank, perm_out, target_bits, nbr_out, tile_bits_out));
+                target_masks, T, (int64_t)align_up((size_t)T, kBM), (int)O, cs, src_of_rank, perm_out,
+                target_bits, nbr_out, tile_bits_out));
   return MN_OK;
 }
 
@@ -709,8 +817,8 @@ extern "C" mn_status mn_sparse_convolution_forward_implicit(
                    targets_out != nullptr && status_dev != nullptr && (S == 0 || sources != nullptr),
                "implicit forward: null pointer");
   MN_CHECK_ARG(((reinterpret_cast<uintptr_t>(sources) | reinterpret_cast<uintptr_t>(targets_out) |
-                 reinterpret_cast<uintptr_t>(residual)) & 15) == 0,
-               "implicit forward: feature arrays must be 16-byte aligned");
+                 reinterpret_cast<uintptr_t>(residual) | reinterpret_cast<uintptr_t>(nbr)) & 15) == 0,
+               "implicit forward: feature arrays and the neighbour table must be 16-byte aligned");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const bool bf16 = dtype == MN_BF16;
   Workspace ws(ws_ptr, ws_bytes);
@@ -739,43 +847,42 @@ extern "C" mn_status mn_sparse_convolution_forward_implicit(
   a.n_pad = (int)align_up((size_t)c_out, 16);
   a.k_blocks = (int)div_up(c_in, kBK);
   a.n_tiles128 = (int)div_up(T, kBM);
-  // Sub-tiles per CTA tile.  Every sub-tile of a CTA tile reuses the weight tile of a stage,
-  // at the price of a shallower ring and, past 512 / (2 * n_pad) sub-tiles, a single
-  // accumulator buffer (the epilogue then no longer overlaps the next tile's MMAs).  The
-  // automatic choice is the one that measured fastest per output width on maps with two or
-  // more pairs per row (1 sub-tile at 64 columns, 2 at 32, 128 and 256); sparse
-  // maps keep small CTA tiles and several CTAs per SM.  Callers that have timed the layer
+  // Sub-tiles per CTA tile.  The two sub-tiles of a CTA tile share the weight tile of a
+  // stage, at the price of a shallower ring; at 256 columns they also leave no room for a
+  // second accumulator set (the epilogue then no longer overlaps the next tile's MMAs).
+  // Measured on maps with 3.5 to 17 pairs per row (1 / 2 sub-tiles): 64 columns 155 / 191 us,
+  // 128 columns 399 / 366 us, 256 columns 535 / 593 us.  Callers that have timed the layer
   // pass their own choice.
   int sub = sub_hint;
   if (sub <= 0) {
     sub = 1;
-    if (pairs_per_row >= 2.0) sub = a.n_pad >= 128 ? 2 : a.n_pad >= 64 ? 1 : 2;
+    if (pairs_per_row >= 2.0 && a.n_pad > 64 && a.n_pad <= 128) sub = 2;
     while (sub > 1 && (sub * a.n_pad > 512 || a.n_tiles128 < 2 * sub * kNumSMs ||
-                       2 * (sub * kBM * kBK * 2 + a.n_pad * kBK * 2) + 4 * 8192 + 2048 > 227 * 1024))
+                       2 * (sub * kBM * kBK * 2 + a.n_pad * kBK * 2) + 2048 > 227 * 1024))
       sub--;
   }
-  MN_CHECK_ARG(sub >= 1 && sub <= kMaxSub && sub * a.n_pad <= 512,
-               "implicit forward: %d sub-tiles of %d columns do not fit TMEM", sub, a.n_pad);
-  a.sub = sub;
-  a.acc_bufs = 2 * a.sub * a.n_pad <= 512 ? 2 : 1;
-  a.a_bytes = a.sub * kBM * kBK * 2;
+  MN_CHECK_ARG(sub_hint <= 4 && (sub_hint <= 0 || sub_hint * a.n_pad <= 512),
+               "implicit forward: %d sub-tiles of %d columns do not fit TMEM", sub_hint, a.n_pad);
+  sub = std::min(sub, kMaxSub);
+  a.pitch = (int64_t)align_up((size_t)T, kBM);
+  a.acc_bufs = 2 * sub * a.n_pad <= 512 ? 2 : 1;
+  a.a_bytes = sub * kBM * kBK * 2;
   a.stage_bytes = a.a_bytes + a.n_pad * kBK * 2;
-  const TcSizing sizing = size_tc_kernel(a.stage_bytes, a.acc_bufs * a.sub * a.n_pad, kMaxStages, kImCtas);
+  const TcSizing sizing = size_tc_kernel(a.stage_bytes, a.acc_bufs * sub * a.n_pad, kMaxStages, kImCtas, kIdxSlots * kMaxSub * kBM * 4, kMaxStages);
   a.stages = sizing.stages;
   a.tmem_cols = sizing.tmem_cols;
   a.num_offsets = (int)O;
   a.elem_is_bf16 = bf16 ? 1 : 0;
-  a.num_tiles = (int)div_up(a.n_tiles128, a.sub);
+  a.num_tiles = (int)div_up(a.n_tiles128, sub);
   a.relu = relu ? 1 : 0;
+  a.wide = c_out % 16 == 0 && ((reinterpret_cast<uintptr_t>(targets_out) |
+                                reinterpret_cast<uintptr_t>(residual)) & 31) == 0;
 
-  CUtensorMap map_b, map_out;
+  CUtensorMap map_b;
   MN_RETURN_IF(make_kmajor_map(&map_b, weights_t, bf16, c_in, c_out, O, a.n_pad));
-  MN_RETURN_IF(make_kmajor_map(&map_out, targets_out, bf16, c_out, T, 0, 32));
-  const size_t smem = sizing.smem_bytes;
-  MN_CHECK_CUDA(cudaFuncSetAttribute(conv_implicit_kernel,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const int grid = std::min(a.num_tiles, kNumSMs * sizing.ctas_per_sm);
-  MN_LAUNCH("conv_implicit_kernel", st,
-            conv_implicit_kernel<<<grid, kImThreads, smem, st>>>(a, map_b, map_out));
-  return MN_OK;
+  if (sub == 1)
+    return c_in <= 32 ? launch_implicit<1, 4, false>(a, sizing, map_b, st)
+                      : launch_implicit<1, 8, false>(a, sizing, map_b, st);
+  return c_in <= 32 ? launch_implicit<2, 4, false>(a, sizing, map_b, st)
+                    : launch_implicit<2, 8, false>(a, sizing, map_b, st);
 }

@@ -602,14 +602,12 @@ mn_status launch_gemm_tc_impl(const GemmTable &tab_in, const TcOperands &ops, in
   const size_t smem = sizing.smem_bytes;
   const int grid = std::min(total_tiles, kNumSMs * sizing.ctas_per_sm);
   if (bf16) {
-    MN_CHECK_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<__nv_bfloat16>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    MN_RETURN_IF(allow_max_shared_memory(reinterpret_cast<const void *>(gemm_tc_kernel<__nv_bfloat16>)));
     MN_LAUNCH("gemm_tc_kernel", st,
               gemm_tc_kernel<__nv_bfloat16><<<grid, kTcThreads, smem, st>>>(
                   tab, args, map_a, map_direct, map_b, map_c, map_c_direct, epilogue));
   } else {
-    MN_CHECK_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<__half>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    MN_RETURN_IF(allow_max_shared_memory(reinterpret_cast<const void *>(gemm_tc_kernel<__half>)));
     MN_LAUNCH("gemm_tc_kernel", st,
               gemm_tc_kernel<__half><<<grid, kTcThreads, smem, st>>>(tab, args, map_a, map_direct,
                                                                     map_b, map_c, map_c_direct,

@@ -42,6 +42,20 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
   return ok != 0;
 }
 
+// Non-blocking probe: unlike try_wait it never suspends the thread, which must not happen
+// between a probe of the next stage and the work on the current one.
+__device__ __forceinline__ bool mbar_test(uint64_t *bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+
 // Bounded wait: false when the limit expired or another role already gave up.
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volatile int *abort_flag,
                                           int32_t *status) {
@@ -52,6 +66,14 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volati
   *abort_flag = 1;
   atomicOr(status, 4);
   return false;
+}
+
+// The same for a converged warp whose lanes go on together: every lane gets the same answer.
+// `ready`: an earlier probe of the same phase that succeeded.
+__device__ __forceinline__ bool mbar_wait_warp(bool ready, uint64_t *bar, uint32_t parity,
+                                               volatile int *abort_flag, int32_t *status) {
+  if (__all_sync(0xffffffffu, ready)) return true;
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status));
 }
 
 __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, int x, int y,
@@ -88,6 +110,24 @@ __device__ __forceinline__ uint64_t umma_desc(uint32_t smem_addr) {
   return d;
 }
 
+// The same descriptor from its constant upper word and a lower word that differs from
+// another descriptor's by (byte distance / 16).
+__device__ __forceinline__ uint64_t umma_desc_at(uint32_t hi, uint32_t lo) {
+  return ((uint64_t)hi << 32) | lo;
+}
+
+// One lane of a converged warp: the code around it stays warp-uniform, so that descriptors
+// and addresses live in uniform registers, where tcgen05.mma and the TMA read them.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t leader;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(leader));
+  return leader != 0u;
+}
+
 __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b,
                                          uint32_t idesc, uint32_t accumulate) {
   asm volatile(
@@ -117,6 +157,15 @@ __device__ __forceinline__ void tmem_ld_32x32(uint32_t taddr, uint32_t (&r)[32])
       : "r"(taddr));
 }
 
+__device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+        "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr));
+}
 
 }  // namespace tc
 
@@ -132,22 +181,39 @@ struct TcSizing {
   size_t smem_bytes;  // dynamic shared memory per CTA
 };
 inline TcSizing size_tc_kernel(int stage_bytes, int acc_cols, int max_stages, int max_ctas,
-                               int extra_bytes = 0) {
+                               int staging_bytes = 4 * 8192, int shared_sm_stages = 4) {
   TcSizing z{};
   z.tmem_cols = 32;
   while (z.tmem_cols < acc_cols) z.tmem_cols *= 2;
-  const int extra = 4 * 8192 + 1024 + extra_bytes;   // epilogue staging tiles + alignment slack
+  const int extra = staging_bytes + 1024;   // epilogue staging tiles + alignment slack
   for (int ctas = std::min(max_ctas, 512 / z.tmem_cols); ctas >= 1; ctas--) {
-    const int budget = (227 * 1024) / ctas - 2048;   // static shared memory and reserve
+    const int budget = (227 * 1024) / ctas - 4096;   // static shared memory and reserve
     const int stages = std::min(max_stages, (budget - extra) / stage_bytes);
     if (stages >= 2 || ctas == 1) {
       z.ctas_per_sm = ctas;
-      z.stages = std::max(2, ctas == 1 ? stages : std::min(stages, 4));
+      z.stages = std::max(2, ctas == 1 ? stages : std::min(stages, shared_sm_stages));
       break;
     }
   }
   z.smem_bytes = (size_t)z.stages * stage_bytes + extra;
   return z;
+}
+
+// Lets a kernel use all the dynamic shared memory that size_tc_kernel may give it.  The limit
+// is a property of the kernel on a device, whichever thread sets it, so every thread sets
+// the same value, once.
+constexpr int kMaxDynamicShared = 227 * 1024 - 4096;
+inline mn_status allow_max_shared_memory(const void *kernel) {
+  struct Seen { const void *kernel; int device; };
+  static thread_local Seen seen[32];
+  static thread_local int count = 0;
+  int device = 0;
+  MN_CHECK_CUDA(cudaGetDevice(&device));
+  for (int i = 0; i < count; i++)
+    if (seen[i].kernel == kernel && seen[i].device == device) return MN_OK;
+  MN_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicShared));
+  if (count < 32) seen[count++] = Seen{kernel, device};
+  return MN_OK;
 }
 
 // ---- pair-list forward (mn_conv_pairs.cu) -------------------------------------------

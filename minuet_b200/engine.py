@@ -373,7 +373,8 @@ def neighbor_table(source_masks: torch.Tensor, target_masks: torch.Tensor,
     O, S = source_masks.shape
     T = target_masks.shape[1]
     device = source_masks.device
-    nbr = torch.empty((O, T), dtype=torch.int32, device=device)
+    # rows of the table start on 128-row tiles (the kernels read whole tiles)
+    nbr = torch.empty((O, -(-T // 128) * 128), dtype=torch.int32, device=device)[:, :T]
     tile_bits = torch.empty((T + 127) // 128, dtype=torch.int32, device=device)
     perm = torch.empty(T, dtype=torch.int32, device=device) if bits is not None else None
     ws = workspace(lib().mn_neighbor_table_workspace_bytes(np_ptr(sizes_host), O, T), device)

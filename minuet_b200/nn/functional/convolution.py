@@ -381,14 +381,14 @@ def estimate_ms(algorithm: str, S, T, O, c_in, c_out, pairs, shortcut: bool) -> 
     """Rough cost of one 16-bit forward pass, from fits to measured layers of the
     benchmark network on a B200.  Pair lists move every non-centre pair row three
     times (16-bit read, fp32 product written and read back) at about 2.7 TB/s.  The
-    fused kernel pays about 3.3 ns per (128-row tile, offset present in the tile,
-    64-channel block) plus 10 ns per tile; with the rows sorted by hit word a tile of a
+    fused kernel pays about 2.4 ns per (128-row tile, offset present in the tile,
+    64-channel block) plus 8 ns per tile; with the rows sorted by hit word a tile of a
     map with E/T pairs per row holds about 1 + 2.2 (E/T - 1) of the O offsets.  Only
     the ORDER of the two estimates matters."""
     if algorithm == "implicit":
         tiles = math.ceil(T / 128)
         present = min(float(O), 1.0 + 2.2 * max(pairs / max(T, 1) - 1.0, 0.0)) if REORDER_ROWS else O
-        return 0.03 + 1.0e-5 * tiles + 3.3e-6 * tiles * present * math.ceil(c_in / 64) * \
+        return 0.03 + 8.0e-6 * tiles + 2.4e-6 * tiles * present * math.ceil(c_in / 64) * \
             (0.7 + 0.3 * c_out / 128)
     rest = pairs - (min(S, T) if shortcut else 0)
     return 0.05 + (rest * (8.0 * c_out + 2.0 * c_in) + 2.0 * (S * c_in + T * c_out)) / 2.7e9

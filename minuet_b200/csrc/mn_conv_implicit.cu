@@ -90,8 +90,9 @@ __device__ __forceinline__ int pair_row_of_tile(const ImArgs &a, int tile) {
   return lo;
 }
 
-// 16-byte asynchronous copy; src_bytes = 0 writes 16 zero bytes instead (the fill
-// travels the same path as the copies, so no proxy fence is needed for it)
+// 16-byte asynchronous copy; src_bytes = 0 writes 16 zero bytes instead.  It writes through the
+// generic proxy, like a store: the MMA issuer fences after the stage barrier (without the fence
+// one tile in some ten thousand was multiplied with a few rows missing).
 __device__ __forceinline__ void cp_async_16(uint32_t dst, const void *src, uint32_t src_bytes) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(src_bytes)
                : "memory");
@@ -301,6 +302,7 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
       for (int o = 0; alive && o < n_offsets; o++) {
         for (int kb = 0; kb < args.k_blocks; kb++) {
           if (!mbar_wait_warp(ready, &bar_full[stage], phase, abort_flag, args.status)) { alive = false; break; }
+          fence_generic_to_async();
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           const uint32_t lo = desc_lo + (uint32_t)stage * stage_step;
           const int nk = kb + 1 < args.k_blocks ? kBK / kUmmaK : last_nk;

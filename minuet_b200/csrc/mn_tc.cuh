@@ -56,6 +56,12 @@ __device__ __forceinline__ bool mbar_test(uint64_t *bar, uint32_t parity) {
   return ok != 0;
 }
 
+// Shared-memory writes of the generic proxy that a barrier wait of this thread has made visible
+// (cp.async copies, ordinary stores) -> the tensor-core and TMA instructions it issues next.
+__device__ __forceinline__ void fence_generic_to_async() {
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
+
 // Bounded wait: false when the limit expired or another role already gave up.
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volatile int *abort_flag,
                                           int32_t *status) {

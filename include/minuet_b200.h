@@ -89,7 +89,7 @@ typedef struct {
 /* Version of this interface; mn_version() returns the value the library was
  * built with.  A binding should refuse a library whose version differs from the
  * header it was written against: argument lists change between versions. */
-#define MN_ABI_VERSION 15
+#define MN_ABI_VERSION 16
 
 const char *mn_last_error(void);
 int mn_version(void);
@@ -306,8 +306,9 @@ mn_status mn_conv_stage(int stage, int64_t S, int64_t T, int64_t O, int64_t c_in
  * fp16/bf16, at most 32 offsets, channels multiple of 8, c_out <= 256. */
 int mn_implicit_supported(int64_t O, int64_t c_in, int64_t c_out, mn_dtype dtype);
 
-/* Neighbour table of a kernel map given as masks: nbr_out int32 [O, T] holds the
- * source row feeding target t under mask row p, or -1; tile_bits_out uint32
+/* Neighbour table of a kernel map given as masks: nbr_out int32 [O, T rounded up to 128]
+ * holds the source row feeding target t under mask row p, or -1 (also past T);
+ * tile_bits_out uint32
  * [ceil(T/128)] has bit p set when any target of that 128-row tile has a
  * source under mask row p.  sizes_host: HOST sizes of the mask rows. */
 size_t mn_neighbor_table_workspace_bytes(const int32_t *sizes_host, int64_t O, int64_t T);
@@ -338,6 +339,27 @@ mn_status mn_sparse_convolution_forward_implicit(
     const uint32_t *tile_bits, const int32_t *perm, const int32_t *order, const float *scale, const float *shift,
     const void *residual, int relu, double pairs_per_row, int sub_tiles, void *targets_out,
     int32_t *status_dev, void *ws, size_t ws_bytes, void *stream);
+
+/* ---- weight gradients (no reference counterpart) ---------------------------------
+ * Pair lists: entry row_begin[p] + r holds the source (target) row of the pair with rank r
+ * under mask row p, row_begin[p] = sum over q < p of sizes[q] rounded up to 128, -1 in the
+ * padding.  mn_pair_list_rows: entries of each list.  source_bits / target_bits: hit words
+ * of the two sides (each may be NULL; up to 32 offsets).  sizes_host: HOST sizes. */
+int64_t mn_pair_list_rows(const int32_t *sizes_host, int64_t O);
+mn_status mn_build_pair_lists(const int32_t *source_masks, const int32_t *target_masks,
+                              const uint32_t *source_bits, const uint32_t *target_bits,
+                              const int32_t *sizes_host, int64_t O, int64_t S, int64_t T,
+                              int32_t *pair_src_out, int32_t *pair_dst_out, void *stream);
+/* grad_weights_out[order ? order[p] : p] = sum over the pairs (s, t) of mask row p of
+ * sources[s]^T grad_targets[t], [c_in, c_out] in the feature dtype, sums in fp32 in a fixed
+ * order. */
+size_t mn_weight_gradient_workspace_bytes(const int32_t *sizes_host, int64_t O, int64_t c_in,
+                                          int64_t c_out, mn_dtype dtype);
+mn_status mn_sparse_convolution_weight_gradient(
+    int64_t S, int64_t T, int64_t O, int64_t c_in, int64_t c_out, mn_dtype dtype, const void *sources,
+    const void *grad_targets, const int32_t *pair_src, const int32_t *pair_dst, const int32_t *order,
+    const int32_t *sizes_host, void *grad_weights_out, int32_t *status_dev, void *ws,
+    size_t ws_bytes, void *stream);
 
 /* weights_t_out[o, n, k] = weights[o, k, n]: the K-major weight layout the tensor-core
  * kernels read.  The three 16-bit forward entry points (implicit, pairs, dense) take

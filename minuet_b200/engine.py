@@ -426,3 +426,27 @@ def pair_list(source_masks: torch.Tensor, target_masks: torch.Tensor, sizes_host
 
     _pair_lists[key] = (weakref.ref(source_masks, drop), weakref.ref(target_masks, drop), pair_src)
     return pair_src
+
+
+def pair_lists(source_masks: torch.Tensor, target_masks: torch.Tensor, sizes_host: np.ndarray):
+    """``(pair_src, pair_dst)`` int32: the source and the target row of every pair of the
+    kernel map, mask row by mask row in rank order (each mask row padded with -1 to a
+    multiple of 128); built on first use and kept for as long as the masks live."""
+    key = (id(source_masks), id(target_masks), "both")
+    hit = _pair_lists.get(key)
+    if hit is not None and hit[0]() is source_masks and hit[1]() is target_masks:
+        return hit[2]
+    O, S = source_masks.shape
+    T = target_masks.shape[1]
+    rows = max(int(lib().mn_pair_list_rows(np_ptr(sizes_host), O)), 1)
+    lists = torch.empty((2, rows), dtype=torch.int32, device=source_masks.device)
+    _lib.check(lib().mn_build_pair_lists(
+        ptr(source_masks), ptr(target_masks), ptr(hit_bits(source_masks)), ptr(hit_bits(target_masks)),
+        np_ptr(sizes_host), O, S, T, ptr(lists[0]), ptr(lists[1]),
+        stream_ptr(source_masks.device)), "build_pair_lists")
+
+    def drop(_ref, k=key):
+        _pair_lists.pop(k, None)
+
+    _pair_lists[key] = (weakref.ref(source_masks, drop), weakref.ref(target_masks, drop), lists)
+    return lists

@@ -126,9 +126,8 @@ class _SparseConvolution(torch.autograd.Function):
     With pairs ``(s, t)`` under offset ``k``: ``out[t] += x[s] W[k]``, hence
     ``dx[s] += dout[t] W[k]^T`` -- the same convolution with the two masks swapped and
     every weight matrix transposed, run by the same kernels -- and
-    ``dW[k] = sum over the pairs of x[s]^T dout[t]``, computed per offset from the pair
-    rows in rank order (index selection and one fp32 product per offset; written for
-    correctness, not tuned)."""
+    ``dW[k] = sum over the pairs of x[s]^T dout[t]``, one launch over the pairs of all
+    offsets and one that adds its partial matrices."""
 
     @staticmethod
     def forward(ctx, sources, weights, source_masks, target_masks, order, sizes, gather_tile,
@@ -151,30 +150,35 @@ class _SparseConvolution(torch.autograd.Function):
         od = od if ctx.has_order else None
         gather_tile, scatter_tile, shortcut, threshold, algorithm, sub_tiles = ctx.args
         grad_out = grad_out.contiguous()
-        O = sm.shape[0]
         sizes_host = engine.host_copy(sizes, np.int32)
         grad_x = grad_w = None
         if ctx.needs_input_grad[0]:
+            # [O, c_out, c_in] weights; their transpose, which the tensor-core kernels read, is w
             grad_x = _forward(grad_out, w.transpose(1, 2).contiguous(), tm, sm, od, sizes_host,
                               scatter_tile, gather_tile, shortcut, threshold, algorithm=algorithm,
-                              sub_tiles=sub_tiles)
+                              sub_tiles=sub_tiles, weights_t=w)
         if ctx.needs_input_grad[1]:
-            grad_w = torch.zeros_like(w, dtype=torch.float32)
-            for p in range(O):
-                n = int(sizes_host[p])
-                if n == 0:
-                    continue
-                k = p if od is None else int(od[p])
-                s_rows = torch.nonzero(sm[p] >= 0).squeeze(1)
-                t_rows = torch.nonzero(tm[p] >= 0).squeeze(1)
-                # pair r of this mask row is (source with rank r, target with rank r)
-                s_by_rank = torch.empty(n, dtype=torch.int64, device=x.device)
-                t_by_rank = torch.empty(n, dtype=torch.int64, device=x.device)
-                s_by_rank[sm[p, s_rows].long()] = s_rows
-                t_by_rank[tm[p, t_rows].long()] = t_rows
-                grad_w[k] = x[s_by_rank].float().t() @ grad_out[t_by_rank].float()
-            grad_w = grad_w.to(w.dtype)
+            grad_w = _weight_gradient(x, grad_out, w, sm, tm, od, sizes_host)
         return (grad_x, grad_w) + (None,) * 10
+
+
+def _weight_gradient(x, grad_out, weights, sm, tm, order, sizes_host):
+    O, S = sm.shape
+    T = tm.shape[1]
+    c_in, c_out = weights.shape[1], weights.shape[2]
+    code = engine.dtype_code(weights.dtype)
+    device = x.device
+    lib = engine.lib()
+    pair_src, pair_dst = engine.pair_lists(sm, tm, sizes_host)
+    grad_w = torch.empty_like(weights)
+    ws = engine.workspace(lib.mn_weight_gradient_workspace_bytes(engine.np_ptr(sizes_host), O, c_in,
+                                                                 c_out, code), device)
+    _lib.check(lib.mn_sparse_convolution_weight_gradient(
+        S, T, O, c_in, c_out, code, engine.ptr(x), engine.ptr(grad_out), engine.ptr(pair_src),
+        engine.ptr(pair_dst), engine.ptr(order), engine.np_ptr(sizes_host), engine.ptr(grad_w),
+        engine.ptr(engine.status_word(device)), engine.ptr(ws), ws.numel(),
+        engine.stream_ptr(device)), "sparse_convolution_weight_gradient")
+    return grad_w
 
 
 def sparse_convolution_forward_fused(sources: torch.Tensor, weights: torch.Tensor,

@@ -89,7 +89,7 @@ typedef struct {
 /* Version of this interface; mn_version() returns the value the library was
  * built with.  A binding should refuse a library whose version differs from the
  * header it was written against: argument lists change between versions. */
-#define MN_ABI_VERSION 16
+#define MN_ABI_VERSION 17
 
 const char *mn_last_error(void);
 int mn_version(void);
@@ -339,6 +339,17 @@ mn_status mn_sparse_convolution_forward_implicit(
     const uint32_t *tile_bits, const int32_t *perm, const int32_t *order, const float *scale, const float *shift,
     const void *residual, int relu, double pairs_per_row, int sub_tiles, void *targets_out,
     int32_t *status_dev, void *ws, size_t ws_bytes, void *stream);
+
+/* The same function in fp32 on FFMA units (sums in fp32, any channel counts, at most 32
+ * offsets), every offset's product by itself and the products added in mask-row order: one
+ * output-stationary kernel over the neighbour table, plus one launch that adds the offsets'
+ * products where the rows alone do not fill the GPU (the workspace is for those). */
+size_t mn_implicit_fp32_workspace_bytes(int64_t T, int64_t O, int64_t c_out);
+mn_status mn_sparse_convolution_forward_implicit_fp32(
+    int64_t S, int64_t T, int64_t O, int64_t c_in, int64_t c_out, const float *sources,
+    const float *weights, const int32_t *nbr, const uint32_t *tile_bits, const int32_t *perm,
+    const int32_t *order, const float *scale, const float *shift, const float *residual, int relu,
+    float *targets_out, void *ws, size_t ws_bytes, void *stream);
 
 /* ---- weight gradients (no reference counterpart) ---------------------------------
  * Pair lists: entry row_begin[p] + r holds the source (target) row of the pair with rank r

@@ -15,7 +15,7 @@ MN_F32, MN_F16, MN_BF16 = 0, 1, 2
 MN_MAX_NDIM = 4
 MN_MAX_OFFSETS = 128
 MN_CTRL_WORDS = 1024
-ABI_VERSION = 16         # must equal MN_ABI_VERSION of the header the library was built from
+ABI_VERSION = 17         # must equal MN_ABI_VERSION of the header the library was built from
 
 c_i32p = ctypes.c_void_p
 c_ptr = ctypes.c_void_p
@@ -91,6 +91,11 @@ PROTOTYPES = {
                                                        c_ptr, c_ptr, c_ptr, c_ptr, c_ptr, c_ptr,
                                                        c_ptr, c_ptr, c_ptr, c_ptr, c_int, c_dbl,
                                                        c_int, c_ptr, c_ptr, c_ptr, c_size, c_ptr]),
+    "mn_implicit_fp32_workspace_bytes": (c_size, [c_i64, c_i64, c_i64]),
+    "mn_sparse_convolution_forward_implicit_fp32": (c_int, [c_i64, c_i64, c_i64, c_i64, c_i64, c_ptr,
+                                                            c_ptr, c_ptr, c_ptr, c_ptr, c_ptr, c_ptr,
+                                                            c_ptr, c_ptr, c_int, c_ptr, c_ptr,
+                                                            c_size, c_ptr]),
     "mn_pair_list_rows": (c_i64, [c_ptr, c_i64]),
     "mn_build_pair_lists": (c_int, [c_ptr, c_ptr, c_ptr, c_ptr, c_ptr, c_i64, c_i64, c_i64, c_ptr,
                                     c_ptr, c_ptr]),

@@ -381,6 +381,27 @@ def _implicit_forward(sources, weights, source_masks, target_masks, order, sizes
     return out
 
 
+def _implicit_forward_fp32(sources, weights, source_masks, target_masks, order, sizes_host, out,
+                           scale=None, shift=None, residual=None, relu=False):
+    O, S = source_masks.shape
+    T = target_masks.shape[1]
+    c_in, c_out = weights.shape[1], weights.shape[2]
+    device = sources.device
+    nbr, tile_bits, perm = engine.neighbor_table(source_masks, target_masks, sizes_host,
+                                                 reorder=REORDER_ROWS)
+    if engine.LAYER_LOG:
+        engine.LAYER_LOG[-1]["tile_bits"] = tile_bits
+    lib = engine.lib()
+    ws = engine.workspace(lib.mn_implicit_fp32_workspace_bytes(T, O, c_out), device)
+    _lib.check(lib.mn_sparse_convolution_forward_implicit_fp32(
+        S, T, O, c_in, c_out, engine.ptr(sources), engine.ptr(weights), engine.ptr(nbr),
+        engine.ptr(tile_bits), engine.ptr(perm), engine.ptr(order), engine.ptr(scale),
+        engine.ptr(shift), engine.ptr(residual), int(bool(relu)), engine.ptr(out),
+        engine.ptr(ws), ws.numel(), engine.stream_ptr(device)),
+        "sparse_convolution_forward_implicit_fp32")
+    return out
+
+
 def estimate_ms(algorithm: str, S, T, O, c_in, c_out, pairs, shortcut: bool) -> float:
     """Rough cost of one 16-bit forward pass, from fits to measured layers of the
     benchmark network on a B200.  Pair lists move every non-centre pair row three
@@ -409,6 +430,11 @@ def _pick_algorithm(weights, sm, tm, sizes_host, allow_shortcut_matmul, algorith
     if algorithm not in ("auto", "explicit", "implicit"):
         raise ValueError(f"unknown sparse convolution algorithm {algorithm!r}")
     code = engine.dtype_code(weights.dtype)
+    if weights.dtype == torch.float32:
+        # one kernel for any channel counts, whose sums are the explicit path's bit for bit, so
+        # that a call (or a tuned configuration) that asks for that path gets its result too;
+        # the path itself is for more than 32 offsets
+        return "implicit" if 0 < T and O <= 32 else "explicit"
     if algorithm == "explicit" or T == 0 or not engine.lib().mn_implicit_supported(
             O, c_in, c_out, code):
         return "explicit"
@@ -455,6 +481,9 @@ def _forward(sources, weights, sm, tm, order, sizes_host, gather_tile_size, scat
         return out
 
     def run_implicit():
+        if weights.dtype == torch.float32:
+            return _implicit_forward_fp32(sources, weights, sm, tm, order, sizes_host, out, scale,
+                                          shift, residual, relu)
         return _implicit_forward(sources, weights, sm, tm, order, sizes_host, out, scale, shift,
                                  residual, relu, sub_tiles, weights_t)
 

@@ -148,6 +148,26 @@ def load():
     return _lib
 
 
+_host = None
+
+
+def host():
+    """The native host path (csrc/host.cpp), bound to the library that :func:`load` loaded."""
+    global _host
+    if _host is None:
+        load()
+        import torch  # noqa: F401  (its libraries must be in the process first)
+        try:
+            from minuet_b200 import _host as module
+        except ImportError as error:
+            raise ImportError(
+                f"minuet_b200/_host.so is missing or does not fit this torch ({error}): build it "
+                "with `python -m minuet_b200.build`. minuet_b200 has no fallback.") from error
+        module.bind(LIB_PATH)
+        _host = module
+    return _host
+
+
 def last_error() -> str:
     return load().mn_last_error().decode(errors="replace")
 

@@ -126,22 +126,13 @@ STATUS_KEY_BOX = 2
 STATUS_TC_TIMEOUT = 4
 STATUS_KEY_BITS = 8
 STATUS_GRID_TIMEOUT = 16
-_status = {}
-_pending_status = {}
 
 
 def control_block(device) -> torch.Tensor:
     """The ``MN_CTRL_WORDS`` int32 control block of (device, current stream): word 0
     is the status word, the rest is grid-barrier state of the cooperative kernels.
     One block per stream, because kernels of different streams may overlap."""
-    index = _device_index(device)
-    key = (index, raw_stream(index))
-    block = _status.get(key)
-    if block is None:
-        block = torch.zeros(_lib.MN_CTRL_WORDS, dtype=torch.int32,
-                            device=torch.device("cuda", index))
-        _status[key] = block
-    return block
+    return _lib.host().control_block(_device_index(device))
 
 
 def status_word(device) -> torch.Tensor:
@@ -191,18 +182,7 @@ def poll_status(device):
     status word into pinned memory and raises for any earlier copy that has
     landed with a non-zero value.  An error therefore surfaces at the latest one
     call after the kernel that raised it, without a host-device synchronisation."""
-    dev = torch.device(device)
-    key = dev.index if dev.index is not None else torch.cuda.current_device()
-    queue = _pending_status.setdefault(key, [])
-    while queue and queue[0][1].query():
-        pinned, _ = queue.pop(0)
-        raise_on_status(int(pinned[0]), device)
-    if len(queue) < 8:
-        pinned = torch.empty(1, dtype=torch.int32, pin_memory=True)
-        pinned.copy_(status_word(device), non_blocking=True)
-        event = torch.cuda.Event()
-        event.record(torch.cuda.current_stream(device))
-        queue.append((pinned, event))
+    raise_on_status(_lib.host().poll_status(_device_index(device)), device)
 
 
 # ---------------------------------------------------------------------------
@@ -231,33 +211,6 @@ def make_keyspec(coord_tensors: Sequence[torch.Tensor], ndim: int, num_clouds: i
     return spec
 
 
-def make_keyspec_device(coords: torch.Tensor, batch_dims: Optional[torch.Tensor], ndim: int,
-                        num_clouds: int, margin: int, with_keys: bool = True):
-    """Bounding box, key layout and (optionally) the keys of ``coords`` in one launch,
-    all left on the device (no read-back).  Returns ``(spec, spec_dev, keys)``: the
-    host struct only carries ndim, margin and the pointer to ``spec_dev``, which
-    must stay alive for as long as the spec is used."""
-    device = coords.device
-    spec = KeySpec()
-    spec_dev = torch.empty(256, dtype=torch.uint8, device=device)
-    keys = torch.empty(coords.shape[0], dtype=torch.int64, device=device) if with_keys else None
-    ws = workspace(lib().mn_map_workspace_bytes(0, 0, 0), device)
-    _lib.check(lib().mn_keyspec_device(ptr(coords), coords.shape[0], ndim, ptr(batch_dims),
-                                       max(int(num_clouds), 1), int(margin), ptr(spec_dev),
-                                       ctypes.byref(spec), ptr(keys), ptr(control_block(device)),
-                                       ptr(ws), ws.numel(), stream_ptr(device)), "keyspec_device")
-    return spec, spec_dev, keys
-
-
-def read_small(t: torch.Tensor) -> np.ndarray:
-    """Blocking device-to-host read of a small tensor through pinned memory (one DMA
-    transfer, no kernel)."""
-    pinned = torch.empty(t.shape, dtype=t.dtype, pin_memory=True)
-    pinned.copy_(t, non_blocking=True)
-    torch.cuda.current_stream(t.device).synchronize()
-    return pinned.numpy().copy()
-
-
 def pack_keys(coords: torch.Tensor, batch_dims: Optional[torch.Tensor], spec: KeySpec,
               tstride: Optional[Sequence[int]] = None) -> torch.Tensor:
     n, ndim = coords.shape
@@ -271,50 +224,55 @@ def pack_keys(coords: torch.Tensor, batch_dims: Optional[torch.Tensor], spec: Ke
 
 
 # ---------------------------------------------------------------------------
-# host copies of small device tensors (kernel-map sizes), keyed by tensor
+# plans of kernel maps (csrc/host.cpp:Plan): pair counts on the host, hit words,
+# neighbour tables and pair lists, kept for as long as the mask tensors live
 # ---------------------------------------------------------------------------
-_host_copies = {}
+_plans = {}        # id(masks) or id(sizes) -> (weak reference, plan, side)
+_foreign = {}      # (id(source masks), id(target masks)) of maps built elsewhere -> the same
+_host_copies = {}  # id(tensor) -> (weak reference, numpy values)
+_SOURCE, _TARGET, _SIZES = range(3)
 
 
-class PendingHostCopy:
-    """Asynchronous device-to-host copy of a small int32 tensor whose LAST element
-    is a snapshot of the status word (one DMA transfer into pinned memory, no
-    kernel); the wait happens when (and if) the host needs the values."""
-
-    _pool = []
-
-    def __init__(self, values_and_status: torch.Tensor):
-        device = values_and_status.device
-        self.device = device
-        n = values_and_status.numel()
-        pinned = None
-        for i, buf in enumerate(self._pool):
-            if buf.numel() >= n:
-                pinned = self._pool.pop(i)
-                break
-        if pinned is None:
-            pinned = torch.empty(max(n, 160), dtype=torch.int32, pin_memory=True)
-        self.pinned = pinned
-        self.n = n
-        pinned[:n].copy_(values_and_status, non_blocking=True)
-        self.event = torch.cuda.Event()
-        self.event.record(torch.cuda.current_stream(device))
-        self.values = None
-
-    def get(self) -> np.ndarray:
-        if self.values is None:
-            self.event.synchronize()
-            host = self.pinned[:self.n].numpy().copy()
-            if len(self._pool) < 64:
-                self._pool.append(self.pinned)
-            self.pinned = None
-            raise_on_status(int(host[-1]), self.device)
-            self.values = np.ascontiguousarray(host[:-1])
-        return self.values
+def _remember(t: torch.Tensor, plan, side: int):
+    key = id(t)
+    _plans[key] = (weakref.ref(t, lambda _r, k=key: _plans.pop(k, None)), plan, side)
 
 
-def remember_host(t: torch.Tensor, values):
-    """``values``: a numpy array or a PendingHostCopy of the tensor's contents."""
+def remember_plan(source_masks, target_masks, sizes, plan):
+    """Find ``plan`` again by the tensors of its map."""
+    _remember(source_masks, plan, _SOURCE)
+    _remember(target_masks, plan, _TARGET)
+    _remember(sizes, plan, _SIZES)
+
+
+def _entry(t: torch.Tensor):
+    hit = _plans.get(id(t))
+    return hit if hit is not None and hit[0]() is t else None
+
+
+def plan_of(source_masks: torch.Tensor, target_masks: torch.Tensor, sizes):
+    """``(plan, swapped)`` of the map that two int32 mask tensors describe; ``swapped`` when
+    they are the map's own with the sides exchanged.  Masks that did not come from this
+    engine get a plan on first use (``sizes``: their pair counts, a tensor or host values)."""
+    s, t = _entry(source_masks), _entry(target_masks)
+    if s is not None and t is not None and s[1] is t[1] and s[2] != t[2]:
+        return s[1], s[2] == _TARGET
+    key = (id(source_masks), id(target_masks))
+    hit = _foreign.get(key)
+    if hit is not None and hit[0]() is source_masks and hit[1]() is target_masks:
+        return hit[2], False
+    plan = _lib.host().Plan(source_masks.shape[0], source_masks.shape[1], target_masks.shape[1])
+    values = host_copy(sizes, np.int32) if isinstance(sizes, torch.Tensor) else sizes
+    plan.set_sizes(np.asarray(values).tolist())
+
+    def drop(_ref, k=key):
+        _foreign.pop(k, None)
+
+    _foreign[key] = (weakref.ref(source_masks, drop), weakref.ref(target_masks, drop), plan)
+    return plan, False
+
+
+def remember_host(t: torch.Tensor, values: np.ndarray):
     key = id(t)
     _host_copies[key] = (weakref.ref(t, lambda _r, k=key: _host_copies.pop(k, None)), values)
 
@@ -322,39 +280,22 @@ def remember_host(t: torch.Tensor, values):
 def host_copy(t: torch.Tensor, dtype=np.int32) -> np.ndarray:
     """Host values of ``t``: the remembered copy when the tensor came from this
     engine, otherwise a blocking device-to-host read."""
+    entry = _entry(t)
+    if entry is not None and entry[2] == _SIZES:
+        return np.asarray(entry[1].sizes(), dtype=dtype)
     hit = _host_copies.get(id(t))
     if hit is not None and hit[0]() is t:
-        values = hit[1].get() if isinstance(hit[1], PendingHostCopy) else hit[1]
-        return np.ascontiguousarray(values.astype(dtype, copy=False))
+        return np.ascontiguousarray(np.asarray(hit[1]).astype(dtype, copy=False))
     return np.ascontiguousarray(t.detach().cpu().numpy().astype(dtype, copy=False))
 
 
-# ---------------------------------------------------------------------------
-# per-row hit words of kernel maps, keyed by the mask tensors they belong to
-# ---------------------------------------------------------------------------
-_hit_bits = {}
-
-
-def remember_bits(source_masks, target_masks, source_bits, target_bits):
-    """Keep the per-row hit words (bit p set <=> mask row p has an entry for the row)
-    that the fused map build produced, for as long as the masks live."""
-    for masks, bits in ((source_masks, source_bits), (target_masks, target_bits)):
-        key = id(masks)
-        _hit_bits[key] = (weakref.ref(masks, lambda _r, k=key: _hit_bits.pop(k, None)), bits)
-
-
 def hit_bits(masks: torch.Tensor) -> Optional[torch.Tensor]:
-    """Hit words of a mask tensor that came from the fused map build, else None."""
-    hit = _hit_bits.get(id(masks))
-    if hit is not None and hit[0]() is masks:
-        return hit[1]
-    return None
-
-
-# ---------------------------------------------------------------------------
-# neighbour tables of kernel maps (fused forward), keyed by the mask tensors
-# ---------------------------------------------------------------------------
-_neighbor_tables = {}
+    """Hit words (bit p set <=> mask row p has an entry for the row) of a mask tensor that
+    came from the fused map build, else None."""
+    entry = _entry(masks)
+    if entry is None or entry[2] == _SIZES:
+        return None
+    return entry[1].source_bits if entry[2] == _SOURCE else entry[1].target_bits
 
 
 def neighbor_table(source_masks: torch.Tensor, target_masks: torch.Tensor,
@@ -365,88 +306,5 @@ def neighbor_table(source_masks: torch.Tensor, target_masks: torch.Tensor,
     and gets its own table).  With ``reorder`` and a map that carries hit words, the
     table's rows are the targets sorted by hit word (``perm[r]`` = target at position
     ``r``), so that 128-row tiles skip the offsets none of their rows has."""
-    bits = hit_bits(target_masks) if reorder else None
-    key = (id(source_masks), id(target_masks), bits is not None)
-    hit = _neighbor_tables.get(key)
-    if hit is not None and hit[0]() is source_masks and hit[1]() is target_masks:
-        return hit[2], hit[3], hit[4]
-    O, S = source_masks.shape
-    T = target_masks.shape[1]
-    device = source_masks.device
-    # rows of the table start on 128-row tiles (the kernels read whole tiles)
-    nbr = torch.empty((O, -(-T // 128) * 128), dtype=torch.int32, device=device)[:, :T]
-    tile_bits = torch.empty((T + 127) // 128, dtype=torch.int32, device=device)
-    perm = torch.empty(T, dtype=torch.int32, device=device) if bits is not None else None
-    ws = workspace(lib().mn_neighbor_table_workspace_bytes(np_ptr(sizes_host), O, T), device)
-    _lib.check(lib().mn_build_neighbor_table(ptr(source_masks), ptr(target_masks),
-                                             np_ptr(sizes_host), O, S, T,
-                                             ptr(hit_bits(source_masks) if bits is not None else None),
-                                             ptr(bits), ptr(nbr),
-                                             ptr(tile_bits), ptr(perm), ptr(control_block(device)),
-                                             ptr(ws), ws.numel(), stream_ptr(device)),
-               "build_neighbor_table")
-
-    def drop(_ref, k=key):
-        _neighbor_tables.pop(k, None)
-
-    _neighbor_tables[key] = (weakref.ref(source_masks, drop), weakref.ref(target_masks, drop),
-                             nbr, tile_bits, perm)
-    return nbr, tile_bits, perm
-
-
-# ---------------------------------------------------------------------------
-# pair lists of kernel maps (pair-list forward), keyed by the mask tensors
-# ---------------------------------------------------------------------------
-_pair_lists = {}
-
-
-def pair_list(source_masks: torch.Tensor, target_masks: torch.Tensor, sizes_host: np.ndarray,
-              allow_shortcut: bool):
-    """``pair_src`` int32 ``[R]`` (the source row of every product row, -1 in the
-    padding) of the kernel map the masks describe, or None when the map did not come
-    with hit words; built on first use and kept for as long as the masks live."""
-    bits = hit_bits(source_masks)
-    if bits is None or hit_bits(target_masks) is None:
-        return None
-    key = (id(source_masks), id(target_masks), bool(allow_shortcut))
-    hit = _pair_lists.get(key)
-    if hit is not None and hit[0]() is source_masks and hit[1]() is target_masks:
-        return hit[2]
-    O, S = source_masks.shape
-    T = target_masks.shape[1]
-    device = source_masks.device
-    rows = int(lib().mn_pair_rows(np_ptr(sizes_host), O, S, T, int(bool(allow_shortcut))))
-    pair_src = torch.empty(max(rows, 1), dtype=torch.int32, device=device)
-    _lib.check(lib().mn_build_pair_list(ptr(source_masks), ptr(bits), np_ptr(sizes_host), O, S, T,
-                                        int(bool(allow_shortcut)), ptr(pair_src),
-                                        stream_ptr(device)), "build_pair_list")
-
-    def drop(_ref, k=key):
-        _pair_lists.pop(k, None)
-
-    _pair_lists[key] = (weakref.ref(source_masks, drop), weakref.ref(target_masks, drop), pair_src)
-    return pair_src
-
-
-def pair_lists(source_masks: torch.Tensor, target_masks: torch.Tensor, sizes_host: np.ndarray):
-    """``(pair_src, pair_dst)`` int32: the source and the target row of every pair of the
-    kernel map, mask row by mask row in rank order (each mask row padded with -1 to a
-    multiple of 128); built on first use and kept for as long as the masks live."""
-    key = (id(source_masks), id(target_masks), "both")
-    hit = _pair_lists.get(key)
-    if hit is not None and hit[0]() is source_masks and hit[1]() is target_masks:
-        return hit[2]
-    O, S = source_masks.shape
-    T = target_masks.shape[1]
-    rows = max(int(lib().mn_pair_list_rows(np_ptr(sizes_host), O)), 1)
-    lists = torch.empty((2, rows), dtype=torch.int32, device=source_masks.device)
-    _lib.check(lib().mn_build_pair_lists(
-        ptr(source_masks), ptr(target_masks), ptr(hit_bits(source_masks)), ptr(hit_bits(target_masks)),
-        np_ptr(sizes_host), O, S, T, ptr(lists[0]), ptr(lists[1]),
-        stream_ptr(source_masks.device)), "build_pair_lists")
-
-    def drop(_ref, k=key):
-        _pair_lists.pop(k, None)
-
-    _pair_lists[key] = (weakref.ref(source_masks, drop), weakref.ref(target_masks, drop), lists)
-    return lists
+    plan, swapped = plan_of(source_masks, target_masks, sizes_host)
+    return plan.neighbours(swapped, reorder, source_masks, target_masks)

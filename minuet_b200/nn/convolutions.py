@@ -13,6 +13,7 @@ from torch.nn import Module
 
 from minuet_b200 import _lib, engine
 from minuet_b200.nn import functional as F
+from minuet_b200.nn.functional import convolution as conv_functional
 from minuet_b200.tensors import SparseTensor
 from minuet_b200.utils.helpers import as_tuple, generate_kernel_offsets
 
@@ -44,9 +45,9 @@ class KernelMapCache(object):
         self._kernel_maps_cache = dict()
         self._coordinates_cache = dict()
         self._offsets_cache = dict()
+        self._layers = dict()        # (tensor stride, layer geometry) -> what SparseConv looks up
         self._keys = dict()          # stride -> (coordinates tensor, keys tensor)
-        self._spec = None
-        self._spec_dev = None        # device copy of the key layout (kept alive with the spec)
+        self._spec = None            # key layout of this forward pass
         self._root_keys = None       # (coordinates tensor, keys) of the first tensor seen
         self._root = None            # (coords int32, batch_dims int64, num_clouds)
 
@@ -54,19 +55,21 @@ class KernelMapCache(object):
     def reset(self):
         self._coordinates_cache.clear()
         self._kernel_maps_cache.clear()
+        self._layers.clear()
         self._keys.clear()
         self._spec = None
-        self._spec_dev = None
         self._root_keys = None
         self._root = None
 
-    def _get_kernel_offsets(self, source_stride, kernel_size, kernel_dilation) -> np.ndarray:
+    def _get_kernel_offsets(self, source_stride, kernel_size, kernel_dilation):
+        """The offset table of a geometry, as an array and in native form."""
         key = (source_stride, kernel_size, kernel_dilation)
         if key not in self._offsets_cache:
             table = generate_kernel_offsets(ndim=self._ndim, kernel_size=kernel_size,
                                             source_stride=source_stride,
                                             dilation=kernel_dilation, layout=self._layout)
-            self._offsets_cache[key] = np.ascontiguousarray(table, dtype=np.int32)
+            table = np.ascontiguousarray(table, dtype=np.int32)
+            self._offsets_cache[key] = (table, _lib.host().Offsets(table.tolist(), self._ndim))
         return self._offsets_cache[key]
 
     def _ensure_spec(self, coordinates, batch_dims, margin: int):
@@ -80,8 +83,8 @@ class KernelMapCache(object):
             coords, bd, num_clouds = self._root
             # bounding box, key layout and the keys of the first tensor in one launch;
             # all of it stays on the device: no read-back here
-            self._spec, self._spec_dev, keys = engine.make_keyspec_device(
-                coords, bd, self._ndim, num_clouds, max(int(margin), engine.DEFAULT_MARGIN))
+            self._spec, keys = _lib.host().root_keys(coords, bd, num_clouds,
+                                                     max(int(margin), engine.DEFAULT_MARGIN))
             self._keys.clear()
             self._root_keys = (coordinates, keys)
         return self._spec
@@ -93,8 +96,8 @@ class KernelMapCache(object):
         if self._root_keys is not None and self._root_keys[0] is coordinates:
             self._keys[stride] = self._root_keys
             return self._root_keys[1]
-        keys = engine.pack_keys(engine.as_i32_coords(coordinates), engine.as_i64(batch_dims),
-                                self._spec)
+        keys = _lib.host().pack_keys(engine.as_i32_coords(coordinates), engine.as_i64(batch_dims),
+                                     self._spec)
         self._keys[stride] = (coordinates, keys)
         return keys
 
@@ -123,36 +126,19 @@ class KernelMapCache(object):
                                "non-transposed layer before its execution")
 
         engine.require_cuda(source_coordinates, source_batch_dims)
-        coords = engine.as_i32_coords(source_coordinates)
-        bd = engine.as_i64(source_batch_dims)
-        nb = 1 if bd is None else bd.numel() - 1
-        n = coords.shape[0]
-        device = coords.device
         spec = self._ensure_spec(source_coordinates, source_batch_dims, max(target_stride) - 1)
-        ts = np.asarray(target_stride, dtype=np.int32)
-        unique = torch.empty((n, ndim), dtype=torch.int32, device=device)
-        keys = torch.empty(n, dtype=torch.int64, device=device)
-        meta = torch.empty(nb + 3, dtype=torch.int64, device=device)  # count, batch_dims, status
-        lib = engine.lib()
-        ws = engine.workspace(lib.mn_map_workspace_bytes(n, n, 1), device)
-        _lib.check(lib.mn_downsample_coordinates(
-            engine.ptr(coords), n, ndim, engine.ptr(bd), nb, engine.np_ptr(ts), ctypes.byref(spec),
-            engine.ptr(unique), engine.ptr(keys), engine.ptr(meta),
-            engine.ptr(engine.control_block(device)), engine.ptr(ws), ws.numel(),
-            engine.stream_ptr(device)), "downsample_coordinates")
-        # the one blocking read of a strided level: the number of output rows sets
-        # the shapes of everything that follows
-        host = engine.read_small(meta)
-        engine.raise_on_status(int(host[-1]), device)
-        count = int(host[0])
-        target_coordinates = unique[:count]
+        # the one blocking read of a strided level is in here: the number of output rows
+        # sets the shapes of everything that follows
+        target_coordinates, keys, starts, starts_host = _lib.host().downsample(
+            engine.as_i32_coords(source_coordinates), engine.as_i64(source_batch_dims),
+            target_stride, spec)
         if source_coordinates.dtype != torch.int32:
             target_coordinates = target_coordinates.to(source_coordinates.dtype)
         target_batch_dims = None
         if source_batch_dims is not None:
-            target_batch_dims = meta[1:nb + 2].to(source_batch_dims.dtype)
-            engine.remember_host(target_batch_dims, host[1:nb + 2].copy())
-        self._keys[target_stride] = (target_coordinates, keys[:count])
+            target_batch_dims = starts.to(source_batch_dims.dtype)
+            engine.remember_host(target_batch_dims, np.asarray(starts_host, dtype=np.int64))
+        self._keys[target_stride] = (target_coordinates, keys)
         self._coordinates_cache[target_stride] = (target_coordinates, target_stride,
                                                   target_batch_dims)
         return self._coordinates_cache[target_stride]
@@ -182,74 +168,67 @@ class KernelMapCache(object):
                                "non-transposed layer before its execution")
 
         engine.require_cuda(source_coordinates, target_coordinates)
-        offsets = self._get_kernel_offsets(source_stride, kernel_size, kernel_dilation)
+        table, offsets = self._get_kernel_offsets(source_stride, kernel_size, kernel_dilation)
         reorder = not (self._disable_reordering or disable_reordering)
-        margin = int(np.abs(offsets).max()) + max(max(source_stride), max(target_stride)) - 1
+        margin = offsets.reach + max(max(source_stride), max(target_stride)) - 1
         spec = self._ensure_spec(source_coordinates, source_batch_dims, margin)
         skeys = self._keys_of(source_coordinates, source_batch_dims, source_stride)
         if target_coordinates is source_coordinates:
             tkeys = skeys
         else:
             tkeys = self._keys_of(target_coordinates, target_batch_dims, target_stride)
-        result = build_kernel_map(skeys, tkeys, offsets, spec, reorder)
+        result = build_kernel_map(skeys, tkeys, table, offsets, spec, reorder)
         self._kernel_maps_cache[key] = result
         return result
 
 
-def build_kernel_map(source_keys: torch.Tensor, target_keys: torch.Tensor, offsets: np.ndarray,
-                     spec, reorder: bool):
+def build_kernel_map(source_keys: torch.Tensor, target_keys: torch.Tensor, table: np.ndarray,
+                     offsets, spec, reorder: bool):
     """Masks, order and sizes from packed keys.  Up to 32 offsets take the fused
     build; larger kernels go through a materialised kernel map."""
+    if offsets.count <= 32:
+        source_masks, target_masks, order, sizes, plan = _lib.host().build_map(
+            source_keys, target_keys, offsets, spec, reorder)
+    else:
+        source_masks, target_masks, order, sizes, plan = _build_large_kernel_map(
+            source_keys, target_keys, table, spec, reorder)
+    engine.remember_plan(source_masks, target_masks, sizes, plan)
+    return source_masks, target_masks, (order if reorder else None), sizes
+
+
+def _build_large_kernel_map(source_keys, target_keys, table, spec, reorder):
     device = source_keys.device
-    S, T, O = source_keys.numel(), target_keys.numel(), offsets.shape[0]
+    S, T, O = source_keys.numel(), target_keys.numel(), table.shape[0]
     lib = engine.lib()
+    stream = engine.stream_ptr(device)
     source_masks = torch.empty((O, S), dtype=torch.int32, device=device)
     target_masks = torch.empty((O, T), dtype=torch.int32, device=device)
-    # one allocation for the small outputs: order [O], sizes + status word [O + 1] and the
-    # per-row hit words [S], [T] (each part starts on a 256-byte boundary)
-    pad = lambda n: -(-n // 64) * 64
-    small = torch.empty(2 * pad(O + 1) + pad(S) + pad(T), dtype=torch.int32, device=device)
-    order = small[:O]
-    sizes_status = small[pad(O + 1):pad(O + 1) + O + 1]                  # sizes, status word
+    sizes_status = torch.empty(O + 1, dtype=torch.int32, device=device)   # sizes, status word
     sizes = sizes_status[:O]
     ws = engine.workspace(lib.mn_map_workspace_bytes(S, T, O), device)
-    stream = engine.stream_ptr(device)
-    if O <= 32:
-        # per-row hit words in mask-row order, kept with the masks for the forward kernels
-        base = 2 * pad(O + 1)
-        source_bits = small[base:base + S]
-        target_bits = small[base + pad(S):base + pad(S) + T]
-        same = source_keys.data_ptr() == target_keys.data_ptr() and S == T
-        _lib.check(lib.mn_build_kernel_map(
-            engine.ptr(source_keys), S, engine.ptr(source_keys if same else target_keys), T,
-            engine.np_ptr(offsets), O, ctypes.byref(spec), int(reorder), engine.ptr(source_masks),
-            engine.ptr(target_masks), engine.ptr(order), engine.ptr(sizes_status),
-            engine.ptr(source_bits), engine.ptr(target_bits),
-            engine.ptr(engine.control_block(device)), engine.ptr(ws), ws.numel(), stream),
-            "build_kernel_map")
-        engine.remember_bits(source_masks, target_masks, source_bits, target_bits)
+    kernel_map = torch.empty((O, T), dtype=torch.int32, device=device)
+    _lib.check(lib.mn_query_sorted_index_with_offsets(
+        engine.ptr(source_keys), S, engine.ptr(target_keys), T, engine.np_ptr(table), O,
+        ctypes.cast(spec.address, ctypes.POINTER(_lib.KeySpec)), engine.ptr(kernel_map), stream),
+        "query_sorted_index_with_offsets")
+    _lib.check(lib.mn_compute_kernel_map_sizes(engine.ptr(kernel_map), O, T, engine.ptr(sizes),
+                                               stream), "compute_kernel_map_sizes")
+    if reorder:
+        sorted_sizes, order64 = torch.sort(sizes, stable=True)
+        sizes.copy_(sorted_sizes)
+        order = order64.to(torch.int32)
+        kernel_map = kernel_map[order64]
     else:
-        kernel_map = torch.empty((O, T), dtype=torch.int32, device=device)
-        _lib.check(lib.mn_query_sorted_index_with_offsets(
-            engine.ptr(source_keys), S, engine.ptr(target_keys), T, engine.np_ptr(offsets), O,
-            ctypes.byref(spec), engine.ptr(kernel_map), stream), "query_sorted_index_with_offsets")
-        _lib.check(lib.mn_compute_kernel_map_sizes(engine.ptr(kernel_map), O, T, engine.ptr(sizes),
-                                                   stream), "compute_kernel_map_sizes")
-        if reorder:
-            sorted_sizes, order64 = torch.sort(sizes, stable=True)
-            sizes.copy_(sorted_sizes)
-            order = order64.to(torch.int32)
-            kernel_map = kernel_map[order64]
-        else:
-            order = torch.arange(O, dtype=torch.int32, device=device)
-        sizes_status[O:].copy_(engine.status_word(device))
-        _lib.check(lib.mn_compute_kernel_map_masks(
-            engine.ptr(kernel_map), O, S, T, engine.ptr(source_masks), engine.ptr(target_masks),
-            engine.ptr(ws), ws.numel(), stream), "compute_kernel_map_masks")
+        order = torch.arange(O, dtype=torch.int32, device=device)
+    sizes_status[O:].copy_(engine.status_word(device))
+    _lib.check(lib.mn_compute_kernel_map_masks(
+        engine.ptr(kernel_map), O, S, T, engine.ptr(source_masks), engine.ptr(target_masks),
+        engine.ptr(ws), ws.numel(), stream), "compute_kernel_map_masks")
     # the GEMM plan needs the sizes on the host: start the copy (sizes + status
     # word) now, wait for it only when a convolution asks
-    engine.remember_host(sizes, engine.PendingHostCopy(sizes_status))
-    return source_masks, target_masks, (order if reorder else None), sizes
+    plan = _lib.host().Plan(O, S, T)
+    plan.expect_sizes(sizes_status)
+    return source_masks, target_masks, order, sizes, plan
 
 
 class SparseConv(Module):
@@ -286,6 +265,7 @@ class SparseConv(Module):
         self.stride = as_tuple(stride, size=ndim, name="stride")
         self.dilation = as_tuple(dilation, size=ndim, name="dilation")
         self.transposed = transposed
+        self._geometry = (self.kernel_size, self.stride, self.dilation, transposed)
         volume = int(np.prod(self.kernel_size))
         self.kernel = torch.nn.Parameter(
             torch.empty(volume, in_channels, out_channels, dtype=dtype, device=device))
@@ -307,6 +287,8 @@ class SparseConv(Module):
         self._tuning_maps = None
         self._tuning_epilogue = (False, False, False, False)
         self._frozen_kernel_t = None
+        self._native_options = None
+        self._trivial = all(v == 1 for v in self.stride + self.dilation + self.kernel_size)
 
     def reset_parameters(self):
         """Uniform init in ``+-1/sqrt(fan * K^D)`` with ``fan`` the input channels
@@ -345,7 +327,7 @@ class SparseConv(Module):
 
     @property
     def is_trivial(self) -> bool:
-        return all(v == 1 for v in self.stride + self.dilation + self.kernel_size)
+        return self._trivial
 
     @property
     def _allow_shortcut_matmul(self) -> bool:
@@ -485,22 +467,43 @@ class SparseConv(Module):
         return out_c, out_s, out_bd
 
     def _lookup(self, inputs: SparseTensor):
-        """Output coordinates and the kernel map of this layer for ``inputs``."""
+        """Output coordinates, the kernel map of this layer for ``inputs`` and its plan:
+        found in the cache's own record of layers after the first time."""
         cache = self._kernel_map_cache
         if cache is None:
             raise ValueError("Kernel map cache must be specified")
-        coordinates, stride, batch_dims = cache.get_target_coordinates(
-            source_coordinates=inputs.C, source_batch_dims=inputs.batch_dims,
-            source_stride=inputs.stride, kernel_stride=self.stride, transposed=self.transposed)
-        source_masks, target_masks, order, sizes = cache.get_kernel_map(
-            source_coordinates=inputs.C, source_stride=inputs.stride,
-            source_batch_dims=inputs.batch_dims, target_coordinates=coordinates,
-            target_stride=stride, target_batch_dims=batch_dims, kernel_size=self.kernel_size,
-            kernel_dilation=self.dilation, transposed=self.transposed)
+        key = (inputs.stride, self._geometry)
+        hit = cache._layers.get(key)
+        if hit is None:
+            coordinates, stride, batch_dims = cache.get_target_coordinates(
+                source_coordinates=inputs.C, source_batch_dims=inputs.batch_dims,
+                source_stride=inputs.stride, kernel_stride=self.stride, transposed=self.transposed)
+            source_masks, target_masks, order, sizes = cache.get_kernel_map(
+                source_coordinates=inputs.C, source_stride=inputs.stride,
+                source_batch_dims=inputs.batch_dims, target_coordinates=coordinates,
+                target_stride=stride, target_batch_dims=batch_dims, kernel_size=self.kernel_size,
+                kernel_dilation=self.dilation, transposed=self.transposed)
+            plan, swapped = engine.plan_of(source_masks, target_masks, sizes)
+            hit = (coordinates, stride, batch_dims, source_masks, target_masks, order, sizes, plan, swapped)
+            cache._layers[key] = hit
         if self._tuning_data is not None:
+            _, _, _, source_masks, target_masks, order, sizes, _, _ = hit
             self._tuning_data.append((source_masks, target_masks, sizes))
             self._tuning_maps.append((source_masks, target_masks, order, sizes))
-        return coordinates, stride, batch_dims, source_masks, target_masks, order, sizes
+        return hit
+
+    def _options(self, relu: bool = False):
+        """The call options of this layer in native form (made once per configuration)."""
+        c = self._tunable_config
+        key = (conv_functional.ALGORITHM, conv_functional.IMPLICIT_SUB_TILES,
+               conv_functional.REORDER_ROWS, c.get("algorithm"), c.get("sub_tiles"),
+               c["gather_tile_size"], c["scatter_tile_size"], c["threshold"],
+               self._kernel_map_cache._disable_reordering, relu)
+        if self._native_options is None or self._native_options[0] != key:
+            self._native_options = (key, conv_functional.native_options(
+                c["gather_tile_size"], c["scatter_tile_size"], self._allow_shortcut_matmul,
+                c["threshold"], c.get("algorithm"), c.get("sub_tiles"), relu))
+        return self._native_options[1]
 
     def forward(self, inputs: SparseTensor) -> SparseTensor:
         features = inputs.F
@@ -516,19 +519,10 @@ class SparseConv(Module):
             out = F.dense_forward(features, self.kernel.view(self.in_channels, self.out_channels),
                                   shift=bias, weights_t=self._frozen_kernel_t)
             return SparseTensor(out, inputs.C, stride=inputs.stride, batch_dims=inputs.batch_dims)
-        else:
-            coordinates, stride, batch_dims, source_masks, target_masks, order, sizes = \
-                self._lookup(inputs)
-            out = F.sparse_convolution_forward(
-                sources=features, weights=self.kernel, source_masks=source_masks,
-                target_masks=target_masks, kernel_map_order=order, kernel_map_sizes=sizes,
-                gather_tile_size=self._tunable_config["gather_tile_size"],
-                scatter_tile_size=self._tunable_config["scatter_tile_size"],
-                allow_shortcut_matmul=self._allow_shortcut_matmul,
-                threshold=self._tunable_config["threshold"],
-                algorithm=self._tunable_config.get("algorithm"),
-                sub_tiles=self._tunable_config.get("sub_tiles"),
-                weights_t=self._frozen_kernel_t)
+        coordinates, stride, batch_dims, source_masks, target_masks, order, _, plan, swapped = \
+            self._lookup(inputs)
+        out = conv_functional.run(plan, swapped, features, self.kernel, source_masks, target_masks,
+                                  order, self._options(), self._frozen_kernel_t)
         if self.bias is not None:
             out += self.bias
         return SparseTensor(out, coordinates, stride=stride, batch_dims=batch_dims)
@@ -549,20 +543,14 @@ class SparseConv(Module):
             out = F.dense_forward(features, self.kernel.view(self.in_channels, self.out_channels),
                                   scale, shift, residual, relu, weights_t=self._frozen_kernel_t)
             return SparseTensor(out, inputs.C, stride=inputs.stride, batch_dims=inputs.batch_dims)
-        coordinates, stride, batch_dims, source_masks, target_masks, order, sizes = \
+        coordinates, stride, batch_dims, source_masks, target_masks, order, _, plan, swapped = \
             self._lookup(inputs)
         if self._tuning_data is not None:     # the tuner times the layer with the epilogue it runs
             self._tuning_epilogue = (scale is not None, shift is not None, residual is not None,
                                      bool(relu))
-        out = F.sparse_convolution_forward_fused(
-            sources=features, weights=self.kernel, source_masks=source_masks,
-            target_masks=target_masks, kernel_map_order=order, kernel_map_sizes=sizes,
-            gather_tile_size=self._tunable_config["gather_tile_size"],
-            scatter_tile_size=self._tunable_config["scatter_tile_size"],
-            allow_shortcut_matmul=self._allow_shortcut_matmul,
-            threshold=self._tunable_config["threshold"], scale=scale, shift=shift,
-            residual=residual, relu=relu, algorithm=self._tunable_config.get("algorithm"),
-            sub_tiles=self._tunable_config.get("sub_tiles"), weights_t=self._frozen_kernel_t)
+        out = conv_functional.run_fused(plan, swapped, features, self.kernel, source_masks,
+                                        target_masks, order, self._options(bool(relu)),
+                                        self._frozen_kernel_t, scale, shift, residual)
         return SparseTensor(out, coordinates, stride=stride, batch_dims=batch_dims)
 
 

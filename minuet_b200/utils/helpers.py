@@ -17,6 +17,8 @@ from torch.nn import Module
 def as_tuple(value, *, size: int = 3, name: Optional[str] = None):
     """``value`` repeated ``size`` times when it is a scalar, else checked to have
     ``size`` elements (minuet/utils/helpers.py:138-162)."""
+    if type(value) is tuple and len(value) == size:
+        return value
     if not isinstance(value, Iterable):
         return (value,) * size
     value = tuple(value)

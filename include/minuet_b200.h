@@ -60,6 +60,7 @@ typedef enum { MN_F32 = 0, MN_F16 = 1, MN_BF16 = 2 } mn_dtype;
 #define MN_CTRL_BARRIER_COUNT 32      /* byte offset 128 */
 #define MN_CTRL_BARRIER_GEN 64        /* copy k at word MN_CTRL_BARRIER_GEN + 32 * k */
 #define MN_CTRL_GEN_COPIES 16
+#define MN_CTRL_TICKET 640            /* arrival count that wraps to zero by itself */
 
 #define MN_STATUS_KEY_BOX 2       /* a coordinate fell outside the key box              */
 #define MN_STATUS_TC_TIMEOUT 4    /* a bounded barrier wait of a tensor-core kernel ran out */
@@ -89,7 +90,7 @@ typedef struct {
 /* Version of this interface; mn_version() returns the value the library was
  * built with.  A binding should refuse a library whose version differs from the
  * header it was written against: argument lists change between versions. */
-#define MN_ABI_VERSION 17
+#define MN_ABI_VERSION 18
 
 const char *mn_last_error(void);
 int mn_version(void);
@@ -199,18 +200,35 @@ mn_status mn_unique_coordinates_static(const int32_t *coords, int64_t n, int ndi
 
 /* Fused target-coordinate build of a strided convolution
  * (KernelMapCache.get_target_coordinates, minuet/nn/convolutions.py:85-96):
- * floor to the target stride, sort, unique; two launches.  Outputs: unique_out
+ * floor to the target stride, sort, unique.  Outputs: unique_out
  * int32 [n, ndim], keys_out uint64 [n] (sorted unique keys), and meta_out int64
- * [num_clouds + 3] = { number of unique rows, batch_dims of the result
- * [num_clouds + 1], copy of the status word }, so that one small read brings
- * back everything the host needs.  batch_dims == NULL means one cloud
- * (meta_out then has 4 entries).  ctrl: the control block. */
+ * [num_clouds + 4] = { number of unique rows, batch_dims of the result
+ * [num_clouds + 1], copy of the status word, key bits of the layout }, so that one
+ * small read brings back everything the host needs.  A spec whose total_bits is
+ * positive saves the launches of the digits that a layout known only to the device
+ * might have.  batch_dims == NULL means one cloud
+ * (meta_out then has 5 entries).  ctrl: the control block. */
 mn_status mn_downsample_coordinates(const int32_t *coords, int64_t n, int ndim,
                                     const int64_t *batch_dims, int64_t num_clouds,
                                     const int32_t *tstride, const mn_keyspec *spec,
                                     int32_t *unique_out, uint64_t *keys_out,
                                     int64_t *meta_out, int32_t *ctrl, void *ws,
                                     size_t ws_bytes, void *stream);
+
+/* Voxelisation of floating-point points (float, or double with points_are_double):
+ * voxels_out int32 [n, ndim] = the distinct floor(point / voxel_size) (HOST [ndim]; the
+ * arithmetic is the points' own type), cloud-major, then lexicographic; inverse_out int64 [n]
+ * (may be NULL): the voxel of every point; means_out [n, channels] (with features): mean feature
+ * of every voxel, summed in sorted order in fp32.  meta_out as mn_downsample_coordinates; only
+ * its first entry's worth of rows of voxels_out and means_out is written.  The result is valid
+ * when the key bits of the layout (last entry of meta_out) plus ceil(log2 n) (at least 1) are at
+ * most 64; boxes wider than that take arg sort, unique and mn_voxel_mean one by one. */
+size_t mn_voxelize_workspace_bytes(int64_t n);
+mn_status mn_voxelize(const void *points, int points_are_double, int64_t n, int ndim,
+                      const double *voxel_size, const int64_t *batch_dims, int64_t num_clouds,
+                      const void *features, int64_t channels, mn_dtype dtype, int32_t *voxels_out,
+                      int64_t *inverse_out, void *means_out, int64_t *meta_out, int32_t *ctrl,
+                      void *ws, size_t ws_bytes, void *stream);
 
 /* _C.cuda_query_sorted_index_with_offsets / _C.cuda_multi_query_...
  * (csrc/minuet/torch/cuda_sparse_convolution_mapping.cu:9-100) on packed keys:

@@ -46,7 +46,7 @@ namespace {
   X(mn_conv_workspace_bytes) X(mn_sparse_convolution_forward) X(mn_apply_epilogue)                \
   X(mn_dense_supported) X(mn_dense_workspace_bytes) X(mn_dense_forward) X(mn_dense_forward_simt)  \
   X(mn_pair_list_rows) X(mn_build_pair_lists) X(mn_weight_gradient_workspace_bytes)               \
-  X(mn_sparse_convolution_weight_gradient)
+  X(mn_sparse_convolution_weight_gradient) X(mn_voxelize_workspace_bytes) X(mn_voxelize)
 
 struct Api {
 #define MN_DECLARE(name) decltype(&::name) name = nullptr;
@@ -219,6 +219,26 @@ int poll_status(int device) {
 struct KeyLayout {
   mn_keyspec spec{};
   Tensor dev;      // device copy of the layout, alive as long as this object
+
+  ~KeyLayout() { pinned_pool().give(bits_); }
+  // The width of the keys follows on a copy of its own: where it has landed by the time a sort is
+  // launched, no digit too many is (a digit pass that finds nothing to do is 2-4 us).
+  void expect_bits(cudaStream_t st) {
+    bits_ = pinned_pool().take(dev.get_device());
+    check_cuda(cudaMemcpyAsync(bits_.host, static_cast<char *>(dev.data_ptr()) + offsetof(mn_keyspec, total_bits),
+                               sizeof(int32_t), cudaMemcpyDeviceToHost, st), "key layout");
+    check_cuda(cudaEventRecord(bits_.event, st), "key layout");
+  }
+  void look_for_bits() {
+    if (spec.total_bits > 0 || bits_.host == nullptr) return;
+    if (cudaEventQuery(bits_.event) == cudaSuccess)
+      spec.total_bits = *static_cast<int32_t *>(bits_.host);
+    else
+      (void)cudaGetLastError();   // "not ready" of a query is not an error of this thread
+  }
+
+ private:
+  PinnedPool::Buffer bits_;
 };
 
 struct Offsets {
@@ -254,6 +274,7 @@ std::pair<std::shared_ptr<KeyLayout>, Tensor> root_keys(const Tensor &coords, co
                               raw<uint64_t>(keys), ctrl_of(coords), ws.data_ptr(), (size_t)ws.numel(),
                               stream_of(coords)),
         "keyspec_device");
+  layout->expect_bits(stream_of(coords));
   return {layout, keys};
 }
 
@@ -309,18 +330,58 @@ std::tuple<Tensor, Tensor, Tensor, std::vector<int64_t>> downsample(const Tensor
   const int64_t nb = batch_dims.has_value() ? batch_dims->numel() - 1 : 1;
   Tensor unique = empty_on(coords, {n, ndim}, at::kInt);
   Tensor keys = empty_on(coords, {n}, at::kLong);
-  Tensor meta = empty_on(coords, {nb + 3}, at::kLong);   // count, cloud starts, status
+  Tensor meta = empty_on(coords, {nb + 4}, at::kLong);   // count, cloud starts, status, key bits
   Tensor ws = workspace(coords, api.mn_map_workspace_bytes(n, n, 1));
+  layout.look_for_bits();
   check(api.mn_downsample_coordinates(raw<int32_t>(coords), n, (int)ndim, raw<int64_t>(batch_dims), nb,
                                       tstride.data(), &layout.spec, raw<int32_t>(unique), raw<uint64_t>(keys),
                                       raw<int64_t>(meta), ctrl_of(coords), ws.data_ptr(), (size_t)ws.numel(),
                                       stream_of(coords)),
         "downsample_coordinates");
-  std::vector<int64_t> host = read_back(meta);
+  const std::vector<int64_t> host = read_back(meta);
   if (host[(size_t)nb + 2] != 0) raise_device_status((int)host[(size_t)nb + 2], coords.get_device());
+  layout.spec.total_bits = (int32_t)host[(size_t)nb + 3];   // later levels launch no digit too many
   const int64_t count = host[0];
   return {unique.narrow(0, 0, count), keys.narrow(0, 0, count), meta.narrow(0, 1, nb + 1),
           std::vector<int64_t>(host.begin() + 1, host.begin() + nb + 2)};
+}
+
+// Distinct voxels of floating-point points: (voxels, cloud starts, inverse or None, means or None), or
+// None when the voxels' box is too wide for keys that carry the point's index.
+std::optional<std::tuple<Tensor, Tensor, OptTensor, OptTensor>> voxelize(const Tensor &points_in,
+                                                                         const std::vector<double> &voxel_size,
+                                                                         const OptTensor &batch_dims, bool inverse,
+                                                                         const OptTensor &features_in) {
+  at::NoGradGuard no_grad;
+  if (!points_in.is_cuda()) not_on_gpu();
+  c10::cuda::CUDAGuard guard(points_in.get_device());
+  const Tensor points = points_in.contiguous();
+  const int64_t n = points.size(0), ndim = points.size(1);
+  const int64_t nb = batch_dims.has_value() ? batch_dims->numel() - 1 : 1;
+  OptTensor features, means, inv;
+  if (features_in.has_value()) {
+    if (!features_in->is_cuda()) not_on_gpu();
+    features = features_in->contiguous();
+    means = empty_on(*features, {n, features->size(1)}, features->scalar_type());
+  }
+  if (inverse) inv = empty_on(points, {n}, at::kLong);
+  Tensor voxels = empty_on(points, {n, ndim}, at::kInt);
+  Tensor meta = empty_on(points, {nb + 4}, at::kLong);
+  Tensor ws = workspace(points, api.mn_voxelize_workspace_bytes(n));
+  check(api.mn_voxelize(points.data_ptr(), points.scalar_type() == at::kDouble, n, (int)ndim, voxel_size.data(),
+                        raw<int64_t>(batch_dims), nb, raw<void>(features), features.has_value() ? features->size(1) : 0,
+                        features.has_value() ? dtype_code(features->scalar_type()) : MN_F32, raw<int32_t>(voxels),
+                        raw<int64_t>(inv), raw<void>(means), raw<int64_t>(meta), ctrl_of(points), ws.data_ptr(),
+                        (size_t)ws.numel(), stream_of(points)),
+        "voxelize");
+  const std::vector<int64_t> host = read_back(meta);
+  int index_bits = 1;
+  while ((1ll << index_bits) < n) index_bits++;
+  if (host[(size_t)nb + 3] + index_bits > 64) return std::nullopt;
+  if (host[(size_t)nb + 2] != 0) raise_device_status((int)host[(size_t)nb + 2], points.get_device());
+  const int64_t count = host[0];
+  if (means.has_value()) means = means->narrow(0, 0, count);
+  return std::make_tuple(voxels.narrow(0, 0, count), meta.narrow(0, 1, nb + 1), inv, means);
 }
 
 // ---------------------------------------------------------------------------
@@ -784,6 +845,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("root_keys", &root_keys);
   m.def("pack_keys", &pack_keys);
   m.def("downsample", &downsample, NoGil());
+  m.def("voxelize", &voxelize, NoGil());
   py::class_<Plan, PlanPtr>(m, "Plan")
       .def(py::init<int64_t, int64_t, int64_t>())
       .def("set_sizes", &Plan::set_sizes)

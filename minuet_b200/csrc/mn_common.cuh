@@ -196,11 +196,5 @@ struct SortSource {
   int ndim;
   const int32_t *tstride;   // host, may be NULL
 };
-mn_status launch_radix_sort(uint64_t *keys, uint64_t *keys_tmp, int32_t *vals, int32_t *vals_tmp,
-                            bool iota_vals, int64_t n, int begin_bit, int end_bit,
-                            const mn_keyspec &spec, const SortSource *source, int32_t *ctrl,
-                            int32_t *result_in_second_dev, Workspace &ws, bool *result_in_tmp,
-                            cudaStream_t st);
-size_t radix_sort_workspace_bytes(int64_t n);
 
 }  // namespace mn

@@ -28,6 +28,7 @@
 // from a divergent lane-0 branch every MMA took about 150 cycles of register moves), a
 // lane reads the indices of all its rows with one load, two offsets ahead, and the next
 // stage's barrier is probed before the current stage is worked on.
+#include "mn_sort.cuh"
 #include "mn_tc.cuh"
 
 #include <algorithm>
@@ -644,24 +645,6 @@ neighbor_table_kernel(const int32_t *__restrict__ target_masks, int64_t T, int64
   if (threadIdx.x == 0) tile_bits[blockIdx.x] = s_bits;
 }
 
-// sort keys of the row permutation: the row's hit word with its bits reversed (rows with
-// the same set of offsets become neighbours, so whole tiles can skip the offsets none of
-// their rows has).  Mask rows are in ascending size order, so the reversal makes the RARE
-// offsets the most significant key bits: the few rows that have a rare offset end up
-// together instead of sprinkling it over many tiles (15 against 20 offsets per tile on a
-// map with 9 pairs per row).
-__global__ void hit_word_keys_kernel(const uint32_t *__restrict__ bits, int64_t n, int num_offsets,
-                                     uint64_t *__restrict__ keys) {
-  const int64_t gsz = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gsz) {
-    // position of the reversed word in the reflected Gray sequence: neighbouring keys then
-    // differ in one offset instead of many (2-5 % fewer offsets per tile than binary order)
-    uint32_t r = __brev(__ldg(bits + i)) >> (32 - num_offsets);
-    r ^= r >> 1; r ^= r >> 2; r ^= r >> 4; r ^= r >> 8; r ^= r >> 16;
-    keys[i] = (uint64_t)r;
-  }
-}
-
 }  // namespace
 
 namespace {
@@ -733,7 +716,7 @@ extern "C" size_t mn_neighbor_table_workspace_bytes(const int32_t *sizes_host, i
   int64_t e = 0;
   for (int64_t p = 0; p < O; p++) e += sizes_host[p];
   const size_t n = (size_t)std::max<int64_t>(T, 1);
-  const size_t sort = 2 * align_up(n * 8, 256) + 2 * align_up(n * 4, 256) + radix_sort_workspace_bytes(T);
+  const size_t sort = 2 * align_up(n * 8, 256) + rsort::workspace_bytes(T);
   return align_up((size_t)std::max<int64_t>(e, 1) * sizeof(int32_t), 256) + sort + 1024;
 }
 
@@ -765,17 +748,15 @@ extern "C" mn_status mn_build_neighbor_table(const int32_t *source_masks,
   if (perm_out != nullptr) {
     // stable sort of the rows by hit word: perm[r] = target row at position r
     uint64_t *keys = ws.take<uint64_t>(T), *keys_tmp = ws.take<uint64_t>(T);
-    int32_t *vals = ws.take<int32_t>(T), *vals_tmp = ws.take<int32_t>(T);
     MN_CHECK_WS(ws);
-    const int blocks = (int)std::min<int64_t>(kNumSMs * 8, div_up(T, 256));
-    MN_LAUNCH("hit_word_keys_kernel", st,
-              hit_word_keys_kernel<<<blocks, 256, 0, st>>>(target_bits, T, (int)O, keys));
-    const mn_keyspec no_spec{};
-    bool in_tmp = false;
-    MN_RETURN_IF(launch_radix_sort(keys, keys_tmp, vals, vals_tmp, true, T, 0, (int)O, no_spec,
-                                   nullptr, ctrl, nullptr, ws, &in_tmp, st));
-    MN_CHECK_CUDA(cudaMemcpyAsync(perm_out, in_tmp ? vals_tmp : vals, (size_t)T * sizeof(int32_t),
-                                  cudaMemcpyDeviceToDevice, st));
+    rsort::Args a{};
+    a.keys[0] = keys; a.keys[1] = keys_tmp;
+    a.n = T;
+    a.first_bit = rsort::bits_for(T);
+    a.bits = (int)O;
+    a.status = ctrl + MN_CTRL_STATUS;
+    a.index32 = perm_out;
+    MN_RETURN_IF(rsort::run(a, HitWordKeys{target_bits, (int32_t)O, a.first_bit}, ws, st));
   }
   // a scattered 4-byte read costs a 32-byte sector: worth it while the pairs are fewer than
   // an eighth of the mask entries

@@ -36,7 +36,7 @@
 // no separate scan kernel.  For submanifold maps (sources == targets,
 // symmetric offsets) the source mask of offset o is read off the hit bits of
 // the mirrored offset.
-#include "mn_grid.cuh"
+#include "mn_sort.cuh"
 
 #include <algorithm>
 #include <vector>
@@ -899,7 +899,7 @@ using namespace mn;
 extern "C" size_t mn_map_workspace_bytes(int64_t S, int64_t T, int64_t O) {
   const int64_t n = std::max<int64_t>(std::max(S, T), 1);
   size_t sort = 2 * align_up((size_t)n * 8, 256) + 2 * align_up((size_t)n * 4, 256) +
-                radix_sort_workspace_bytes(n) + align_up((size_t)div_up(n, 2048) * 4, 256) + 512;
+                rsort::workspace_bytes(n) + align_up((size_t)div_up(n, 2048) * 4, 256) + 512;
   const int64_t tiles = div_up(S, kMTile) + div_up(T, kMTile) + 2;
   size_t map = align_up((size_t)S * 4, 256) + align_up((size_t)T * 4, 256) +
                2 * align_up((size_t)std::max<int64_t>(O, 1) * tiles * 4, 256) +

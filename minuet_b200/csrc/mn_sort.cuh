@@ -1,0 +1,378 @@
+// Stable radix sort of 64-bit keys, shared by the map step, voxelisation and the neighbour
+// tables: one launch that makes the keys and counts their digits, then one launch per 8-bit
+// digit.
+//
+// A digit pass moves every key once: a block takes the next tile of keys, ranks them in
+// registers (equal digits of a warp find each other with match.any), learns how many keys of
+// each digit the tiles before it hold by looking back over their published counts (every thread
+// follows one digit; a tile publishes its own count at once and the running total as soon as it
+// knows it), reorders the tile in shared memory and writes it out in runs.  Tiles are numbered
+// in the order in which blocks start, so a block only ever waits for blocks that already run;
+// the waits are bounded all the same (status bit 4).  An index that travels with the keys sits
+// in their low bits where both fit 64 bits (8 bytes per key and pass instead of 12), in an array
+// of its own otherwise.
+//
+// A pass is bound by latency at small sizes (two dependent rounds of loads and the look-back)
+// and by instruction issue at large ones.  The kernel it replaces, one cooperative launch with
+// two grid-wide barriers per pass and every block reading every block's counts, took 12 us per
+// pass at 120 000 keys and 147 us at 7.3 million.
+#pragma once
+
+#include "mn_grid.cuh"
+#include "mn_pack.cuh"
+
+#include <algorithm>
+
+namespace mn {
+namespace rsort {
+
+constexpr int kThreads = 256;
+constexpr int kWarps = kThreads / 32;
+constexpr int kBits = 8;
+constexpr int kDigits = 1 << kBits;           // == kThreads: a thread per digit
+constexpr int kMaxPasses = 8;
+constexpr uint32_t kSpinLimit = 1u << 22;
+
+struct Args {
+  uint64_t *keys[2];          // ping-pong buffers; the keys start in [0]
+  int32_t *vals[2];           // index array of its own, or NULL
+  int64_t n;
+  int32_t first_bit;          // lowest key bit that is sorted on
+  int32_t bits;               // sorted bits; < 0: the key layout's total_bits
+  SpecRef spec;
+  uint32_t *hist;             // [kMaxPasses][kDigits], zeroed
+  uint32_t *next_tile;        // [kMaxPasses], zeroed
+  uint32_t *state;            // [passes][tiles][kDigits], zeroed
+  int32_t *result_in_second;  // out (may be NULL): 1 when the result is in keys[1]
+  int32_t *status;            // device status word
+  int32_t tiles;
+  // the last pass may write the index (low `first_bit` bits of the key, or vals) instead of keys
+  int32_t *index32;
+  int64_t *index64;
+};
+
+__device__ __forceinline__ int passes_of(const Args &a) {
+  const int bits = a.bits >= 0 ? a.bits : spec_of(a.spec).total_bits;
+  const int p = (bits + kBits - 1) / kBits;
+  return p < 1 ? 1 : (p > kMaxPasses ? kMaxPasses : p);
+}
+
+__device__ __forceinline__ unsigned lanes_below() {
+  unsigned m;
+  asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
+  return m;
+}
+
+// Makes the keys and counts the digits of all passes.  A digit that a whole warp shares (the high
+// digits of sorted input, most digits of hit words) is added once.
+template <typename Source>
+__global__ void __launch_bounds__(kThreads)
+sort_keys_kernel(const __grid_constant__ Args a, const __grid_constant__ Source source) {
+  __shared__ uint32_t s_hist[kMaxPasses][kDigits];
+  const int passes = passes_of(a);
+  for (int i = threadIdx.x; i < passes * kDigits; i += kThreads) (&s_hist[0][0])[i] = 0u;
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  const int64_t gsz = (int64_t)gridDim.x * kThreads;
+  for (int64_t i0 = (int64_t)blockIdx.x * kThreads; i0 < a.n; i0 += gsz) {
+    const int64_t i = i0 + threadIdx.x;
+    const bool valid = i < a.n;
+    const uint64_t key = valid ? source(i) : 0ull;
+    if (valid) {
+      a.keys[0][i] = key;
+      if (a.vals[0] != nullptr) a.vals[0][i] = (int32_t)i;
+    }
+    const unsigned live = __ballot_sync(0xffffffffu, valid);
+    if (live == 0u) continue;
+    const int leader = __ffs(live) - 1;
+    for (int p = 0; p < passes; p++) {
+      const unsigned d = (unsigned)(key >> (a.first_bit + p * kBits)) & (kDigits - 1);
+      const unsigned d0 = __shfl_sync(0xffffffffu, d, leader);
+      if (__all_sync(0xffffffffu, d == d0 || !valid)) {
+        if (lane == leader) atomicAdd(&s_hist[p][d0], (uint32_t)__popc(live));
+      } else if (valid) {
+        atomicAdd(&s_hist[p][d], 1u);
+      }
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < passes * kDigits; i += kThreads) {
+    const uint32_t v = (&s_hist[0][0])[i];
+    if (v != 0u) atomicAdd(a.hist + i, v);
+  }
+}
+
+// exclusive prefix of one value per thread over the block; s_part: [kWarps]
+__device__ __forceinline__ uint32_t block_exclusive(uint32_t v, uint32_t *s_part, int lane, int warp) {
+  uint32_t inc = v;
+#pragma unroll
+  for (int s = 1; s < 32; s <<= 1) {
+    const uint32_t t = __shfl_up_sync(0xffffffffu, inc, s);
+    if (lane >= s) inc += t;
+  }
+  if (lane == 31) s_part[warp] = inc;
+  __syncthreads();
+  uint32_t before = 0;
+  for (int w = 0; w < warp; w++) before += s_part[w];
+  __syncthreads();
+  return before + inc - v;
+}
+
+template <int kItems, bool kVals>
+__global__ void __launch_bounds__(kThreads)
+sort_pass_kernel(const __grid_constant__ Args a, int pass) {
+  constexpr int kTile = kThreads * kItems;
+  __shared__ uint64_t s_key[kTile];
+  __shared__ uint32_t s_cnt[kWarps][kDigits];     // counts, then first position, per warp and digit
+  __shared__ uint32_t s_local[kDigits];              // first position of a digit inside the tile
+  __shared__ uint32_t s_dest[kDigits];               // its first position in the output, minus s_local
+  __shared__ uint32_t s_part[kWarps];
+  __shared__ int s_tile;
+  const int passes = passes_of(a);
+  if (pass >= passes) return;
+  const bool last_pass = pass + 1 == passes;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const unsigned lt = lanes_below();
+  if (tid == 0) s_tile = (int)atomicAdd(a.next_tile + pass, 1u);
+#pragma unroll
+  for (int w = 0; w < kWarps; w++) s_cnt[w][tid] = 0u;
+  // where the digit starts in the output (every block adds up the 256 totals itself)
+  const uint32_t digit_start = block_exclusive(__ldcg(a.hist + pass * kDigits + tid), s_part, lane, warp);
+  const int tile = s_tile;
+  if (tile >= a.tiles) return;
+  if (tile == 0 && tid == 0 && last_pass && a.result_in_second != nullptr) *a.result_in_second = passes & 1;
+
+  const uint64_t *kin = a.keys[pass & 1];
+  const int shift = a.first_bit + pass * kBits;
+  const int64_t base = (int64_t)tile * kTile + warp * (kItems * 32) + lane;
+  uint64_t key[kItems];
+#pragma unroll
+  for (int j = 0; j < kItems; j++) key[j] = base + j * 32 < a.n ? __ldcg(kin + base + j * 32) : ~0ull;
+  // ---- rank inside the warp: position among the equal digits of the warp's slice ------------
+  uint16_t rank[kItems];
+  uint32_t *mine = s_cnt[warp];
+#pragma unroll
+  for (int j = 0; j < kItems; j++) {
+    const bool valid = base + j * 32 < a.n;
+    const unsigned d = valid ? (unsigned)(key[j] >> shift) & (kDigits - 1) : (unsigned)kDigits;
+    const unsigned peers = __match_any_sync(0xffffffffu, d);
+    uint32_t before = 0;
+    if (valid) before = mine[d];
+    __syncwarp();
+    if (valid && (peers & lt) == 0u) mine[d] = before + __popc(peers);
+    rank[j] = (uint16_t)(before + __popc(peers & lt));
+    __syncwarp();
+  }
+  __syncthreads();
+  // ---- per digit: the warps' first positions, the tile's count ---------------------------------
+  uint32_t count = 0;
+#pragma unroll
+  for (int w = 0; w < kWarps; w++) {
+    const uint32_t c = s_cnt[w][tid];
+    s_cnt[w][tid] = count;
+    count += c;
+  }
+  // a published word: 2 * value + (running total ? 1 : 0) + 1; 0: nothing yet
+  volatile uint32_t *state = a.state + ((size_t)pass * a.tiles) * kDigits + tid;
+  state[(size_t)tile * kDigits] = 2u * count + (tile == 0 ? 2u : 1u);
+  const uint32_t local = block_exclusive(count, s_part, lane, warp);
+  // ---- look back: keys of this digit in the tiles before ----------------------------------------
+  uint32_t before = 0;
+  if (tile > 0) {
+    uint32_t spins = 0;
+    for (int prev = tile - 1; prev >= 0;) {
+      const uint32_t v = state[(size_t)prev * kDigits];
+      if (v == 0u) {
+        if (++spins > kSpinLimit) { atomicOr(a.status, MN_STATUS_GRID_TIMEOUT); break; }
+        continue;
+      }
+      before += (v - 1u) >> 1;
+      if (((v - 1u) & 1u) != 0u) break;
+      prev--;
+    }
+    state[(size_t)tile * kDigits] = 2u * (before + count) + 2u;
+  }
+  s_local[tid] = local;
+  s_dest[tid] = digit_start + before - local;
+  __syncthreads();
+  // ---- reorder in shared memory, write in runs -------------------------------------------------
+#pragma unroll
+  for (int j = 0; j < kItems; j++) {
+    if (base + j * 32 < a.n) {
+      const unsigned d = (unsigned)(key[j] >> shift) & (kDigits - 1);
+      const uint32_t pos = s_local[d] + s_cnt[warp][d] + rank[j];
+      rank[j] = (uint16_t)pos;
+      s_key[pos] = key[j];
+    }
+  }
+  __syncthreads();
+  const int in_tile = (int)min((int64_t)kTile, a.n - (int64_t)tile * kTile);
+  const bool write_index = last_pass && (a.index32 != nullptr || a.index64 != nullptr);
+  uint64_t *kout = a.keys[(pass & 1) ^ 1];
+  const uint64_t index_mask = (1ull << a.first_bit) - 1ull;
+  uint32_t dest[kItems];
+#pragma unroll
+  for (int j = 0; j < kItems; j++) {
+    const int i = j * kThreads + tid;
+    if (i < in_tile) {
+      const uint64_t k = s_key[i];
+      // a timed-out look-back (status bit 4) must not write outside the arrays
+      dest[j] = min(s_dest[(unsigned)(k >> shift) & (kDigits - 1)] + (uint32_t)i, (uint32_t)a.n - 1u);
+      if (!write_index) kout[dest[j]] = k;
+      else if (!kVals && a.index32 != nullptr) a.index32[dest[j]] = (int32_t)(k & index_mask);
+      else if (!kVals) a.index64[dest[j]] = (int64_t)(k & index_mask);
+    }
+  }
+  if (kVals) {
+    // the index array follows the same way
+    int32_t *s_val = reinterpret_cast<int32_t *>(s_key);
+    const int32_t *vin = a.vals[pass & 1];
+    int32_t val[kItems];
+#pragma unroll
+    for (int j = 0; j < kItems; j++) val[j] = base + j * 32 < a.n ? __ldcg(vin + base + j * 32) : 0;
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < kItems; j++)
+      if (base + j * 32 < a.n) s_val[rank[j]] = val[j];
+    __syncthreads();
+    int32_t *vout = a.vals[(pass & 1) ^ 1];
+#pragma unroll
+    for (int j = 0; j < kItems; j++) {
+      const int i = j * kThreads + tid;
+      if (i < in_tile) {
+        const int32_t v = s_val[i];
+        if (!write_index) vout[dest[j]] = v;
+        else if (a.index32 != nullptr) a.index32[dest[j]] = v;
+        else a.index64[dest[j]] = v;
+      }
+    }
+  }
+}
+
+// 4096 keys per tile; 1024 where those would leave SMs without a tile (a pass is then a chain of
+// latencies, and smaller tiles shorten every link).
+inline int items_of(int64_t n) { return n < 4096ll * kNumSMs ? 4 : 16; }
+inline int64_t tiles_of(int64_t n) { return div_up(std::max<int64_t>(n, 1), (int64_t)kThreads * items_of(n)); }
+inline size_t control_words(int64_t n, int passes) {
+  return (size_t)kMaxPasses * kDigits + 64 + (size_t)passes * tiles_of(n) * kDigits;
+}
+inline size_t workspace_bytes(int64_t n) { return align_up(control_words(n, kMaxPasses) * sizeof(uint32_t), 256) + 256; }
+
+inline int bits_for(int64_t values) {    // bits that tell `values` different values apart, at least 1
+  int b = 1;
+  while ((1ll << b) < values) b++;
+  return b;
+}
+
+template <int kItems>
+mn_status launch_passes(const Args &a, int launches, cudaStream_t st) {
+  for (int p = 0; p < launches; p++) {
+    if (a.vals[0] != nullptr) {
+      MN_LAUNCH("sort_pass_kernel", st, sort_pass_kernel<kItems, true><<<a.tiles, kThreads, 0, st>>>(a, p));
+    } else {
+      MN_LAUNCH("sort_pass_kernel", st, sort_pass_kernel<kItems, false><<<a.tiles, kThreads, 0, st>>>(a, p));
+    }
+  }
+  return MN_OK;
+}
+
+// Stable sort on key bits [first_bit, first_bit + bits) (bits < 0: the key layout's, known on
+// the device).  `a` comes with keys, n, bits, spec and what the last pass writes.
+template <typename Source>
+mn_status run(Args a, const Source &source, Workspace &ws, cudaStream_t st) {
+  MN_CHECK_ARG(a.n > 0 && a.n < (1ll << 31) - 1, "radix sort: n = %lld exceeds 2^31-2", (long long)a.n);
+  a.tiles = (int32_t)tiles_of(a.n);
+  const int launches = a.bits >= 0 ? std::min(kMaxPasses, std::max(1, (a.bits + kBits - 1) / kBits)) : kMaxPasses;
+  uint32_t *control = ws.take<uint32_t>(control_words(a.n, kMaxPasses));
+  MN_CHECK_WS(ws);
+  a.hist = control;
+  a.next_tile = control + kMaxPasses * kDigits;
+  a.state = a.next_tile + 64;
+  MN_CHECK_CUDA(cudaMemsetAsync(control, 0, control_words(a.n, launches) * sizeof(uint32_t), st));
+  const int blocks = (int)std::min<int64_t>(kNumSMs * 8, div_up(a.n, kThreads));
+  MN_LAUNCH("sort_keys_kernel", st, sort_keys_kernel<Source><<<blocks, kThreads, 0, st>>>(a, source));
+  return items_of(a.n) == 4 ? launch_passes<4>(a, launches, st) : launch_passes<16>(a, launches, st);
+}
+
+}  // namespace rsort
+
+// Where keys come from.  (Outside any unnamed namespace: kernels are instantiated on these.)
+struct CoordKeys {            // coordinate rows, floored to a target stride and packed
+  const int32_t *coords;
+  const int64_t *batch_dims;
+  int32_t ndim, num_clouds, index_bits;   // index_bits > 0: the row index goes below the key
+  PackParams pack;
+  int32_t *status;
+  __device__ __forceinline__ uint64_t operator()(int64_t r) const {
+    const mn_keyspec &spec = spec_of(pack.spec);
+    int c[4] = {0, 0, 0, 0};
+    for (int k = 0; k < ndim; k++) c[k] = __ldg(coords + r * ndim + k);
+    const uint64_t g = batch_dims != nullptr ? cloud_of(batch_dims, num_clouds, r) : 0;
+    bool bad = false;
+    const uint64_t key = pack_one(c, ndim, g, spec, pack, bad);
+    if (bad) atomicOr(status, MN_STATUS_KEY_BOX);
+    return index_bits > 0 ? (key << index_bits) | (uint64_t)r : key;
+  }
+};
+
+// Keys of one pass of the dimension-by-dimension sort: the coordinate of dimension `dim`
+// (dim >= 0; sign bit flipped, so that unsigned order is signed order) or the cloud (dim < 0) of
+// the row that currently sits at position i, the row itself below.
+struct DimensionKeys {
+  const int32_t *coords;
+  const int32_t *perm;
+  const int64_t *batch_dims;
+  int32_t ndim, dim, num_clouds, index_bits;
+  __device__ __forceinline__ uint64_t operator()(int64_t i) const {
+    const int64_t row = perm != nullptr ? perm[i] : i;
+    const uint64_t k = dim >= 0 ? (uint64_t)((uint32_t)__ldg(coords + row * ndim + dim) ^ 0x80000000u)
+                                : (uint64_t)cloud_of(batch_dims, num_clouds, row);
+    return (k << index_bits) | (uint64_t)row;
+  }
+};
+
+// Sort keys of a neighbour table's row permutation: the row's hit word with its bits reversed, so
+// that rows with the same set of offsets become neighbours and whole tiles can skip the offsets
+// none of their rows has.  Mask rows are in ascending size order, so the reversal makes the RARE
+// offsets the most significant key bits: the few rows that have a rare offset end up together
+// instead of sprinkling it over many tiles.  The key is the reversed word's position in the
+// reflected Gray sequence: neighbouring keys differ in one offset instead of many (2-5 % fewer
+// offsets per tile than binary order).  The row itself sits below.
+struct HitWordKeys {
+  const uint32_t *bits;
+  int32_t num_offsets, index_bits;
+  __device__ __forceinline__ uint64_t operator()(int64_t i) const {
+    uint32_t r = __brev(__ldg(bits + i)) >> (32 - num_offsets);
+    r ^= r >> 1; r ^= r >> 2; r ^= r >> 4; r ^= r >> 8; r ^= r >> 16;
+    return ((uint64_t)r << index_bits) | (uint64_t)i;
+  }
+};
+
+// Voxels of floating-point points: floor(point / size) in the points' own type.
+template <typename F>
+struct VoxelPoints {
+  const F *points;
+  F size[4];
+  int32_t ndim;
+  __device__ __forceinline__ void operator()(int64_t r, int (&c)[4]) const {
+#pragma unroll
+    for (int k = 0; k < 4; k++) c[k] = k < ndim ? (int)floor(__ldg(points + r * ndim + k) / size[k]) : 0;
+  }
+};
+
+template <typename F>
+struct VoxelKeys {
+  VoxelPoints<F> voxel;
+  const int64_t *batch_dims;
+  int32_t num_clouds, index_bits;
+  PackParams pack;
+  __device__ __forceinline__ uint64_t operator()(int64_t r) const {
+    int c[4];
+    voxel(r, c);
+    const uint64_t g = batch_dims != nullptr ? cloud_of(batch_dims, num_clouds, r) : 0;
+    bool bad = false;
+    return (pack_one(c, voxel.ndim, g, spec_of(pack.spec), pack, bad) << index_bits) | (uint64_t)r;
+  }
+};
+
+}  // namespace mn

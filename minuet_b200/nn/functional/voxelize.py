@@ -30,6 +30,12 @@ def voxelize(coordinates: torch.Tensor, voxel_size, batch_dims: Optional[torch.T
     """
     if coordinates.ndim != 2:
         raise ValueError(f"coordinates must be [N, D] but found {coordinates.ndim}-D")
+    if features is not None and (features.ndim != 2 or features.shape[0] != coordinates.shape[0]):
+        raise ValueError("features must be [N, C] with one row per point")
+    native = _native(coordinates, voxel_size, batch_dims, return_inverse, features)
+    if native is not None:
+        return native
+    # other point types, sizes in tensors, boxes too wide for one key: step by step
     size = torch.as_tensor(voxel_size, dtype=coordinates.dtype, device=coordinates.device)
     voxels = torch.floor(coordinates / size).to(torch.int32)
     index = build_sorted_index(voxels, batch_dims=batch_dims)
@@ -46,8 +52,6 @@ def voxelize(coordinates: torch.Tensor, voxel_size, batch_dims: Optional[torch.T
         inverse[index] = run_ids
         result.append(inverse)
     if features is not None:
-        if features.ndim != 2 or features.shape[0] != coordinates.shape[0]:
-            raise ValueError("features must be [N, C] with one row per point")
         engine.require_cuda(features)
         feats = features.contiguous()
         means = torch.empty((unique.shape[0], feats.shape[1]), dtype=feats.dtype,
@@ -56,5 +60,33 @@ def voxelize(coordinates: torch.Tensor, voxel_size, batch_dims: Optional[torch.T
             engine.ptr(feats), feats.shape[0], feats.shape[1], engine.dtype_code(feats.dtype),
             engine.ptr(index.to(torch.int64).contiguous()), engine.ptr(run_ids), engine.ptr(means),
             engine.stream_ptr(feats.device)), "voxel_mean")
+        result.append(means)
+    return tuple(result)
+
+
+def _native(coordinates, voxel_size, batch_dims, return_inverse, features):
+    """The whole of it in a handful of launches and one read of the number of voxels; None
+    where that path does not apply."""
+    n, ndim = coordinates.shape
+    if not coordinates.is_cuda or coordinates.dtype not in (torch.float32, torch.float64) or \
+            n == 0 or ndim > _lib.MN_MAX_NDIM or isinstance(voxel_size, torch.Tensor):
+        return None
+    if features is not None and (features.shape[1] == 0 or features.dtype not in (
+            torch.float32, torch.float16, torch.bfloat16)):
+        return None
+    sizes = [float(v) for v in (voxel_size if hasattr(voxel_size, "__len__") else (voxel_size,))]
+    if len(sizes) == 1:
+        sizes = sizes * ndim
+    if len(sizes) != ndim:
+        return None
+    out = _lib.host().voxelize(coordinates.detach(), sizes, engine.as_i64(batch_dims), return_inverse,
+                               features)
+    if out is None:
+        return None
+    voxels, starts, inverse, means = out
+    result = [voxels, None if batch_dims is None else starts.to(batch_dims.dtype)]
+    if return_inverse:
+        result.append(inverse)
+    if features is not None:
         result.append(means)
     return tuple(result)

@@ -140,15 +140,22 @@ __device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t b
       : "memory");
 }
 
-// Offset bits of the sub-tiles of a CTA tile (pair mode: one offset each).
+// Offset bits of the sub-tiles of a CTA tile, in two steps: the request (unconditional, from a
+// clamped index: a load under a condition is waited for where the branch joins, a thousand cycles
+// per tile) and, a tile later, the value (pair mode: one offset each).
 template <int kSub, bool kPairs>
-__device__ __forceinline__ void load_tile_bits(const ImArgs &args, int tile, uint32_t (&hb)[kSub]) {
+__device__ __forceinline__ void request_bits(const ImArgs &args, int tile, uint32_t (&raw)[kSub]) {
 #pragma unroll
-  for (int h = 0; h < kSub; h++) {
-    hb[h] = 0u;
-    if (tile < args.num_tiles && tile * kSub + h < args.n_tiles128)
-      hb[h] = kPairs ? 1u : (uint32_t)load_ahead_1(args.tile_bits + tile * kSub + h);
-  }
+  for (int h = 0; h < kSub; h++)
+    raw[h] = kPairs ? 1u : (uint32_t)load_ahead_1(args.tile_bits + min(tile * kSub + h, args.n_tiles128 - 1));
+}
+
+template <int kSub>
+__device__ __forceinline__ void take_bits(const ImArgs &args, int tile, const uint32_t (&raw)[kSub],
+                                          uint32_t (&hb)[kSub]) {
+#pragma unroll
+  for (int h = 0; h < kSub; h++)
+    hb[h] = tile < args.num_tiles && tile * kSub + h < args.n_tiles128 ? raw[h] : 0u;
 }
 
 template <int kSub>
@@ -290,12 +297,14 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
     int stage = 0, acc = 0;
     uint32_t phase = 0, acc_phase = 0;
     bool alive = true;
-    uint32_t hb_next[kSub];
-    load_tile_bits<kSub, kPairs>(args, (int)blockIdx.x, hb_next);
+    uint32_t raw[kSub];
+    request_bits<kSub, kPairs>(args, (int)blockIdx.x, raw);
     bool ready = mbar_test(&bar_full[0], 0u);
     for (int tile = blockIdx.x; alive && tile < args.num_tiles; tile += gridDim.x) {
-      const int n_offsets = __popc(union_of<kSub>(hb_next));
-      load_tile_bits<kSub, kPairs>(args, tile + (int)gridDim.x, hb_next);
+      uint32_t hb[kSub];
+      take_bits<kSub>(args, tile, raw, hb);
+      const int n_offsets = __popc(union_of<kSub>(hb));
+      request_bits<kSub, kPairs>(args, tile + (int)gridDim.x, raw);
       if (!mbar_wait_warp(false, &bar_acc_empty[acc], acc_phase ^ 1u, abort_flag, args.status)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t tmem_d = tmem_base + (uint32_t)(acc * kSub * args.n_pad);
@@ -341,16 +350,15 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
     const int my_order = lane < args.num_offsets && args.order != nullptr ? __ldg(args.order + lane) : lane;
     bool alive = true;
     int itile = (int)blockIdx.x - (int)gridDim.x, slot = 0;
-    uint32_t irest = 0u, slot_phase = 0, ihb[kSub], ihb_next[kSub];
-    load_tile_bits<kSub, kPairs>(args, (int)blockIdx.x, ihb_next);
+    uint32_t irest = 0u, slot_phase = 0, ihb[kSub], iraw[kSub];
+    request_bits<kSub, kPairs>(args, (int)blockIdx.x, iraw);
     bool more = true;          // false once the end mark is out
     auto send_indices = [&]() {
       while (irest == 0u && itile < args.num_tiles) {
         itile += (int)gridDim.x;
-#pragma unroll
-        for (int h = 0; h < kSub; h++) ihb[h] = ihb_next[h];
+        take_bits<kSub>(args, itile, iraw, ihb);
         irest = union_of<kSub>(ihb);
-        load_tile_bits<kSub, kPairs>(args, itile + (int)gridDim.x, ihb_next);
+        request_bits<kSub, kPairs>(args, itile + (int)gridDim.x, iraw);
       }
       if (!mbar_wait_warp(false, &bar_idx_empty[slot], slot_phase ^ 1u, abort_flag, args.status)) {
         alive = false;
@@ -386,12 +394,14 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
 
     int stage = 0;
     uint32_t phase = 0;
-    uint32_t hb_next[kSub];
-    load_tile_bits<kSub, kPairs>(args, (int)blockIdx.x, hb_next);
+    uint32_t raw[kSub];
+    request_bits<kSub, kPairs>(args, (int)blockIdx.x, raw);
     bool ready = mbar_test(&bar_empty[0], 1u);
     for (int tile = blockIdx.x; alive && tile < args.num_tiles; tile += gridDim.x) {
-      uint32_t rest = union_of<kSub>(hb_next);
-      load_tile_bits<kSub, kPairs>(args, tile + (int)gridDim.x, hb_next);
+      uint32_t hb[kSub];
+      take_bits<kSub>(args, tile, raw, hb);
+      uint32_t rest = union_of<kSub>(hb);
+      request_bits<kSub, kPairs>(args, tile + (int)gridDim.x, raw);
       const int pair_row = kPairs ? pair_row_of_tile(args, tile) : 0;
       while (alive && rest != 0u) {
         const int p = kPairs ? pair_row : __ffs(rest) - 1;
@@ -425,28 +435,42 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
     const bool affine = args.scale != nullptr || args.shift != nullptr;
     int acc = 0;
     uint32_t acc_phase = 0;
-    uint32_t hb_next[kSub];
-    load_tile_bits<kSub, kPairs>(args, (int)blockIdx.x, hb_next);
-    // row of the output (and of the residual) that this lane's accumulator row belongs to, per
-    // sub-tile (-1: none), requested a tile ahead
-    int32_t grow_next[kSub];
-    auto load_rows = [&](int tile) {
+    uint32_t raw[kSub];
+    request_bits<kSub, kPairs>(args, (int)blockIdx.x, raw);
+    // Row of the output (and of the residual) that this lane's accumulator row belongs to, per
+    // sub-tile (-1: none): requested two tiles ahead, so that the residual rows of the next tile
+    // can be on their way to L2 while this one is worked on.
+    const bool permuted = !kPairs && args.perm != nullptr;
+    auto table_row = [&](int tile, int h) { return ((int64_t)tile * kSub + h) * kBM + quarter * 32 + lane; };
+    auto request_rows = [&](int tile, int32_t (&rows)[kSub]) {
 #pragma unroll
-      for (int h = 0; h < kSub; h++) {
-        const int64_t row = ((int64_t)tile * kSub + h) * kBM + quarter * 32 + lane;
-        grow_next[h] = -1;
-        if (tile < args.num_tiles && row < args.T)
-          grow_next[h] = !kPairs && args.perm != nullptr ? load_ahead_1(args.perm + row) : (int32_t)row;
-      }
+      for (int h = 0; h < kSub; h++)
+        if (permuted) rows[h] = load_ahead_1(args.perm + min(table_row(tile, h), args.T - 1));
     };
-    load_rows((int)blockIdx.x);
+    auto take_row = [&](int tile, int h, int32_t raw_row) {
+      const int64_t row = table_row(tile, h);
+      return tile < args.num_tiles && row < args.T ? (permuted ? raw_row : (int32_t)row) : -1;
+    };
+    int32_t grow[kSub], rows_1[kSub] = {}, rows_2[kSub] = {};
+    request_rows((int)blockIdx.x, rows_1);
+    request_rows((int)(blockIdx.x + gridDim.x), rows_2);
     for (int tile = blockIdx.x; tile < args.num_tiles; tile += gridDim.x) {
-      const bool empty_tile = union_of<kSub>(hb_next) == 0u;   // no MMA ran: the rows are zero
-      load_tile_bits<kSub, kPairs>(args, tile + (int)gridDim.x, hb_next);
-      int32_t grow[kSub];
+      uint32_t hb[kSub];
+      take_bits<kSub>(args, tile, raw, hb);
+      const bool empty_tile = union_of<kSub>(hb) == 0u;   // no MMA ran: the rows are zero
+      request_bits<kSub, kPairs>(args, tile + (int)gridDim.x, raw);
 #pragma unroll
-      for (int h = 0; h < kSub; h++) grow[h] = grow_next[h];
-      load_rows(tile + (int)gridDim.x);
+      for (int h = 0; h < kSub; h++) { grow[h] = take_row(tile, h, rows_1[h]); rows_1[h] = rows_2[h]; }
+      request_rows(tile + 2 * (int)gridDim.x, rows_2);
+      if (!kPairs && args.residual != nullptr) {
+#pragma unroll
+        for (int h = 0; h < kSub; h++) {
+          const int32_t next = take_row(tile + (int)gridDim.x, h, rows_1[h]);
+          if (next < 0) continue;
+          const uint8_t *row = args.residual + (int64_t)next * n * 2;
+          for (int off = 0; off < n * 2; off += 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(row + off));
+        }
+      }
       uint32_t res[2][8];
       auto load_residual = [&](uint32_t (&r)[8], int h, int c) {
 #pragma unroll
@@ -473,7 +497,13 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
           __syncwarp();
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
           const bool more = q + 1 < pieces;
-          if (more) tmem_ld_32x16(taddr + (uint32_t)(q + 1) * 16, nxt);
+          if (more) {
+            tmem_ld_32x16(taddr + (uint32_t)(q + 1) * 16, nxt);
+          } else if (h + 1 == kSub) {
+            // the last read of this accumulator set: the next tile's MMAs may have it
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            if (lane == 0) mbar_arrive(&bar_acc_empty[acc]);
+          }
           if (!kPairs) {
             if (more) load_residual(nxt_res, h, (q + 1) * 16);
             else if (h + 1 < kSub) load_residual(nxt_res, h + 1, 0);
@@ -491,29 +521,52 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
                                 __uint_as_float(cur[4 * i + 2]), __uint_as_float(cur[4 * i + 3]));
             return;
           }
-          uint32_t out[8];
+          // one uniform branch per step of the epilogue and 16 independent values inside each: with
+          // the branches inside the loop over the values a piece took 1300 cycles of latencies
+          float f[16];
 #pragma unroll
-          for (int i = 0; i < 8; i++) {
-            float lo = empty_tile ? 0.f : __uint_as_float(cur[2 * i]);
-            float hi = empty_tile ? 0.f : __uint_as_float(cur[2 * i + 1]);
-            if (affine) {
-              const float2 sc = *reinterpret_cast<const float2 *>(s_scale + c + 2 * i);
-              const float2 sh = *reinterpret_cast<const float2 *>(s_shift + c + 2 * i);
-              lo = lo * sc.x + sh.x;
-              hi = hi * sc.y + sh.y;
+          for (int i = 0; i < 16; i++) f[i] = empty_tile ? 0.f : __uint_as_float(cur[i]);
+          if (affine) {
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+              const float4 sc = *reinterpret_cast<const float4 *>(s_scale + c + 4 * i);
+              const float4 sh = *reinterpret_cast<const float4 *>(s_shift + c + 4 * i);
+              f[4 * i] = f[4 * i] * sc.x + sh.x;
+              f[4 * i + 1] = f[4 * i + 1] * sc.y + sh.y;
+              f[4 * i + 2] = f[4 * i + 2] * sc.z + sh.z;
+              f[4 * i + 3] = f[4 * i + 3] * sc.w + sh.w;
             }
-            if (args.residual != nullptr) {
-              const uint32_t w = cur_res[i];
-              const uint16_t a = (uint16_t)(w & 0xffffu), b = (uint16_t)(w >> 16);
-              lo += args.elem_is_bf16 ? elem_to_f32<true>(a) : elem_to_f32<false>(a);
-              hi += args.elem_is_bf16 ? elem_to_f32<true>(b) : elem_to_f32<false>(b);
-            }
-            if (args.relu) { lo = fmaxf(lo, 0.f); hi = fmaxf(hi, 0.f); }
+          }
+          if (args.residual != nullptr) {
             if (args.elem_is_bf16) {
-              __nv_bfloat162 pk = __floats2bfloat162_rn(lo, hi);
-              out[i] = *reinterpret_cast<uint32_t *>(&pk);
+#pragma unroll
+              for (int i = 0; i < 8; i++) {
+                f[2 * i] += elem_to_f32<true>((uint16_t)(cur_res[i] & 0xffffu));
+                f[2 * i + 1] += elem_to_f32<true>((uint16_t)(cur_res[i] >> 16));
+              }
             } else {
-              __half2 pk = __floats2half2_rn(lo, hi);
+#pragma unroll
+              for (int i = 0; i < 8; i++) {
+                f[2 * i] += elem_to_f32<false>((uint16_t)(cur_res[i] & 0xffffu));
+                f[2 * i + 1] += elem_to_f32<false>((uint16_t)(cur_res[i] >> 16));
+              }
+            }
+          }
+          if (args.relu) {
+#pragma unroll
+            for (int i = 0; i < 16; i++) f[i] = fmaxf(f[i], 0.f);
+          }
+          uint32_t out[8];
+          if (args.elem_is_bf16) {
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+              __nv_bfloat162 pk = __floats2bfloat162_rn(f[2 * i], f[2 * i + 1]);
+              out[i] = *reinterpret_cast<uint32_t *>(&pk);
+            }
+          } else {
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+              __half2 pk = __floats2half2_rn(f[2 * i], f[2 * i + 1]);
               out[i] = *reinterpret_cast<uint32_t *>(&pk);
             }
           }
@@ -540,9 +593,6 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
           }
         }
       }
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&bar_acc_empty[acc]);
       if (++acc == args.acc_bufs) { acc = 0; acc_phase ^= 1u; }
     }
   }

@@ -695,6 +695,22 @@ neighbor_table_kernel(const int32_t *__restrict__ target_masks, int64_t T, int64
   if (threadIdx.x == 0) tile_bits[blockIdx.x] = s_bits;
 }
 
+// Rows of a neighbour table are sorted by hit word inside chunks of 2^shift rows (rows come in
+// coordinate order, so a chunk is a region of space).  Over the whole table the order is best for
+// skipping offsets, but a tile then gathers from everywhere, and once the feature rows outgrow the
+// 126 MB L2 each of a row's pairs is a DRAM access of its own: 4.7M rows of 128 channels with 9.3
+// pairs each took 4.5 ms (1.35 slots computed per pair); in chunks of 2^17 or 2^18 rows they take
+// 2.8 ms (1.7 slots per pair), 1.9M rows of 256 channels 4.7 -> 4.15 ms.  Chunks from 2^16 to 2^19
+// rows differ by less than 5 %.  With fewer than three pairs a row there is little to find again
+// in L2 and the skipped offsets are worth more (7.1M rows of 32 channels, 1.6 pairs: 0.57 ms
+// without chunks, 0.65 with), and half a million rows fit L2.  At most 32 chunks, and 32 key bits
+// in all: another pass of the sort would cost more than smaller chunks give.
+inline int row_chunk_shift(int64_t T, int64_t pairs, int64_t O) {
+  const int chunk_bits = (int)std::min<int64_t>(5, 32 - O);
+  if (T < (1 << 19) || pairs < 3 * T || chunk_bits <= 0) return 31;
+  return std::max(17, rsort::bits_for(T) - chunk_bits);
+}
+
 }  // namespace
 
 namespace {
@@ -803,10 +819,11 @@ extern "C" mn_status mn_build_neighbor_table(const int32_t *source_masks,
     a.keys[0] = keys; a.keys[1] = keys_tmp;
     a.n = T;
     a.first_bit = rsort::bits_for(T);
-    a.bits = (int)O;
+    const int chunk_shift = row_chunk_shift(T, cs.cum[O], O);
+    a.bits = (int)O + (T > (1ll << chunk_shift) ? rsort::bits_for(((T - 1) >> chunk_shift) + 1) : 0);
     a.status = ctrl + MN_CTRL_STATUS;
     a.index32 = perm_out;
-    MN_RETURN_IF(rsort::run(a, HitWordKeys{target_bits, (int32_t)O, a.first_bit}, ws, st));
+    MN_RETURN_IF(rsort::run(a, HitWordKeys{target_bits, (int32_t)O, a.first_bit, chunk_shift}, ws, st));
   }
   // a scattered 4-byte read costs a 32-byte sector: worth it while the pairs are fewer than
   // an eighth of the mask entries

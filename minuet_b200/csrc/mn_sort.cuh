@@ -337,14 +337,15 @@ struct DimensionKeys {
 // offsets the most significant key bits: the few rows that have a rare offset end up together
 // instead of sprinkling it over many tiles.  The key is the reversed word's position in the
 // reflected Gray sequence: neighbouring keys differ in one offset instead of many (2-5 % fewer
-// offsets per tile than binary order).  The row itself sits below.
+// offsets per tile than binary order).  Rows stay within their chunk of 2^chunk_shift rows, whose
+// number sits on top.  The row itself sits below.
 struct HitWordKeys {
   const uint32_t *bits;
-  int32_t num_offsets, index_bits;
+  int32_t num_offsets, index_bits, chunk_shift;
   __device__ __forceinline__ uint64_t operator()(int64_t i) const {
     uint32_t r = __brev(__ldg(bits + i)) >> (32 - num_offsets);
     r ^= r >> 1; r ^= r >> 2; r ^= r >> 4; r ^= r >> 8; r ^= r >> 16;
-    return ((uint64_t)r << index_bits) | (uint64_t)i;
+    return ((((uint64_t)(i >> chunk_shift) << num_offsets) | (uint64_t)r) << index_bits) | (uint64_t)i;
   }
 };
 

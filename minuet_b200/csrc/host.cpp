@@ -535,21 +535,24 @@ Tensor pair_sources(Plan &plan, bool swapped, bool shortcut, const Tensor &sm) {
 // ---------------------------------------------------------------------------
 enum Algorithm { kAuto = 0, kExplicit = 1, kImplicit = 2 };
 
-// Rough cost of one 16-bit forward pass in milliseconds, from fits to measured layers of the
-// benchmark network.  Pair lists move every non-centre pair row three times (16-bit read, fp32
-// product written and read back) at about 2.7 TB/s.  The fused kernel pays about 2.4 ns per
-// (128-row tile, offset present in the tile, 64-channel block) plus 8 ns per tile; with the rows
-// sorted by hit word a tile of a map with E/T pairs per row holds about 1 + 2.2 (E/T - 1) of the
-// O offsets.  Only the ORDER of the two estimates matters.
+// Rough cost of one 16-bit forward pass in milliseconds, fitted to 144 layers of 2 500 to 918 000
+// rows, 8 to 256 channels and 1 to 20 pairs per row (the fused kernel within 25 % of most, pair
+// lists within a factor of two; of the 144 choices four are wrong, all at 12 000 rows and by less
+// than 3 us).  Pair lists move every non-centre pair row three times (16-bit read, fp32 product
+// written and read back) and every row twice in the centre product.  The fused kernel pays per
+// 128-row tile and per offset of a tile, of which the row permutation leaves a tile a little over
+// the pairs per row.  It is the faster one nearly everywhere, up to 9 times where pairs are many;
+// the neighbour table it needs is built once per map.
 double estimate_ms(bool implicit, double S, double T, double O, double c_in, double c_out, double pairs,
                    bool shortcut, bool reorder) {
   if (implicit) {
     const double tiles = std::ceil(T / 128);
-    const double present = reorder ? std::min(O, 1.0 + 2.2 * std::max(pairs / std::max(T, 1.0) - 1.0, 0.0)) : O;
-    return 0.03 + 8.0e-6 * tiles + 2.4e-6 * tiles * present * std::ceil(c_in / 64) * (0.7 + 0.3 * c_out / 128);
+    const double present = reorder ? std::min(O, 1.0 + 1.4 * std::max(pairs / std::max(T, 1.0) - 1.0, 0.0)) : O;
+    return 0.0177 + tiles * (4.0e-6 + 1.7e-8 * (c_in + c_out)) +
+           1.6e-6 * tiles * present * std::ceil(c_in / 64) * (1.05 + c_out / 128);
   }
   const double rest = pairs - (shortcut ? std::min(S, T) : 0.0);
-  return 0.05 + (rest * (8.0 * c_out + 2.0 * c_in) + 2.0 * (S * c_in + T * c_out)) / 2.7e9;
+  return 0.022 + (rest * (8.0 * c_out + 2.0 * c_in) + 2.0 * (S * std::max(c_in, 32.0) + T * std::max(c_out, 32.0))) / 1.8e9;
 }
 
 struct ConvOptions {

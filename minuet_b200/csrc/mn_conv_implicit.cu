@@ -6,15 +6,15 @@
 // crosses HBM four times.  Here one persistent kernel owns 128 consecutive TARGET
 // rows at a time and accumulates ALL kernel offsets of that tile in one TMEM
 // accumulator:
-//   warps 0..7   producers: warp w fetches, for every active offset and k-block, the
-//                128-byte slices of the source rows that feed target rows 16w..16w+15
-//                (cp.async straight into the 128-byte-swizzled A tile, zeros where the
-//                kernel map has no entry)
-//   warp 8       allocates TMEM and issues tcgen05.mma over (offset, k-block)
-//   warp 9       starts the copy of every step's index block and the TMA load of every
-//                stage's transposed weight tile
-//   warps 10..13 epilogue: TMEM -> registers -> optional per-channel scale/shift
-//                (folded BatchNorm or bias), residual add, ReLU -> the output rows
+//   producers   (4 or 8 warps): warp w fetches, for every active offset and k-block, the
+//               128-byte slices of the source rows that feed its share of the target rows
+//               (cp.async straight into the 128-byte-swizzled A tile, zeros where the
+//               kernel map has no entry)
+//   MMA warp    allocates TMEM and issues tcgen05.mma over (offset, k-block)
+//   TMA warp    starts the copy of every step's index block and the TMA load of every
+//               stage's transposed weight tile
+//   epilogue    (8 or 4 warps): TMEM -> registers -> optional per-channel scale/shift
+//               (folded BatchNorm or bias), residual add, ReLU -> the output rows
 // so that features are read once per pair (mostly from L2), outputs are written
 // once, and no pair-row buffer exists.  Offsets with no pair inside a tile are
 // skipped through a per-tile bit mask.  The neighbour table [O, T] (source row
@@ -39,12 +39,8 @@ namespace {
 
 using namespace tc;
 
-constexpr int kProdWarps = 8;          // producer warps: warp w owns 128 / kProdWarps rows of a sub-tile
-constexpr int kProdRows = 128 / kProdWarps;
-constexpr int kMmaWarp = kProdWarps;
-constexpr int kTmaWarp = kProdWarps + 1;
-constexpr int kEpiWarp = kProdWarps + 2;   // the first of four
-constexpr int kImThreads = (kProdWarps + 6) * 32;
+constexpr int kGatherWarps = 12;       // producer and epilogue warps together: 8 + 4 or 4 + 8
+constexpr int kImThreads = (kGatherWarps + 2) * 32;
 constexpr int kImCtas = 2;             // CTAs per SM the register file allows
 constexpr int kBM = 128;
 constexpr int kBK = 64;
@@ -92,8 +88,7 @@ __device__ __forceinline__ int pair_row_of_tile(const ImArgs &a, int tile) {
 }
 
 // 16-byte asynchronous copy; src_bytes = 0 writes 16 zero bytes instead.  It writes through the
-// generic proxy, like a store: the MMA issuer fences after the stage barrier (without the fence
-// one tile in some ten thousand was multiplied with a few rows missing).
+// generic proxy, like a store: the MMA issuer fences after the stage barrier.
 __device__ __forceinline__ void cp_async_16(uint32_t dst, const void *src, uint32_t src_bytes) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(src_bytes)
                : "memory");
@@ -168,11 +163,14 @@ __device__ __forceinline__ uint32_t union_of(const uint32_t (&hb)[kSub]) {
 
 // kSub: sub-tiles per CTA tile (they share every weight tile); kLpr: lanes that copy one
 // 128-byte slice (4 where a source row has at most 64 bytes: half the copies, twice the rows
-// per copy); kPairs: pair mode.
-template <int kSub, int kLpr, bool kPairs>
+// per copy); kProdWarps: 4 producer and 8 epilogue warps or 8 and 4; kPairs: pair mode.
+template <int kSub, int kLpr, int kProdWarps, bool kPairs>
 __global__ void __launch_bounds__(kImThreads, kImCtas)
 conv_implicit_kernel(const __grid_constant__ ImArgs args,
                      const __grid_constant__ CUtensorMap map_b) {   // weights^T [O, N, K]
+  constexpr int kProdRows = 128 / kProdWarps;               // rows of a sub-tile per producer warp
+  constexpr int kMmaWarp = kProdWarps, kTmaWarp = kProdWarps + 1, kEpiWarp = kProdWarps + 2;
+  constexpr int kEpiCols = (kGatherWarps - kProdWarps) / 4;   // epilogue warps per quarter of the rows
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   __shared__ uint64_t bar_full[kMaxStages], bar_empty[kMaxStages];
   __shared__ uint64_t bar_acc_full[2], bar_acc_empty[2];
@@ -194,7 +192,7 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
       mbar_init(&bar_full[s], kProdWarps * 32 + 1);   // every producer lane + the weight tile's expect_tx
       mbar_init(&bar_empty[s], 1);
     }
-    for (int a = 0; a < 2; a++) { mbar_init(&bar_acc_full[a], 1); mbar_init(&bar_acc_empty[a], 4); }
+    for (int a = 0; a < 2; a++) { mbar_init(&bar_acc_full[a], 1); mbar_init(&bar_acc_empty[a], 4 * kEpiCols); }
     for (int i = 0; i < kIdxSlots; i++) { mbar_init(&bar_idx_full[i], 1); mbar_init(&bar_idx_empty[i], kProdWarps); }
     s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -245,16 +243,29 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
 #pragma unroll
       for (int h = 0; h < kSub; h++) {
         const int32_t *at = idx_ring + (slot * kSub + h) * kBM + r0;
-        if (kRpl == 4) {
-          const int4 v = *reinterpret_cast<const int4 *>(at);
-          q[h][0] = v.x; q[h][1] = v.y; q[h][kRpl - 2] = v.z; q[h][kRpl - 1] = v.w;
-        } else {
+        if (kRpl == 2) {
           const int2 v = *reinterpret_cast<const int2 *>(at);
           q[h][0] = v.x; q[h][1] = v.y;
+        } else {
+#pragma unroll
+          for (int i = 0; i + 3 < kRpl; i += 4) {
+            const int4 v = *reinterpret_cast<const int4 *>(at + i);
+            q[h][i] = v.x; q[h][i + 1] = v.y; q[h][i + 2] = v.z; q[h][i + 3] = v.w;
+          }
         }
       }
+      // The slot may be refilled only once the loads above have RETURNED, not when they have been
+      // issued: behind a queue of copies they were overtaken by the arrival and read the block of
+      // eight steps later (one launch in a hundred on freshly built tables).  So the arrival's
+      // address depends on the values (their OR is -1 or non-negative: `never` is 0).
+      int32_t seen = 0;
+#pragma unroll
+      for (int h = 0; h < kSub; h++)
+#pragma unroll
+        for (int i = 0; i < kRpl; i++) seen |= q[h][i];
+      const int never = seen == (int32_t)0x80000001 ? 1 : 0;
       __syncwarp();
-      if (lane == 0) mbar_arrive(&bar_idx_empty[slot]);
+      if (lane == 0) mbar_arrive(&bar_idx_empty[slot] + never);
       if (++slot == kIdxSlots) { slot = 0; slot_phase ^= 1u; }
       for (int kb = 0; kb < args.k_blocks; kb++) {
         if (!ready && !mbar_wait(&bar_empty[stage], phase ^ 1u, abort_flag, args.status)) {
@@ -426,11 +437,16 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
     // ------------------------------ epilogue ----------------------------------
     // A lane owns one accumulator row and takes it 16 columns at a time: one 32-byte store
     // (a whole sector of the output row, wherever perm puts it) and, with a residual, one
-    // 32-byte load requested a piece ahead; the TMEM read of the next piece is in flight while
-    // one is worked on.  No shared-memory staging: its barriers and index shuffles cost more
-    // than the wider stores gave (a tile of 32 columns took 3400 cycles of SM time, most of it
-    // here), and the 32 KB are worth more as ring stages.
-    const int quarter = warp & 3;
+    // 32-byte load requested while the piece before is rounded and stored.  Two warps share a
+    // quarter of the rows where there are eight: they take alternate pieces.  No shared-memory
+    // staging: its barriers and index shuffles cost more than the wider stores gave, and the
+    // 32 KB are worth more as ring stages.
+    // This role bounds the levels with few pairs a row, and what it costs is instruction
+    // latency: every piece is a chain of some 100 dependent instructions.  It must not spill:
+    // next to 200 KB of shared memory L1 keeps no local memory, and each reload of a spilled
+    // register was a trip to L2 (with 32 bytes of spills 918k rows 32->32 took 66 us, without
+    // 52; the pieces' registers are therefore single, not double, buffered).
+    const int quarter = warp & 3, first_piece = (warp - kEpiWarp) >> 2;
     const int n = args.N, pieces = args.n_pad / 16;
     const bool affine = args.scale != nullptr || args.shift != nullptr;
     int acc = 0;
@@ -471,46 +487,40 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
           for (int off = 0; off < n * 2; off += 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(row + off));
         }
       }
-      uint32_t res[2][8];
-      auto load_residual = [&](uint32_t (&r)[8], int h, int c) {
+      uint32_t res[8];
+      auto load_residual = [&](int h, int c) {
 #pragma unroll
-        for (int i = 0; i < 8; i++) r[i] = 0u;
+        for (int i = 0; i < 8; i++) res[i] = 0u;
         if (args.residual == nullptr || grow[h] < 0) return;
         const uint8_t *src = args.residual + ((int64_t)grow[h] * n + c) * 2;
         if (args.wide && c + 16 <= n) {
-          ld_global_32(src, r);
+          ld_global_32(src, res);
         } else {
-          if (c < n) ld_global_16(src, r);
-          if (c + 8 < n) ld_global_16(src + 16, r + 4);
+          if (c < n) ld_global_16(src, res);
+          if (c + 8 < n) ld_global_16(src + 16, res + 4);
         }
       };
-      if (!kPairs) load_residual(res[0], 0, 0);
+      if (!kPairs) load_residual(0, first_piece * 16);
       if (!mbar_wait_warp(false, &bar_acc_full[acc], acc_phase, abort_flag, args.status)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      uint32_t v[2][16];
 #pragma unroll
       for (int h = 0; h < kSub; h++) {
         const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) +
                                (uint32_t)((acc * kSub + h) * args.n_pad);
-        auto piece = [&](uint32_t (&cur)[16], uint32_t (&cur_res)[8], uint32_t (&nxt)[16],
-                         uint32_t (&nxt_res)[8], int q) {
+        auto piece = [&](int q) {
+          uint32_t cur[16];
           __syncwarp();
+          tmem_ld_32x16(taddr + (uint32_t)q * 16, cur);
+          const bool more = q + kEpiCols < pieces;
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-          const bool more = q + 1 < pieces;
-          if (more) {
-            tmem_ld_32x16(taddr + (uint32_t)(q + 1) * 16, nxt);
-          } else if (h + 1 == kSub) {
+          if (!more && h + 1 == kSub) {
             // the last read of this accumulator set: the next tile's MMAs may have it
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             if (lane == 0) mbar_arrive(&bar_acc_empty[acc]);
           }
-          if (!kPairs) {
-            if (more) load_residual(nxt_res, h, (q + 1) * 16);
-            else if (h + 1 < kSub) load_residual(nxt_res, h + 1, 0);
-          }
           const int c = q * 16;
-          if (grow[h] < 0) return;
           if (kPairs) {
+            if (grow[h] < 0) return;
             // pair mode: the fp32 accumulators of this row go out as they are
             float *dst = args.out_f32 + (int64_t)grow[h] * n + c;
 #pragma unroll
@@ -541,21 +551,24 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
             if (args.elem_is_bf16) {
 #pragma unroll
               for (int i = 0; i < 8; i++) {
-                f[2 * i] += elem_to_f32<true>((uint16_t)(cur_res[i] & 0xffffu));
-                f[2 * i + 1] += elem_to_f32<true>((uint16_t)(cur_res[i] >> 16));
+                f[2 * i] += elem_to_f32<true>((uint16_t)(res[i] & 0xffffu));
+                f[2 * i + 1] += elem_to_f32<true>((uint16_t)(res[i] >> 16));
               }
             } else {
 #pragma unroll
               for (int i = 0; i < 8; i++) {
-                f[2 * i] += elem_to_f32<false>((uint16_t)(cur_res[i] & 0xffffu));
-                f[2 * i + 1] += elem_to_f32<false>((uint16_t)(cur_res[i] >> 16));
+                f[2 * i] += elem_to_f32<false>((uint16_t)(res[i] & 0xffffu));
+                f[2 * i + 1] += elem_to_f32<false>((uint16_t)(res[i] >> 16));
               }
             }
           }
+          if (more) load_residual(h, (q + kEpiCols) * 16);
+          else if (h + 1 < kSub) load_residual(h + 1, first_piece * 16);
           if (args.relu) {
 #pragma unroll
             for (int i = 0; i < 16; i++) f[i] = fmaxf(f[i], 0.f);
           }
+          if (grow[h] < 0) return;
           uint32_t out[8];
           if (args.elem_is_bf16) {
 #pragma unroll
@@ -578,20 +591,12 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
             if (c + 8 < n) *reinterpret_cast<uint4 *>(dst + 16) = make_uint4(out[4], out[5], out[6], out[7]);
           }
         };
-        __syncwarp();
-        tmem_ld_32x16(taddr, v[0]);
-        int q = 0;
-        for (; q + 1 < pieces; q += 2) {
-          piece(v[0], res[0], v[1], res[1], q);
-          piece(v[1], res[1], v[0], res[0], q + 1);
+        int q = first_piece;
+        if (kEpiCols > 1 && q >= pieces && h + 1 == kSub) {   // no columns for this warp
+          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          if (lane == 0) mbar_arrive(&bar_acc_empty[acc]);
         }
-        if (q < pieces) {
-          piece(v[0], res[0], v[1], res[1], q);
-          if (h + 1 < kSub) {   // the next sub-tile's first residual piece landed in the other set
-#pragma unroll
-            for (int i = 0; i < 8; i++) res[0][i] = res[1][i];
-          }
-        }
+        for (; q < pieces; q += kEpiCols) piece(q);
       }
       if (++acc == args.acc_bufs) { acc = 0; acc_phase ^= 1u; }
     }
@@ -715,10 +720,10 @@ inline int row_chunk_shift(int64_t T, int64_t pairs, int64_t O) {
 
 namespace {
 
-template <int kSub, int kLpr, bool kPairs>
+template <int kSub, int kLpr, int kProdWarps, bool kPairs>
 mn_status launch_implicit(const ImArgs &a, const TcSizing &sizing, const CUtensorMap &map_b,
                           cudaStream_t st) {
-  auto kernel = conv_implicit_kernel<kSub, kLpr, kPairs>;
+  auto kernel = conv_implicit_kernel<kSub, kLpr, kProdWarps, kPairs>;
   MN_RETURN_IF(allow_max_shared_memory(reinterpret_cast<const void *>(kernel)));
   const int grid = std::min(a.num_tiles, kNumSMs * sizing.ctas_per_sm);
   MN_LAUNCH(kPairs ? "conv_implicit_kernel<pairs>" : "conv_implicit_kernel", st,
@@ -765,8 +770,8 @@ mn_status launch_pair_products(const PairPlan &plan, int64_t S, int64_t c_in, in
   a.out_f32 = products;
   CUtensorMap map_b;
   MN_RETURN_IF(make_kmajor_map(&map_b, weights_t, bf16, c_in, c_out, O, a.n_pad));
-  return c_in <= 32 ? launch_implicit<1, 4, true>(a, sizing, map_b, st)
-                    : launch_implicit<1, 8, true>(a, sizing, map_b, st);
+  return c_in <= 32 ? launch_implicit<1, 4, 8, true>(a, sizing, map_b, st)
+                    : launch_implicit<1, 8, 8, true>(a, sizing, map_b, st);
 }
 
 }  // namespace mn
@@ -897,6 +902,10 @@ extern "C" mn_status mn_sparse_convolution_forward_implicit(
   a.n_pad = (int)align_up((size_t)c_out, 16);
   a.k_blocks = (int)div_up(c_in, kBK);
   a.n_tiles128 = (int)div_up(T, kBM);
+  // One sub-tile: four producer and eight epilogue warps (918k rows 32->32 52 -> 50 us against
+  // eight and four, 243k rows 128->256 with stride 2 90 -> 78 us, 64->64 with 3.5 pairs a row
+  // 164 -> 158 us, 256->256 the same); two sub-tiles: twice the rows to fetch per step, eight
+  // producers (128->128 with 9.4 pairs a row 387 against 395 us).
   // Sub-tiles per CTA tile.  The two sub-tiles of a CTA tile share the weight tile of a
   // stage, at the price of a shallower ring; at 256 columns they also leave no room for a
   // second accumulator set (the epilogue then no longer overlaps the next tile's MMAs).
@@ -931,8 +940,8 @@ extern "C" mn_status mn_sparse_convolution_forward_implicit(
   CUtensorMap map_b;
   MN_RETURN_IF(make_kmajor_map(&map_b, weights_t, bf16, c_in, c_out, O, a.n_pad));
   if (sub == 1)
-    return c_in <= 32 ? launch_implicit<1, 4, false>(a, sizing, map_b, st)
-                      : launch_implicit<1, 8, false>(a, sizing, map_b, st);
-  return c_in <= 32 ? launch_implicit<2, 4, false>(a, sizing, map_b, st)
-                    : launch_implicit<2, 8, false>(a, sizing, map_b, st);
+    return c_in <= 32 ? launch_implicit<1, 4, 4, false>(a, sizing, map_b, st)
+                      : launch_implicit<1, 8, 4, false>(a, sizing, map_b, st);
+  return c_in <= 32 ? launch_implicit<2, 4, 8, false>(a, sizing, map_b, st)
+                    : launch_implicit<2, 8, 8, false>(a, sizing, map_b, st);
 }

@@ -47,3 +47,23 @@ def test_rows_are_sorted_inside_chunks(n, spacing, shift):
         finally:
             conv_mod.REORDER_ROWS = True
     assert torch.equal(got, want)      # the same sums in the same order, other rows per tile
+
+
+@pytest.mark.parametrize("c_in,c_out", [(32, 16), (128, 256)])
+def test_first_pass_on_a_fresh_table(c_in, c_out):
+    """The first launch after a table was built finds it, and the features, in no cache."""
+    gen = torch.Generator(device=DEV).manual_seed(c_in)
+    c = torch.unique(torch.randint(0, 72, (60_000, 3), generator=gen, device=DEV, dtype=torch.int32), dim=0)
+    bounds = torch.tensor([0, len(c)], device=DEV)
+    conv = minuet.nn.SparseConv3d(c_in, c_out, 3, dtype=torch.float16, device=DEV).eval()
+    cache = minuet.nn.KernelMapCache(ndim=3, dtype=torch.int32, device=DEV)
+    minuet.set_kernel_map_cache(conv, cache)
+    conv.tunable_config.update(algorithm="implicit")
+    feats = torch.randn(len(c), c_in, generator=gen, device=DEV).half()
+    want = None
+    with torch.no_grad():
+        for _ in range(60):
+            cache.reset()
+            got = conv(minuet.SparseTensor(feats.clone(), c, batch_dims=bounds)).F
+            want = got if want is None else want
+            assert torch.equal(got, want)

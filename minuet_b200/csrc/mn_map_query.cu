@@ -25,15 +25,13 @@
 // or, for the fused build, one 32-bit word of per-offset hit bits per row.
 //
 // emit_masks_kernel (cooperative launch, all blocks resident): every block
-// owns a contiguous range of 512-row tiles.  Phase 1 counts the hits per
-// offset of its range (32x32 bit-matrix transposes turn 32 hit words into 32
-// per-offset row masks); one grid barrier later every block knows its rank
-// offset per offset and the total sizes, hence the stable size order; phase 2
-// turns each tile's row masks into ranks in a shared-memory staging tile
-// (pre-filled with -1, only the hits are patched) and writes every mask row
-// segment with one bulk asynchronous copy (cp.async.bulk shared -> global),
-// whatever the alignment of the row pitch.  No memset, no select, no scatter,
-// no separate scan kernel.  For submanifold maps (sources == targets,
+// and every warp of it owns a contiguous range of 32-row segments.  Phase 1
+// counts the hits per offset of the range (32x32 bit-matrix transposes turn 32
+// hit words into 32 per-offset row masks); one grid barrier later every block
+// knows its rank offset per offset and the total sizes, hence the stable size
+// order; phase 2 turns each segment's row masks into ranks and writes every
+// mask row of it with one 128-byte store per warp.  No memset, no select, no
+// scatter, no separate scan kernel.  For submanifold maps (sources == targets,
 // symmetric offsets) the source mask of offset o is read off the hit bits of
 // the mirrored offset.
 #include "mn_sort.cuh"
@@ -451,9 +449,8 @@ search_kernel(const __grid_constant__ SearchPair sp) {
 // ---------------------------------------------------------------------------
 constexpr int kEThreads = 512;
 constexpr int kEWarps = kEThreads / 32;
-constexpr int kETile = 512;           // rows per tile: one 32-row segment per warp
-constexpr int kEPitch = kETile + 4;   // staging row pitch (elements), a multiple of 4
-constexpr int kEBatch = 8;            // tiles whose hit words are fetched together
+constexpr int kESegs = 4;             // 32-row segments a warp takes at a time
+constexpr int kEUnit = kESegs * 32;
 
 struct EmitArgs {
   const uint32_t *words_t;   // [T] hit bits of target rows
@@ -464,12 +461,11 @@ struct EmitArgs {
   int32_t *sizes_out;        // [O + 1] size of mask row p, then a copy of the status word
   uint32_t *bits_t;          // optional [T]: bit p set when mask row p has an entry for the target
   uint32_t *bits_s;          // optional [S]: the same for the sources
-  int32_t *agg;              // workspace [64 pairs][grid]: hit counts of every block's tile
-                             // range, then their exclusive prefix; pair = direction * 32 + offset
-  int32_t *total;            // workspace [64]
+  int32_t *agg;              // workspace [64 pairs][grid]: hit counts of every block's rows;
+                             // pair = direction * 32 + offset
   int32_t *ctrl;
   int64_t T, S;
-  int32_t tiles_t, tiles_s;
+  int32_t units_t, units_s;  // kEUnit-row units of the targets / the sources
   int32_t num_offsets;
   int32_t reorder;
   uint8_t mirror[32];        // source direction: which offset's bit to read
@@ -488,102 +484,93 @@ __device__ __forceinline__ uint32_t transpose32(uint32_t x, int lane) {
   return x;
 }
 
-__device__ __forceinline__ void bulk_store(void *dst_global, const void *src_shared, uint32_t bytes) {
-  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst_global),
-               "r"((uint32_t)__cvta_generic_to_shared(src_shared)), "r"(bytes)
-               : "memory");
-}
-
-__global__ void __launch_bounds__(kEThreads)
+// A warp owns consecutive 128-row units of the target rows followed by the source rows, lane p
+// the running rank of mask row p; a mask row of a unit is four 128-byte stores of the whole warp.
+// After the grid-wide barrier no warp waits for another one: with 512-row tiles staged in shared
+// memory and three block barriers a tile the kernel spent half its time in those barriers where
+// the masks are narrow (7.3M + 7.1M rows, 8 offsets: 301 us, now 160; 464k + 464k rows 28, now
+// 18 us).  With 27 offsets it is bound by the bytes it writes (1.58 GB in 355 us either way).
+// More than two blocks of 16 warps per SM make it slower: too many rows are open at a time.
+__global__ void __launch_bounds__(kEThreads, 2)
 emit_masks_kernel(const __grid_constant__ EmitArgs e) {
-  extern __shared__ __align__(16) int32_t s_stage[];   // [O][kEPitch]
-  __shared__ int32_t s_wcnt[32][kEWarps + 1];           // per offset: warp counts, then warp bases
-  __shared__ int32_t s_run[2][32];                      // rank of the next hit, per direction / offset
-  __shared__ int32_t s_size[32], s_pos[32], s_ord[32];
-  __shared__ int32_t s_mis[32];
-  __shared__ uint32_t s_words[kEBatch][kETile];         // hit words of up to kEBatch tiles
+  __shared__ int32_t s_wcnt[2][32][kEWarps + 1];        // per direction / offset: warp counts, then warp bases
+  __shared__ int32_t s_first[2][32], s_size[32], s_ord[32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int O = e.num_offsets;
   const int G = (int)gridDim.x, b = (int)blockIdx.x;
-  const int total_tiles = e.tiles_t + e.tiles_s;
-  const int t_begin = (int)((int64_t)total_tiles * b / G);
-  const int t_end = (int)((int64_t)total_tiles * (b + 1) / G);
+  const int64_t total_units = (int64_t)e.units_t + e.units_s, workers = (int64_t)G * kEWarps;
+  const int64_t me = (int64_t)b * kEWarps + warp;
+  const int begin = (int)(total_units * me / workers), end = (int)(total_units * (me + 1) / workers);
   const unsigned lt = lanemask_lt();
   const int my_mirror = lane < O ? e.mirror[lane] : 0;
 
   MN_MARK(g_marks_emit, 0);
-  // hit words of tiles [first, first + kEBatch) of this block's range: all loads are in
-  // flight together; a thread only ever reads back the words it loaded itself
-  auto fetch_words = [&](int first) {
+  auto fetch_words = [&](int unit, uint32_t (&w)[kESegs]) {
+    const int dir = unit >= e.units_t ? 1 : 0;
+    const int64_t n = unit < end ? (dir ? e.S : e.T) : 0;
+    const int64_t r = (int64_t)(unit - (dir ? e.units_t : 0)) * kEUnit + lane;
+    const uint32_t *words = dir ? e.words_s : e.words_t;
 #pragma unroll
-    for (int k = 0; k < kEBatch; k++) {
-      const int tile = first + k;
-      uint32_t w = 0u;
-      if (tile < t_end) {
-        const int dir = tile >= e.tiles_t ? 1 : 0;
-        const int64_t r = (int64_t)(tile - dir * e.tiles_t) * kETile + tid;
-        const int64_t n = dir ? e.S : e.T;
-        if (r < n) w = __ldg((dir ? e.words_s : e.words_t) + r);
-      }
-      s_words[k][tid] = w;
-    }
+    for (int k = 0; k < kESegs; k++) w[k] = r + 32 * k < n ? __ldg(words + r + 32 * k) : 0u;
   };
 
-  // ---- phase 1: hits per offset of this block's tile range ---------------------
-  int cnt0 = 0, cnt1 = 0;   // lane o: hits of offset o, per direction
-  for (int first = t_begin; first < t_end; first += kEBatch) {
-    fetch_words(first);
-    for (int tile = first; tile < min(first + kEBatch, t_end); tile++) {
-      const int dir = tile >= e.tiles_t ? 1 : 0;
-      const uint32_t w = s_words[tile - first][tid];
-      if (__ballot_sync(0xffffffffu, w != 0u) == 0u) continue;
-      uint32_t plane = transpose32(w, lane);
-      if (dir) plane = __shfl_sync(0xffffffffu, plane, my_mirror);
-      if (dir) cnt1 += __popc(plane); else cnt0 += __popc(plane);
+  // ---- phase 1: hits per offset of this warp's rows -------------------------------
+  {
+    int cnt0 = 0, cnt1 = 0;   // lane o: hits of offset o, per direction
+    uint32_t w[kESegs], next[kESegs];
+    fetch_words(begin, w);
+    for (int unit = begin; unit < end; unit++) {
+      fetch_words(unit + 1, next);
+#pragma unroll
+      for (int k = 0; k < kESegs; k++) {
+        const int c = __popc(transpose32(w[k], lane));
+        if (unit >= e.units_t) cnt1 += c; else cnt0 += c;
+        w[k] = next[k];
+      }
     }
+    cnt1 = __shfl_sync(0xffffffffu, cnt1, my_mirror);
+    if (lane < O) { s_wcnt[0][lane][warp] = cnt0; s_wcnt[1][lane][warp] = cnt1; }
   }
-  for (int d = 0; d < 2; d++) {
-    if (lane < O) s_wcnt[lane][warp] = d ? cnt1 : cnt0;
-    __syncthreads();
-    if (tid < 32) {
-      int sum = 0;
-      if (tid < O)
-        for (int w = 0; w < kEWarps; w++) sum += s_wcnt[tid][w];
-      e.agg[(int64_t)(d * 32 + tid) * G + b] = sum;
-    }
-    __syncthreads();
+  __syncthreads();
+  if (tid < 64) {
+    int sum = 0;
+    if ((tid & 31) < O)
+      for (int w = 0; w < kEWarps; w++) {
+        const int c = s_wcnt[tid >> 5][tid & 31][w];
+        s_wcnt[tid >> 5][tid & 31][w] = sum;
+        sum += c;
+      }
+    e.agg[(int64_t)tid * G + b] = sum;
   }
+  __syncthreads();
   MN_MARK(g_marks_emit, 1);
   grid_barrier(e.ctrl, (unsigned)G);
   MN_MARK(g_marks_emit, 2);
 
-  // ---- one warp per (direction, offset): exclusive prefix over the blocks ----------
-  for (int pair = b * kEWarps + warp; pair < 64; pair += G * kEWarps) {
-    {
-      int32_t *row = e.agg + (int64_t)pair * G;
-      int carry = 0;
-      for (int b0 = 0; b0 < G; b0 += 32) {
-        const int bb = b0 + lane;
-        const int v = bb < G ? __ldcg(row + bb) : 0;
-        int inc = v;
+  // ---- totals and this block's first ranks: every block adds up the other blocks' counts
+  // itself (a few hundred 4-byte reads per pair), which is cheaper than a second barrier ------
+  for (int pair = warp; pair < 64; pair += kEWarps) {
+    if ((pair & 31) >= O) continue;
+    const int32_t *row = e.agg + (int64_t)pair * G;
+    int all = 0, before = 0;
+    for (int b0 = 0; b0 < G; b0 += 160) {
+      int v[5];
 #pragma unroll
-        for (int s = 1; s < 32; s <<= 1) {
-          const int t = __shfl_up_sync(0xffffffffu, inc, s);
-          if (lane >= s) inc += t;
-        }
-        if (bb < G) row[bb] = carry + inc - v;
-        carry += __shfl_sync(0xffffffffu, inc, 31);
+      for (int i = 0; i < 5; i++) v[i] = b0 + 32 * i + lane < G ? __ldcg(row + b0 + 32 * i + lane) : 0;
+#pragma unroll
+      for (int i = 0; i < 5; i++) {
+        all += v[i];
+        before += b0 + 32 * i + lane < b ? v[i] : 0;
       }
-      if (lane == 0) e.total[pair] = carry;
+    }
+    all = __reduce_add_sync(0xffffffffu, all);
+    before = __reduce_add_sync(0xffffffffu, before);
+    if (lane == 0) {
+      s_first[pair >> 5][pair & 31] = before;
+      if (pair < 32) s_size[pair] = all;
     }
   }
-  MN_MARK(g_marks_emit, 3);
-  grid_barrier(e.ctrl, (unsigned)G);
-  MN_MARK(g_marks_emit, 4);
-
-  // ---- rank offsets of this block, total sizes, size order ---------------------
-  if (tid < 64) s_run[tid >> 5][tid & 31] = __ldcg(e.agg + (int64_t)tid * G + b);
-  if (tid < 32) s_size[tid] = __ldcg(e.total + tid);
+  if (tid < 32) s_ord[tid] = 0;
   __syncthreads();
   if (tid < O) {
     int pos = tid;
@@ -596,7 +583,6 @@ emit_masks_kernel(const __grid_constant__ EmitArgs e) {
         pos += (other < mine) || (other == mine && j < tid);
       }
     }
-    s_pos[tid] = pos;
     s_ord[pos] = tid;
     if (b == 0) {
       e.order_out[pos] = tid;
@@ -605,106 +591,63 @@ emit_masks_kernel(const __grid_constant__ EmitArgs e) {
   }
   if (b == 0 && tid == 0) e.sizes_out[O] = e.ctrl[MN_CTRL_STATUS];
   __syncthreads();
+  // from here on lane p stands for mask row p
+  const int ord = s_ord[lane];
+  const int plane_of[2] = {ord, __shfl_sync(0xffffffffu, my_mirror, ord)};
+  int run[2];
+#pragma unroll
+  for (int d = 0; d < 2; d++)
+    run[d] = lane < O ? s_first[d][ord] + s_wcnt[d][ord][warp] : 0;
 
   MN_MARK(g_marks_emit, 5);
-  // ---- phase 2: ranks, staged per tile, one bulk copy per mask row segment ------
-  bool pending = false;   // threads < O: a bulk group of mine may still be reading the stage
-  for (int tile = t_begin; tile < t_end; tile++) {
-    // the words of the first kEBatch tiles are still in shared memory from phase 1
-    if (tile != t_begin && (tile - t_begin) % kEBatch == 0) fetch_words(tile);
-    if (tile == t_begin && t_end - t_begin > kEBatch) fetch_words(tile);
-    const int dir = tile >= e.tiles_t ? 1 : 0;
-    const int64_t tile_row0 = (int64_t)(tile - dir * e.tiles_t) * kETile;
-    const int64_t n = dir ? e.S : e.T;
-    int32_t *out = dir ? e.source_masks : e.target_masks;
-    const int rows_here = (int)min((int64_t)kETile, n - tile_row0);
-    const int seg = warp * 32;
-
-    uint32_t plane = transpose32(s_words[(tile - t_begin) % kEBatch][tid], lane);
-    if (dir) plane = __shfl_sync(0xffffffffu, plane, my_mirror);
-    if (lane >= O) plane = 0u;
-    {
+  // ---- phase 2: ranks ------------------------------------------------------------------
+  uint32_t w[kESegs], next[kESegs];
+  fetch_words(begin, w);
+  for (int unit = begin; unit < end; unit++) {
+    fetch_words(unit + 1, next);
+    const int dir = unit >= e.units_t ? 1 : 0;
+    const int64_t n = dir ? e.S : e.T, r = (int64_t)(unit - (dir ? e.units_t : 0)) * kEUnit + lane;
+    const int left = (int)min(n - r, (int64_t)kEUnit);   // rows from this lane's first one on
+    uint32_t *bits_out = dir ? e.bits_s : e.bits_t;
+    uint32_t plane[kESegs], seen = 0u;
+    int count = 0;
+#pragma unroll
+    for (int k = 0; k < kESegs; k++) {
+      plane[k] = __shfl_sync(0xffffffffu, transpose32(w[k], lane), dir ? plane_of[1] : plane_of[0]);
+      if (lane >= O) plane[k] = 0u;
+      seen |= plane[k];
+      count += __popc(plane[k]);
       // hit word of every row in mask-row order (bit p <-> mask row p), for the
       // convolution kernels that walk a row's pairs without scanning the masks
-      uint32_t *bits_out = dir ? e.bits_s : e.bits_t;
       if (bits_out != nullptr) {
-        uint32_t by_row = __shfl_sync(0xffffffffu, plane, lane < O ? s_ord[lane] : 0);
-        if (lane >= O) by_row = 0u;
-        by_row = transpose32(by_row, lane);
-        if (tile_row0 + seg + lane < n) bits_out[tile_row0 + seg + lane] = by_row;
+        const uint32_t by_row = transpose32(plane[k], lane);
+        if (32 * k < left) bits_out[r + 32 * k] = by_row;
       }
+      w[k] = next[k];
     }
-    if (lane < O) s_wcnt[lane][warp] = __popc(plane);
-    // the previous tile's copies must have read the stage before it is refilled
-    if (pending) {
-      asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-      pending = false;
-    }
-    __syncthreads();
-    if (tid < O) {
-      // exclusive prefix over the warps on top of the running rank; where the
-      // row segment of this offset starts relative to a 16-byte boundary
-      int run = s_run[dir][tid];
+    const unsigned any = __ballot_sync(0xffffffffu, seen != 0u);
+    const int first_rank = dir ? run[1] : run[0];
+    int32_t *dst = (dir ? e.source_masks : e.target_masks) + r;
+    for (int p = 0; p < O; p++, dst += n) {
+      int v[kESegs];
 #pragma unroll
-      for (int w = 0; w < kEWarps; w++) {
-        const int c = s_wcnt[tid][w];
-        s_wcnt[tid][w] = run;
-        run += c;
+      for (int k = 0; k < kESegs; k++) v[k] = -1;
+      if ((any >> p) & 1u) {
+        int rank = __shfl_sync(0xffffffffu, first_rank, p);
+#pragma unroll
+        for (int k = 0; k < kESegs; k++) {
+          const uint32_t pl = __shfl_sync(0xffffffffu, plane[k], p);
+          if ((pl >> lane) & 1u) v[k] = rank + __popc(pl & lt);
+          rank += __popc(pl);
+        }
       }
-      s_run[dir][tid] = run;
-      const int64_t g0 = (int64_t)s_pos[tid] * n + tile_row0;
-      s_mis[tid] = (int)(((reinterpret_cast<uintptr_t>(out) >> 2) + (uint64_t)g0) & 3u);
+#pragma unroll
+      for (int k = 0; k < kESegs; k++)
+        if (32 * k < left) dst[32 * k] = v[k];
     }
-    {
-      int4 *fill = reinterpret_cast<int4 *>(s_stage);
-      const int n_vec = O * kEPitch / 4;
-      for (int i = tid; i < n_vec; i += kEThreads) fill[i] = make_int4(-1, -1, -1, -1);
-    }
-    __syncthreads();
-    // sparse planes: the owning lane walks its hits; dense planes: all lanes, one row each
-    {
-      int base = 0;
-      int32_t *row = s_stage;
-      if (lane < O) {
-        base = s_wcnt[lane][warp];
-        row = s_stage + lane * kEPitch + s_mis[lane] + seg;
-      }
-      const bool dense = __popc(plane) > 6;
-      uint32_t p = dense ? 0u : plane;
-      int r = base;
-      while (p != 0u) {
-        row[__ffs(p) - 1] = r++;
-        p &= p - 1u;
-      }
-      uint32_t todo = __ballot_sync(0xffffffffu, dense);
-      while (todo != 0u) {
-        const int o = __ffs(todo) - 1;
-        todo &= todo - 1u;
-        const uint32_t pl = __shfl_sync(0xffffffffu, plane, o);
-        const int bs = __shfl_sync(0xffffffffu, base, o);
-        if ((pl >> lane) & 1u) s_stage[o * kEPitch + s_mis[o] + seg + lane] = bs + __popc(pl & lt);
-      }
-    }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    __syncthreads();
-    if (tid < O) {
-      const int mis = s_mis[tid];
-      const int32_t *src = s_stage + tid * kEPitch + mis;
-      int32_t *dst = out + (int64_t)s_pos[tid] * n + tile_row0;
-      const int head = min((4 - mis) & 3, rows_here);
-      const int body = (rows_here - head) & ~3;
-      if (body > 0) {
-        bulk_store(dst + head, src + head, (uint32_t)body * 4u);
-        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-        pending = true;
-      }
-      for (int i = 0; i < head; i++) dst[i] = src[i];
-      for (int i = head + body; i < rows_here; i++) dst[i] = src[i];
-    }
+    if (dir) run[1] += count; else run[0] += count;
   }
   MN_MARK(g_marks_emit, 6);
-  if (pending) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
-  MN_MARK(g_marks_emit, 7);
 }
 
 __global__ void identity_order_kernel(int O, int32_t *order_out, int32_t *sizes_out,
@@ -1027,30 +970,26 @@ extern "C" mn_status mn_build_kernel_map(const uint64_t *source_keys, int64_t S,
   const bool mirrored = symmetric && source_keys == target_keys && S == T;
 
   // grid of the cooperative emission kernel: every block resident at once
-  const size_t stage_bytes = (size_t)O * kEPitch * sizeof(int32_t);
-  static thread_local int coresident_for[kMaxDevices][33] = {{0}};
+  static thread_local int coresident_for[kMaxDevices] = {0};
   int device = 0;
   MN_CHECK_CUDA(cudaGetDevice(&device));
   MN_CHECK_ARG(device >= 0 && device < kMaxDevices, "build_kernel_map: device index %d out of range", device);
-  int &coresident = coresident_for[device][O];
+  int &coresident = coresident_for[device];
   if (coresident == 0) {
-    MN_CHECK_CUDA(cudaFuncSetAttribute(emit_masks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       32 * kEPitch * (int)sizeof(int32_t)));
-    coresident = std::min(kMaxCoopBlocks, max_coresident_blocks(emit_masks_kernel, kEThreads, stage_bytes));
+    coresident = std::min(kMaxCoopBlocks, max_coresident_blocks(emit_masks_kernel, kEThreads, 0));
     if (coresident <= 0) {
       coresident = 0;
       set_error("build_kernel_map: cannot size the cooperative grid");
       return MN_ERR_CUDA;
     }
   }
-  const int tiles_t = (int)div_up(T, kETile), tiles_s = (int)div_up(S, kETile);
-  const int grid = std::min(tiles_t + tiles_s, coresident);
+  const int units_t = (int)div_up(T, kEUnit), units_s = (int)div_up(S, kEUnit);
+  const int grid = (int)std::min<int64_t>(div_up((int64_t)units_t + units_s, 2), coresident);
 
   Workspace ws(ws_ptr, ws_bytes);
   uint32_t *words_t = ws.take<uint32_t>(T);
   uint32_t *words_s = mirrored ? words_t : ws.take<uint32_t>(S);
   int32_t *agg = ws.take<int32_t>((size_t)grid * 64);
-  int32_t *total = ws.take<int32_t>(64);
   MN_CHECK_WS(ws);
 
   SearchArgs fwd_args;
@@ -1068,16 +1007,16 @@ extern "C" mn_status mn_build_kernel_map(const uint64_t *source_keys, int64_t S,
   EmitArgs e{};
   e.words_t = words_t; e.words_s = words_s;
   e.target_masks = target_masks_out; e.source_masks = source_masks_out;
-  e.order_out = order_out; e.sizes_out = sizes_out; e.agg = agg; e.total = total; e.ctrl = ctrl;
+  e.order_out = order_out; e.sizes_out = sizes_out; e.agg = agg; e.ctrl = ctrl;
   e.bits_t = target_bits_out; e.bits_s = source_bits_out;
-  e.T = T; e.S = S; e.tiles_t = tiles_t; e.tiles_s = tiles_s;
+  e.T = T; e.S = S; e.units_t = units_t; e.units_s = units_s;
   e.num_offsets = (int)O; e.reorder = reorder ? 1 : 0;
   for (int64_t o = 0; o < O; o++) e.mirror[o] = mirrored ? neg[o] : (uint8_t)o;
   void *params[] = {&e};
   {
     LaunchScope scope("emit_masks_kernel", st);
     MN_CHECK_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void *>(emit_masks_kernel), dim3(grid),
-                                              dim3(kEThreads), params, stage_bytes, st));
+                                              dim3(kEThreads), params, 0, st));
   }
   MN_CHECK_LAUNCH();
   return MN_OK;

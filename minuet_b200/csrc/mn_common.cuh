@@ -3,6 +3,7 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <utility>
 #include <cuda_fp16.h>
 #include <cuda_bf16.h>
 
@@ -76,6 +77,36 @@ struct LaunchScope {
     }                                             \
     MN_CHECK_LAUNCH();                            \
   } while (0)
+
+// Dependent launches.  A kernel launched with launch_early may be given to the SMs while the kernel
+// before it in the stream still drains; it starts with begin_early(), which returns when that
+// kernel is complete and its writes are visible, and then lets the next one do the same.  Every
+// block calls it before anything else that touches global memory or allocates tensor memory,
+// and before any return, so that "complete" covers all the kernels before it.  It takes launch
+// latency, block scheduling and the first instruction fetches out of the chains of short kernels
+// that a map or a network is made of.
+__device__ __forceinline__ void wait_for_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void release_successor() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void begin_early() {
+  wait_for_predecessor();
+  release_successor();
+}
+
+template <typename... Params, typename... Args>
+inline void launch_early(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                         Args &&...args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  (void)cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);   // errors: MN_CHECK_LAUNCH
+}
 
 // Optional phase timing of a kernel (builds with -DMN_PHASE_TIMING only): thread 0
 // of the first blocks stores its SM cycle counter at numbered points into a

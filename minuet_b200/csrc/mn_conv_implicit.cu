@@ -197,6 +197,7 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
     s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  wait_for_predecessor();
   if (!kPairs && (args.scale != nullptr || args.shift != nullptr)) {
     for (int c = threadIdx.x; c < args.n_pad; c += kImThreads) {
       s_scale[c] = args.scale != nullptr && c < args.N ? __ldg(args.scale + c) : 1.f;
@@ -212,6 +213,7 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  release_successor();   // every block has its tensor memory before another kernel's block can ask for some
   const uint32_t tmem_base = s_tmem_base;
   volatile int *abort_flag = &s_abort;
 
@@ -626,6 +628,7 @@ struct CumSizes {
 __global__ void __launch_bounds__(256)
 rank_to_source_kernel(const int32_t *__restrict__ source_masks, int64_t S, int O,
                       const __grid_constant__ CumSizes cs, int32_t *__restrict__ src_of_rank) {
+  begin_early();
   const int p = blockIdx.y;
   const int64_t gsz = (int64_t)gridDim.x * blockDim.x;
   for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < S; s += gsz) {
@@ -640,6 +643,7 @@ __global__ void __launch_bounds__(256)
 rank_to_source_bits_kernel(const int32_t *__restrict__ source_masks,
                            const uint32_t *__restrict__ source_bits, int64_t S,
                            const __grid_constant__ CumSizes cs, int32_t *__restrict__ src_of_rank) {
+  begin_early();
   const int64_t gsz = (int64_t)gridDim.x * blockDim.x;
   for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < S; s += gsz) {
     for (uint32_t rest = __ldg(source_bits + s); rest != 0u; rest &= rest - 1u) {
@@ -663,6 +667,7 @@ neighbor_table_kernel(const int32_t *__restrict__ target_masks, int64_t T, int64
                       const int32_t *__restrict__ src_of_rank, const int32_t *__restrict__ perm,
                       const uint32_t *__restrict__ bits, int32_t *__restrict__ nbr,
                       uint32_t *__restrict__ tile_bits) {
+  begin_early();
   __shared__ uint32_t s_bits;
   if (threadIdx.x == 0) s_bits = 0u;
   __syncthreads();
@@ -727,7 +732,7 @@ mn_status launch_implicit(const ImArgs &a, const TcSizing &sizing, const CUtenso
   MN_RETURN_IF(allow_max_shared_memory(reinterpret_cast<const void *>(kernel)));
   const int grid = std::min(a.num_tiles, kNumSMs * sizing.ctas_per_sm);
   MN_LAUNCH(kPairs ? "conv_implicit_kernel<pairs>" : "conv_implicit_kernel", st,
-            kernel<<<grid, kImThreads, sizing.smem_bytes, st>>>(a, map_b));
+            launch_early(kernel, grid, kImThreads, sizing.smem_bytes, st, a, map_b));
   return MN_OK;
 }
 
@@ -835,15 +840,15 @@ extern "C" mn_status mn_build_neighbor_table(const int32_t *source_masks,
   if (S > 0 && source_bits != nullptr && cs.cum[O] * 8 < O * S) {
     const int blocks = (int)std::min<int64_t>(kNumSMs * 16, div_up(S, 256));
     MN_LAUNCH("rank_to_source_bits_kernel", st,
-              rank_to_source_bits_kernel<<<blocks, 256, 0, st>>>(source_masks, source_bits, S, cs,
+              launch_early(rank_to_source_bits_kernel, blocks, 256, 0, st, source_masks, source_bits, S, cs,
                                                                   src_of_rank));
   } else if (S > 0) {
     const dim3 grid((unsigned)std::min<int64_t>(kNumSMs * 4, div_up(S, 256)), (unsigned)O);
     MN_LAUNCH("rank_to_source_kernel", st,
-              rank_to_source_kernel<<<grid, 256, 0, st>>>(source_masks, S, (int)O, cs, src_of_rank));
+              launch_early(rank_to_source_kernel, grid, 256, 0, st, source_masks, S, (int)O, cs, src_of_rank));
   }
   MN_LAUNCH("neighbor_table_kernel", st,
-            neighbor_table_kernel<<<(unsigned)div_up(T, 128), 128, 0, st>>>(
+            launch_early(neighbor_table_kernel, (unsigned)div_up(T, 128), 128, 0, st, 
                 target_masks, T, (int64_t)align_up((size_t)T, kBM), (int)O, cs, src_of_rank, perm_out,
                 target_bits, nbr_out, tile_bits_out));
   return MN_OK;

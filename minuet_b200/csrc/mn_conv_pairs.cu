@@ -38,6 +38,7 @@ __global__ void __launch_bounds__(256)
 pair_list_kernel(const int32_t *__restrict__ source_masks, const uint32_t *__restrict__ bits,
                  int64_t S, uint32_t keep, const __grid_constant__ PairPlan plan,
                  int32_t *__restrict__ pair_src) {
+  begin_early();
   const int64_t gsz = (int64_t)gridDim.x * blockDim.x;
   for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < S; s += gsz) {
     uint32_t w = __ldg(bits + s) & keep;
@@ -169,7 +170,7 @@ extern "C" mn_status mn_build_pair_list(const int32_t *source_masks, const uint3
   MN_CHECK_CUDA(cudaMemsetAsync(pair_src_out, 0xff, sizeof(int32_t) * plan.total_rows, st));
   const int blocks = (int)std::min<int64_t>(kNumSMs * 8, div_up(S, 256));
   MN_LAUNCH("pair_list_kernel", st,
-            pair_list_kernel<<<blocks, 256, 0, st>>>(source_masks, source_bits, S, plan.keep, plan,
+            launch_early(pair_list_kernel, blocks, 256, 0, st, source_masks, source_bits, S, plan.keep, plan,
                                                      pair_src_out));
   return MN_OK;
 }

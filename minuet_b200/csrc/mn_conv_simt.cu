@@ -77,6 +77,7 @@ __device__ __forceinline__ float4 cs_epilogue(float4 v, const CsArgs &a, int64_t
 template <int BM, int BN, int kStages, bool kVec>
 __global__ void __launch_bounds__(BM * BN / 32, BN == 32 ? 12 : 3)
 conv_simt_kernel(const __grid_constant__ CsArgs a) {
+  begin_early();
   constexpr int kThreads = BM * BN / 32, kWarps = kThreads / 32;
   constexpr int kRows = BM / kWarps;                   // rows of a warp: 32 or 16
   constexpr int kStageFloats = BM * kCsPitch + kCsK * BN;
@@ -270,6 +271,7 @@ conv_simt_kernel(const __grid_constant__ CsArgs a) {
 // out[perm[r]] = epilogue(sum of the products of row r's pairs, in mask-row order)
 __global__ void __launch_bounds__(256)
 conv_simt_add_kernel(const __grid_constant__ CsArgs a) {
+  begin_early();
   const int per_row = (a.N + 3) / 4;
   const int64_t total = a.T * per_row, gsz = (int64_t)gridDim.x * blockDim.x;
   const bool vec = a.N % 4 == 0;
@@ -337,9 +339,9 @@ mn_status launch_cs(const CsArgs &a, int64_t O, cudaStream_t st) {
     sized[device] = true;
   }
   if (vec) {
-    MN_LAUNCH("conv_simt_kernel", st, conv_simt_kernel<BM, BN, kStages, true><<<grid, BM * BN / 32, smem, st>>>(a));
+    MN_LAUNCH("conv_simt_kernel", st, launch_early(conv_simt_kernel<BM, BN, kStages, true>, grid, BM * BN / 32, smem, st, a));
   } else {
-    MN_LAUNCH("conv_simt_kernel", st, conv_simt_kernel<BM, BN, kStages, false><<<grid, BM * BN / 32, smem, st>>>(a));
+    MN_LAUNCH("conv_simt_kernel", st, launch_early(conv_simt_kernel<BM, BN, kStages, false>, grid, BM * BN / 32, smem, st, a));
   }
   return MN_OK;
 }
@@ -390,7 +392,7 @@ extern "C" mn_status mn_sparse_convolution_forward_implicit_fp32(
   if (s.splits > 1) {
     const int64_t total = T * div_up(c_out, 4);
     const int blocks = (int)std::min<int64_t>(kNumSMs * 8, div_up(total, 256));
-    MN_LAUNCH("conv_simt_add_kernel", st, conv_simt_add_kernel<<<blocks, 256, 0, st>>>(a));
+    MN_LAUNCH("conv_simt_add_kernel", st, launch_early(conv_simt_add_kernel, blocks, 256, 0, st, a));
   }
   return MN_OK;
 }

@@ -66,6 +66,7 @@ __device__ __forceinline__ int row_of_item(const WgradPlan &plan, int item) {
 __global__ void __launch_bounds__(256)
 pair_side_kernel(const int32_t *__restrict__ masks, const uint32_t *__restrict__ bits, int64_t rows,
                  const __grid_constant__ WgradPlan plan, int32_t *__restrict__ list) {
+  begin_early();
   const int64_t gsz = (int64_t)gridDim.x * blockDim.x;
   for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < rows; r += gsz) {
     if (bits != nullptr) {
@@ -142,6 +143,7 @@ wgrad_tc_kernel(const __grid_constant__ WgradArgs a, const __grid_constant__ Wgr
     s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  wait_for_predecessor();
   if (warp == kWgMmaWarp) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                      smem_u32(&s_tmem_base)), "r"((uint32_t)a.tmem_cols)
@@ -151,6 +153,7 @@ wgrad_tc_kernel(const __grid_constant__ WgradArgs a, const __grid_constant__ Wgr
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  release_successor();   // every block has its tensor memory before another kernel's block can ask for some
   const uint32_t tmem_base = s_tmem_base;
   volatile int *abort_flag = &s_abort;
 
@@ -320,6 +323,7 @@ constexpr int kWsStages = 3;
 template <typename T, int BM, int BN, bool kVec>
 __global__ void __launch_bounds__(kWsThreads)
 wgrad_simt_kernel(const __grid_constant__ WgradArgs a, const __grid_constant__ WgradPlan plan, int n_tiles) {
+  begin_early();
   constexpr int kTileThreads = BM * BN / 32;
   constexpr int kGroups = kWsThreads / kTileThreads;
   constexpr int kStageFloats = kWsRows * (BM + BN);
@@ -434,6 +438,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 wgrad_reduce_kernel(const float *__restrict__ partial, const __grid_constant__ WgradPlan plan,
                     const int32_t *__restrict__ order, int64_t matrix, T *__restrict__ grad_w) {
+  begin_early();
   const int p = blockIdx.y;
   const int k = order != nullptr ? __ldg(order + p) : p;
   const int begin = plan.item_prefix[p], end = plan.item_prefix[p + 1];
@@ -502,12 +507,12 @@ mn_status run_wgrad_simt(const WgradArgs &a, const WgradPlan &plan, int items, c
   if constexpr (sizeof(T) == 4) {
     if (vec) {
       MN_LAUNCH("wgrad_simt_kernel", st,
-                wgrad_simt_kernel<T, BM, BN, true><<<grid, kWsThreads, smem, st>>>(a, plan, n_tiles));
+                launch_early(wgrad_simt_kernel<T, BM, BN, true>, grid, kWsThreads, smem, st, a, plan, n_tiles));
       return MN_OK;
     }
   }
   MN_LAUNCH("wgrad_simt_kernel", st,
-            wgrad_simt_kernel<T, BM, BN, false><<<grid, kWsThreads, smem, st>>>(a, plan, n_tiles));
+            launch_early(wgrad_simt_kernel<T, BM, BN, false>, grid, kWsThreads, smem, st, a, plan, n_tiles));
   return MN_OK;
 }
 
@@ -525,7 +530,7 @@ mn_status run_wgrad_reduce(const float *partial, const WgradPlan &plan, const in
                            int64_t matrix, void *grad_w, cudaStream_t st) {
   const dim3 grid((unsigned)std::min<int64_t>(div_up(matrix, 256), 64), (unsigned)O);
   MN_LAUNCH("wgrad_reduce_kernel", st,
-            wgrad_reduce_kernel<T><<<grid, 256, 0, st>>>(partial, plan, order, matrix, static_cast<T *>(grad_w)));
+            launch_early(wgrad_reduce_kernel<T>, grid, 256, 0, st, partial, plan, order, matrix, static_cast<T *>(grad_w)));
   return MN_OK;
 }
 
@@ -565,7 +570,7 @@ extern "C" mn_status mn_build_pair_lists(const int32_t *source_masks, const int3
     MN_CHECK_CUDA(cudaMemsetAsync(list, 0xff, sizeof(int32_t) * rows, st));   // padding: no row
     const dim3 grid((unsigned)std::min<int64_t>(kNumSMs * 8, div_up(n, 256)), bits != nullptr ? 1u : (unsigned)O);
     MN_LAUNCH("pair_side_kernel", st,
-              pair_side_kernel<<<grid, 256, 0, st>>>(side ? target_masks : source_masks, bits, n, plan, list));
+              launch_early(pair_side_kernel, grid, 256, 0, st, side ? target_masks : source_masks, bits, n, plan, list));
   }
   return MN_OK;
 }
@@ -614,7 +619,7 @@ extern "C" mn_status mn_sparse_convolution_weight_gradient(
       a.tmem_cols = z.tmem_cols;
       MN_RETURN_IF(allow_max_shared_memory(reinterpret_cast<const void *>(wgrad_tc_kernel)));
       const dim3 grid((unsigned)items, (unsigned)div_up(c_in, 256));
-      MN_LAUNCH("wgrad_tc_kernel", st, wgrad_tc_kernel<<<grid, kWgThreads, z.smem_bytes, st>>>(a, plan));
+      MN_LAUNCH("wgrad_tc_kernel", st, launch_early(wgrad_tc_kernel, grid, kWgThreads, z.smem_bytes, st, a, plan));
     } else if (dtype == MN_F32) {
       MN_RETURN_IF(run_wgrad_simt_t<float>(a, plan, items, st));
     } else if (dtype == MN_F16) {

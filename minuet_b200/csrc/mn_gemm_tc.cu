@@ -97,6 +97,7 @@ gemm_tc_kernel(const __grid_constant__ GemmTable tab, const __grid_constant__ Tc
     s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  wait_for_predecessor();
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                      smem_u32(&s_tmem_base)), "r"(tmem_cols)
@@ -106,6 +107,7 @@ gemm_tc_kernel(const __grid_constant__ GemmTable tab, const __grid_constant__ Tc
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  release_successor();   // every block has its tensor memory before another kernel's block can ask for some
   const uint32_t tmem_base = s_tmem_base;
   volatile int *abort_flag = &s_abort;
 
@@ -385,6 +387,7 @@ gemm_tc_kernel(const __grid_constant__ GemmTable tab, const __grid_constant__ Tc
 template <typename T>
 __global__ void __launch_bounds__(256)
 transpose_weights_kernel(const T *__restrict__ w, T *__restrict__ wt, int K, int N) {
+  begin_early();
   __shared__ T tile[32][33];
   const int o = blockIdx.z;
   const int k0 = blockIdx.y * 32, n0 = blockIdx.x * 32;
@@ -450,12 +453,12 @@ mn_status launch_transpose_weights(const void *weights, void *weights_t, int O, 
   const dim3 grid((unsigned)div_up(c_out, 32), (unsigned)div_up(c_in, 32), (unsigned)O);
   if (bf16) {
     MN_LAUNCH("transpose_weights_kernel", st,
-              transpose_weights_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(
+              launch_early(transpose_weights_kernel<__nv_bfloat16>, grid, 256, 0, st, 
                   static_cast<const __nv_bfloat16 *>(weights),
                   static_cast<__nv_bfloat16 *>(weights_t), c_in, c_out));
   } else {
     MN_LAUNCH("transpose_weights_kernel", st,
-              transpose_weights_kernel<__half><<<grid, 256, 0, st>>>(
+              launch_early(transpose_weights_kernel<__half>, grid, 256, 0, st, 
                   static_cast<const __half *>(weights), static_cast<__half *>(weights_t), c_in,
                   c_out));
   }
@@ -604,12 +607,12 @@ mn_status launch_gemm_tc_impl(const GemmTable &tab_in, const TcOperands &ops, in
   if (bf16) {
     MN_RETURN_IF(allow_max_shared_memory(reinterpret_cast<const void *>(gemm_tc_kernel<__nv_bfloat16>)));
     MN_LAUNCH("gemm_tc_kernel", st,
-              gemm_tc_kernel<__nv_bfloat16><<<grid, kTcThreads, smem, st>>>(
+              launch_early(gemm_tc_kernel<__nv_bfloat16>, grid, kTcThreads, smem, st, 
                   tab, args, map_a, map_direct, map_b, map_c, map_c_direct, epilogue));
   } else {
     MN_RETURN_IF(allow_max_shared_memory(reinterpret_cast<const void *>(gemm_tc_kernel<__half>)));
     MN_LAUNCH("gemm_tc_kernel", st,
-              gemm_tc_kernel<__half><<<grid, kTcThreads, smem, st>>>(tab, args, map_a, map_direct,
+              launch_early(gemm_tc_kernel<__half>, grid, kTcThreads, smem, st, tab, args, map_a, map_direct,
                                                                     map_b, map_c, map_c_direct,
                                                                     epilogue));
   }

@@ -565,6 +565,7 @@ template <typename T, int kVecElems>
 __global__ void __launch_bounds__(256)
 epilogue_kernel(T *__restrict__ x, int64_t n_vec, int vec_per_row, const float *__restrict__ scale,
                 const float *__restrict__ shift, const T *__restrict__ residual, int relu) {
+  begin_early();
   using V = typename Chunk<kVecElems * sizeof(T)>::type;
   const int64_t gsz = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_vec; i += gsz) {
@@ -598,13 +599,13 @@ mn_status run_epilogue(void *x, int64_t rows, int64_t c, const float *scale, con
     const int64_t n_vec = n / kVec;
     const int blocks = (int)std::min<int64_t>(kNumSMs * 16, div_up(n_vec, 256));
     MN_LAUNCH("epilogue_kernel", st,
-              epilogue_kernel<T, kVec><<<blocks, 256, 0, st>>>(
+              launch_early(epilogue_kernel<T, kVec>, blocks, 256, 0, st, 
                   static_cast<T *>(x), n_vec, (int)(c / kVec), scale, shift,
                   static_cast<const T *>(residual), relu));
   } else {
     const int blocks = (int)std::min<int64_t>(kNumSMs * 16, div_up(n, 256));
     MN_LAUNCH("epilogue_kernel", st,
-              epilogue_kernel<T, 1><<<blocks, 256, 0, st>>>(static_cast<T *>(x), n, (int)c, scale,
+              launch_early(epilogue_kernel<T, 1>, blocks, 256, 0, st, static_cast<T *>(x), n, (int)c, scale,
                                                             shift, static_cast<const T *>(residual),
                                                             relu));
   }

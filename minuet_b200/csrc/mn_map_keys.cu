@@ -191,6 +191,7 @@ struct RootArgs {
 
 __global__ void __launch_bounds__(kBBoxThreads)
 root_keys_kernel(const __grid_constant__ RootArgs a) {
+  release_successor();
   __shared__ int s[kBBoxThreads / 32][8];
   __shared__ int32_t s_mm[8];
   __shared__ PackParams s_p;

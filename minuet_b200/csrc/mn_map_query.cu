@@ -146,6 +146,7 @@ __device__ __forceinline__ uint32_t insert_cell(uint2 *slots, uint32_t c, uint32
 template <int kMode>
 __global__ void __launch_bounds__(kQThreads, kMode == kBits ? 5 : 4)
 search_kernel(const __grid_constant__ SearchPair sp) {
+  begin_early();
   constexpr bool kPos = kMode != kBits;   // table positions are needed
   // blocks [0, tiles0) serve direction 0, the rest direction 1 (rows and table swapped)
   const int dir = (int)blockIdx.x >= sp.tiles0 ? 1 : 0;
@@ -493,6 +494,7 @@ __device__ __forceinline__ uint32_t transpose32(uint32_t x, int lane) {
 // More than two blocks of 16 warps per SM make it slower: too many rows are open at a time.
 __global__ void __launch_bounds__(kEThreads, 2)
 emit_masks_kernel(const __grid_constant__ EmitArgs e) {
+  release_successor();
   __shared__ int32_t s_wcnt[2][32][kEWarps + 1];        // per direction / offset: warp counts, then warp bases
   __shared__ int32_t s_first[2][32], s_size[32], s_ord[32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -781,9 +783,9 @@ mn_status run_search(int mode, const mn_keyspec &spec, const SearchArgs &first,
   {
     LaunchScope scope(mode == kMap ? "search_kernel<map>" : mode == kBits ? "search_kernel<bits>"
                                                                          : "search_kernel<bits,rev>", st);
-    if (mode == kMap) search_kernel<kMap><<<blocks, kQThreads, 0, st>>>(sp);
-    else if (mode == kBits) search_kernel<kBits><<<blocks, kQThreads, 0, st>>>(sp);
-    else search_kernel<kBitsRev><<<blocks, kQThreads, 0, st>>>(sp);
+    if (mode == kMap) launch_early(search_kernel<kMap>, blocks, kQThreads, 0, st, sp);
+    else if (mode == kBits) launch_early(search_kernel<kBits>, blocks, kQThreads, 0, st, sp);
+    else launch_early(search_kernel<kBitsRev>, blocks, kQThreads, 0, st, sp);
   }
   MN_CHECK_LAUNCH();
   return MN_OK;

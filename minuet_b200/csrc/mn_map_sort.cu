@@ -197,6 +197,7 @@ constexpr int kUkStep = kUkThreads * kUkRounds;       // 8192 keys per block and
 
 __global__ void __launch_bounds__(kUkThreads, 1)
 unique_keys_kernel(const __grid_constant__ UniqueKeysArgs a) {
+  release_successor();
   __shared__ uint32_t s_cnt[kUkRounds][kUkWarps];     // openers per (round, warp), then their prefix
   __shared__ uint32_t s_before, s_total, s_step_total;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -616,6 +617,7 @@ voxel_run_mean_kernel(const T *__restrict__ features, int channels, int lanes, c
                       const uint64_t *keys1, const int32_t *which, int index_bits,
                       const int32_t *__restrict__ run_start, const int64_t *__restrict__ meta, int64_t n,
                       T *__restrict__ out) {
+  begin_early();
   const int64_t count = __ldg(meta);
   const uint64_t *keys = (*which & 1) ? keys1 : keys0;
   const uint64_t mask = (1ull << index_bits) - 1ull;
@@ -656,7 +658,7 @@ mn_status run_mean(const void *features, int64_t channels, const Runs &r, void *
   while (lanes < 32 && lanes * 4 < channels) lanes *= 2;
   const int blocks = (int)std::min<int64_t>(kNumSMs * 32, div_up(r.n, 256 / lanes));
   MN_LAUNCH("voxel_run_mean_kernel", st,
-            voxel_run_mean_kernel<T><<<blocks, 256, 0, st>>>(static_cast<const T *>(features), (int)channels, lanes,
+            launch_early(voxel_run_mean_kernel<T>, blocks, 256, 0, st, static_cast<const T *>(features), (int)channels, lanes,
                                                              r.keys, r.keys_tmp, r.which, r.index_bits, r.run_start,
                                                              r.meta, r.n, static_cast<T *>(out)));
   return MN_OK;

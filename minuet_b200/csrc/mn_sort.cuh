@@ -68,6 +68,7 @@ __device__ __forceinline__ unsigned lanes_below() {
 template <typename Source>
 __global__ void __launch_bounds__(kThreads)
 sort_keys_kernel(const __grid_constant__ Args a, const __grid_constant__ Source source) {
+  begin_early();
   __shared__ uint32_t s_hist[kMaxPasses][kDigits];
   const int passes = passes_of(a);
   for (int i = threadIdx.x; i < passes * kDigits; i += kThreads) (&s_hist[0][0])[i] = 0u;
@@ -121,6 +122,7 @@ __device__ __forceinline__ uint32_t block_exclusive(uint32_t v, uint32_t *s_part
 template <int kItems, bool kVals>
 __global__ void __launch_bounds__(kThreads)
 sort_pass_kernel(const __grid_constant__ Args a, int pass) {
+  begin_early();
   constexpr int kTile = kThreads * kItems;
   __shared__ uint64_t s_key[kTile];
   __shared__ uint32_t s_cnt[kWarps][kDigits];     // counts, then first position, per warp and digit
@@ -268,9 +270,9 @@ template <int kItems>
 mn_status launch_passes(const Args &a, int launches, cudaStream_t st) {
   for (int p = 0; p < launches; p++) {
     if (a.vals[0] != nullptr) {
-      MN_LAUNCH("sort_pass_kernel", st, sort_pass_kernel<kItems, true><<<a.tiles, kThreads, 0, st>>>(a, p));
+      MN_LAUNCH("sort_pass_kernel", st, launch_early(sort_pass_kernel<kItems, true>, a.tiles, kThreads, 0, st, a, p));
     } else {
-      MN_LAUNCH("sort_pass_kernel", st, sort_pass_kernel<kItems, false><<<a.tiles, kThreads, 0, st>>>(a, p));
+      MN_LAUNCH("sort_pass_kernel", st, launch_early(sort_pass_kernel<kItems, false>, a.tiles, kThreads, 0, st, a, p));
     }
   }
   return MN_OK;
@@ -290,7 +292,7 @@ mn_status run(Args a, const Source &source, Workspace &ws, cudaStream_t st) {
   a.state = a.next_tile + 64;
   MN_CHECK_CUDA(cudaMemsetAsync(control, 0, control_words(a.n, launches) * sizeof(uint32_t), st));
   const int blocks = (int)std::min<int64_t>(kNumSMs * 8, div_up(a.n, kThreads));
-  MN_LAUNCH("sort_keys_kernel", st, sort_keys_kernel<Source><<<blocks, kThreads, 0, st>>>(a, source));
+  MN_LAUNCH("sort_keys_kernel", st, launch_early(sort_keys_kernel<Source>, blocks, kThreads, 0, st, a, source));
   return items_of(a.n) == 4 ? launch_passes<4>(a, launches, st) : launch_passes<16>(a, launches, st);
 }
 

@@ -1,11 +1,11 @@
 // Stable radix sort of 64-bit keys, shared by the map step, voxelisation and the neighbour
-// tables: one launch that makes the keys and counts their digits, then one launch per 8-bit
+// tables: one launch that makes the keys and counts their digits, then one launch per 9-bit
 // digit.
 //
 // A digit pass moves every key once: a block takes the next tile of keys, ranks them in
 // registers (equal digits of a warp find each other with match.any), learns how many keys of
 // each digit the tiles before it hold by looking back over their published counts (every thread
-// follows one digit; a tile publishes its own count at once and the running total as soon as it
+// follows two digits; a tile publishes its own count at once and the running total as soon as it
 // knows it), reorders the tile in shared memory and writes it out in runs.  Tiles are numbered
 // in the order in which blocks start, so a block only ever waits for blocks that already run;
 // the waits are bounded all the same (status bit 4).  An index that travels with the keys sits
@@ -28,9 +28,9 @@ namespace rsort {
 
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
-constexpr int kBits = 8;
-constexpr int kDigits = 1 << kBits;           // == kThreads: a thread per digit
-constexpr int kMaxPasses = 8;
+constexpr int kBits = 9;
+constexpr int kDigits = 1 << kBits;           // == 2 * kThreads: a thread per pair of digits
+constexpr int kMaxPasses = 8;                 // more than 64 / kBits
 constexpr uint32_t kSpinLimit = 1u << 22;
 
 struct Args {
@@ -125,7 +125,8 @@ sort_pass_kernel(const __grid_constant__ Args a, int pass) {
   begin_early();
   constexpr int kTile = kThreads * kItems;
   __shared__ uint64_t s_key[kTile];
-  __shared__ uint32_t s_cnt[kWarps][kDigits];     // counts, then first position, per warp and digit
+  // counts, then first positions inside the tile's digit, per warp and digit (at most kTile)
+  __shared__ __align__(8) uint16_t s_cnt[kWarps][kDigits];
   __shared__ uint32_t s_local[kDigits];              // first position of a digit inside the tile
   __shared__ uint32_t s_dest[kDigits];               // its first position in the output, minus s_local
   __shared__ uint32_t s_part[kWarps];
@@ -137,9 +138,10 @@ sort_pass_kernel(const __grid_constant__ Args a, int pass) {
   const unsigned lt = lanes_below();
   if (tid == 0) s_tile = (int)atomicAdd(a.next_tile + pass, 1u);
 #pragma unroll
-  for (int w = 0; w < kWarps; w++) s_cnt[w][tid] = 0u;
-  // where the digit starts in the output (every block adds up the 256 totals itself)
-  const uint32_t digit_start = block_exclusive(__ldcg(a.hist + pass * kDigits + tid), s_part, lane, warp);
+  for (int w = 0; w < kWarps; w++) reinterpret_cast<uint32_t *>(s_cnt[w])[tid] = 0u;
+  // where this thread's two digits start in the output (every block adds up the totals itself)
+  const uint2 totals = __ldcg(reinterpret_cast<const uint2 *>(a.hist + pass * kDigits) + tid);
+  const uint32_t digit_start = block_exclusive(totals.x + totals.y, s_part, lane, warp);
   const int tile = s_tile;
   if (tile >= a.tiles) return;
   if (tile == 0 && tid == 0 && last_pass && a.result_in_second != nullptr) *a.result_in_second = passes & 1;
@@ -152,7 +154,7 @@ sort_pass_kernel(const __grid_constant__ Args a, int pass) {
   for (int j = 0; j < kItems; j++) key[j] = base + j * 32 < a.n ? __ldcg(kin + base + j * 32) : ~0ull;
   // ---- rank inside the warp: position among the equal digits of the warp's slice ------------
   uint16_t rank[kItems];
-  uint32_t *mine = s_cnt[warp];
+  uint16_t *mine = s_cnt[warp];
 #pragma unroll
   for (int j = 0; j < kItems; j++) {
     const bool valid = base + j * 32 < a.n;
@@ -161,41 +163,52 @@ sort_pass_kernel(const __grid_constant__ Args a, int pass) {
     uint32_t before = 0;
     if (valid) before = mine[d];
     __syncwarp();
-    if (valid && (peers & lt) == 0u) mine[d] = before + __popc(peers);
+    if (valid && (peers & lt) == 0u) mine[d] = (uint16_t)(before + __popc(peers));
     rank[j] = (uint16_t)(before + __popc(peers & lt));
     __syncwarp();
   }
   __syncthreads();
   // ---- per digit: the warps' first positions, the tile's count ---------------------------------
-  uint32_t count = 0;
+  uint2 count = make_uint2(0u, 0u);
 #pragma unroll
   for (int w = 0; w < kWarps; w++) {
-    const uint32_t c = s_cnt[w][tid];
-    s_cnt[w][tid] = count;
-    count += c;
+    uint32_t *at = reinterpret_cast<uint32_t *>(s_cnt[w]) + tid;    // two digits
+    const uint32_t c = *at;
+    *at = count.x | (count.y << 16);
+    count.x += c & 0xffffu;
+    count.y += c >> 16;
   }
-  // a published word: 2 * value + (running total ? 1 : 0) + 1; 0: nothing yet
-  volatile uint32_t *state = a.state + ((size_t)pass * a.tiles) * kDigits + tid;
-  state[(size_t)tile * kDigits] = 2u * count + (tile == 0 ? 2u : 1u);
-  const uint32_t local = block_exclusive(count, s_part, lane, warp);
-  // ---- look back: keys of this digit in the tiles before ----------------------------------------
-  uint32_t before = 0;
+  // a published word: 2 * value + (running total ? 1 : 0) + 1; 0: nothing yet.  A thread's two
+  // words are one 8-byte access, so both say the same about what they hold.
+  volatile uint64_t *state = reinterpret_cast<uint64_t *>(a.state + ((size_t)pass * a.tiles) * kDigits) + tid;
+  constexpr int kPairs = kDigits / 2;
+  auto publish = [&](uint32_t x, uint32_t y, uint32_t mark) {
+    state[(size_t)tile * kPairs] = (uint64_t)(2u * x + mark) | ((uint64_t)(2u * y + mark) << 32);
+  };
+  publish(count.x, count.y, tile == 0 ? 2u : 1u);
+  const uint32_t local = block_exclusive(count.x + count.y, s_part, lane, warp);
+  // ---- look back: keys of these digits in the tiles before --------------------------------------
+  uint2 before = make_uint2(0u, 0u);
   if (tile > 0) {
     uint32_t spins = 0;
     for (int prev = tile - 1; prev >= 0;) {
-      const uint32_t v = state[(size_t)prev * kDigits];
-      if (v == 0u) {
+      const uint64_t v = state[(size_t)prev * kPairs];
+      const uint32_t x = (uint32_t)v, y = (uint32_t)(v >> 32);
+      if (x == 0u) {
         if (++spins > kSpinLimit) { atomicOr(a.status, MN_STATUS_GRID_TIMEOUT); break; }
         continue;
       }
-      before += (v - 1u) >> 1;
-      if (((v - 1u) & 1u) != 0u) break;
+      before.x += (x - 1u) >> 1;
+      before.y += (y - 1u) >> 1;
+      if (((x - 1u) & 1u) != 0u) break;
       prev--;
     }
-    state[(size_t)tile * kDigits] = 2u * (before + count) + 2u;
+    publish(before.x + count.x, before.y + count.y, 2u);
   }
-  s_local[tid] = local;
-  s_dest[tid] = digit_start + before - local;
+  s_local[2 * tid] = local;
+  s_local[2 * tid + 1] = local + count.x;
+  s_dest[2 * tid] = digit_start + before.x - local;
+  s_dest[2 * tid + 1] = digit_start + totals.x + before.y - (local + count.x);
   __syncthreads();
   // ---- reorder in shared memory, write in runs -------------------------------------------------
 #pragma unroll
@@ -284,7 +297,9 @@ template <typename Source>
 mn_status run(Args a, const Source &source, Workspace &ws, cudaStream_t st) {
   MN_CHECK_ARG(a.n > 0 && a.n < (1ll << 31) - 1, "radix sort: n = %lld exceeds 2^31-2", (long long)a.n);
   a.tiles = (int32_t)tiles_of(a.n);
-  const int launches = a.bits >= 0 ? std::min(kMaxPasses, std::max(1, (a.bits + kBits - 1) / kBits)) : kMaxPasses;
+  // bits that only the device knows: no more than fit above the index
+  const int bits = a.bits >= 0 ? a.bits : 64 - a.first_bit;
+  const int launches = std::min(kMaxPasses, std::max(1, (bits + kBits - 1) / kBits));
   uint32_t *control = ws.take<uint32_t>(control_words(a.n, kMaxPasses));
   MN_CHECK_WS(ws);
   a.hist = control;

@@ -109,6 +109,7 @@ __device__ __forceinline__ void pack_rows(const int32_t *__restrict__ coords, in
                                           int num_clouds, const mn_keyspec &spec,
                                           const PackParams &p, uint64_t *__restrict__ keys,
                                           int64_t thread, int64_t nthreads, bool &bad) {
+  int hint = 0;
   if (ndim == 3) {
     const bool aligned = ((reinterpret_cast<uintptr_t>(coords) | reinterpret_cast<uintptr_t>(keys)) & 15) == 0;
     const int64_t q_begin = r_begin >> 2;
@@ -121,10 +122,10 @@ __device__ __forceinline__ void pack_rows(const int32_t *__restrict__ coords, in
       const int64_t r = q << 2;
       uint64_t g0 = 0, g1 = 0, g2 = 0, g3 = 0;
       if (bd != nullptr) {
-        g0 = cloud_of(bd, num_clouds, r);
-        g3 = cloud_of(bd, num_clouds, r + 3);
-        g1 = g0 == g3 ? g0 : cloud_of(bd, num_clouds, r + 1);
-        g2 = g0 == g3 ? g0 : cloud_of(bd, num_clouds, r + 2);
+        g0 = cloud_near(bd, num_clouds, r, hint);
+        g1 = cloud_near(bd, num_clouds, r + 1, hint);
+        g2 = cloud_near(bd, num_clouds, r + 2, hint);
+        g3 = cloud_near(bd, num_clouds, r + 3, hint);
       }
       ulonglong2 lo, hi;
       lo.x = pack_one(c0, 3, g0, spec, p, bad);
@@ -137,14 +138,14 @@ __device__ __forceinline__ void pack_rows(const int32_t *__restrict__ coords, in
     }
     for (int64_t r = (q_end << 2) + thread; r < r_end; r += nthreads) {
       int c[4] = {coords[r * 3], coords[r * 3 + 1], coords[r * 3 + 2], 0};
-      uint64_t g = bd != nullptr ? cloud_of(bd, num_clouds, r) : 0;
+      uint64_t g = bd != nullptr ? cloud_near(bd, num_clouds, r, hint) : 0;
       keys[r] = pack_one(c, 3, g, spec, p, bad);
     }
   } else {
     for (int64_t r = r_begin + thread; r < r_end; r += nthreads) {
       int c[4] = {0, 0, 0, 0};
       for (int k = 0; k < ndim; k++) c[k] = coords[r * ndim + k];
-      uint64_t g = bd != nullptr ? cloud_of(bd, num_clouds, r) : 0;
+      uint64_t g = bd != nullptr ? cloud_near(bd, num_clouds, r, hint) : 0;
       keys[r] = pack_one(c, ndim, g, spec, p, bad);
     }
   }

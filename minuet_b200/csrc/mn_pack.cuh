@@ -40,6 +40,7 @@ __host__ __device__ inline bool compute_keyspec(const int32_t *minmax, int ndim,
 
 #ifdef __CUDACC__
 __device__ __forceinline__ int floor_to(int c, int s) {
+  if ((s & (s - 1)) == 0) return c & -s;
   int q = c / s;
   if ((c % s != 0) && (c < 0)) q--;
   return q * s;
@@ -53,6 +54,12 @@ __device__ __forceinline__ int cloud_of(const int64_t *bd, int num_clouds, int64
     if (bd[mid] <= row) lo = mid; else hi = mid;
   }
   return lo;
+}
+
+// The same where rows come in order: `hint` is the cloud of the caller's row before (0 at first).
+__device__ __forceinline__ int cloud_near(const int64_t *bd, int num_clouds, int64_t row, int &hint) {
+  if (row < bd[hint] || (hint + 1 < num_clouds && row >= bd[hint + 1])) hint = cloud_of(bd, num_clouds, row);
+  return hint;
 }
 
 struct PackParams {

@@ -50,6 +50,10 @@ constexpr int kMaxN = 256;
 constexpr int kIdxSlots = 8;           // steps the index blocks run ahead
 constexpr int kMaxSub = 2;             // 128-row sub-tiles per CTA tile
 
+// What feeds the kernel: a kernel map; the product rows of a pair list; the rows of one dense
+// product (the 1x1x1 convolution), whose tiles TMA fetches whole.
+enum ImMode { kMap = 0, kPairRows = 1, kDense = 2 };
+
 struct ImArgs {
   const uint8_t *in;          // [S, K] 16-bit
   const int32_t *nbr;         // [O, pitch]
@@ -138,11 +142,11 @@ __device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t b
 // Offset bits of the sub-tiles of a CTA tile, in two steps: the request (unconditional, from a
 // clamped index: a load under a condition is waited for where the branch joins, a thousand cycles
 // per tile) and, a tile later, the value (pair mode: one offset each).
-template <int kSub, bool kPairs>
+template <int kSub, int kMode>
 __device__ __forceinline__ void request_bits(const ImArgs &args, int tile, uint32_t (&raw)[kSub]) {
 #pragma unroll
   for (int h = 0; h < kSub; h++)
-    raw[h] = kPairs ? 1u : (uint32_t)load_ahead_1(args.tile_bits + min(tile * kSub + h, args.n_tiles128 - 1));
+    raw[h] = kMode != kMap ? 1u : (uint32_t)load_ahead_1(args.tile_bits + min(tile * kSub + h, args.n_tiles128 - 1));
 }
 
 template <int kSub>
@@ -163,11 +167,13 @@ __device__ __forceinline__ uint32_t union_of(const uint32_t (&hb)[kSub]) {
 
 // kSub: sub-tiles per CTA tile (they share every weight tile); kLpr: lanes that copy one
 // 128-byte slice (4 where a source row has at most 64 bytes: half the copies, twice the rows
-// per copy); kProdWarps: 4 producer and 8 epilogue warps or 8 and 4; kPairs: pair mode.
-template <int kSub, int kLpr, int kProdWarps, bool kPairs>
+// per copy); kProdWarps: 4 producer and 8 epilogue warps or 8 and 4.
+template <int kSub, int kLpr, int kProdWarps, int kMode>
 __global__ void __launch_bounds__(kImThreads, kImCtas)
 conv_implicit_kernel(const __grid_constant__ ImArgs args,
+                     const __grid_constant__ CUtensorMap map_a,     // kDense: features [S, K]
                      const __grid_constant__ CUtensorMap map_b) {   // weights^T [O, N, K]
+  constexpr bool kPairs = kMode == kPairRows;
   constexpr int kProdRows = 128 / kProdWarps;               // rows of a sub-tile per producer warp
   constexpr int kMmaWarp = kProdWarps, kTmaWarp = kProdWarps + 1, kEpiWarp = kProdWarps + 2;
   constexpr int kEpiCols = (kGatherWarps - kProdWarps) / 4;   // epilogue warps per quarter of the rows
@@ -189,7 +195,8 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < stages; s++) {
-      mbar_init(&bar_full[s], kProdWarps * 32 + 1);   // every producer lane + the weight tile's expect_tx
+      // every producer lane + the weight tile's expect_tx
+      mbar_init(&bar_full[s], kMode == kDense ? 1 : kProdWarps * 32 + 1);
       mbar_init(&bar_empty[s], 1);
     }
     for (int a = 0; a < 2; a++) { mbar_init(&bar_acc_full[a], 1); mbar_init(&bar_acc_empty[a], 4 * kEpiCols); }
@@ -237,7 +244,7 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
     uint32_t phase = 0, slot_phase = 0;
     bool alive = true;
     bool ready = mbar_test(&bar_empty[0], 1u);
-    while (alive) {
+    while (kMode != kDense && alive) {
       if (!mbar_wait(&bar_idx_full[slot], slot_phase, abort_flag, args.status)) break;
       const uint32_t has = s_idx_has[slot];        // sub-tiles that have this offset; 0: no more steps
       if (has == 0u) break;
@@ -311,13 +318,13 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
     uint32_t phase = 0, acc_phase = 0;
     bool alive = true;
     uint32_t raw[kSub];
-    request_bits<kSub, kPairs>(args, (int)blockIdx.x, raw);
+    request_bits<kSub, kMode>(args, (int)blockIdx.x, raw);
     bool ready = mbar_test(&bar_full[0], 0u);
     for (int tile = blockIdx.x; alive && tile < args.num_tiles; tile += gridDim.x) {
       uint32_t hb[kSub];
       take_bits<kSub>(args, tile, raw, hb);
       const int n_offsets = __popc(union_of<kSub>(hb));
-      request_bits<kSub, kPairs>(args, tile + (int)gridDim.x, raw);
+      request_bits<kSub, kMode>(args, tile + (int)gridDim.x, raw);
       if (!mbar_wait_warp(false, &bar_acc_empty[acc], acc_phase ^ 1u, abort_flag, args.status)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t tmem_d = tmem_base + (uint32_t)(acc * kSub * args.n_pad);
@@ -325,7 +332,7 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
       for (int o = 0; alive && o < n_offsets; o++) {
         for (int kb = 0; kb < args.k_blocks; kb++) {
           if (!mbar_wait_warp(ready, &bar_full[stage], phase, abort_flag, args.status)) { alive = false; break; }
-          fence_generic_to_async();
+          if (kMode != kDense) fence_generic_to_async();
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           const uint32_t lo = desc_lo + (uint32_t)stage * stage_step;
           const int nk = kb + 1 < args.k_blocks ? kBK / kUmmaK : last_nk;
@@ -364,14 +371,14 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
     bool alive = true;
     int itile = (int)blockIdx.x - (int)gridDim.x, slot = 0;
     uint32_t irest = 0u, slot_phase = 0, ihb[kSub], iraw[kSub];
-    request_bits<kSub, kPairs>(args, (int)blockIdx.x, iraw);
-    bool more = true;          // false once the end mark is out
+    request_bits<kSub, kMode>(args, (int)blockIdx.x, iraw);
+    bool more = kMode != kDense;   // false once the end mark is out
     auto send_indices = [&]() {
       while (irest == 0u && itile < args.num_tiles) {
         itile += (int)gridDim.x;
         take_bits<kSub>(args, itile, iraw, ihb);
         irest = union_of<kSub>(ihb);
-        request_bits<kSub, kPairs>(args, itile + (int)gridDim.x, iraw);
+        request_bits<kSub, kMode>(args, itile + (int)gridDim.x, iraw);
       }
       if (!mbar_wait_warp(false, &bar_idx_empty[slot], slot_phase ^ 1u, abort_flag, args.status)) {
         alive = false;
@@ -408,13 +415,13 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
     int stage = 0;
     uint32_t phase = 0;
     uint32_t raw[kSub];
-    request_bits<kSub, kPairs>(args, (int)blockIdx.x, raw);
+    request_bits<kSub, kMode>(args, (int)blockIdx.x, raw);
     bool ready = mbar_test(&bar_empty[0], 1u);
     for (int tile = blockIdx.x; alive && tile < args.num_tiles; tile += gridDim.x) {
       uint32_t hb[kSub];
       take_bits<kSub>(args, tile, raw, hb);
       uint32_t rest = union_of<kSub>(hb);
-      request_bits<kSub, kPairs>(args, tile + (int)gridDim.x, raw);
+      request_bits<kSub, kMode>(args, tile + (int)gridDim.x, raw);
       const int pair_row = kPairs ? pair_row_of_tile(args, tile) : 0;
       while (alive && rest != 0u) {
         const int p = kPairs ? pair_row : __ffs(rest) - 1;
@@ -427,7 +434,8 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
           if (++stage == stages) { stage = 0; phase ^= 1u; }
           ready = mbar_test(&bar_empty[stage], phase ^ 1u);
           if (elect_one()) {
-            mbar_expect_tx(full, b_bytes);
+            mbar_expect_tx(full, b_bytes + (kMode == kDense ? (uint32_t)args.a_bytes : 0u));
+            if (kMode == kDense) tma_load_2d(sb - args.a_bytes, &map_a, kb * kBK, tile * kBM, full);
             tma_load_3d(sb, &map_b, kb * kBK, 0, widx, full);
           }
           __syncwarp();
@@ -454,11 +462,11 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
     int acc = 0;
     uint32_t acc_phase = 0;
     uint32_t raw[kSub];
-    request_bits<kSub, kPairs>(args, (int)blockIdx.x, raw);
+    request_bits<kSub, kMode>(args, (int)blockIdx.x, raw);
     // Row of the output (and of the residual) that this lane's accumulator row belongs to, per
     // sub-tile (-1: none): requested two tiles ahead, so that the residual rows of the next tile
     // can be on their way to L2 while this one is worked on.
-    const bool permuted = !kPairs && args.perm != nullptr;
+    const bool permuted = kMode == kMap && args.perm != nullptr;
     auto table_row = [&](int tile, int h) { return ((int64_t)tile * kSub + h) * kBM + quarter * 32 + lane; };
     auto request_rows = [&](int tile, int32_t (&rows)[kSub]) {
 #pragma unroll
@@ -476,7 +484,7 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
       uint32_t hb[kSub];
       take_bits<kSub>(args, tile, raw, hb);
       const bool empty_tile = union_of<kSub>(hb) == 0u;   // no MMA ran: the rows are zero
-      request_bits<kSub, kPairs>(args, tile + (int)gridDim.x, raw);
+      request_bits<kSub, kMode>(args, tile + (int)gridDim.x, raw);
 #pragma unroll
       for (int h = 0; h < kSub; h++) { grow[h] = take_row(tile, h, rows_1[h]); rows_1[h] = rows_2[h]; }
       request_rows(tile + 2 * (int)gridDim.x, rows_2);
@@ -725,14 +733,15 @@ inline int row_chunk_shift(int64_t T, int64_t pairs, int64_t O) {
 
 namespace {
 
-template <int kSub, int kLpr, int kProdWarps, bool kPairs>
-mn_status launch_implicit(const ImArgs &a, const TcSizing &sizing, const CUtensorMap &map_b,
-                          cudaStream_t st) {
-  auto kernel = conv_implicit_kernel<kSub, kLpr, kProdWarps, kPairs>;
+template <int kSub, int kLpr, int kProdWarps, int kMode>
+mn_status launch_implicit(const ImArgs &a, const TcSizing &sizing, const CUtensorMap &map_a,
+                          const CUtensorMap &map_b, cudaStream_t st) {
+  auto kernel = conv_implicit_kernel<kSub, kLpr, kProdWarps, kMode>;
   MN_RETURN_IF(allow_max_shared_memory(reinterpret_cast<const void *>(kernel)));
   const int grid = std::min(a.num_tiles, kNumSMs * sizing.ctas_per_sm);
-  MN_LAUNCH(kPairs ? "conv_implicit_kernel<pairs>" : "conv_implicit_kernel", st,
-            launch_early(kernel, grid, kImThreads, sizing.smem_bytes, st, a, map_b));
+  MN_LAUNCH(kMode == kPairRows ? "conv_implicit_kernel<pairs>" : kMode == kDense ? "conv_implicit_kernel<dense>"
+                                                                                 : "conv_implicit_kernel", st,
+            launch_early(kernel, grid, kImThreads, sizing.smem_bytes, st, a, map_a, map_b));
   return MN_OK;
 }
 
@@ -775,8 +784,40 @@ mn_status launch_pair_products(const PairPlan &plan, int64_t S, int64_t c_in, in
   a.out_f32 = products;
   CUtensorMap map_b;
   MN_RETURN_IF(make_kmajor_map(&map_b, weights_t, bf16, c_in, c_out, O, a.n_pad));
-  return c_in <= 32 ? launch_implicit<1, 4, 8, true>(a, sizing, map_b, st)
-                    : launch_implicit<1, 8, 8, true>(a, sizing, map_b, st);
+  return c_in <= 32 ? launch_implicit<1, 4, 8, kPairRows>(a, sizing, map_b, map_b, st)
+                    : launch_implicit<1, 8, 8, kPairRows>(a, sizing, map_b, map_b, st);
+}
+
+// out = relu?((features @ weights) * scale + shift + residual), c_out a multiple of 8
+mn_status launch_dense_rows(int64_t rows, int64_t c_in, int64_t c_out, bool bf16, const void *features,
+                            const void *weights_t, const float *scale, const float *shift, const void *residual,
+                            bool relu, void *out, int32_t *status_dev, cudaStream_t st) {
+  ImArgs a{};
+  a.scale = scale;
+  a.shift = shift;
+  a.residual = static_cast<const uint8_t *>(residual);
+  a.out16 = static_cast<uint8_t *>(out);
+  a.status = status_dev;
+  a.T = rows;
+  a.K = (int)c_in;
+  a.N = (int)c_out;
+  a.n_pad = (int)align_up((size_t)c_out, 16);
+  a.k_blocks = (int)div_up(c_in, kBK);
+  a.n_tiles128 = a.num_tiles = (int)div_up(rows, kBM);
+  a.acc_bufs = 2;
+  a.a_bytes = kBM * kBK * 2;
+  a.stage_bytes = a.a_bytes + a.n_pad * kBK * 2;
+  const TcSizing sizing = size_tc_kernel(a.stage_bytes, a.acc_bufs * a.n_pad, kMaxStages, kImCtas, kIdxSlots * kMaxSub * kBM * 4, kMaxStages);
+  a.stages = sizing.stages;
+  a.tmem_cols = sizing.tmem_cols;
+  a.num_offsets = 1;
+  a.elem_is_bf16 = bf16 ? 1 : 0;
+  a.relu = relu ? 1 : 0;
+  a.wide = c_out % 16 == 0 && ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(residual)) & 31) == 0;
+  CUtensorMap map_a, map_b;
+  MN_RETURN_IF(make_kmajor_map(&map_a, features, bf16, c_in, rows, 0, kBM));
+  MN_RETURN_IF(make_kmajor_map(&map_b, weights_t, bf16, c_in, c_out, 1, a.n_pad));
+  return launch_implicit<1, 8, 4, kDense>(a, sizing, map_a, map_b, st);
 }
 
 }  // namespace mn
@@ -945,8 +986,8 @@ extern "C" mn_status mn_sparse_convolution_forward_implicit(
   CUtensorMap map_b;
   MN_RETURN_IF(make_kmajor_map(&map_b, weights_t, bf16, c_in, c_out, O, a.n_pad));
   if (sub == 1)
-    return c_in <= 32 ? launch_implicit<1, 4, 4, false>(a, sizing, map_b, st)
-                      : launch_implicit<1, 8, 4, false>(a, sizing, map_b, st);
-  return c_in <= 32 ? launch_implicit<2, 4, 8, false>(a, sizing, map_b, st)
-                    : launch_implicit<2, 8, 8, false>(a, sizing, map_b, st);
+    return c_in <= 32 ? launch_implicit<1, 4, 4, kMap>(a, sizing, map_b, map_b, st)
+                      : launch_implicit<1, 8, 4, kMap>(a, sizing, map_b, map_b, st);
+  return c_in <= 32 ? launch_implicit<2, 4, 8, kMap>(a, sizing, map_b, map_b, st)
+                    : launch_implicit<2, 8, 8, kMap>(a, sizing, map_b, map_b, st);
 }

@@ -257,7 +257,7 @@ gemm_tc_kernel(const __grid_constant__ GemmTable tab, const __grid_constant__ Tc
 #pragma unroll
                   for (int i = 0; i < 8; i++) f[i] = __uint_as_float(r[v * 8 + i]);
                   if (ep.scale != nullptr) {
-                    if (c + 8 <= n) {
+                    if (c + 8 <= n && (reinterpret_cast<uintptr_t>(ep.scale) & 15) == 0) {
                       const float4 s0 = __ldg(reinterpret_cast<const float4 *>(ep.scale + c));
                       const float4 s1 = __ldg(reinterpret_cast<const float4 *>(ep.scale + c) + 1);
                       f[0] *= s0.x; f[1] *= s0.y; f[2] *= s0.z; f[3] *= s0.w;
@@ -267,7 +267,7 @@ gemm_tc_kernel(const __grid_constant__ GemmTable tab, const __grid_constant__ Tc
                     }
                   }
                   if (ep.shift != nullptr) {
-                    if (c + 8 <= n) {
+                    if (c + 8 <= n && (reinterpret_cast<uintptr_t>(ep.shift) & 15) == 0) {
                       const float4 s0 = __ldg(reinterpret_cast<const float4 *>(ep.shift + c));
                       const float4 s1 = __ldg(reinterpret_cast<const float4 *>(ep.shift + c) + 1);
                       f[0] += s0.x; f[1] += s0.y; f[2] += s0.z; f[3] += s0.w;
@@ -276,7 +276,9 @@ gemm_tc_kernel(const __grid_constant__ GemmTable tab, const __grid_constant__ Tc
                       for (int i = 0; i < 8 && c + i < n; i++) f[i] += __ldg(ep.shift + c + i);
                     }
                   }
-                  if (ep.residual != nullptr && c + 8 <= n) {
+                  // rows of 8-channel pieces only: another pitch leaves them off 16-byte boundaries
+                  if (ep.residual != nullptr && n % 8 == 0 &&
+                      (reinterpret_cast<uintptr_t>(ep.residual) & 15) == 0) {
                     const uint4 rv = __ldg(reinterpret_cast<const uint4 *>(
                         static_cast<const uint8_t *>(ep.residual) + (t * n + c) * 2));
                     const uint16_t *r16 = reinterpret_cast<const uint16_t *>(&rv);

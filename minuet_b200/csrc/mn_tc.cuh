@@ -253,6 +253,9 @@ struct PairEpilogue {
 };
 
 // step 1: products[r, :] = sources[pair_src[r], :] @ weights_t[order[p(r)]]^T, fp32
+mn_status launch_dense_rows(int64_t rows, int64_t c_in, int64_t c_out, bool bf16, const void *features,
+                            const void *weights_t, const float *scale, const float *shift, const void *residual,
+                            bool relu, void *out, int32_t *status_dev, cudaStream_t st);
 mn_status launch_pair_products(const PairPlan &plan, int64_t S, int64_t c_in, int64_t c_out, bool bf16,
                                const void *sources, const void *weights_t, int O,
                                const int32_t *pair_src, const int32_t *order, float *products,

@@ -498,6 +498,20 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
         }
       }
       uint32_t res[8];
+      // rows that are no whole number of 16-byte pieces (kDense): 8-byte pieces
+      auto load_narrow = [&](const uint8_t *src, int c) {
+        if (kMode == kDense && (n & 7) != 0) {
+#pragma unroll
+          for (int i = 0; i < 4; i++)
+            if (c + 4 * i < n) {
+              const uint2 v = *reinterpret_cast<const uint2 *>(src + 8 * i);
+              res[2 * i] = v.x; res[2 * i + 1] = v.y;
+            }
+          return;
+        }
+        if (c < n) ld_global_16(src, res);
+        if (c + 8 < n) ld_global_16(src + 16, res + 4);
+      };
       auto load_residual = [&](int h, int c) {
 #pragma unroll
         for (int i = 0; i < 8; i++) res[i] = 0u;
@@ -506,8 +520,7 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
         if (args.wide && c + 16 <= n) {
           ld_global_32(src, res);
         } else {
-          if (c < n) ld_global_16(src, res);
-          if (c + 8 < n) ld_global_16(src + 16, res + 4);
+          load_narrow(src, c);
         }
       };
       if (!kPairs) load_residual(0, first_piece * 16);
@@ -596,6 +609,10 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
           uint8_t *dst = args.out16 + ((int64_t)grow[h] * n + c) * 2;
           if (args.wide && c + 16 <= n) {
             st_global_32(dst, out);
+          } else if (kMode == kDense && (n & 7) != 0) {
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+              if (c + 4 * i < n) *reinterpret_cast<uint2 *>(dst + 8 * i) = make_uint2(out[2 * i], out[2 * i + 1]);
           } else {
             if (c < n) *reinterpret_cast<uint4 *>(dst) = make_uint4(out[0], out[1], out[2], out[3]);
             if (c + 8 < n) *reinterpret_cast<uint4 *>(dst + 16) = make_uint4(out[4], out[5], out[6], out[7]);
@@ -788,7 +805,7 @@ mn_status launch_pair_products(const PairPlan &plan, int64_t S, int64_t c_in, in
                     : launch_implicit<1, 8, 8, kPairRows>(a, sizing, map_b, map_b, st);
 }
 
-// out = relu?((features @ weights) * scale + shift + residual), c_out a multiple of 8
+// out = relu?((features @ weights) * scale + shift + residual), c_out a multiple of 4
 mn_status launch_dense_rows(int64_t rows, int64_t c_in, int64_t c_out, bool bf16, const void *features,
                             const void *weights_t, const float *scale, const float *shift, const void *residual,
                             bool relu, void *out, int32_t *status_dev, cudaStream_t st) {

@@ -13,7 +13,7 @@ DEV = "cuda:0"
 
 
 @pytest.mark.parametrize("rows", [1, 127, 128, 129, 80_001])
-@pytest.mark.parametrize("c_in,c_out", [(8, 8), (32, 20), (72, 24), (64, 32), (256, 128), (40, 256)])
+@pytest.mark.parametrize("c_in,c_out", [(8, 8), (32, 20), (16, 6), (72, 24), (64, 32), (256, 128), (40, 256)])
 @pytest.mark.parametrize("dtype,unit", [(torch.float16, 2.0 ** -11), (torch.bfloat16, 2.0 ** -8)])
 def test_dense_rows(rows, c_in, c_out, dtype, unit):
     gen = torch.Generator(device=DEV).manual_seed(rows + c_in + c_out)

@@ -49,10 +49,12 @@ constexpr int kMaxStages = 8;
 constexpr int kMaxN = 256;
 constexpr int kIdxSlots = 8;           // steps the index blocks run ahead
 constexpr int kMaxSub = 2;             // 128-row sub-tiles per CTA tile
+constexpr int kNBlock = kBK * 128;     // kMapNMajor: bytes of one block of 64 columns of a weight tile
 
-// What feeds the kernel: a kernel map; the product rows of a pair list; the rows of one dense
-// product (the 1x1x1 convolution), whose tiles TMA fetches whole.
-enum ImMode { kMap = 0, kPairRows = 1, kDense = 2 };
+// What feeds the kernel: a kernel map; the same with weights as they are, [O, K, N], as N-major
+// tiles; the product rows of a pair list; the rows of one dense product (the 1x1x1 convolution),
+// whose tiles TMA fetches whole.
+enum ImMode { kMap = 0, kMapNMajor = 1, kPairRows = 2, kDense = 3 };
 
 struct ImArgs {
   const uint8_t *in;          // [S, K] 16-bit
@@ -146,7 +148,7 @@ template <int kSub, int kMode>
 __device__ __forceinline__ void request_bits(const ImArgs &args, int tile, uint32_t (&raw)[kSub]) {
 #pragma unroll
   for (int h = 0; h < kSub; h++)
-    raw[h] = kMode != kMap ? 1u : (uint32_t)load_ahead_1(args.tile_bits + min(tile * kSub + h, args.n_tiles128 - 1));
+    raw[h] = kMode > kMapNMajor ? 1u : (uint32_t)load_ahead_1(args.tile_bits + min(tile * kSub + h, args.n_tiles128 - 1));
 }
 
 template <int kSub>
@@ -172,8 +174,8 @@ template <int kSub, int kLpr, int kProdWarps, int kMode>
 __global__ void __launch_bounds__(kImThreads, kImCtas)
 conv_implicit_kernel(const __grid_constant__ ImArgs args,
                      const __grid_constant__ CUtensorMap map_a,     // kDense: features [S, K]
-                     const __grid_constant__ CUtensorMap map_b) {   // weights^T [O, N, K]
-  constexpr bool kPairs = kMode == kPairRows;
+                     const __grid_constant__ CUtensorMap map_b) {   // weights^T [O, N, K]; kMapNMajor: weights [O, K, N]
+  constexpr bool kPairs = kMode == kPairRows, kNMajor = kMode == kMapNMajor;
   constexpr int kProdRows = 128 / kProdWarps;               // rows of a sub-tile per producer warp
   constexpr int kMmaWarp = kProdWarps, kTmaWarp = kProdWarps + 1, kEpiWarp = kProdWarps + 2;
   constexpr int kEpiCols = (kGatherWarps - kProdWarps) / 4;   // epilogue warps per quarter of the rows
@@ -309,10 +311,14 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
     // ------------------------------ MMA issuer --------------------------------
     const uint32_t fmt = args.elem_is_bf16 ? 1u : 0u;
     const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) |
-                           ((uint32_t)(args.n_pad >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
+                           ((uint32_t)(args.n_pad >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24) |
+                           (kNMajor ? 1u << 16 : 0u);
     const uint64_t desc0 = umma_desc(smem_u32(stage_base));
+    const uint64_t desc_b = kNMajor ? mn_major_desc(smem_u32(stage_base), kNBlock) : desc0;
+    const uint32_t b_hi = (uint32_t)(desc_b >> 32), b_lo = (uint32_t)desc_b + ((uint32_t)args.a_bytes >> 4);
+    constexpr uint32_t b_next = kNMajor ? kUmmaK * 128 / 16 : kUmmaK * 2 / 16;   // 16 steps along K
     const uint32_t desc_hi = (uint32_t)(desc0 >> 32), desc_lo = (uint32_t)desc0;
-    const uint32_t stage_step = (uint32_t)args.stage_bytes >> 4, b_step = (uint32_t)args.a_bytes >> 4;
+    const uint32_t stage_step = (uint32_t)args.stage_bytes >> 4;
     const int last_nk = (args.K - (args.k_blocks - 1) * kBK + kUmmaK - 1) / kUmmaK;
     int stage = 0, acc = 0;
     uint32_t phase = 0, acc_phase = 0;
@@ -334,7 +340,7 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
           if (!mbar_wait_warp(ready, &bar_full[stage], phase, abort_flag, args.status)) { alive = false; break; }
           if (kMode != kDense) fence_generic_to_async();
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t lo = desc_lo + (uint32_t)stage * stage_step;
+          const uint32_t lo = desc_lo + (uint32_t)stage * stage_step, lo_b = b_lo + (uint32_t)stage * stage_step;
           const int nk = kb + 1 < args.k_blocks ? kBK / kUmmaK : last_nk;
           uint64_t *empty = &bar_empty[stage];
           if (++stage == stages) { stage = 0; phase ^= 1u; }
@@ -343,7 +349,7 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
 #pragma unroll
             for (int k = 0; k < kBK / kUmmaK; k++) {
               if (k < nk) {
-                const uint64_t db = umma_desc_at(desc_hi, lo + b_step + k * (kUmmaK * 2 / 16));
+                const uint64_t db = umma_desc_at(b_hi, lo_b + k * b_next);
 #pragma unroll
                 for (int h = 0; h < kSub; h++)                 // one weight tile, all sub-tiles
                   umma_f16(tmem_d + (uint32_t)(h * args.n_pad),
@@ -436,7 +442,12 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
           if (elect_one()) {
             mbar_expect_tx(full, b_bytes + (kMode == kDense ? (uint32_t)args.a_bytes : 0u));
             if (kMode == kDense) tma_load_2d(sb - args.a_bytes, &map_a, kb * kBK, tile * kBM, full);
-            tma_load_3d(sb, &map_b, kb * kBK, 0, widx, full);
+            if (kNMajor) {
+              for (int n = 0; n < args.n_pad; n += 64)
+                tma_load_3d(sb + n / 64 * kNBlock, &map_b, n, kb * kBK, widx, full);
+            } else {
+              tma_load_3d(sb, &map_b, kb * kBK, 0, widx, full);
+            }
           }
           __syncwarp();
         }
@@ -466,7 +477,7 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
     // Row of the output (and of the residual) that this lane's accumulator row belongs to, per
     // sub-tile (-1: none): requested two tiles ahead, so that the residual rows of the next tile
     // can be on their way to L2 while this one is worked on.
-    const bool permuted = kMode == kMap && args.perm != nullptr;
+    const bool permuted = kMode <= kMapNMajor && args.perm != nullptr;
     auto table_row = [&](int tile, int h) { return ((int64_t)tile * kSub + h) * kBM + quarter * 32 + lane; };
     auto request_rows = [&](int tile, int32_t (&rows)[kSub]) {
 #pragma unroll
@@ -939,9 +950,20 @@ extern "C" mn_status mn_sparse_convolution_forward_implicit(
                "implicit forward: feature arrays and the neighbour table must be 16-byte aligned");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const bool bf16 = dtype == MN_BF16;
+  // Weights that were not transposed once are read as they are, as N-major tiles, where a call has
+  // few steps: the transposition is a launch of 3 to 10 us, an N-major step a little slower than a
+  // K-major one.  With fewer than two pairs a row the MMAs wait for the rest anyway (464k rows
+  // 64->64, 1.15 pairs: 56.3 -> 53.8 us; 168k rows 64->128, 1.4 pairs: 23.4 -> 20.5 us); up to two
+  // tiles per CTA the launch is what counts (53k rows 256->256: 95.5 -> 92.1 us, 30k rows 32->96:
+  // 13.9 -> 12.0 us); 200k rows 64->64 with 3 pairs and both gradients lose 1 of 115 us.  TMA needs
+  // them on a 16-byte boundary.
   Workspace ws(ws_ptr, ws_bytes);
   const void *weights_t = weights_t_in;
-  if (weights_t == nullptr) {
+  const bool n_major = weights_t == nullptr && (reinterpret_cast<uintptr_t>(weights) & 15) == 0 &&
+                       (pairs_per_row < 2.0 || div_up(T, kBM) <= 4 * kNumSMs);
+  if (n_major) {
+    weights_t = weights;
+  } else if (weights_t == nullptr) {
     char *mine = ws.take<char>(align_up((size_t)O * c_in * c_out * 2, 1024));
     MN_CHECK_WS(ws);
     MN_RETURN_IF(launch_transpose_weights(weights, mine, (int)O, (int)c_in, (int)c_out, bf16, st));
@@ -989,7 +1011,7 @@ extern "C" mn_status mn_sparse_convolution_forward_implicit(
   a.pitch = (int64_t)align_up((size_t)T, kBM);
   a.acc_bufs = 2 * sub * a.n_pad <= 512 ? 2 : 1;
   a.a_bytes = sub * kBM * kBK * 2;
-  a.stage_bytes = a.a_bytes + a.n_pad * kBK * 2;
+  a.stage_bytes = a.a_bytes + (n_major ? (int)div_up(a.n_pad, 64) * kNBlock : a.n_pad * kBK * 2);
   const TcSizing sizing = size_tc_kernel(a.stage_bytes, a.acc_bufs * sub * a.n_pad, kMaxStages, kImCtas, kIdxSlots * kMaxSub * kBM * 4, kMaxStages);
   a.stages = sizing.stages;
   a.tmem_cols = sizing.tmem_cols;
@@ -1001,7 +1023,15 @@ extern "C" mn_status mn_sparse_convolution_forward_implicit(
                                 reinterpret_cast<uintptr_t>(residual)) & 31) == 0;
 
   CUtensorMap map_b;
-  MN_RETURN_IF(make_kmajor_map(&map_b, weights_t, bf16, c_in, c_out, O, a.n_pad));
+  MN_RETURN_IF(n_major ? make_kmajor_map(&map_b, weights_t, bf16, c_out, c_in, O, kBK)
+                       : make_kmajor_map(&map_b, weights_t, bf16, c_in, c_out, O, a.n_pad));
+  if (n_major) {
+    if (sub == 1)
+      return c_in <= 32 ? launch_implicit<1, 4, 4, kMapNMajor>(a, sizing, map_b, map_b, st)
+                        : launch_implicit<1, 8, 4, kMapNMajor>(a, sizing, map_b, map_b, st);
+    return c_in <= 32 ? launch_implicit<2, 4, 8, kMapNMajor>(a, sizing, map_b, map_b, st)
+                      : launch_implicit<2, 8, 8, kMapNMajor>(a, sizing, map_b, map_b, st);
+  }
   if (sub == 1)
     return c_in <= 32 ? launch_implicit<1, 4, 4, kMap>(a, sizing, map_b, map_b, st)
                       : launch_implicit<1, 8, 4, kMap>(a, sizing, map_b, map_b, st);

@@ -93,18 +93,6 @@ constexpr int kWgRows = 64;             // pairs per stage
 constexpr int kWgBlock = kWgRows * 128; // bytes of 64 pairs x 64 channels
 constexpr int kWgMaxStages = 8;
 
-// M/N-major tile with 128-byte swizzle: rows of 128 bytes are K (pairs), 8-row groups 1024
-// bytes apart (stride offset), 64-channel blocks `block` bytes apart (leading offset).
-__device__ __forceinline__ uint64_t mn_major_desc(uint32_t smem_addr, uint32_t block) {
-  uint64_t d = 0;
-  d |= (uint64_t)((smem_addr & 0x3ffffu) >> 4);
-  d |= (uint64_t)(block >> 4) << 16;
-  d |= (uint64_t)(1024 >> 4) << 32;
-  d |= (uint64_t)1 << 46;
-  d |= (uint64_t)2 << 61;
-  return d;
-}
-
 __device__ __forceinline__ void wg_copy_16(uint32_t dst, const void *src, uint32_t src_bytes) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(src_bytes)
                : "memory");

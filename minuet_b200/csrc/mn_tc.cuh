@@ -105,6 +105,18 @@ __device__ __forceinline__ void tma_store_2d(const CUtensorMap *map, int x, int 
                : "memory");
 }
 
+// M/N-major tile with 128-byte swizzle: rows of 128 bytes are K, 8-row groups 1024
+// bytes apart (stride offset), 64-channel blocks `block` bytes apart (leading offset).
+__device__ __forceinline__ uint64_t mn_major_desc(uint32_t smem_addr, uint32_t block) {
+  uint64_t d = 0;
+  d |= (uint64_t)((smem_addr & 0x3ffffu) >> 4);
+  d |= (uint64_t)(block >> 4) << 16;
+  d |= (uint64_t)(1024 >> 4) << 32;
+  d |= (uint64_t)1 << 46;
+  d |= (uint64_t)2 << 61;
+  return d;
+}
+
 // Shared-memory matrix descriptor of a K-major tile with 128-byte swizzle:
 // rows of 128 bytes, 8-row groups 1024 bytes apart.
 __device__ __forceinline__ uint64_t umma_desc(uint32_t smem_addr) {

@@ -88,6 +88,18 @@ inline void check_cuda(cudaError_t e, const char *what) {
   throw py::error_already_set();
 }
 
+// A kernel follows the operand's pointer: one on the host, or on another GPU than `like`, would be
+// an illegal access there.
+void require_device(const Tensor &t, const Tensor &like, const char *what) {
+  if (!t.is_cuda()) not_on_gpu();
+  if (t.get_device() != like.get_device())
+    throw std::runtime_error(std::string(what) + " must be on the device of its input (cuda:" +
+                             std::to_string(like.get_device()) + ") but is on cuda:" + std::to_string(t.get_device()));
+}
+void require_device(const OptTensor &t, const Tensor &like, const char *what) {
+  if (t.has_value() && t->defined()) require_device(*t, like, what);
+}
+
 // ---------------------------------------------------------------------------
 // memory, streams
 // ---------------------------------------------------------------------------
@@ -264,6 +276,7 @@ std::shared_ptr<Offsets> make_offsets(const std::vector<std::vector<int32_t>> &r
 std::pair<std::shared_ptr<KeyLayout>, Tensor> root_keys(const Tensor &coords, const OptTensor &batch_dims,
                                                         int64_t num_clouds, int margin) {
   if (!coords.is_cuda()) not_on_gpu();
+  require_device(batch_dims, coords, "batch_dims");
   c10::cuda::CUDAGuard guard(coords.get_device());
   auto layout = std::make_shared<KeyLayout>();
   layout->dev = empty_on(coords, {256}, at::kByte);
@@ -280,6 +293,7 @@ std::pair<std::shared_ptr<KeyLayout>, Tensor> root_keys(const Tensor &coords, co
 
 Tensor pack_keys(const Tensor &coords, const OptTensor &batch_dims, KeyLayout &layout) {
   if (!coords.is_cuda()) not_on_gpu();
+  require_device(batch_dims, coords, "batch_dims");
   c10::cuda::CUDAGuard guard(coords.get_device());
   Tensor keys = empty_on(coords, {coords.size(0)}, at::kLong);
   const int64_t nb = batch_dims.has_value() ? batch_dims->numel() - 1 : 1;
@@ -325,6 +339,7 @@ std::tuple<Tensor, Tensor, Tensor, std::vector<int64_t>> downsample(const Tensor
                                                                     const std::vector<int32_t> &tstride,
                                                                     KeyLayout &layout) {
   if (!coords.is_cuda()) not_on_gpu();
+  require_device(batch_dims, coords, "batch_dims");
   c10::cuda::CUDAGuard guard(coords.get_device());
   const int64_t n = coords.size(0), ndim = coords.size(1);
   const int64_t nb = batch_dims.has_value() ? batch_dims->numel() - 1 : 1;
@@ -354,13 +369,14 @@ std::optional<std::tuple<Tensor, Tensor, OptTensor, OptTensor>> voxelize(const T
                                                                          const OptTensor &features_in) {
   at::NoGradGuard no_grad;
   if (!points_in.is_cuda()) not_on_gpu();
+  require_device(batch_dims, points_in, "batch_dims");
+  require_device(features_in, points_in, "features");
   c10::cuda::CUDAGuard guard(points_in.get_device());
   const Tensor points = points_in.contiguous();
   const int64_t n = points.size(0), ndim = points.size(1);
   const int64_t nb = batch_dims.has_value() ? batch_dims->numel() - 1 : 1;
   OptTensor features, means, inv;
   if (features_in.has_value()) {
-    if (!features_in->is_cuda()) not_on_gpu();
     features = features_in->contiguous();
     means = empty_on(*features, {n, features->size(1)}, features->scalar_type());
   }

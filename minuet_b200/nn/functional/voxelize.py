@@ -30,8 +30,10 @@ def voxelize(coordinates: torch.Tensor, voxel_size, batch_dims: Optional[torch.T
     """
     if coordinates.ndim != 2:
         raise ValueError(f"coordinates must be [N, D] but found {coordinates.ndim}-D")
+    engine.require_cuda(coordinates, batch_dims)
     if features is not None and (features.ndim != 2 or features.shape[0] != coordinates.shape[0]):
         raise ValueError("features must be [N, C] with one row per point")
+    engine.require_cuda(features)
     native = _native(coordinates, voxel_size, batch_dims, return_inverse, features)
     if native is not None:
         return native
@@ -52,7 +54,6 @@ def voxelize(coordinates: torch.Tensor, voxel_size, batch_dims: Optional[torch.T
         inverse[index] = run_ids
         result.append(inverse)
     if features is not None:
-        engine.require_cuda(features)
         feats = features.contiguous()
         means = torch.empty((unique.shape[0], feats.shape[1]), dtype=feats.dtype,
                             device=feats.device)

@@ -680,9 +680,32 @@ Tensor run_forward(Plan &plan, bool swapped, Tensor x, Tensor w, const Tensor &s
   return out;
 }
 
-// Shapes, types and layouts that every forward needs; the messages are the reference's.
-void check_operands(const Plan &plan, bool swapped, const Tensor &x, const Tensor &w) {
+// Per-channel factors and sums of an epilogue.
+void check_channels(const OptTensor &v, const Tensor &like, int64_t c_out, const char *what) {
+  if (!v.has_value()) return;
+  require_device(v, like, what);
+  if (v->numel() < c_out)
+    throw std::runtime_error(std::string(what) + " must have one value per output channel (" + std::to_string(c_out) +
+                             ") but has " + std::to_string(v->numel()));
+}
+
+void check_transposed(const OptTensor &w_t, const Tensor &w) {
+  if (!w_t.has_value()) return;
+  require_device(w_t, w, "weights_t");
+  if (w_t->numel() != w.numel() || w_t->scalar_type() != w.scalar_type() || !w_t->is_contiguous())
+    throw std::runtime_error("weights_t must be transpose_weights(weights)");
+}
+
+// Devices, shapes, types and layouts that every forward needs; the messages are the reference's.
+void check_operands(const Plan &plan, bool swapped, const Tensor &x, const Tensor &w, const Tensor &sm,
+                    const Tensor &tm, const OptTensor &order) {
   if (!x.is_cuda()) not_on_gpu();
+  require_device(w, x, "weights");
+  require_device(sm, x, "source_masks");
+  require_device(tm, x, "target_masks");
+  require_device(order, x, "kernel_map_order");
+  if (order.has_value() && order->numel() < plan.O)
+    throw std::runtime_error("kernel_map_order must have one entry per offset (" + std::to_string(plan.O) + ")");
   if (w.dim() != 3) throw std::runtime_error("weights must be a 3-D tensor but found " + std::to_string(w.dim()) + "-D");
   if (w.size(0) != plan.O)
     throw std::runtime_error("source_masks, weights and kernel_map_sizes must have one row per offset (" +
@@ -707,10 +730,14 @@ Tensor conv_forward(const PlanPtr &plan, bool swapped, const Tensor &x, const Te
                     const Tensor &tm, const OptTensor &order, const OptTensor &w_t, const OptTensor &scale,
                     const OptTensor &shift, const OptTensor &residual, const ConvOptions &o) {
   at::NoGradGuard no_grad;
-  check_operands(*plan, swapped, x, w);
+  check_operands(*plan, swapped, x, w, sm, tm, order);
+  check_transposed(w_t, w);
+  check_channels(scale, x, w.size(2), "scale");
+  check_channels(shift, x, w.size(2), "shift");
   c10::cuda::CUDAGuard guard(x.get_device());
   OptTensor res;
   if (residual.has_value()) {
+    require_device(residual, x, "residual");
     res = residual->contiguous();
     const int64_t T = swapped ? plan->S : plan->T;
     if (res->dim() != 2 || res->size(0) != T || res->size(1) != w.size(2) || res->scalar_type() != w.scalar_type())
@@ -806,7 +833,7 @@ struct Convolution : torch::autograd::Function<Convolution> {
 
 Tensor conv_autograd(const PlanPtr &plan, bool swapped, const Tensor &x, const Tensor &w, const Tensor &sm,
                      const Tensor &tm, const OptTensor &order, const ConvOptions &o) {
-  check_operands(*plan, swapped, x, w);
+  check_operands(*plan, swapped, x, w, sm, tm, order);
   auto holder = c10::make_intrusive<PlanHolder>();
   holder->plan = plan;
   holder->options = o;
@@ -821,6 +848,18 @@ std::pair<Tensor, bool> dense_forward(const Tensor &features_in, const Tensor &w
                                       const OptTensor &w_t) {
   at::NoGradGuard no_grad;
   if (!features_in.is_cuda()) not_on_gpu();
+  require_device(weight_in, features_in, "weight");
+  if (features_in.dim() != 2 || weight_in.dim() != 2 || features_in.size(1) != weight_in.size(0))
+    throw std::runtime_error("features must be [N, C_in] and weight [C_in, C_out]");
+  check_transposed(w_t, weight_in);
+  check_channels(scale, features_in, weight_in.size(1), "scale");
+  check_channels(shift, features_in, weight_in.size(1), "shift");
+  if (residual.has_value()) {
+    require_device(residual, features_in, "residual");
+    if (residual->numel() != features_in.size(0) * weight_in.size(1) ||
+        residual->scalar_type() != features_in.scalar_type())
+      throw std::runtime_error("residual must be [N, C_out] in the feature dtype");
+  }
   c10::cuda::CUDAGuard guard(features_in.get_device());
   const Tensor features = features_in.contiguous(), weight = weight_in.contiguous();
   const int64_t rows = features.size(0), c_in = features.size(1), c_out = weight.size(1);

@@ -201,7 +201,7 @@ def sparse_convolution_forward_fused(sources: torch.Tensor, weights: torch.Tenso
 def apply_epilogue(features: torch.Tensor, scale=None, shift=None, residual=None,
                    relu: bool = False) -> torch.Tensor:
     """In place ``features = relu?(features * scale[c] + shift[c] + residual)``."""
-    engine.require_cuda(features)
+    engine.require_cuda(features, scale, shift, residual)
     rows, channels = features.shape
     _lib.check(engine.lib().mn_apply_epilogue(
         engine.ptr(features), rows, channels, engine.dtype_code(features.dtype),

@@ -90,7 +90,7 @@ typedef struct {
 /* Version of this interface; mn_version() returns the value the library was
  * built with.  A binding should refuse a library whose version differs from the
  * header it was written against: argument lists change between versions. */
-#define MN_ABI_VERSION 18
+#define MN_ABI_VERSION 19
 
 const char *mn_last_error(void);
 int mn_version(void);
@@ -169,6 +169,14 @@ mn_status mn_arg_sort_coordinates_by_dimension(const int32_t *coords, int64_t n,
                                                const int64_t *batch_dims, int64_t num_clouds,
                                                int64_t *index_out, int32_t *ctrl, void *ws,
                                                size_t ws_bytes, void *stream);
+
+/* Stable order of 64-bit keys by their low `bits` bits; bits + ceil(log2 n) (at least 1) must not
+ * exceed 64.  wait_limit: polls after which a block stops waiting for the counts of earlier
+ * blocks (0: the library's own limit of some seconds); status bit 4 is then set and the order is
+ * invalid, but every entry of index_out is in [0, n).  Workspace: mn_map_workspace_bytes(n, n, 1). */
+mn_status mn_arg_sort_keys(const uint64_t *keys, int64_t n, int bits, uint32_t wait_limit,
+                           int64_t *index_out, int32_t *status_dev, void *ws, size_t ws_bytes,
+                           void *stream);
 
 /* _C.cuda_unique_coordinates / _C.cuda_multi_unique_coordinates
  * (csrc/minuet/torch/cuda_unique_coordinates.cu:8-81) on SORTED coordinates:

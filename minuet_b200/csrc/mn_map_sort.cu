@@ -293,7 +293,7 @@ unique_keys_kernel(const __grid_constant__ UniqueKeysArgs a) {
       const uint32_t pos = run + s_cnt[j][warp] + __popc(votes[j] & lt);   // openers before key i
       const bool opens = ((votes[j] >> lane) & 1u) != 0u;
       if (a.inverse != nullptr && i < c1)
-        a.inverse[k[j] & index_mask] = (int64_t)(opens ? pos : pos - 1u);
+        a.inverse[rsort::index_of(k[j], index_mask, a.n)] = (int64_t)(opens ? pos : pos - 1u);
       if (opens) {
         const uint64_t key = k[j] >> ib;
         if (a.keys_out != nullptr) a.keys_out[pos] = key;
@@ -416,6 +416,38 @@ extern "C" mn_status mn_arg_sort_coordinates(const int32_t *coords, int64_t n, i
     a.vals[0] = vals; a.vals[1] = vals_tmp;    // the index does not fit below the key
   }
   return rsort::run(a, k, ws, st);
+}
+
+namespace mn {
+struct GivenKeys {
+  const uint64_t *keys;
+  int32_t index_bits;
+  __device__ __forceinline__ int layout() const { return 0; }
+  __device__ __forceinline__ uint64_t operator()(int64_t i, int, int &) const {
+    return (__ldg(keys + i) << index_bits) | (uint64_t)i;
+  }
+};
+}  // namespace mn
+
+extern "C" mn_status mn_arg_sort_keys(const uint64_t *keys_in, int64_t n, int bits, uint32_t wait_limit,
+                                      int64_t *index_out, int32_t *status_dev, void *ws_ptr, size_t ws_bytes,
+                                      void *stream) {
+  MN_CHECK_ARG(n >= 0 && n < (1ll << 31) - 1, "arg_sort_keys: bad n");
+  if (n == 0) return MN_OK;
+  MN_CHECK_ARG(bits >= 1 && bits + rsort::bits_for(n) <= 64, "arg_sort_keys: the index does not fit below the key");
+  MN_CHECK_ARG(keys_in != nullptr && index_out != nullptr && status_dev != nullptr, "arg_sort_keys: null pointer");
+  Workspace ws(ws_ptr, ws_bytes);
+  rsort::Args a{};
+  a.keys[0] = ws.take<uint64_t>(n);
+  a.keys[1] = ws.take<uint64_t>(n);
+  MN_CHECK_WS(ws);
+  a.n = n;
+  a.first_bit = rsort::bits_for(n);
+  a.bits = bits;
+  a.wait_limit = wait_limit;
+  a.status = status_dev;
+  a.index64 = index_out;
+  return rsort::run(a, GivenKeys{keys_in, a.first_bit}, ws, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" mn_status mn_arg_sort_coordinates_by_dimension(
@@ -630,7 +662,7 @@ voxel_run_mean_kernel(const T *__restrict__ features, int channels, int lanes, c
     for (int c0 = part * 4; c0 < channels; c0 += lanes * 4) {
       float acc[4] = {0.f, 0.f, 0.f, 0.f};
       for (int64_t j = begin; j < end; j++) {
-        const T *row = features + (int64_t)(__ldg(keys + j) & mask) * channels + c0;
+        const T *row = features + rsort::index_of(__ldg(keys + j), mask, n) * channels + c0;
 #pragma unroll
         for (int k = 0; k < 4; k++)
           if (c0 + k < channels) acc[k] += vm_to_f32<T>(row[k]);

@@ -46,6 +46,7 @@ struct Args {
   int32_t *result_in_second;  // out (may be NULL): 1 when the result is in keys[1]
   int32_t *status;            // device status word
   int32_t tiles;
+  uint32_t wait_limit;        // polls of the look-back before it gives up; 0: kSpinLimit
   // the last pass may write the index (low `first_bit` bits of the key, or vals) instead of keys
   int32_t *index32;
   int64_t *index64;
@@ -55,6 +56,11 @@ __device__ __forceinline__ int passes_of(const Args &a) {
   const int bits = a.bits >= 0 ? a.bits : spec_of(a.spec).total_bits;
   const int p = (bits + kBits - 1) / kBits;
   return p < 1 ? 1 : (p > kMaxPasses ? kMaxPasses : p);
+}
+
+// The row that the low bits of a sorted key name.
+__device__ __forceinline__ int64_t index_of(uint64_t key, uint64_t mask, int64_t n) {
+  return min((int64_t)(key & mask), n - 1);
 }
 
 __device__ __forceinline__ unsigned lanes_below() {
@@ -93,6 +99,9 @@ sort_keys_kernel(const __grid_constant__ Args a, const __grid_constant__ Source 
       if (i[j] < end) {
         a.keys[0][i[j]] = key[j];
         if (a.vals[0] != nullptr) a.vals[0][i[j]] = (int32_t)i[j];
+        // slots that a timed-out pass leaves out must hold an index all the same
+        if (a.index32 != nullptr) a.index32[i[j]] = (int32_t)i[j];
+        if (a.index64 != nullptr) a.index64[i[j]] = i[j];
       }
     }
     for (int p = 0; p < passes; p++) {
@@ -210,7 +219,7 @@ sort_pass_kernel(const __grid_constant__ Args a, int pass) {
       const uint64_t v = state[(size_t)prev * kPairs];
       const uint32_t x = (uint32_t)v, y = (uint32_t)(v >> 32);
       if (x == 0u) {
-        if (++spins > kSpinLimit) { atomicOr(a.status, MN_STATUS_GRID_TIMEOUT); break; }
+        if (++spins > a.wait_limit) { atomicOr(a.status, MN_STATUS_GRID_TIMEOUT); break; }
         continue;
       }
       before.x += (x - 1u) >> 1;
@@ -246,11 +255,13 @@ sort_pass_kernel(const __grid_constant__ Args a, int pass) {
     const int i = j * kThreads + tid;
     if (i < in_tile) {
       const uint64_t k = s_key[i];
-      // a timed-out look-back (status bit 4) must not write outside the arrays
+      // After a look-back that timed out (status bit 4) keys may land on one another and leave
+      // slots of the output with what the buffer held before: positions stay inside the arrays here,
+      // and so does every index that is read out of a key, here and in the kernels that follow.
       dest[j] = min(s_dest[(unsigned)(k >> shift) & (kDigits - 1)] + (uint32_t)i, (uint32_t)a.n - 1u);
       if (!write_index) kout[dest[j]] = k;
-      else if (!kVals && a.index32 != nullptr) a.index32[dest[j]] = (int32_t)(k & index_mask);
-      else if (!kVals) a.index64[dest[j]] = (int64_t)(k & index_mask);
+      else if (!kVals && a.index32 != nullptr) a.index32[dest[j]] = (int32_t)index_of(k, index_mask, a.n);
+      else if (!kVals) a.index64[dest[j]] = index_of(k, index_mask, a.n);
     }
   }
   if (kVals) {
@@ -270,7 +281,7 @@ sort_pass_kernel(const __grid_constant__ Args a, int pass) {
     for (int j = 0; j < kItems; j++) {
       const int i = j * kThreads + tid;
       if (i < in_tile) {
-        const int32_t v = s_val[i];
+        const int32_t v = (int32_t)min((uint32_t)s_val[i], (uint32_t)a.n - 1u);
         if (!write_index) vout[dest[j]] = v;
         else if (a.index32 != nullptr) a.index32[dest[j]] = v;
         else a.index64[dest[j]] = v;
@@ -312,6 +323,7 @@ template <typename Source>
 mn_status run(Args a, const Source &source, Workspace &ws, cudaStream_t st) {
   MN_CHECK_ARG(a.n > 0 && a.n < (1ll << 31) - 1, "radix sort: n = %lld exceeds 2^31-2", (long long)a.n);
   a.tiles = (int32_t)tiles_of(a.n);
+  if (a.wait_limit == 0) a.wait_limit = kSpinLimit;
   // bits that only the device knows: no more than fit above the index
   const int bits = a.bits >= 0 ? a.bits : 64 - a.first_bit;
   const int launches = std::min(kMaxPasses, std::max(1, (bits + kBits - 1) / kBits));

@@ -609,6 +609,12 @@ Tensor zero_channels(const Tensor &t, int64_t dim, int64_t pad) {
   return out;
 }
 
+// TMA reads transposed weights, from a 16-byte boundary; off one the call transposes its own (a
+// weight that is a view into a flat parameter buffer, its own transpose in the backward pass).
+void drop_misaligned(OptTensor &w_t) {
+  if (w_t.has_value() && (reinterpret_cast<uintptr_t>(w_t->data_ptr()) & 15) != 0) w_t = std::nullopt;
+}
+
 Tensor run_forward(Plan &plan, bool swapped, Tensor x, Tensor w, const Tensor &sm, const Tensor &tm,
                    const OptTensor &order, OptTensor w_t, const OptTensor &scale, const OptTensor &shift,
                    const OptTensor &residual, const ConvOptions &o) {
@@ -624,6 +630,7 @@ Tensor run_forward(Plan &plan, bool swapped, Tensor x, Tensor w, const Tensor &s
     w = zero_channels(w, 1, pad);
     w_t = std::nullopt;
   }
+  drop_misaligned(w_t);
   const int64_t c_in = w.size(1);
   const auto &sizes = plan.sizes();
   const int choice = pick_algorithm(plan, swapped, c_in, c_out, code, o);
@@ -845,13 +852,14 @@ Tensor conv_autograd(const PlanPtr &plan, bool swapped, const Tensor &x, const T
 // ---------------------------------------------------------------------------
 std::pair<Tensor, bool> dense_forward(const Tensor &features_in, const Tensor &weight_in, const OptTensor &scale,
                                       const OptTensor &shift, const OptTensor &residual, bool relu,
-                                      const OptTensor &w_t) {
+                                      OptTensor w_t) {
   at::NoGradGuard no_grad;
   if (!features_in.is_cuda()) not_on_gpu();
   require_device(weight_in, features_in, "weight");
   if (features_in.dim() != 2 || weight_in.dim() != 2 || features_in.size(1) != weight_in.size(0))
     throw std::runtime_error("features must be [N, C_in] and weight [C_in, C_out]");
   check_transposed(w_t, weight_in);
+  drop_misaligned(w_t);
   check_channels(scale, features_in, weight_in.size(1), "scale");
   check_channels(shift, features_in, weight_in.size(1), "shift");
   if (residual.has_value()) {

@@ -248,13 +248,18 @@ conv_simt_kernel(const __grid_constant__ CsArgs a) {
             store4(out + r * a.N + c, make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]));
         }
       }
+      // A row without this offset multiplied zeros: nothing to add, and a NaN where a weight is not
+      // finite, which must not reach it.
+      const int32_t *idx = s_idx + ((entry >> 8) & 0xff) * BM + warp * kRows + ty;
 #pragma unroll
-      for (int i = 0; i < 8; i++)
+      for (int i = 0; i < 8; i++) {
+        const bool present = idx[i * (kRows / 8)] >= 0;
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-          sum[i][j] += acc[i][j];
+          if (present) sum[i][j] += acc[i][j];
           acc[i][j] = 0.f;
         }
+      }
     }
   }
 

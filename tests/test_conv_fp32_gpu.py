@@ -52,3 +52,28 @@ def test_same_bits_as_gather_gemm_scatter(n, c_in, c_out, kernel, stride):
     ref = torch.relu(want.double() * scale + shift + res)
     bound = 2.0 ** -22 * ((want * scale).abs() + shift.abs() + res.abs()) + 1e-30
     assert bool(((fused.double() - ref).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("n,c_in,c_out", [(900, 16, 24), (60_000, 16, 24), (20_000, 8, 70)])
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+def test_weights_that_are_not_finite_reach_their_pairs_only(n, c_in, c_out, value):
+    rng = np.random.default_rng(n)
+    src, _ = synth.random_small_batch(rng, 1, n, max(2, round((n / 0.25) ** (1 / 3))))
+    c = torch.as_tensor(src, device=DEV)
+    x = torch.as_tensor(rng.standard_normal((len(src), c_in)).astype(np.float32), device=DEV)
+    conv = minuet.nn.SparseConv3d(c_in, c_out, 3, device=DEV)
+    cache = minuet.nn.KernelMapCache(ndim=3, dtype=torch.int32, device=DEV)
+    minuet.set_kernel_map_cache(conv, cache)
+    sm, tm, order, sizes = cache.get_kernel_map(c, 1, None, c, 1, None, 3, 1)
+    clean = conv(minuet.SparseTensor(x, c)).F
+    conv.kernel[5, 3, 4] = value
+    out = conv(minuet.SparseTensor(x, c)).F
+    row = int((order == 5).nonzero())                   # mask row of offset 5
+    hit = tm[row] >= 0
+    assert bool(hit.any()) and not bool(hit.all())
+    bad = torch.zeros_like(out, dtype=torch.bool)
+    bad[hit, 4] = True                                  # no feature is zero: inf or NaN in every one
+    assert torch.equal(~torch.isfinite(out), bad)
+    assert torch.equal(out[~bad], clean[~bad])
+    assert torch.equal(torch.nan_to_num(out), torch.nan_to_num(
+        explicit(x, conv.kernel.detach(), sm, tm, order, engine.host_copy(sizes), True)))

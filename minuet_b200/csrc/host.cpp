@@ -794,6 +794,15 @@ Tensor weight_gradient(Plan &plan, bool swapped, const Tensor &x, const Tensor &
   return grad;
 }
 
+// Counts the writes into tensors that a backward pass will read again (tensors made in inference
+// mode, which cannot be saved for one, keep no count).
+std::vector<int64_t> versions_of(const Tensor &sm, const Tensor &tm, const OptTensor &order) {
+  std::vector<int64_t> v;
+  for (const Tensor &t : {sm, tm, order.value_or(Tensor())})
+    v.push_back(!t.defined() || t.is_inference() ? 0 : (int64_t)t._version());
+  return v;
+}
+
 struct Convolution : torch::autograd::Function<Convolution> {
   static Tensor forward(torch::autograd::AutogradContext *ctx, const Tensor &x_in, const Tensor &w_in,
                         const Tensor &sm, const Tensor &tm, const OptTensor &order, bool swapped,
@@ -804,6 +813,7 @@ struct Convolution : torch::autograd::Function<Convolution> {
     ctx->save_for_backward({x, w});
     ctx->saved_data["masks"] = std::vector<Tensor>{sm, tm};
     if (order.has_value()) ctx->saved_data["order"] = *order;
+    ctx->saved_data["versions"] = versions_of(sm, tm, order);
     ctx->saved_data["swapped"] = swapped;
     ctx->saved_data["plan"] = c10::IValue::make_capsule(holder);
     return run_forward(*holder->plan, swapped, x, w, sm, tm, order, std::nullopt, std::nullopt, std::nullopt,
@@ -820,6 +830,9 @@ struct Convolution : torch::autograd::Function<Convolution> {
     OptTensor order;
     const auto it = ctx->saved_data.find("order");
     if (it != ctx->saved_data.end()) order = it->second.toTensor();
+    if (ctx->saved_data["versions"].toIntVector() != versions_of(sm, tm, order))
+      throw std::runtime_error("one of the variables needed for gradient computation has been modified by an inplace "
+                               "operation: the kernel map of a sparse convolution");
     const bool swapped = ctx->saved_data["swapped"].toBool();
     auto holder = c10::static_intrusive_pointer_cast<PlanHolder>(ctx->saved_data["plan"].toCapsule());
     Plan &plan = *holder->plan;

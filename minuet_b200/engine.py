@@ -227,19 +227,28 @@ def pack_keys(coords: torch.Tensor, batch_dims: Optional[torch.Tensor], spec: Ke
 # plans of kernel maps (csrc/host.cpp:Plan): pair counts on the host, hit words,
 # neighbour tables and pair lists, kept for as long as the mask tensors live
 # ---------------------------------------------------------------------------
-_plans = {}        # id(masks) or id(sizes) -> (weak reference, plan, side)
-_foreign = {}      # (id(source masks), id(target masks)) of maps built elsewhere -> the same
-_host_copies = {}  # id(tensor) -> (weak reference, numpy values)
+_plans = {}        # id(masks) or id(sizes) -> (weak reference, version, plan, side)
+_foreign = {}      # (id(source masks), id(target masks)) of other maps -> (both references, versions, plan)
+_host_copies = {}  # id(tensor) -> (weak reference, version, numpy values)
 _SOURCE, _TARGET, _SIZES = range(3)
+
+
+def version(*tensors):
+    """Changes whenever one of ``tensors`` is written in place (None for tensors made in inference
+    mode, which keep no count)."""
+    try:
+        return [t._version for t in tensors]
+    except RuntimeError:
+        return None
 
 
 def _remember(t: torch.Tensor, plan, side: int):
     key = id(t)
-    _plans[key] = (weakref.ref(t, lambda _r, k=key: _plans.pop(k, None)), plan, side)
+    _plans[key] = (weakref.ref(t, lambda _r, k=key: _plans.pop(k, None)), version(t), plan, side)
 
 
 def remember_plan(source_masks, target_masks, sizes, plan):
-    """Find ``plan`` again by the tensors of its map."""
+    """Find ``plan`` again by the tensors of its map, as long as nobody writes into them."""
     _remember(source_masks, plan, _SOURCE)
     _remember(target_masks, plan, _TARGET)
     _remember(sizes, plan, _SIZES)
@@ -247,45 +256,55 @@ def remember_plan(source_masks, target_masks, sizes, plan):
 
 def _entry(t: torch.Tensor):
     hit = _plans.get(id(t))
-    return hit if hit is not None and hit[0]() is t else None
+    return hit if hit is not None and hit[0]() is t and hit[1] == version(t) else None
 
 
 def plan_of(source_masks: torch.Tensor, target_masks: torch.Tensor, sizes):
-    """``(plan, swapped)`` of the map that two int32 mask tensors describe; ``swapped`` when
-    they are the map's own with the sides exchanged.  Masks that did not come from this
-    engine get a plan on first use (``sizes``: their pair counts, a tensor or host values)."""
+    """``(plan, swapped)`` of the map that two int32 mask tensors and its pair counts (a tensor or
+    host values) describe; ``swapped`` when the masks are the map's own with the sides exchanged.
+    Masks that did not come from this engine, or were written to since, get a plan of their own on
+    first use; it serves until one of them is written to or other counts come with them."""
     s, t = _entry(source_masks), _entry(target_masks)
-    if s is not None and t is not None and s[1] is t[1] and s[2] != t[2]:
-        return s[1], s[2] == _TARGET
+    own = s is not None and t is not None and s[2] is t[2] and s[3] != t[3]
+    if own and isinstance(sizes, torch.Tensor):
+        z = _entry(sizes)
+        if z is not None and z[2] is s[2]:        # the map's own counts: no wait for their copy here
+            return s[2], s[3] == _TARGET
+    values = host_copy(sizes, np.int32) if isinstance(sizes, torch.Tensor) else np.asarray(sizes)
+    values = values.tolist()
+    if own and s[2].sizes() == values:
+        return s[2], s[3] == _TARGET
     key = (id(source_masks), id(target_masks))
+    versions = version(source_masks, target_masks)
     hit = _foreign.get(key)
-    if hit is not None and hit[0]() is source_masks and hit[1]() is target_masks:
-        return hit[2], False
+    if hit is not None and hit[0]() is source_masks and hit[1]() is target_masks and \
+            hit[2] == versions and hit[3].sizes() == values:
+        return hit[3], False
     plan = _lib.host().Plan(source_masks.shape[0], source_masks.shape[1], target_masks.shape[1])
-    values = host_copy(sizes, np.int32) if isinstance(sizes, torch.Tensor) else sizes
-    plan.set_sizes(np.asarray(values).tolist())
+    plan.set_sizes(values)
 
-    def drop(_ref, k=key):
-        _foreign.pop(k, None)
+    def drop(ref, k=key):
+        if k in _foreign and any(r is ref for r in _foreign[k][:2]):
+            del _foreign[k]
 
-    _foreign[key] = (weakref.ref(source_masks, drop), weakref.ref(target_masks, drop), plan)
+    _foreign[key] = (weakref.ref(source_masks, drop), weakref.ref(target_masks, drop), versions, plan)
     return plan, False
 
 
 def remember_host(t: torch.Tensor, values: np.ndarray):
     key = id(t)
-    _host_copies[key] = (weakref.ref(t, lambda _r, k=key: _host_copies.pop(k, None)), values)
+    _host_copies[key] = (weakref.ref(t, lambda _r, k=key: _host_copies.pop(k, None)), version(t), values)
 
 
 def host_copy(t: torch.Tensor, dtype=np.int32) -> np.ndarray:
     """Host values of ``t``: the remembered copy when the tensor came from this
     engine, otherwise a blocking device-to-host read."""
     entry = _entry(t)
-    if entry is not None and entry[2] == _SIZES:
-        return np.asarray(entry[1].sizes(), dtype=dtype)
+    if entry is not None and entry[3] == _SIZES:
+        return np.asarray(entry[2].sizes(), dtype=dtype)
     hit = _host_copies.get(id(t))
-    if hit is not None and hit[0]() is t:
-        return np.ascontiguousarray(np.asarray(hit[1]).astype(dtype, copy=False))
+    if hit is not None and hit[0]() is t and hit[1] == version(t):
+        return np.ascontiguousarray(np.asarray(hit[2]).astype(dtype, copy=False))
     return np.ascontiguousarray(t.detach().cpu().numpy().astype(dtype, copy=False))
 
 
@@ -293,9 +312,9 @@ def hit_bits(masks: torch.Tensor) -> Optional[torch.Tensor]:
     """Hit words (bit p set <=> mask row p has an entry for the row) of a mask tensor that
     came from the fused map build, else None."""
     entry = _entry(masks)
-    if entry is None or entry[2] == _SIZES:
+    if entry is None or entry[3] == _SIZES:
         return None
-    return entry[1].source_bits if entry[2] == _SOURCE else entry[1].target_bits
+    return entry[2].source_bits if entry[3] == _SOURCE else entry[2].target_bits
 
 
 def neighbor_table(source_masks: torch.Tensor, target_masks: torch.Tensor,

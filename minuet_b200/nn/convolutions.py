@@ -478,19 +478,21 @@ class SparseConv(Module):
             coordinates, stride, batch_dims = cache.get_target_coordinates(
                 source_coordinates=inputs.C, source_batch_dims=inputs.batch_dims,
                 source_stride=inputs.stride, kernel_stride=self.stride, transposed=self.transposed)
-            source_masks, target_masks, order, sizes = cache.get_kernel_map(
+            maps = cache.get_kernel_map(
                 source_coordinates=inputs.C, source_stride=inputs.stride,
                 source_batch_dims=inputs.batch_dims, target_coordinates=coordinates,
                 target_stride=stride, target_batch_dims=batch_dims, kernel_size=self.kernel_size,
                 kernel_dilation=self.dilation, transposed=self.transposed)
-            plan, swapped = engine.plan_of(source_masks, target_masks, sizes)
-            hit = (coordinates, stride, batch_dims, source_masks, target_masks, order, sizes, plan, swapped)
+            hit = (coordinates, stride, batch_dims, *maps, None, None, ())
+        versions = engine.version(hit[3], hit[4], hit[6])
+        if versions != hit[9]:      # the first time, and when somebody wrote into the map since
+            hit = (*hit[:7], *engine.plan_of(hit[3], hit[4], hit[6]), versions)
             cache._layers[key] = hit
         if self._tuning_data is not None:
-            _, _, _, source_masks, target_masks, order, sizes, _, _ = hit
+            source_masks, target_masks, order, sizes = hit[3:7]
             self._tuning_data.append((source_masks, target_masks, sizes))
             self._tuning_maps.append((source_masks, target_masks, order, sizes))
-        return hit
+        return hit[:9]
 
     def _options(self, relu: bool = False):
         """The call options of this layer in native form (made once per configuration)."""

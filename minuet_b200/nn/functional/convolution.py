@@ -155,8 +155,8 @@ def sparse_convolution_forward(sources: torch.Tensor,
     del parallel
     engine.require_cuda(sources)
     sm, tm, order = _i32(source_masks), _i32(target_masks), _i32(kernel_map_order)
-    _prepare(weights, sm, tm, kernel_map_sizes)
-    plan, swapped = engine.plan_of(sm, tm, kernel_map_sizes)
+    sizes_host = _prepare(weights, sm, tm, kernel_map_sizes)[-1]
+    plan, swapped = engine.plan_of(sm, tm, sizes_host)
     options = native_options(gather_tile_size, scatter_tile_size, allow_shortcut_matmul, threshold,
                              algorithm, sub_tiles, False)
     return run(plan, swapped, sources, weights, sm, tm, order, options, weights_t)
@@ -190,8 +190,8 @@ def sparse_convolution_forward_fused(sources: torch.Tensor, weights: torch.Tenso
     pass over the output."""
     engine.require_cuda(sources)
     sm, tm, order = _i32(source_masks), _i32(target_masks), _i32(kernel_map_order)
-    _prepare(weights, sm, tm, kernel_map_sizes)
-    plan, swapped = engine.plan_of(sm, tm, kernel_map_sizes)
+    sizes_host = _prepare(weights, sm, tm, kernel_map_sizes)[-1]
+    plan, swapped = engine.plan_of(sm, tm, sizes_host)
     options = native_options(gather_tile_size, scatter_tile_size, allow_shortcut_matmul, threshold,
                              algorithm, sub_tiles, relu)
     return run_fused(plan, swapped, sources, weights, sm, tm, order, options, weights_t, scale,

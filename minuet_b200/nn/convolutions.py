@@ -61,6 +61,12 @@ class KernelMapCache(object):
         self._root_keys = None
         self._root = None
 
+    def __getstate__(self):
+        """A copy starts with the tables that a key layout and native objects are not part of."""
+        if self._spec is not None:
+            raise ValueError("a KernelMapCache that holds keys and maps cannot be copied: reset() it first")
+        return {**self.__dict__, "_offsets_cache": dict(), "_layers": dict()}
+
     def _get_kernel_offsets(self, source_stride, kernel_size, kernel_dilation):
         """The offset table of a geometry, as an array and in native form."""
         key = (source_stride, kernel_size, kernel_dilation)
@@ -253,6 +259,7 @@ class SparseConv(Module):
     __AVAILABLE_THRESHOLD__ = [-1, 0.0, 0.5, None]
     __AVAILABLE_SUB_TILES__ = [1, 2, 3, 4]
     __NUM_TUNING_ROUNDS__ = 10
+    _native_options = None      # the call options in native form, with what they were made from
 
     def __init__(self, ndim: int, in_channels: int, out_channels: int, kernel_size,
                  stride=1, dilation=1, bias: bool = False, transposed: bool = False,
@@ -287,8 +294,10 @@ class SparseConv(Module):
         self._tuning_maps = None
         self._tuning_epilogue = (False, False, False, False)
         self._frozen_kernel_t = None
-        self._native_options = None
         self._trivial = all(v == 1 for v in self.stride + self.dilation + self.kernel_size)
+
+    def __getstate__(self):
+        return {k: v for k, v in self.__dict__.items() if k != "_native_options"}
 
     def reset_parameters(self):
         """Uniform init in ``+-1/sqrt(fan * K^D)`` with ``fan`` the input channels

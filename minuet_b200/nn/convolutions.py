@@ -272,7 +272,6 @@ class SparseConv(Module):
         self.stride = as_tuple(stride, size=ndim, name="stride")
         self.dilation = as_tuple(dilation, size=ndim, name="dilation")
         self.transposed = transposed
-        self._geometry = (self.kernel_size, self.stride, self.dilation, transposed)
         volume = int(np.prod(self.kernel_size))
         self.kernel = torch.nn.Parameter(
             torch.empty(volume, in_channels, out_channels, dtype=dtype, device=device))
@@ -294,7 +293,6 @@ class SparseConv(Module):
         self._tuning_maps = None
         self._tuning_epilogue = (False, False, False, False)
         self._frozen_kernel_t = None
-        self._trivial = all(v == 1 for v in self.stride + self.dilation + self.kernel_size)
 
     def __getstate__(self):
         return {k: v for k, v in self.__dict__.items() if k != "_native_options"}
@@ -336,7 +334,8 @@ class SparseConv(Module):
 
     @property
     def is_trivial(self) -> bool:
-        return self._trivial
+        sizes = self.stride + self.dilation + self.kernel_size
+        return sizes.count(1) == len(sizes)
 
     @property
     def _allow_shortcut_matmul(self) -> bool:
@@ -481,7 +480,7 @@ class SparseConv(Module):
         cache = self._kernel_map_cache
         if cache is None:
             raise ValueError("Kernel map cache must be specified")
-        key = (inputs.stride, self._geometry)
+        key = (inputs.stride, self.kernel_size, self.stride, self.dilation, self.transposed)
         hit = cache._layers.get(key)
         if hit is None:
             coordinates, stride, batch_dims = cache.get_target_coordinates(
@@ -508,7 +507,7 @@ class SparseConv(Module):
         c = self._tunable_config
         key = (conv_functional.ALGORITHM, conv_functional.IMPLICIT_SUB_TILES,
                conv_functional.REORDER_ROWS, c.get("algorithm"), c.get("sub_tiles"),
-               c["gather_tile_size"], c["scatter_tile_size"], c["threshold"],
+               c["gather_tile_size"], c["scatter_tile_size"], c["threshold"], self.stride, self.dilation,
                self._kernel_map_cache._disable_reordering, relu)
         if self._native_options is None or self._native_options[0] != key:
             self._native_options = (key, conv_functional.native_options(

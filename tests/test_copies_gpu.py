@@ -68,3 +68,19 @@ def test_a_cache_in_use_is_not_copied():
     for copying in (copy.deepcopy, pickle.dumps):
         with pytest.raises(ValueError, match="reset"):
             copying(maps)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+def test_a_layer_whose_geometry_is_changed(dtype):
+    """What a layer looks up follows its attributes, not those it was made with."""
+    x = _input(dtype)
+    conv = minuet.nn.SparseConv3d(8, 8, 3, dtype=dtype, device=DEV)
+    minuet.set_kernel_map_cache(conv, _cache())
+    conv(x)
+    for size, stride, dilation in (((2, 2, 2), (1, 1, 1), (1, 1, 1)), ((3, 1, 1), (1, 1, 1), (2, 1, 1)),
+                                   ((2, 2, 2), (2, 2, 2), (1, 1, 1)), ((1, 1, 1), (1, 1, 1), (1, 1, 1))):
+        made = minuet.nn.SparseConv3d(8, 8, size, stride=stride, dilation=dilation, dtype=dtype, device=DEV)
+        minuet.set_kernel_map_cache(made, _cache())
+        conv.kernel_size, conv.stride, conv.dilation, conv.kernel = size, stride, dilation, made.kernel
+        want, got = made(x), conv(x)
+        assert torch.equal(got.F, want.F) and torch.equal(got.C, want.C) and got.stride == want.stride

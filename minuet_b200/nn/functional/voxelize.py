@@ -4,6 +4,7 @@ __all__ = ['voxelize']
 
 from typing import Optional
 
+import numpy as np
 import torch
 
 from minuet_b200 import _lib, engine
@@ -75,7 +76,13 @@ def _native(coordinates, voxel_size, batch_dims, return_inverse, features):
     if features is not None and (features.shape[1] == 0 or features.dtype not in (
             torch.float32, torch.float16, torch.bfloat16)):
         return None
-    sizes = [float(v) for v in (voxel_size if hasattr(voxel_size, "__len__") else (voxel_size,))]
+    # one size or one per dimension; whatever else broadcasts, or is refused, goes step by step
+    try:
+        if np.ndim(voxel_size) > 1:
+            return None
+        sizes = [float(v) for v in (voxel_size if hasattr(voxel_size, "__len__") else (voxel_size,))]
+    except (TypeError, ValueError):
+        return None
     if len(sizes) == 1:
         sizes = sizes * ndim
     if len(sizes) != ndim:

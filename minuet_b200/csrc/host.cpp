@@ -759,16 +759,28 @@ Tensor conv_forward(const PlanPtr &plan, bool swapped, const Tensor &x, const Te
 // ---------------------------------------------------------------------------
 // With pairs (s, t) under offset k: out[t] += x[s] W[k], hence dx[s] += dout[t] W[k]^T -- the
 // same convolution with the two sides exchanged and every weight matrix transposed, run by the
-// same kernels -- and dW[k] = sum over the pairs of x[s]^T dout[t].
+// same kernels -- and dW[k] = sum over the pairs of x[s]^T dout[t].  Both are differentiable in turn:
+// a backward pass that keeps a graph (create_graph) is made of the same two functions, the gradients
+// of dW under u being dx[s] += dout[t] u[k]^T and ddout[t] += x[s] u[k].
 struct PlanHolder : torch::CustomClassHolder {
   PlanPtr plan;
   ConvOptions options;
 };
+using Holder = c10::intrusive_ptr<PlanHolder>;
 
-Tensor weight_gradient(Plan &plan, bool swapped, const Tensor &x, const Tensor &g, const Tensor &w, const Tensor &sm,
+Holder flipped(const Holder &holder) {
+  auto other = c10::make_intrusive<PlanHolder>();
+  other->plan = holder->plan;
+  other->options = holder->options;
+  std::swap(other->options.gather_tile, other->options.scatter_tile);
+  return other;
+}
+
+Tensor weight_gradient(Plan &plan, bool swapped, const Tensor &x, const Tensor &g, const Tensor &sm,
                        const Tensor &tm, const OptTensor &order) {
   const int64_t O = plan.O, S = swapped ? plan.T : plan.S, T = swapped ? plan.S : plan.T;
-  const mn_dtype code = dtype_code(w.scalar_type());
+  const int64_t c_in = x.size(1), c_out = g.size(1);
+  const mn_dtype code = dtype_code(x.scalar_type());
   const auto &sizes = plan.sizes();
   const cudaStream_t st = stream_of(x);
   Plan::Lock lock(plan.mutex);
@@ -785,71 +797,119 @@ Tensor weight_gradient(Plan &plan, bool swapped, const Tensor &x, const Tensor &
   }
   const int32_t *src = raw<int32_t>(plan.lists), *dst = src + plan.lists.size(1);
   if (swapped) std::swap(src, dst);
-  Tensor grad = at::empty(w.sizes(), w.options().requires_grad(false));
-  Tensor ws = workspace(x, api.mn_weight_gradient_workspace_bytes(sizes.data(), O, w.size(1), w.size(2), code));
-  check(api.mn_sparse_convolution_weight_gradient(S, T, O, w.size(1), w.size(2), code, x.data_ptr(), g.data_ptr(),
+  Tensor grad = empty_on(x, {O, c_in, c_out}, x.scalar_type());
+  Tensor ws = workspace(x, api.mn_weight_gradient_workspace_bytes(sizes.data(), O, c_in, c_out, code));
+  check(api.mn_sparse_convolution_weight_gradient(S, T, O, c_in, c_out, code, x.data_ptr(), g.data_ptr(),
                                                   src, dst, raw<int32_t>(order), sizes.data(), grad.data_ptr(),
                                                   ctrl_of(x), ws.data_ptr(), (size_t)ws.numel(), st),
         "sparse_convolution_weight_gradient");
   return grad;
 }
 
-// Counts the writes into tensors that a backward pass will read again (tensors made in inference
-// mode, which cannot be saved for one, keep no count).
-std::vector<int64_t> versions_of(const Tensor &sm, const Tensor &tm, const OptTensor &order) {
-  std::vector<int64_t> v;
-  for (const Tensor &t : {sm, tm, order.value_or(Tensor())})
-    v.push_back(!t.defined() || t.is_inference() ? 0 : (int64_t)t._version());
-  return v;
-}
+// What a function keeps of a kernel map for its backward pass.  The masks are no saved variables
+// (those made in inference mode cannot be), so writes into them are counted here.
+struct MapRef {
+  Tensor sm, tm;
+  OptTensor order;
+  bool swapped;
+  Holder holder;
 
-struct Convolution : torch::autograd::Function<Convolution> {
-  static Tensor forward(torch::autograd::AutogradContext *ctx, const Tensor &x_in, const Tensor &w_in,
-                        const Tensor &sm, const Tensor &tm, const OptTensor &order, bool swapped,
-                        c10::intrusive_ptr<PlanHolder> holder) {
-    at::AutoDispatchBelowADInplaceOrView below;
-    const Tensor x = x_in.contiguous(), w = w_in.contiguous();
-    c10::cuda::CUDAGuard guard(x.get_device());
-    ctx->save_for_backward({x, w});
+  std::vector<int64_t> versions() const {
+    std::vector<int64_t> v;
+    for (const Tensor &t : {sm, tm, order.value_or(Tensor())})
+      v.push_back(!t.defined() || t.is_inference() ? 0 : (int64_t)t._version());
+    return v;
+  }
+  void save(torch::autograd::AutogradContext *ctx) const {
     ctx->saved_data["masks"] = std::vector<Tensor>{sm, tm};
     if (order.has_value()) ctx->saved_data["order"] = *order;
-    ctx->saved_data["versions"] = versions_of(sm, tm, order);
+    ctx->saved_data["versions"] = versions();
     ctx->saved_data["swapped"] = swapped;
     ctx->saved_data["plan"] = c10::IValue::make_capsule(holder);
+  }
+  static MapRef load(torch::autograd::AutogradContext *ctx) {
+    const auto masks = ctx->saved_data["masks"].toTensorVector();
+    MapRef m{masks[0], masks[1], std::nullopt, ctx->saved_data["swapped"].toBool(),
+             c10::static_intrusive_pointer_cast<PlanHolder>(ctx->saved_data["plan"].toCapsule())};
+    const auto it = ctx->saved_data.find("order");
+    if (it != ctx->saved_data.end()) m.order = it->second.toTensor();
+    if (ctx->saved_data["versions"].toIntVector() != m.versions())
+      throw std::runtime_error("one of the variables needed for gradient computation has been modified by an inplace "
+                               "operation: the kernel map of a sparse convolution");
+    return m;
+  }
+};
+
+struct WeightGradient : torch::autograd::Function<WeightGradient> {
+  static Tensor forward(torch::autograd::AutogradContext *ctx, const Tensor &x, const Tensor &g, const Tensor &sm,
+                        const Tensor &tm, const OptTensor &order, bool swapped, Holder holder);
+  static torch::autograd::variable_list backward(torch::autograd::AutogradContext *ctx,
+                                                 torch::autograd::variable_list grads);
+};
+
+struct Convolution : torch::autograd::Function<Convolution> {
+  static Tensor forward(torch::autograd::AutogradContext *ctx, const Tensor &x, const Tensor &w,
+                        const Tensor &sm, const Tensor &tm, const OptTensor &order, bool swapped, Holder holder) {
+    at::AutoDispatchBelowADInplaceOrView below;
+    c10::cuda::CUDAGuard guard(x.get_device());
+    ctx->save_for_backward({x, w});
+    MapRef{sm, tm, order, swapped, holder}.save(ctx);
     return run_forward(*holder->plan, swapped, x, w, sm, tm, order, std::nullopt, std::nullopt, std::nullopt,
                        std::nullopt, holder->options);
   }
   static torch::autograd::variable_list backward(torch::autograd::AutogradContext *ctx,
                                                  torch::autograd::variable_list grads) {
-    at::AutoDispatchBelowADInplaceOrView below;
     const auto saved = ctx->get_saved_variables();
     const Tensor &x = saved[0], &w = saved[1];
     c10::cuda::CUDAGuard guard(x.get_device());
-    const auto masks = ctx->saved_data["masks"].toTensorVector();
-    const Tensor &sm = masks[0], &tm = masks[1];
-    OptTensor order;
-    const auto it = ctx->saved_data.find("order");
-    if (it != ctx->saved_data.end()) order = it->second.toTensor();
-    if (ctx->saved_data["versions"].toIntVector() != versions_of(sm, tm, order))
-      throw std::runtime_error("one of the variables needed for gradient computation has been modified by an inplace "
-                               "operation: the kernel map of a sparse convolution");
-    const bool swapped = ctx->saved_data["swapped"].toBool();
-    auto holder = c10::static_intrusive_pointer_cast<PlanHolder>(ctx->saved_data["plan"].toCapsule());
-    Plan &plan = *holder->plan;
-    const Tensor g = grads[0].to(w.scalar_type()).contiguous();
+    const MapRef m = MapRef::load(ctx);
     Tensor grad_x, grad_w;
-    if (ctx->needs_input_grad(0)) {
-      ConvOptions o = holder->options;
-      std::swap(o.gather_tile, o.scatter_tile);
-      // [O, c_out, c_in] weights; their transpose, which the tensor-core kernels read, is w
-      grad_x = run_forward(plan, !swapped, g, w.transpose(1, 2).contiguous(), tm, sm, order,
-                           w.scalar_type() == at::kFloat ? OptTensor() : OptTensor(w), std::nullopt, std::nullopt,
-                           std::nullopt, o);
+    if (at::GradMode::is_enabled()) {
+      const Tensor g = grads[0].to(w.scalar_type()).contiguous();
+      if (ctx->needs_input_grad(0))
+        grad_x = Convolution::apply(g, w.transpose(1, 2).contiguous(), m.tm, m.sm, m.order, !m.swapped,
+                                    flipped(m.holder));
+      if (ctx->needs_input_grad(1))
+        grad_w = WeightGradient::apply(x, g, m.sm, m.tm, m.order, m.swapped, m.holder);
+      return {grad_x, grad_w, Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
     }
-    if (ctx->needs_input_grad(1)) grad_w = weight_gradient(plan, swapped, x, g, w, sm, tm, order);
+    at::AutoDispatchBelowADInplaceOrView below;
+    Plan &plan = *m.holder->plan;
+    const Tensor g = grads[0].to(w.scalar_type()).contiguous();
+    if (ctx->needs_input_grad(0)) {
+      // [O, c_out, c_in] weights; their transpose, which the tensor-core kernels read, is w
+      grad_x = run_forward(plan, !m.swapped, g, w.transpose(1, 2).contiguous(), m.tm, m.sm, m.order,
+                           w.scalar_type() == at::kFloat ? OptTensor() : OptTensor(w), std::nullopt, std::nullopt,
+                           std::nullopt, flipped(m.holder)->options);
+    }
+    if (ctx->needs_input_grad(1)) grad_w = weight_gradient(plan, m.swapped, x, g, m.sm, m.tm, m.order);
     return {grad_x, grad_w, Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
   }
 };
+
+Tensor WeightGradient::forward(torch::autograd::AutogradContext *ctx, const Tensor &x, const Tensor &g,
+                               const Tensor &sm, const Tensor &tm, const OptTensor &order, bool swapped,
+                               Holder holder) {
+  at::AutoDispatchBelowADInplaceOrView below;
+  c10::cuda::CUDAGuard guard(x.get_device());
+  ctx->save_for_backward({x, g});
+  MapRef{sm, tm, order, swapped, holder}.save(ctx);
+  return weight_gradient(*holder->plan, swapped, x, g, sm, tm, order);
+}
+
+torch::autograd::variable_list WeightGradient::backward(torch::autograd::AutogradContext *ctx,
+                                                        torch::autograd::variable_list grads) {
+  const auto saved = ctx->get_saved_variables();
+  const Tensor &x = saved[0], &g = saved[1];
+  c10::cuda::CUDAGuard guard(x.get_device());
+  const MapRef m = MapRef::load(ctx);
+  const Tensor u = grads[0].to(x.scalar_type()).contiguous();
+  Tensor grad_x, grad_g;
+  if (ctx->needs_input_grad(0))
+    grad_x = Convolution::apply(g, u.transpose(1, 2).contiguous(), m.tm, m.sm, m.order, !m.swapped, flipped(m.holder));
+  if (ctx->needs_input_grad(1)) grad_g = Convolution::apply(x, u, m.sm, m.tm, m.order, m.swapped, m.holder);
+  return {grad_x, grad_g, Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
+}
 
 Tensor conv_autograd(const PlanPtr &plan, bool swapped, const Tensor &x, const Tensor &w, const Tensor &sm,
                      const Tensor &tm, const OptTensor &order, const ConvOptions &o) {
@@ -857,7 +917,7 @@ Tensor conv_autograd(const PlanPtr &plan, bool swapped, const Tensor &x, const T
   auto holder = c10::make_intrusive<PlanHolder>();
   holder->plan = plan;
   holder->options = o;
-  return Convolution::apply(x, w, sm, tm, order, swapped, holder);
+  return Convolution::apply(x.contiguous(), w.contiguous(), sm, tm, order, swapped, holder);
 }
 
 // ---------------------------------------------------------------------------

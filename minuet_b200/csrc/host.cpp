@@ -8,6 +8,8 @@
 // of interpreter and ctypes work, a kernel map 98; from here 14 and 48.
 #include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDACachingAllocator.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <cuda_runtime_api.h>
@@ -403,6 +405,40 @@ std::optional<std::tuple<Tensor, Tensor, OptTensor, OptTensor>> voxelize(const T
 // ---------------------------------------------------------------------------
 // plans of kernel maps
 // ---------------------------------------------------------------------------
+// Device memory that a plan makes on first use belongs to the stream of the call that made it: calls on
+// other streams wait until it is there, and the allocator does not hand it out again before
+// they are through.  (A capture begins on an idle device and may not wait for work outside itself.)
+bool capturing() {
+  return c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None;
+}
+
+class Made {
+ public:
+  Made() = default;
+  Made(const Made &) = delete;
+  ~Made() {
+    if (event_ != nullptr) (void)cudaEventDestroy(event_);
+  }
+  void here(int device) {
+    device_ = device;
+    stream_ = c10::cuda::getCurrentCUDAStream(device).stream();
+    check_cuda(cudaEventCreateWithFlags(&event_, cudaEventDisableTiming), "plan");
+    check_cuda(cudaEventRecord(event_, stream_), "plan");
+  }
+  void join(std::initializer_list<Tensor> memory) const {
+    const c10::cuda::CUDAStream now = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)device_);
+    if (event_ == nullptr || now.stream() == stream_ || capturing()) return;
+    check_cuda(cudaStreamWaitEvent(now.stream(), event_, 0), "plan");
+    for (const Tensor &t : memory)
+      if (t.defined()) c10::cuda::CUDACachingAllocator::recordStream(t.storage().data_ptr(), now);
+  }
+
+ private:
+  int device_ = 0;
+  cudaStream_t stream_ = nullptr;
+  cudaEvent_t event_ = nullptr;
+};
+
 struct Neighbours {
   Tensor nbr, tile_bits, perm;
 };
@@ -413,9 +449,12 @@ struct Neighbours {
 struct Plan {
   int64_t O = 0, S = 0, T = 0;
   Tensor bits_s, bits_t;                 // hit words of the two sides (undefined: none)
+  // what calls have made so far (a call inside a stream capture keeps nothing: its work is not done
+  // before the graph is replayed)
   Neighbours nb[2][2];                   // [swapped][rows sorted by hit word]
   Tensor pair_src[2][2];                 // [swapped][shortcut], of the pair-list forward
   Tensor lists;                          // [2, rows]: source and target row of every pair
+  Made nb_made[2][2], pair_src_made[2][2], lists_made;
   int last_algorithm = 0;                // of the last forward: 1 explicit, 2 implicit
   // held while a call looks things up or makes them: a backward pass runs on a thread of its own.
   // Never waited for with the GIL held (its holder may need the GIL to raise).
@@ -505,12 +544,15 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, PlanPtr> build_map(const Tensor &sour
   return {sm, tm, small.narrow(0, 0, O), small.narrow(0, pad(O + 1), O), plan};
 }
 
-const Neighbours &neighbours(Plan &plan, bool swapped, bool reorder, const Tensor &sm, const Tensor &tm) {
+Neighbours neighbours(Plan &plan, bool swapped, bool reorder, const Tensor &sm, const Tensor &tm) {
   const Tensor &sb = swapped ? plan.bits_t : plan.bits_s, &tb = swapped ? plan.bits_s : plan.bits_t;
   const bool sorted = reorder && tb.defined();
   Plan::Lock lock(plan.mutex);
   Neighbours &n = plan.nb[swapped][sorted];
-  if (n.nbr.defined()) return n;
+  if (n.nbr.defined()) {
+    plan.nb_made[swapped][sorted].join({n.nbr, n.tile_bits, n.perm});
+    return n;
+  }
   c10::cuda::CUDAGuard guard(tm.get_device());
   const int64_t O = plan.O, S = swapped ? plan.T : plan.S, T = swapped ? plan.S : plan.T;
   const auto &sizes = plan.sizes();
@@ -525,10 +567,11 @@ const Neighbours &neighbours(Plan &plan, bool swapped, bool reorder, const Tenso
                                     raw<int32_t>(nbr), raw<uint32_t>(tile_bits), raw<int32_t>(perm), ctrl_of(tm),
                                     ws.data_ptr(), (size_t)ws.numel(), stream_of(tm)),
         "build_neighbor_table");
-  n.tile_bits = tile_bits;
-  n.perm = perm;
-  n.nbr = nbr;
-  return n;
+  if (!capturing()) {
+    plan.nb_made[swapped][sorted].here(tm.get_device());
+    n = {nbr, tile_bits, perm};
+  }
+  return {nbr, tile_bits, perm};
 }
 
 // Source row of every product row of the pair-list forward; undefined when the map has no hit words.
@@ -536,14 +579,21 @@ Tensor pair_sources(Plan &plan, bool swapped, bool shortcut, const Tensor &sm) {
   const Tensor &sb = swapped ? plan.bits_t : plan.bits_s;
   if (!sb.defined()) return {};
   Tensor &t = plan.pair_src[swapped][shortcut];
-  if (t.defined()) return t;
+  if (t.defined()) {
+    plan.pair_src_made[swapped][shortcut].join({t});
+    return t;
+  }
   const int64_t O = plan.O, S = swapped ? plan.T : plan.S, T = swapped ? plan.S : plan.T;
   const auto &sizes = plan.sizes();
   Tensor list = empty_on(sm, {std::max<int64_t>(api.mn_pair_rows(sizes.data(), O, S, T, shortcut), 1)}, at::kInt);
   check(api.mn_build_pair_list(raw<int32_t>(sm), raw<uint32_t>(sb), sizes.data(), O, S, T, shortcut,
                                raw<int32_t>(list), stream_of(sm)),
         "build_pair_list");
-  return t = list;
+  if (!capturing()) {
+    plan.pair_src_made[swapped][shortcut].here(sm.get_device());
+    t = list;
+  }
+  return list;
 }
 
 // ---------------------------------------------------------------------------
@@ -642,7 +692,7 @@ Tensor run_forward(Plan &plan, bool swapped, Tensor x, Tensor w, const Tensor &s
   const float *sc = raw<float>(scale), *sh = raw<float>(shift);
   const void *res = raw<void>(residual);
   if (choice == kImplicit) {
-    const Neighbours &n = neighbours(plan, swapped, o.reorder, sm, tm);
+    const Neighbours n = neighbours(plan, swapped, o.reorder, sm, tm);
     const int32_t *perm = raw<int32_t>(n.perm), *nbr = raw<int32_t>(n.nbr);
     const uint32_t *tiles = raw<uint32_t>(n.tile_bits);
     if (code == MN_F32) {
@@ -784,18 +834,24 @@ Tensor weight_gradient(Plan &plan, bool swapped, const Tensor &x, const Tensor &
   const auto &sizes = plan.sizes();
   const cudaStream_t st = stream_of(x);
   Plan::Lock lock(plan.mutex);
-  if (!plan.lists.defined()) {
+  Tensor lists = plan.lists;
+  if (lists.defined()) {
+    plan.lists_made.join({lists});
+  } else {
     // the two lists in the map's own direction
-    Tensor lists = empty_on(sm, {2, std::max<int64_t>(api.mn_pair_list_rows(sizes.data(), O), 1)}, at::kInt);
+    lists = empty_on(sm, {2, std::max<int64_t>(api.mn_pair_list_rows(sizes.data(), O), 1)}, at::kInt);
     const Tensor &s = swapped ? tm : sm, &t = swapped ? sm : tm;
     int32_t *p = raw<int32_t>(lists);
     check(api.mn_build_pair_lists(raw<int32_t>(s), raw<int32_t>(t), raw<uint32_t>(plan.bits_s),
                                   raw<uint32_t>(plan.bits_t), sizes.data(), O, plan.S, plan.T, p,
                                   p + lists.size(1), st),
           "build_pair_lists");
-    plan.lists = lists;
+    if (!capturing()) {
+      plan.lists_made.here(sm.get_device());
+      plan.lists = lists;
+    }
   }
-  const int32_t *src = raw<int32_t>(plan.lists), *dst = src + plan.lists.size(1);
+  const int32_t *src = raw<int32_t>(lists), *dst = src + lists.size(1);
   if (swapped) std::swap(src, dst);
   Tensor grad = empty_on(x, {O, c_in, c_out}, x.scalar_type());
   Tensor ws = workspace(x, api.mn_weight_gradient_workspace_bytes(sizes.data(), O, c_in, c_out, code));
@@ -995,7 +1051,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def_property_readonly("target_bits", [](Plan &p) { return optional(p.bits_t); })
       .def_readonly("last_algorithm", &Plan::last_algorithm)
       .def("neighbours", [](Plan &p, bool swapped, bool reorder, const Tensor &sm, const Tensor &tm) {
-        const Neighbours &n = neighbours(p, swapped, reorder, sm, tm);
+        const Neighbours n = neighbours(p, swapped, reorder, sm, tm);
         return std::make_tuple(n.nbr, n.tile_bits, optional(n.perm));
       }, NoGil());
   m.def("build_map", &build_map, NoGil());

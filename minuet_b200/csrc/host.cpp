@@ -144,6 +144,14 @@ Tensor control_block(int device) {
 }
 inline int32_t *ctrl_of(const Tensor &t) { return static_cast<int32_t *>(control_block(t.get_device()).data_ptr()); }
 
+// Whether the work before an event has ended.  The "not ready" of such a query is no error of this
+// thread; errors that other calls have left are theirs to report.
+bool ended(cudaEvent_t event) {
+  const cudaError_t e = cudaEventQuery(event);
+  if (e == cudaErrorNotReady && cudaPeekAtLastError() == cudaErrorNotReady) (void)cudaGetLastError();
+  return e == cudaSuccess;
+}
+
 // Small pinned buffers with an event each, for device-to-host copies that the host waits for
 // later (or never).  A buffer given back while its copy is still in flight is not handed out
 // before the copy has ended; at most kKeep are kept.
@@ -160,14 +168,13 @@ class PinnedPool {
     {
       std::lock_guard<std::mutex> lock(mutex_);
       for (size_t i = 0; i < free_.size(); i++) {
-        if (free_[i].device == device && cudaEventQuery(free_[i].event) == cudaSuccess) {
+        if (free_[i].device == device && ended(free_[i].event)) {
           Buffer b = free_[i];
           free_.erase(free_.begin() + (long)i);
           return b;
         }
       }
     }
-    (void)cudaGetLastError();   // "not ready" of a query is not an error of this thread
     Buffer b;
     b.device = device;
     check_cuda(cudaHostAlloc(&b.host, kBytes, cudaHostAllocDefault), "pinned buffer");
@@ -208,13 +215,12 @@ int poll_status(int device) {
   static auto *queues = new std::map<int, std::vector<PinnedPool::Buffer>>;
   std::lock_guard<std::mutex> lock(mutex);
   auto &queue = (*queues)[device];
-  while (!queue.empty() && cudaEventQuery(queue.front().event) == cudaSuccess) {
+  while (!queue.empty() && ended(queue.front().event)) {
     const int value = *static_cast<int32_t *>(queue.front().host);
     pinned_pool().give(queue.front());
     queue.erase(queue.begin());
     if (value != 0) return value;
   }
-  (void)cudaGetLastError();   // "not ready" of a query is not an error of this thread
   if (queue.size() < 8) {
     c10::cuda::CUDAGuard guard(device);
     const cudaStream_t st = c10::cuda::getCurrentCUDAStream(device).stream();
@@ -245,10 +251,7 @@ struct KeyLayout {
   }
   void look_for_bits() {
     if (spec.total_bits > 0 || bits_.host == nullptr) return;
-    if (cudaEventQuery(bits_.event) == cudaSuccess)
-      spec.total_bits = *static_cast<int32_t *>(bits_.host);
-    else
-      (void)cudaGetLastError();   // "not ready" of a query is not an error of this thread
+    if (ended(bits_.event)) spec.total_bits = *static_cast<int32_t *>(bits_.host);
   }
 
  private:

@@ -257,7 +257,8 @@ class SparseConv(Module):
     # grouped GEMM takes every offset at its own size, so the key stays in the config
     # (files written by the reference load) and only these few values are ever timed.
     __AVAILABLE_THRESHOLD__ = [-1, 0.0, 0.5, None]
-    __AVAILABLE_SUB_TILES__ = [1, 2, 3, 4]
+    # What the fused kernel exists with (a larger value in a config file runs as the largest).
+    __AVAILABLE_SUB_TILES__ = [1, 2]
     __NUM_TUNING_ROUNDS__ = 10
     _native_options = None      # the call options in native form, with what they were made from
 
@@ -401,10 +402,13 @@ class SparseConv(Module):
     def autotune(self, free_buffers: bool = True):
         """Record the kernel maps this layer sees inside the ``with`` block, then
         time the candidates for ``__NUM_TUNING_ROUNDS__`` rounds each and keep the
-        fastest (minuet/nn/convolutions.py:337-444): for fp32 layers (gather - grouped
-        GEMM - scatter) ``threshold``, ``gather_tile_size`` and ``scatter_tile_size`` as
-        the reference does; for fp16/bf16 layers ``algorithm`` (pair lists against the
-        fused kernel) and the fused kernel's ``sub_tiles``."""
+        fastest (minuet/nn/convolutions.py:337-444): for fp16/bf16 layers ``algorithm``
+        (pair lists against the fused kernel) and the fused kernel's ``sub_tiles``; for
+        layers that run gather - grouped GEMM - scatter (more than 32 offsets, 16-bit
+        channel counts that the tensor-core paths do not take) ``threshold``,
+        ``gather_tile_size`` and ``scatter_tile_size`` as the reference does.  fp32 layers of
+        up to 32 offsets have one kernel and nothing to tune: ``algorithm`` is recorded as
+        "explicit", whose sums that kernel returns bit for bit."""
         try:
             self._tuning_data = list()
             self._tuning_maps = list()
@@ -424,7 +428,8 @@ class SparseConv(Module):
                 c_in = -(-c_in // 8) * 8
             pairs_ok = self.kernel.dtype != torch.float32 and bool(lib.mn_pairs_supported(
                 volume, c_in, self.out_channels, code))
-            if not pairs_ok:
+            one_kernel = self.kernel.dtype == torch.float32 and volume <= 32
+            if not pairs_ok and not one_kernel:
                 self._sweep(F.cuda_time_gemm, self.__AVAILABLE_THRESHOLD__, 'threshold',
                             'threshold', stop_on_error=True)
                 threshold = self._tunable_config['threshold']

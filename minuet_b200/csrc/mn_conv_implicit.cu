@@ -663,7 +663,9 @@ struct CumSizes {
   int64_t cum[MN_MAX_OFFSETS + 1];
 };
 
-// src_of_rank[cum[p] + source_masks[p, s]] = s
+// src_of_rank[cum[p] + source_masks[p, s]] = s.  Masks without hit words are a caller's own: a rank
+// that their sizes have no place for, or that only one side has, makes no pair (the ranks start
+// as -1).
 __global__ void __launch_bounds__(256)
 rank_to_source_kernel(const int32_t *__restrict__ source_masks, int64_t S, int O,
                       const __grid_constant__ CumSizes cs, int32_t *__restrict__ src_of_rank) {
@@ -672,7 +674,7 @@ rank_to_source_kernel(const int32_t *__restrict__ source_masks, int64_t S, int O
   const int64_t gsz = (int64_t)gridDim.x * blockDim.x;
   for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < S; s += gsz) {
     const int m = __ldg(source_masks + (int64_t)p * S + s);
-    if (m >= 0) src_of_rank[cs.cum[p] + m] = (int32_t)s;
+    if (m >= 0 && m < cs.cum[p + 1] - cs.cum[p]) src_of_rank[cs.cum[p] + m] = (int32_t)s;
   }
 }
 
@@ -722,8 +724,10 @@ neighbor_table_kernel(const int32_t *__restrict__ target_masks, int64_t T, int64
     for (uint32_t rest = tile; rest != 0u; rest &= rest - 1u) {
       const int p = __ffs(rest) - 1;
       int v = -1;
-      if ((mine >> p) & 1u)
-        v = __ldg(src_of_rank + cs.cum[p] + __ldg(target_masks + (int64_t)p * T + t));
+      if ((mine >> p) & 1u) {
+        const int m = __ldg(target_masks + (int64_t)p * T + t);
+        if (m >= 0) v = __ldg(src_of_rank + cs.cum[p] + m);
+      }
       nbr[(int64_t)p * pitch + r] = v;
     }
     return;
@@ -733,7 +737,7 @@ neighbor_table_kernel(const int32_t *__restrict__ target_masks, int64_t T, int64
     int v = -1;
     if (r < T) {
       const int m = __ldg(target_masks + (int64_t)p * T + t);
-      if (m >= 0) v = __ldg(src_of_rank + cs.cum[p] + m);
+      if (m >= 0 && m < cs.cum[p + 1] - cs.cum[p]) v = __ldg(src_of_rank + cs.cum[p] + m);
     }
     nbr[(int64_t)p * pitch + r] = v;
     mine |= (v >= 0 ? 1u : 0u) << p;
@@ -907,6 +911,8 @@ extern "C" mn_status mn_build_neighbor_table(const int32_t *source_masks,
     a.index32 = perm_out;
     MN_RETURN_IF(rsort::run(a, HitWordKeys{target_bits, (int32_t)O, a.first_bit, chunk_shift}, ws, st));
   }
+  if (target_bits == nullptr)
+    MN_CHECK_CUDA(cudaMemsetAsync(src_of_rank, 0xff, sizeof(int32_t) * (size_t)std::max<int64_t>(cs.cum[O], 1), st));
   // a scattered 4-byte read costs a 32-byte sector: worth it while the pairs are fewer than
   // an eighth of the mask entries
   if (S > 0 && source_bits != nullptr && cs.cum[O] * 8 < O * S) {

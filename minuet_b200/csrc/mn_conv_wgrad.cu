@@ -78,7 +78,8 @@ pair_side_kernel(const int32_t *__restrict__ masks, const uint32_t *__restrict__
     } else {
       const int p = blockIdx.y;
       const int m = __ldg(masks + (int64_t)p * rows + r);
-      if (m >= 0) list[plan.row_begin[p] + m] = (int32_t)r;
+      // a caller's own masks: a rank beyond the row's list makes no pair
+      if (m >= 0 && m < plan.row_begin[p + 1] - plan.row_begin[p]) list[plan.row_begin[p] + m] = (int32_t)r;
     }
   }
 }

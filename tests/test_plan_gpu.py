@@ -90,3 +90,31 @@ def test_unwritten_maps_keep_their_plan():
     a, b = sm.clone(), tm.clone()
     other = engine.plan_of(a, b, sizes)[0]
     assert other is not plan and engine.plan_of(a, b, sizes)[0] is other
+
+
+@pytest.mark.needs_grad
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+def test_ranks_without_a_partner_make_no_pair(dtype):
+    """A caller's own masks that do not fit together: entries that one side lacks, or that the counts
+    have no place for, are no pairs, and nothing is read through them."""
+    conv, cache, x, coords, (sm, tm, order, sizes) = _layer(dtype)
+    want_s, want_t, a, b = sm.clone(), tm.clone(), sm.clone(), tm.clone()
+    b[3][b[3] == 2] = -1                       # only the source side has rank 2 of row 3
+    want_s[3][sm[3] == 2] = want_t[3][tm[3] == 2] = -1
+    a[4][a[4] == 7] = -1                       # only the target side has rank 7 of row 4
+    want_s[4][sm[4] == 7] = want_t[4][tm[4] == 7] = -1
+    free_s, free_t = (int((m[26] >= 0).logical_and(m[5] < 0).nonzero()[0]) for m in (sm, tm))
+    a[5, free_s] = b[5, free_t] = 1 << 30      # far behind the row's last rank
+    sums = torch.zeros(len(x), 32, device=DEV)
+    for p in range(27):
+        rank = torch.full((len(x),), -1, device=DEV)
+        s = torch.nonzero(want_s[p] >= 0)[:, 0]
+        rank[want_s[p, s].long()] = s
+        t = torch.nonzero(want_t[p] >= 0)[:, 0]
+        sums[t] += x[rank[want_t[p, t].long()]].float() @ conv.kernel[order[p].long()].detach().float()
+    x.requires_grad_()
+    out = F.sparse_convolution_forward(x, conv.kernel, a, b, order, sizes, 1, 1, algorithm="implicit")
+    gx, gw = torch.autograd.grad(out, (x, conv.kernel), torch.ones_like(out))
+    assert torch.equal(out.float(), sums)
+    assert bool(torch.isfinite(gx).all()) and bool(torch.isfinite(gw).all())
+    torch.cuda.synchronize()

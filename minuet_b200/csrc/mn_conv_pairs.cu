@@ -99,8 +99,12 @@ pair_scatter_kernel(const float *__restrict__ products, const int32_t *__restric
       for (int k = 0; k < 8; k++) f[k] += __ldg(shift + c + k);
     }
     if (residual != nullptr) {
-      const uint4 rv = __ldg(reinterpret_cast<const uint4 *>(residual + t * c_out + c));
-      const T *r = reinterpret_cast<const T *>(&rv);
+      const T *r = residual + t * c_out + c;
+      uint4 rv;
+      if ((reinterpret_cast<uintptr_t>(residual) & 15) == 0) {
+        rv = __ldg(reinterpret_cast<const uint4 *>(r));
+        r = reinterpret_cast<const T *>(&rv);
+      }
 #pragma unroll
       for (int k = 0; k < 8; k++) f[k] += to_f32<T>(r[k]);
     }
@@ -205,6 +209,8 @@ extern "C" mn_status mn_sparse_convolution_forward_pairs(
   MN_CHECK_ARG((weights != nullptr || weights_t_in != nullptr) && target_masks != nullptr &&
                    target_bits != nullptr && targets_out != nullptr && status_dev != nullptr &&
                    (S == 0 || sources != nullptr), "pair-list forward: null pointer");
+  MN_CHECK_ARG((reinterpret_cast<uintptr_t>(targets_out) & 15) == 0,
+               "pair-list forward: the output must be 16-byte aligned");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const bool bf16 = dtype == MN_BF16;
   const PairPlan plan = make_pair_plan(sizes_host, O, S, T, allow_shortcut);

@@ -79,3 +79,20 @@ def test_layer_operands_on_the_host_are_refused(dtype):
                 F.sparse_convolution_forward(**good, weights_t=w_t[:5])
         assert torch.equal(F.sparse_convolution_forward(**good, weights_t=w_t), conv(x).F)
     torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("kernel,stride", [(3, 1), (2, 2)])
+def test_a_residual_off_a_16_byte_boundary_on_pair_lists(dtype, kernel, stride):
+    gen = torch.Generator(device=DEV).manual_seed(4)
+    coords = torch.unique(_points(3000).int(), dim=0)
+    conv = minuet.nn.SparseConv3d(16, 24, kernel, stride=stride, dtype=dtype, device=DEV)
+    cache = minuet.nn.KernelMapCache(ndim=3, dtype=torch.int32, device=DEV)
+    minuet.set_kernel_map_cache(conv, cache)
+    conv.tunable_config.update(algorithm="explicit")
+    x = minuet.SparseTensor(torch.randn(len(coords), 16, generator=gen, device=DEV).to(dtype), coords)
+    residual = torch.randn(len(conv(x).F), 24, generator=gen, device=DEV).to(dtype)
+    want = conv.forward_fused(x, residual=residual, relu=True).F
+    for shift in (1, 2, 4):
+        off = torch.empty(residual.numel() + shift, dtype=dtype, device=DEV)[shift:].view_as(residual).copy_(residual)
+        assert torch.equal(conv.forward_fused(x, residual=off, relu=True).F, want)

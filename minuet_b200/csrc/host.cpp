@@ -15,6 +15,7 @@
 #include <cuda_runtime_api.h>
 #include <dlfcn.h>
 #include <torch/csrc/autograd/custom_function.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 #include <torch/csrc/utils/pybind.h>
 #include <torch/custom_class.h>
 
@@ -88,6 +89,12 @@ inline void check_cuda(cudaError_t e, const char *what) {
   py::gil_scoped_acquire gil;
   PyErr_SetString(PyExc_NotImplementedError, "minuet_b200 runs on CUDA tensors only (no CPU path)");
   throw py::error_already_set();
+}
+
+// A trace would record nothing of a call into this module but its result, as a constant.
+void refuse_tracing() {
+  if (torch::jit::tracer::isTracing())
+    throw std::runtime_error("sparse convolutions cannot be traced by torch.jit.trace");
 }
 
 // A kernel follows the operand's pointer: one on the host, or on another GPU than `like`, would be
@@ -790,6 +797,7 @@ Tensor conv_forward(const PlanPtr &plan, bool swapped, const Tensor &x, const Te
                     const Tensor &tm, const OptTensor &order, const OptTensor &w_t, const OptTensor &scale,
                     const OptTensor &shift, const OptTensor &residual, const ConvOptions &o) {
   at::NoGradGuard no_grad;
+  refuse_tracing();
   check_operands(*plan, swapped, x, w, sm, tm, order);
   check_transposed(w_t, w);
   check_channels(scale, x, w.size(2), "scale");
@@ -972,6 +980,7 @@ torch::autograd::variable_list WeightGradient::backward(torch::autograd::Autogra
 
 Tensor conv_autograd(const PlanPtr &plan, bool swapped, const Tensor &x, const Tensor &w, const Tensor &sm,
                      const Tensor &tm, const OptTensor &order, const ConvOptions &o) {
+  refuse_tracing();
   check_operands(*plan, swapped, x, w, sm, tm, order);
   auto holder = c10::make_intrusive<PlanHolder>();
   holder->plan = plan;
@@ -986,6 +995,7 @@ std::pair<Tensor, bool> dense_forward(const Tensor &features_in, const Tensor &w
                                       const OptTensor &shift, const OptTensor &residual, bool relu,
                                       OptTensor w_t) {
   at::NoGradGuard no_grad;
+  refuse_tracing();
   if (!features_in.is_cuda()) not_on_gpu();
   require_device(weight_in, features_in, "weight");
   if (features_in.dim() != 2 || weight_in.dim() != 2 || features_in.size(1) != weight_in.size(0))

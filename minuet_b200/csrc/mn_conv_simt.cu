@@ -21,6 +21,7 @@
 #include "mn_common.cuh"
 
 #include <algorithm>
+#include <type_traits>
 
 namespace mn {
 
@@ -84,6 +85,7 @@ conv_simt_kernel(const __grid_constant__ CsArgs a) {
   extern __shared__ __align__(16) float s_mem[];      // [stages][A | B], then the index blocks
   __shared__ int32_t s_active[kCsMaxOffsets], s_weight[kCsMaxOffsets];
   __shared__ uint8_t s_warps[kCsMaxOffsets];
+  __shared__ uint32_t s_rows[kCsMaxOffsets][BM / 32];   // bit r: row r has this offset
   __shared__ int32_t s_count;
   int32_t *s_idx = reinterpret_cast<int32_t *>(s_mem + kStages * kStageFloats);   // [active][BM]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -112,6 +114,7 @@ conv_simt_kernel(const __grid_constant__ CsArgs a) {
 #pragma unroll
     for (int i = 0; i < BM / 32; i++) {
       const uint32_t hit = __ballot_sync(0xffffffffu, s_idx[j * BM + i * 32 + lane] >= 0);
+      if (lane == 0) s_rows[j][i] = hit;
       if (kRows == 32) warps |= (hit != 0u ? 1u : 0u) << i;
       else warps |= ((hit & 0xffffu) != 0u ? 1u : 0u) << (2 * i) | ((hit >> 16) != 0u ? 2u : 0u) << (2 * i);
     }
@@ -133,6 +136,14 @@ conv_simt_kernel(const __grid_constant__ CsArgs a) {
   const int o_begin = (int)((int64_t)n_all * blockIdx.z / a.splits);
   const int o_end = (int)((int64_t)n_all * (blockIdx.z + 1) / a.splits);
   const int n_step = (o_end - o_begin) * a.k_steps;
+
+  // rows of this warp that an entry's offset has, and whether it lacks some of them anywhere
+  constexpr uint32_t kAll = kRows == 32 ? 0xffffffffu : 0xffffu;
+  auto rows_of = [&](int entry) {
+    return (s_rows[(entry >> 8) & 0xff][warp * kRows / 32] >> (warp * kRows % 32)) & kAll;
+  };
+  const uint32_t lane_rows = lane < n_all ? rows_of(s_active[lane]) : 0u;
+  const bool lacking = __any_sync(0xffffffffu, lane_rows != 0u && lane_rows != kAll);
 
   // the cursor of the copies: offset, first channel, ring stage
   int l_off = o_begin, l_k = 0, l_stage = 0;
@@ -195,71 +206,88 @@ conv_simt_kernel(const __grid_constant__ CsArgs a) {
     }
   };
   float acc[8][4], sum[8][4];
+  auto run = [&](auto select) {
 #pragma unroll
-  for (int i = 0; i < 8; i++)
+    for (int i = 0; i < 8; i++)
 #pragma unroll
-    for (int j = 0; j < 4; j++) acc[i][j] = sum[i][j] = 0.f;
-  for (int s = 0; s < kStages - 1; s++) {
-    if (s < n_step) load_step();
-    else asm volatile("cp.async.commit_group;" ::: "memory");
-  }
-  int off = o_begin, k0 = 0, stage = 0;
-  for (int step = 0; step < n_step; step++) {
-    asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
-    __syncthreads();
-    if (step + kStages - 1 < n_step) load_step();
-    else asm volatile("cp.async.commit_group;" ::: "memory");
-    const float *sb = s_mem + stage * kStageFloats + BM * kCsPitch;
-    const float *sa = s_mem + stage * kStageFloats + (warp * kRows + ty) * kCsPitch;
-    const int entry = s_active[off];
-    const int kmax = min(kCsK, a.K - k0);                  // zeros up to a multiple of 4
-    const bool complete = k0 + kCsK >= a.K;                // the last step of this offset
-    if (++stage == kStages) stage = 0;
-    k0 += kCsK;
-    if (complete) { k0 = 0; off++; }
-    if (((entry >> (16 + warp)) & 1) == 0) continue;      // none of this warp's rows
+      for (int j = 0; j < 4; j++) acc[i][j] = sum[i][j] = 0.f;
+    for (int s = 0; s < kStages - 1; s++) {
+      if (s < n_step) load_step();
+      else asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    int off = o_begin, k0 = 0, stage = 0;
+    for (int step = 0; step < n_step; step++) {
+      asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
+      __syncthreads();
+      if (step + kStages - 1 < n_step) load_step();
+      else asm volatile("cp.async.commit_group;" ::: "memory");
+      const float *sb = s_mem + stage * kStageFloats + BM * kCsPitch;
+      const float *sa = s_mem + stage * kStageFloats + (warp * kRows + ty) * kCsPitch;
+      const int entry = s_active[off];
+      const int kmax = min(kCsK, a.K - k0);                  // zeros up to a multiple of 4
+      const bool complete = k0 + kCsK >= a.K;                // the last step of this offset
+      if (++stage == kStages) stage = 0;
+      k0 += kCsK;
+      if (complete) { k0 = 0; off++; }
+      if (((entry >> (16 + warp)) & 1) == 0) continue;      // none of this warp's rows
 #pragma unroll 2
-    for (int k = 0; k < kmax; k += 4) {
-      float4 av[8], bv[4];
+      for (int k = 0; k < kmax; k += 4) {
+        float4 av[8], bv[4];
 #pragma unroll
-      for (int i = 0; i < 8; i++)
-        av[i] = *reinterpret_cast<const float4 *>(sa + i * (kRows / 8) * kCsPitch + k);
+        for (int i = 0; i < 8; i++)
+          av[i] = *reinterpret_cast<const float4 *>(sa + i * (kRows / 8) * kCsPitch + k);
 #pragma unroll
-      for (int j = 0; j < 4; j++) bv[j] = *reinterpret_cast<const float4 *>(sb + (k + j) * BN + tx * 4);
+        for (int j = 0; j < 4; j++) bv[j] = *reinterpret_cast<const float4 *>(sb + (k + j) * BN + tx * 4);
 #pragma unroll
-      for (int i = 0; i < 8; i++) {
-        const float ak[4] = {av[i].x, av[i].y, av[i].z, av[i].w};
+        for (int i = 0; i < 8; i++) {
+          const float ak[4] = {av[i].x, av[i].y, av[i].z, av[i].w};
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-          acc[i][0] = fmaf(ak[j], bv[j].x, acc[i][0]);
-          acc[i][1] = fmaf(ak[j], bv[j].y, acc[i][1]);
-          acc[i][2] = fmaf(ak[j], bv[j].z, acc[i][2]);
-          acc[i][3] = fmaf(ak[j], bv[j].w, acc[i][3]);
+          for (int j = 0; j < 4; j++) {
+            acc[i][0] = fmaf(ak[j], bv[j].x, acc[i][0]);
+            acc[i][1] = fmaf(ak[j], bv[j].y, acc[i][1]);
+            acc[i][2] = fmaf(ak[j], bv[j].z, acc[i][2]);
+            acc[i][3] = fmaf(ak[j], bv[j].w, acc[i][3]);
+          }
+        }
+      }
+      if (complete) {
+        if (a.products != nullptr) {
+          float *out = a.products + (int64_t)(entry & 0xff) * a.T * a.N;
+#pragma unroll
+          for (int i = 0; i < 8; i++) {
+            const int64_t r = r0 + warp * kRows + ty + i * (kRows / 8);
+            if (c < a.N && r < a.T)
+              store4(out + r * a.N + c, make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]));
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+          const bool add = !decltype(select)::value || ((rows_of(entry) >> (ty + i * (kRows / 8))) & 1u) != 0u;
+#pragma unroll
+          for (int j = 0; j < 4; j++) {
+            if (add) sum[i][j] += acc[i][j];
+            acc[i][j] = 0.f;
+          }
         }
       }
     }
-    if (complete) {
-      if (a.products != nullptr) {
-        float *out = a.products + (int64_t)(entry & 0xff) * a.T * a.N;
+  };
+  // A row of a warp that lacks an offset multiplies zeros, which adds NaN to it where a weight is not
+  // finite.  Such a NaN must not reach it, and a select per row and offset costs 4 % of a dense
+  // layer: a block whose sums end with a NaN, and where some rows lack an offset, runs once more
+  // with the select.  (Products that go to the buffer are picked by row when they are added.)
+  run(std::false_type());
+  if (a.products == nullptr) {
+    bool bad = false;
+    if (lacking) {
 #pragma unroll
-        for (int i = 0; i < 8; i++) {
-          const int64_t r = r0 + warp * kRows + ty + i * (kRows / 8);
-          if (c < a.N && r < a.T)
-            store4(out + r * a.N + c, make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]));
-        }
-      }
-      // A row without this offset multiplied zeros: nothing to add, and a NaN where a weight is not
-      // finite, which must not reach it.
-      const int32_t *idx = s_idx + ((entry >> 8) & 0xff) * BM + warp * kRows + ty;
+      for (int i = 0; i < 8; i++)
 #pragma unroll
-      for (int i = 0; i < 8; i++) {
-        const bool present = idx[i * (kRows / 8)] >= 0;
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-          if (present) sum[i][j] += acc[i][j];
-          acc[i][j] = 0.f;
-        }
-      }
+        for (int j = 0; j < 4; j++) bad |= sum[i][j] != sum[i][j];
+    }
+    if (__syncthreads_or(bad)) {
+      l_off = o_begin; l_k = 0; l_stage = 0;
+      run(std::true_type());
     }
   }
 

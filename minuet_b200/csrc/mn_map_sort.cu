@@ -662,7 +662,7 @@ voxel_run_mean_kernel(const T *__restrict__ features, int channels, int lanes, c
     for (int c0 = part * 4; c0 < channels; c0 += lanes * 4) {
       float acc[4] = {0.f, 0.f, 0.f, 0.f};
       for (int64_t j = begin; j < end; j++) {
-        const T *row = features + rsort::index_of(__ldg(keys + j), mask, n) * channels + c0;
+        const T *row = features + (int64_t)rsort::index_of(__ldg(keys + j), mask, n) * channels + c0;
 #pragma unroll
         for (int k = 0; k < 4; k++)
           if (c0 + k < channels) acc[k] += vm_to_f32<T>(row[k]);

@@ -58,9 +58,9 @@ __device__ __forceinline__ int passes_of(const Args &a) {
   return p < 1 ? 1 : (p > kMaxPasses ? kMaxPasses : p);
 }
 
-// The row that the low bits of a sorted key name.
-__device__ __forceinline__ int64_t index_of(uint64_t key, uint64_t mask, int64_t n) {
-  return min((int64_t)(key & mask), n - 1);
+// The row that the low bits of a sorted key name (31 at most).
+__device__ __forceinline__ int32_t index_of(uint64_t key, uint64_t mask, int64_t n) {
+  return (int32_t)min((uint32_t)key & (uint32_t)mask, (uint32_t)n - 1u);
 }
 
 __device__ __forceinline__ unsigned lanes_below() {
@@ -260,7 +260,7 @@ sort_pass_kernel(const __grid_constant__ Args a, int pass) {
       // and so does every index that is read out of a key, here and in the kernels that follow.
       dest[j] = min(s_dest[(unsigned)(k >> shift) & (kDigits - 1)] + (uint32_t)i, (uint32_t)a.n - 1u);
       if (!write_index) kout[dest[j]] = k;
-      else if (!kVals && a.index32 != nullptr) a.index32[dest[j]] = (int32_t)index_of(k, index_mask, a.n);
+      else if (!kVals && a.index32 != nullptr) a.index32[dest[j]] = index_of(k, index_mask, a.n);
       else if (!kVals) a.index64[dest[j]] = index_of(k, index_mask, a.n);
     }
   }

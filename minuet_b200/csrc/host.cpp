@@ -429,22 +429,22 @@ class Made {
   ~Made() {
     if (event_ != nullptr) (void)cudaEventDestroy(event_);
   }
-  void here(int device) {
+  void here(c10::DeviceIndex device) {
     device_ = device;
     stream_ = c10::cuda::getCurrentCUDAStream(device).stream();
     check_cuda(cudaEventCreateWithFlags(&event_, cudaEventDisableTiming), "plan");
     check_cuda(cudaEventRecord(event_, stream_), "plan");
   }
+  bool elsewhere() const { return c10::cuda::getCurrentCUDAStream(device_).stream() != stream_ && !capturing(); }
   void join(std::initializer_list<Tensor> memory) const {
-    const c10::cuda::CUDAStream now = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)device_);
-    if (event_ == nullptr || now.stream() == stream_ || capturing()) return;
+    const c10::cuda::CUDAStream now = c10::cuda::getCurrentCUDAStream(device_);
     check_cuda(cudaStreamWaitEvent(now.stream(), event_, 0), "plan");
     for (const Tensor &t : memory)
       if (t.defined()) c10::cuda::CUDACachingAllocator::recordStream(t.storage().data_ptr(), now);
   }
 
  private:
-  int device_ = 0;
+  c10::DeviceIndex device_ = 0;
   cudaStream_t stream_ = nullptr;
   cudaEvent_t event_ = nullptr;
 };
@@ -560,7 +560,8 @@ Neighbours neighbours(Plan &plan, bool swapped, bool reorder, const Tensor &sm, 
   Plan::Lock lock(plan.mutex);
   Neighbours &n = plan.nb[swapped][sorted];
   if (n.nbr.defined()) {
-    plan.nb_made[swapped][sorted].join({n.nbr, n.tile_bits, n.perm});
+    const Made &made = plan.nb_made[swapped][sorted];
+    if (made.elsewhere()) made.join({n.nbr, n.tile_bits, n.perm});
     return n;
   }
   c10::cuda::CUDAGuard guard(tm.get_device());
@@ -578,7 +579,7 @@ Neighbours neighbours(Plan &plan, bool swapped, bool reorder, const Tensor &sm, 
                                     ws.data_ptr(), (size_t)ws.numel(), stream_of(tm)),
         "build_neighbor_table");
   if (!capturing()) {
-    plan.nb_made[swapped][sorted].here(tm.get_device());
+    plan.nb_made[swapped][sorted].here((c10::DeviceIndex)tm.get_device());
     n = {nbr, tile_bits, perm};
   }
   return {nbr, tile_bits, perm};
@@ -590,7 +591,8 @@ Tensor pair_sources(Plan &plan, bool swapped, bool shortcut, const Tensor &sm) {
   if (!sb.defined()) return {};
   Tensor &t = plan.pair_src[swapped][shortcut];
   if (t.defined()) {
-    plan.pair_src_made[swapped][shortcut].join({t});
+    const Made &made = plan.pair_src_made[swapped][shortcut];
+    if (made.elsewhere()) made.join({t});
     return t;
   }
   const int64_t O = plan.O, S = swapped ? plan.T : plan.S, T = swapped ? plan.S : plan.T;
@@ -600,7 +602,7 @@ Tensor pair_sources(Plan &plan, bool swapped, bool shortcut, const Tensor &sm) {
                                raw<int32_t>(list), stream_of(sm)),
         "build_pair_list");
   if (!capturing()) {
-    plan.pair_src_made[swapped][shortcut].here(sm.get_device());
+    plan.pair_src_made[swapped][shortcut].here((c10::DeviceIndex)sm.get_device());
     t = list;
   }
   return list;
@@ -847,7 +849,7 @@ Tensor weight_gradient(Plan &plan, bool swapped, const Tensor &x, const Tensor &
   Plan::Lock lock(plan.mutex);
   Tensor lists = plan.lists;
   if (lists.defined()) {
-    plan.lists_made.join({lists});
+    if (plan.lists_made.elsewhere()) plan.lists_made.join({lists});
   } else {
     // the two lists in the map's own direction
     lists = empty_on(sm, {2, std::max<int64_t>(api.mn_pair_list_rows(sizes.data(), O), 1)}, at::kInt);
@@ -858,7 +860,7 @@ Tensor weight_gradient(Plan &plan, bool swapped, const Tensor &x, const Tensor &
                                   p + lists.size(1), st),
           "build_pair_lists");
     if (!capturing()) {
-      plan.lists_made.here(sm.get_device());
+      plan.lists_made.here((c10::DeviceIndex)sm.get_device());
       plan.lists = lists;
     }
   }

@@ -261,6 +261,7 @@ class SparseConv(Module):
     __AVAILABLE_SUB_TILES__ = [1, 2]
     __NUM_TUNING_ROUNDS__ = 10
     _native_options = None      # the call options in native form, with what they were made from
+    _native_shape = None        # see _shape
 
     def __init__(self, ndim: int, in_channels: int, out_channels: int, kernel_size,
                  stride=1, dilation=1, bias: bool = False, transposed: bool = False,
@@ -296,7 +297,7 @@ class SparseConv(Module):
         self._frozen_kernel_t = None
 
     def __getstate__(self):
-        return {k: v for k, v in self.__dict__.items() if k != "_native_options"}
+        return {k: v for k, v in self.__dict__.items() if not k.startswith("_native_")}
 
     def reset_parameters(self):
         """Uniform init in ``+-1/sqrt(fan * K^D)`` with ``fan`` the input channels
@@ -333,10 +334,21 @@ class SparseConv(Module):
     def tunable_config(self) -> Dict[str, Any]:
         return self._tunable_config
 
+    def _shape(self):
+        """``(kernel size, stride, dilation, transposed, trivial)``, made again when one of the
+        attributes is replaced."""
+        s = self._native_shape
+        if s is None or s[0] is not self.kernel_size or s[1] is not self.stride or \
+                s[2] is not self.dilation or s[3] is not self.transposed:
+            sizes = self.stride + self.dilation + self.kernel_size
+            s = (self.kernel_size, self.stride, self.dilation, self.transposed, sizes.count(1) == len(sizes))
+            if all(type(v) is tuple for v in s[:3]):
+                self._native_shape = s
+        return s
+
     @property
     def is_trivial(self) -> bool:
-        sizes = self.stride + self.dilation + self.kernel_size
-        return sizes.count(1) == len(sizes)
+        return self._shape()[4]
 
     @property
     def _allow_shortcut_matmul(self) -> bool:
@@ -485,7 +497,7 @@ class SparseConv(Module):
         cache = self._kernel_map_cache
         if cache is None:
             raise ValueError("Kernel map cache must be specified")
-        key = (inputs.stride, self.kernel_size, self.stride, self.dilation, self.transposed)
+        key = (inputs.stride, self._shape())
         hit = cache._layers.get(key)
         if hit is None:
             coordinates, stride, batch_dims = cache.get_target_coordinates(
@@ -497,7 +509,10 @@ class SparseConv(Module):
                 target_stride=stride, target_batch_dims=batch_dims, kernel_size=self.kernel_size,
                 kernel_dilation=self.dilation, transposed=self.transposed)
             hit = (coordinates, stride, batch_dims, *maps, None, None, ())
-        versions = engine.version(hit[3], hit[4], hit[6])
+        try:
+            versions = (hit[3]._version, hit[4]._version, hit[6]._version)
+        except RuntimeError:        # made in inference mode: not counted
+            versions = None
         if versions != hit[9]:      # the first time, and when somebody wrote into the map since
             hit = (*hit[:7], *engine.plan_of(hit[3], hit[4], hit[6]), versions)
             cache._layers[key] = hit
@@ -505,14 +520,14 @@ class SparseConv(Module):
             source_masks, target_masks, order, sizes = hit[3:7]
             self._tuning_data.append((source_masks, target_masks, sizes))
             self._tuning_maps.append((source_masks, target_masks, order, sizes))
-        return hit[:9]
+        return hit
 
     def _options(self, relu: bool = False):
         """The call options of this layer in native form (made once per configuration)."""
         c = self._tunable_config
         key = (conv_functional.ALGORITHM, conv_functional.IMPLICIT_SUB_TILES,
                conv_functional.REORDER_ROWS, c.get("algorithm"), c.get("sub_tiles"),
-               c["gather_tile_size"], c["scatter_tile_size"], c["threshold"], self.stride, self.dilation,
+               c["gather_tile_size"], c["scatter_tile_size"], c["threshold"], self._shape(),
                self._kernel_map_cache._disable_reordering, relu)
         if self._native_options is None or self._native_options[0] != key:
             self._native_options = (key, conv_functional.native_options(
@@ -522,19 +537,20 @@ class SparseConv(Module):
 
     def forward(self, inputs: SparseTensor) -> SparseTensor:
         features = inputs.F
-        if self.is_trivial and torch.is_grad_enabled() and (
+        trivial = self._shape()[4]
+        if trivial and torch.is_grad_enabled() and (
                 features.requires_grad or self.kernel.requires_grad):
             # training: the plain product, differentiated by autograd
             out = features @ self.kernel.view(self.in_channels, self.out_channels)
             if self.bias is not None:
                 out = out + self.bias
             return SparseTensor(out, inputs.C, stride=inputs.stride, batch_dims=inputs.batch_dims)
-        if self.is_trivial:
+        if trivial:
             bias = None if self.bias is None else self.bias.detach().float()
             out = F.dense_forward(features, self.kernel.view(self.in_channels, self.out_channels),
                                   shift=bias, weights_t=self._frozen_kernel_t)
             return SparseTensor(out, inputs.C, stride=inputs.stride, batch_dims=inputs.batch_dims)
-        coordinates, stride, batch_dims, source_masks, target_masks, order, _, plan, swapped = \
+        coordinates, stride, batch_dims, source_masks, target_masks, order, _, plan, swapped, _ = \
             self._lookup(inputs)
         out = conv_functional.run(plan, swapped, features, self.kernel, source_masks, target_masks,
                                   order, self._options(), self._frozen_kernel_t)
@@ -558,7 +574,7 @@ class SparseConv(Module):
             out = F.dense_forward(features, self.kernel.view(self.in_channels, self.out_channels),
                                   scale, shift, residual, relu, weights_t=self._frozen_kernel_t)
             return SparseTensor(out, inputs.C, stride=inputs.stride, batch_dims=inputs.batch_dims)
-        coordinates, stride, batch_dims, source_masks, target_masks, order, _, plan, swapped = \
+        coordinates, stride, batch_dims, source_masks, target_masks, order, _, plan, swapped, _ = \
             self._lookup(inputs)
         if self._tuning_data is not None:     # the tuner times the layer with the epilogue it runs
             self._tuning_epilogue = (scale is not None, shift is not None, residual is not None,

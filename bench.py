@@ -311,8 +311,10 @@ def kernel_bytes(name, S, T2, num_clouds):
             total += 8 * (S + T) + 4 * (S + T)        # both key arrays read, both word arrays written
     if name == "root_keys_kernel":
         total = 12 * S + 8 * S                        # coordinates read, packed keys written
-    elif name == "radix_sort_kernel":
-        total = 12 * S + 8 * S                        # coordinates read (floored + packed on the fly), sorted keys written
+    elif name == "sort_keys_kernel":
+        total = 12 * S + 8 * S                        # coordinates read, floored + packed keys written
+    elif name == "sort_pass_kernel":
+        total = 16 * S                                # unsorted keys read, sorted keys written: once, whatever the passes
     elif name == "unique_keys_kernel":
         total = 8 * S + (12 + 8) * T2 + 8 * (num_clouds + 3)   # keys read, coordinates + keys written
     return total
@@ -667,7 +669,7 @@ def gms_sweep(torch, minuet, lib, cache, d_coords, d_bd, channels=(16, 32, 64, 1
             layer["pairs_kernels_ms"] = {k: round(v["ms"], 4) for k, v in got.items()}
         if lib.mn_implicit_supported(O, c, c, code):
             n_pad = -(-c // 16) * 16
-            for sub in (1, 2, 3, 4):
+            for sub in minuet.nn.SparseConv.__AVAILABLE_SUB_TILES__:
                 if sub * n_pad > 512:
                     break
                 F.time_forward(algorithm="implicit", sub_tiles=sub, **fw)

@@ -620,7 +620,9 @@ enum Algorithm { kAuto = 0, kExplicit = 1, kImplicit = 2 };
 // written and read back) and every row twice in the centre product.  The fused kernel pays per
 // 128-row tile and per offset of a tile, of which the row permutation leaves a tile a little over
 // the pairs per row.  It is the faster one nearly everywhere, up to 9 times where pairs are many;
-// the neighbour table it needs is built once per map.
+// the neighbour table it needs is built once per map.  Of maps with a pair or more per row (8 and 27
+// offsets, 500 to 8 million rows, 8 to 256 channels) the estimate gives none to the pair lists: they
+// run on request, and where most targets have no pair at all.
 double estimate_ms(bool implicit, double S, double T, double O, double c_in, double c_out, double pairs,
                    bool shortcut, bool reorder) {
   if (implicit) {

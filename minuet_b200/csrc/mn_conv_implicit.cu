@@ -21,13 +21,15 @@
 // of target t under mask row p, or -1) is derived once per kernel map from the
 // masks by mn_build_neighbor_table.  Every barrier wait is bounded (status bit 2).
 //
-// What bounds it: the control code between two stages.  A 128 x 64 stage is 256 cycles
-// of tensor time at 128 output columns and about 280 of L2 time, but a warp needs five
-// cycles per dependent instruction, so every role's loop is kept short: the issuing
-// warps stay converged and elect one lane only around the instruction itself (issued
-// from a divergent lane-0 branch every MMA took about 150 cycles of register moves), a
-// lane reads the indices of all its rows with one load, two offsets ahead, and the next
-// stage's barrier is probed before the current stage is worked on.
+// What bounds it.  Maps with three or more pairs a row: a 128 x 64 stage at 128 output columns
+// takes 795 cycles, of which shared memory explains 520 (256 of operand reads by the MMAs, 200 of
+// gathered rows, 64 of weights and the rest); what the other 275 are is not known.  Sparser
+// maps: the epilogue's chain of instructions (see there).  A warp needs five cycles per dependent
+// instruction, so every role's loop is kept short: the issuing warps stay converged and elect
+// one lane only around the instruction itself (issued from a divergent lane-0 branch every MMA
+// took about 150 cycles of register moves), the index blocks arrive eight steps ahead and a lane
+// reads the indices of all its rows with one load, and the next stage's barrier is probed before
+// the current stage is worked on.
 #include "mn_sort.cuh"
 #include "mn_tc.cuh"
 
@@ -962,10 +964,11 @@ extern "C" mn_status mn_sparse_convolution_forward_implicit(
   // Weights that were not transposed once are read as they are, as N-major tiles, where a call has
   // few steps: the transposition is a launch of 3 to 10 us, an N-major step a little slower than a
   // K-major one.  With fewer than two pairs a row the MMAs wait for the rest anyway (464k rows
-  // 64->64, 1.15 pairs: 56.3 -> 53.8 us; 168k rows 64->128, 1.4 pairs: 23.4 -> 20.5 us); up to two
-  // tiles per CTA the launch is what counts (53k rows 256->256: 95.5 -> 92.1 us, 30k rows 32->96:
-  // 13.9 -> 12.0 us); 200k rows 64->64 with 3 pairs and both gradients lose 1 of 115 us.  TMA needs
-  // them on a 16-byte boundary.
+  // 64->64, 1.15 pairs: 56.3 -> 53.8 us; 168k rows 64->128, 1.4 pairs: 23.4 -> 20.5 us); up to four
+  // tiles per SM (two per CTA where two CTAs share one) the launch is what counts (53k rows
+  // 256->256: 95.5 -> 92.1 us, 30k rows 32->96: 13.9 -> 12.0 us).  The line is drawn through these few
+  // layers: 200k rows 64->64 with 3 pairs a row would lose 1 of 115 us beyond it.  TMA needs the
+  // weights on a 16-byte boundary.
   Workspace ws(ws_ptr, ws_bytes);
   const void *weights_t = weights_t_in;
   const bool n_major = weights_t == nullptr && (reinterpret_cast<uintptr_t>(weights) & 15) == 0 &&

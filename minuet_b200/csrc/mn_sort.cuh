@@ -1,6 +1,7 @@
 // Stable radix sort of 64-bit keys, shared by the map step, voxelisation and the neighbour
 // tables: one launch that makes the keys and counts their digits, then one launch per 9-bit
-// digit.
+// digit.  The scheme is published: one sweep per digit (Adinets and Merrill, "Onesweep", 2022) with
+// decoupled look-back (Merrill and Garland, 2016).
 //
 // A digit pass moves every key once: a block takes the next tile of keys, ranks them in
 // registers (equal digits of a warp find each other with match.any), learns how many keys of

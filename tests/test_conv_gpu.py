@@ -449,3 +449,33 @@ def test_benchmark_size_tiles_with_full_epilogue(oracle_lib, algorithm, c_in, c_
     assert_close(plain.F, ref, torch.float16)
     ref = np.maximum(ref * scale + shift + rt.float().cpu().numpy(), 0)
     assert_close(out.F, ref, torch.float16)
+
+
+@pytest.mark.parametrize("dtype,c_in,c_out,kernel", [(torch.float32, 12, 24, 5), (torch.float16, 12, 24, 5),
+                                                     (torch.float16, 6, 3, 3), (torch.bfloat16, 6, 3, 3)])
+def test_tile_sizes_of_the_stages_do_not_change_results(dtype, c_in, c_out, kernel):
+    """Layers that run gather - GEMM - scatter (more than 32 offsets, 16-bit channels off the tensor-core
+    paths): the same bits with every tile size."""
+    gen = torch.Generator(device=DEV).manual_seed(kernel)
+    i = torch.randperm(14 ** 3, generator=gen, device=DEV)[:1000].sort().values
+    coords = torch.stack([i // 196, i // 14 % 14, i % 14], 1).int()
+    conv = minuet.nn.SparseConv3d(c_in, c_out, kernel, dtype=dtype, device=DEV)
+    cache = minuet.nn.KernelMapCache(ndim=3, dtype=torch.int32, device=DEV)
+    minuet.set_kernel_map_cache(conv, cache)
+    x = minuet.SparseTensor(torch.randn(1000, c_in, generator=gen, device=DEV).to(dtype), coords)
+    want = None
+    for gather in [t for t in range(1, c_in + 1) if c_in % t == 0]:
+        for scatter in [t for t in range(1, c_out + 1) if c_out % t == 0]:
+            conv.tunable_config.update(gather_tile_size=gather, scatter_tile_size=scatter)
+            got = conv(x).F
+            want = got if want is None else want
+            assert torch.equal(got, want)
+    maps = cache.get_kernel_map(coords, 1, None, coords, 1, None, kernel, 1)
+    sm, tm, order, _ = maps
+    sums = torch.zeros(1000, c_out, dtype=torch.float64, device=DEV)
+    for p in range(len(sm)):
+        s, t = (torch.nonzero(m[p] >= 0)[:, 0] for m in (sm, tm))
+        sums[t[tm[p, t].argsort()]] += x.F[s[sm[p, s].argsort()]].double() @ conv.kernel[order[p].long()].double()
+    # 16-bit products are rounded once per offset there
+    bound = {torch.float32: 1e-5, torch.float16: 2.0 ** -10, torch.bfloat16: 2.0 ** -7}[dtype]
+    assert float((want.double() - sums).norm() / sums.norm()) < bound

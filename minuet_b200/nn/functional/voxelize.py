@@ -77,16 +77,19 @@ def _native(coordinates, voxel_size, batch_dims, return_inverse, features):
             torch.float32, torch.float16, torch.bfloat16)):
         return None
     # one size or one per dimension; whatever else broadcasts, or is refused, goes step by step
-    try:
-        if np.ndim(voxel_size) > 1:
+    if type(voxel_size) is float:
+        sizes = [voxel_size] * ndim
+    else:
+        try:
+            if np.ndim(voxel_size) > 1:
+                return None
+            sizes = [float(v) for v in (voxel_size if hasattr(voxel_size, "__len__") else (voxel_size,))]
+        except (TypeError, ValueError):
             return None
-        sizes = [float(v) for v in (voxel_size if hasattr(voxel_size, "__len__") else (voxel_size,))]
-    except (TypeError, ValueError):
-        return None
-    if len(sizes) == 1:
-        sizes = sizes * ndim
-    if len(sizes) != ndim:
-        return None
+        if len(sizes) == 1:
+            sizes = sizes * ndim
+        if len(sizes) != ndim:
+            return None
     out = _lib.host().voxelize(coordinates.detach(), sizes, engine.as_i64(batch_dims), return_inverse,
                                features)
     if out is None:

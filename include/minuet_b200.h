@@ -367,9 +367,8 @@ mn_status mn_sparse_convolution_forward_implicit(
     int32_t *status_dev, void *ws, size_t ws_bytes, void *stream);
 
 /* The same function in fp32 on FFMA units (sums in fp32, any channel counts, at most 32
- * offsets), every offset's product by itself and the products added in mask-row order: one
- * output-stationary kernel over the neighbour table, plus one launch that adds the offsets'
- * products where the rows alone do not fill the GPU (the workspace is for those). */
+ * offsets), every offset's product by itself and the products added in mask-row order, by one
+ * output-stationary kernel over the neighbour table.  (It keeps nothing in the workspace.) */
 size_t mn_implicit_fp32_workspace_bytes(int64_t T, int64_t O, int64_t c_out);
 mn_status mn_sparse_convolution_forward_implicit_fp32(
     int64_t S, int64_t T, int64_t O, int64_t c_in, int64_t c_out, const float *sources,

@@ -90,7 +90,7 @@ typedef struct {
 /* Version of this interface; mn_version() returns the value the library was
  * built with.  A binding should refuse a library whose version differs from the
  * header it was written against: argument lists change between versions. */
-#define MN_ABI_VERSION 19
+#define MN_ABI_VERSION 20
 
 const char *mn_last_error(void);
 int mn_version(void);
@@ -133,12 +133,13 @@ mn_status mn_keyspec_make(const int32_t *minmax_host, int ndim,
  * key bits raises MN_STATUS_KEY_BITS in the status word.  Same role as mn_bbox +
  * mn_keyspec_make + mn_pack_keys without the device-to-host read between them
  * (the reference blocks on that read, arg_sort_coodrinates.cu:286-287).
- * ctrl: the control block. */
+ * bits_host (may be NULL): host memory that the GPU can write (pinned), receives
+ * total_bits when the launch ends.  ctrl: the control block. */
 mn_status mn_keyspec_device(const int32_t *coords, int64_t n, int ndim,
                             const int64_t *batch_dims, int64_t num_clouds,
                             int32_t margin, void *spec_dev, mn_keyspec *spec,
-                            uint64_t *keys_out, int32_t *ctrl, void *ws, size_t ws_bytes,
-                            void *stream);
+                            uint64_t *keys_out, int32_t *bits_host, int32_t *ctrl, void *ws,
+                            size_t ws_bytes, void *stream);
 
 /* Pack coordinates into keys.  tstride (host, may be NULL) floors every
  * coordinate to a multiple of tstride[k] first, as
@@ -215,28 +216,30 @@ mn_status mn_unique_coordinates_static(const int32_t *coords, int64_t n, int ndi
  * small read brings back everything the host needs.  A spec whose total_bits is
  * positive saves the launches of the digits that a layout known only to the device
  * might have.  batch_dims == NULL means one cloud
- * (meta_out then has 5 entries).  ctrl: the control block. */
+ * (meta_out then has 5 entries).  meta_host (may be NULL): pinned host memory that receives the
+ * same entries, which saves the read a copy.  ctrl: the control block. */
 mn_status mn_downsample_coordinates(const int32_t *coords, int64_t n, int ndim,
                                     const int64_t *batch_dims, int64_t num_clouds,
                                     const int32_t *tstride, const mn_keyspec *spec,
                                     int32_t *unique_out, uint64_t *keys_out,
-                                    int64_t *meta_out, int32_t *ctrl, void *ws,
-                                    size_t ws_bytes, void *stream);
+                                    int64_t *meta_out, int64_t *meta_host, int32_t *ctrl,
+                                    void *ws, size_t ws_bytes, void *stream);
 
 /* Voxelisation of floating-point points (float, or double with points_are_double):
  * voxels_out int32 [n, ndim] = the distinct floor(point / voxel_size) (HOST [ndim]; the
  * arithmetic is the points' own type), cloud-major, then lexicographic; inverse_out int64 [n]
  * (may be NULL): the voxel of every point; means_out [n, channels] (with features): mean feature
- * of every voxel, summed in sorted order in fp32.  meta_out as mn_downsample_coordinates; only
- * its first entry's worth of rows of voxels_out and means_out is written.  The result is valid
+ * of every voxel, summed in sorted order in fp32.  meta_out and meta_host as
+ * mn_downsample_coordinates; meta_event (cudaEvent_t, may be NULL) is recorded as soon as they are
+ * complete, before the means.  Only meta_out's first entry's worth of rows of voxels_out and means_out is written.  The result is valid
  * when the key bits of the layout (last entry of meta_out) plus ceil(log2 n) (at least 1) are at
  * most 64; boxes wider than that take arg sort, unique and mn_voxel_mean one by one. */
 size_t mn_voxelize_workspace_bytes(int64_t n);
 mn_status mn_voxelize(const void *points, int points_are_double, int64_t n, int ndim,
                       const double *voxel_size, const int64_t *batch_dims, int64_t num_clouds,
                       const void *features, int64_t channels, mn_dtype dtype, int32_t *voxels_out,
-                      int64_t *inverse_out, void *means_out, int64_t *meta_out, int32_t *ctrl,
-                      void *ws, size_t ws_bytes, void *stream);
+                      int64_t *inverse_out, void *means_out, int64_t *meta_out, int64_t *meta_host,
+                      void *meta_event, int32_t *ctrl, void *ws, size_t ws_bytes, void *stream);
 
 /* _C.cuda_query_sorted_index_with_offsets / _C.cuda_multi_query_...
  * (csrc/minuet/torch/cuda_sparse_convolution_mapping.cu:9-100) on packed keys:
@@ -269,7 +272,8 @@ mn_status mn_compute_kernel_map_masks(const int32_t *kernel_map, int64_t O, int6
  * target_bits_out uint32 [T] (each may be NULL) receive one word per row whose
  * bit p is set when mask row p has an entry for that row: the forward kernels
  * walk a row's pairs through these words instead of scanning O mask rows.
- * ctrl: the control block. */
+ * sizes_host (may be NULL): pinned host memory [O + 1] that receives the same values as
+ * sizes_out.  ctrl: the control block. */
 mn_status mn_build_kernel_map(const uint64_t *source_keys, int64_t S,
                               const uint64_t *target_keys, int64_t T,
                               const int32_t *offsets, int64_t O,
@@ -277,7 +281,8 @@ mn_status mn_build_kernel_map(const uint64_t *source_keys, int64_t S,
                               int32_t *source_masks_out, int32_t *target_masks_out,
                               int32_t *order_out, int32_t *sizes_out,
                               uint32_t *source_bits_out, uint32_t *target_bits_out,
-                              int32_t *ctrl, void *ws, size_t ws_bytes, void *stream);
+                              int32_t *sizes_host, int32_t *ctrl, void *ws, size_t ws_bytes,
+                              void *stream);
 
 /* Upper bound of the workspace any Map-step entry point needs. */
 size_t mn_map_workspace_bytes(int64_t S, int64_t T, int64_t O);

@@ -15,7 +15,7 @@ MN_F32, MN_F16, MN_BF16 = 0, 1, 2
 MN_MAX_NDIM = 4
 MN_MAX_OFFSETS = 128
 MN_CTRL_WORDS = 1024
-ABI_VERSION = 19         # must equal MN_ABI_VERSION of the header the library was built from
+ABI_VERSION = 20         # must equal MN_ABI_VERSION of the header the library was built from
 
 c_i32p = ctypes.c_void_p
 c_ptr = ctypes.c_void_p
@@ -58,10 +58,10 @@ PROTOTYPES = {
                                       c_size, c_ptr]),
     "mn_unique_coordinates_static": (c_int, [c_ptr, c_i64, c_int, c_ptr, c_i64, c_ptr, c_ptr, c_ptr]),
     "mn_downsample_coordinates": (c_int, [c_ptr, c_i64, c_int, c_ptr, c_i64, c_ptr,
-                                          ctypes.POINTER(KeySpec), c_ptr, c_ptr, c_ptr, c_ptr,
+                                          ctypes.POINTER(KeySpec), c_ptr, c_ptr, c_ptr, c_ptr, c_ptr,
                                           c_ptr, c_size, c_ptr]),
     "mn_keyspec_device": (c_int, [c_ptr, c_i64, c_int, c_ptr, c_i64, ctypes.c_int32, c_ptr,
-                                  ctypes.POINTER(KeySpec), c_ptr, c_ptr, c_ptr, c_size, c_ptr]),
+                                  ctypes.POINTER(KeySpec), c_ptr, c_ptr, c_ptr, c_ptr, c_size, c_ptr]),
     "mn_query_sorted_index_with_offsets": (c_int, [c_ptr, c_i64, c_ptr, c_i64, c_ptr, c_i64,
                                                    ctypes.POINTER(KeySpec), c_ptr, c_ptr]),
     "mn_compute_kernel_map_sizes": (c_int, [c_ptr, c_i64, c_i64, c_ptr, c_ptr]),
@@ -69,7 +69,7 @@ PROTOTYPES = {
                                             c_size, c_ptr]),
     "mn_build_kernel_map": (c_int, [c_ptr, c_i64, c_ptr, c_i64, c_ptr, c_i64,
                                     ctypes.POINTER(KeySpec), c_int, c_ptr, c_ptr, c_ptr, c_ptr,
-                                    c_ptr, c_ptr, c_ptr, c_ptr, c_size, c_ptr]),
+                                    c_ptr, c_ptr, c_ptr, c_ptr, c_ptr, c_size, c_ptr]),
     "mn_map_workspace_bytes": (c_size, [c_i64, c_i64, c_i64]),
     "mn_plan_buckets": (c_int, [c_ptr, c_i64, c_int, c_dbl, c_ptr, c_ptr, c_ptr]),
     "mn_conv_workspace_bytes": (c_size, [c_ptr, c_i64, c_i64, c_i64, c_i64, c_i64, c_int, c_int,
@@ -118,7 +118,7 @@ PROTOTYPES = {
                                                      c_ptr, c_size, c_ptr]),
     "mn_voxelize_workspace_bytes": (c_size, [c_i64]),
     "mn_voxelize": (c_int, [c_ptr, c_int, c_i64, c_int, c_ptr, c_ptr, c_i64, c_ptr, c_i64, c_int, c_ptr,
-                            c_ptr, c_ptr, c_ptr, c_ptr, c_ptr, c_size, c_ptr]),
+                            c_ptr, c_ptr, c_ptr, c_ptr, c_ptr, c_ptr, c_ptr, c_size, c_ptr]),
     "mn_voxel_mean": (c_int, [c_ptr, c_i64, c_i64, c_int, c_ptr, c_ptr, c_ptr, c_ptr]),
     "mn_dense_forward_simt": (c_int, [c_i64, c_i64, c_i64, c_int, c_ptr, c_ptr, c_ptr, c_ptr, c_ptr,
                                       c_int, c_ptr, c_ptr]),

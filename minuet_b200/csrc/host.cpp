@@ -209,6 +209,42 @@ PinnedPool &pinned_pool() {
   return *pool;
 }
 
+// Host memory that the kernels of one library call write a few values to, and the event after it: the
+// read needs no copy (a copy of a few bytes is 3 us on the stream, and 2 to 9 us pass before it starts).
+// Not used (host() is NULL) for more than a buffer holds and inside a stream capture, where a
+// replay would write to memory that has been given back.
+class Reply {
+ public:
+  Reply(const Tensor &like, size_t bytes) : stream_(stream_of(like)) {
+    if (bytes <= PinnedPool::kBytes && c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None)
+      buffer_ = pinned_pool().take(like.get_device());
+  }
+  Reply(const Reply &) = delete;
+  ~Reply() {
+    if (used()) pinned_pool().give(written());   // a call that has failed may have launched some of its kernels
+  }
+  bool used() const { return buffer_.host != nullptr; }
+  template <typename T>
+  T *host() const { return static_cast<T *>(buffer_.host); }
+  // for a call that records the event itself, once the values are complete
+  cudaEvent_t event() {
+    recorded_ = used();
+    return buffer_.event;
+  }
+  // The buffer, its event recorded behind the call; empty if it is not used.
+  PinnedPool::Buffer written() {
+    if (used() && !recorded_) (void)cudaEventRecord(buffer_.event, stream_);
+    PinnedPool::Buffer b = buffer_;
+    buffer_ = {};
+    return b;
+  }
+
+ private:
+  cudaStream_t stream_;
+  PinnedPool::Buffer buffer_;
+  bool recorded_ = false;
+};
+
 [[noreturn]] void raise_device_status(int value, int device) {
   py::gil_scoped_acquire gil;
   py::module_::import("minuet_b200.engine").attr("raise_on_status")(value, device);
@@ -248,14 +284,9 @@ struct KeyLayout {
   Tensor dev;      // device copy of the layout, alive as long as this object
 
   ~KeyLayout() { pinned_pool().give(bits_); }
-  // The width of the keys follows on a copy of its own: where it has landed by the time a sort is
+  // The kernel also writes the width of the keys here: where it has landed by the time a sort is
   // launched, no digit too many is (a digit pass that finds nothing to do is 2-4 us).
-  void expect_bits(cudaStream_t st) {
-    bits_ = pinned_pool().take(dev.get_device());
-    check_cuda(cudaMemcpyAsync(bits_.host, static_cast<char *>(dev.data_ptr()) + offsetof(mn_keyspec, total_bits),
-                               sizeof(int32_t), cudaMemcpyDeviceToHost, st), "key layout");
-    check_cuda(cudaEventRecord(bits_.event, st), "key layout");
-  }
+  void expect_bits(PinnedPool::Buffer written) { bits_ = written; }
   void look_for_bits() {
     if (spec.total_bits > 0 || bits_.host == nullptr) return;
     if (ended(bits_.event)) spec.total_bits = *static_cast<int32_t *>(bits_.host);
@@ -294,12 +325,13 @@ std::pair<std::shared_ptr<KeyLayout>, Tensor> root_keys(const Tensor &coords, co
   layout->dev = empty_on(coords, {256}, at::kByte);
   Tensor keys = empty_on(coords, {coords.size(0)}, at::kLong);
   Tensor ws = workspace(coords, api.mn_map_workspace_bytes(0, 0, 0));
+  Reply bits(coords, sizeof(int32_t));
   check(api.mn_keyspec_device(raw<int32_t>(coords), coords.size(0), (int)coords.size(1), raw<int64_t>(batch_dims),
                               std::max<int64_t>(num_clouds, 1), margin, layout->dev.data_ptr(), &layout->spec,
-                              raw<uint64_t>(keys), ctrl_of(coords), ws.data_ptr(), (size_t)ws.numel(),
-                              stream_of(coords)),
+                              raw<uint64_t>(keys), bits.host<int32_t>(), ctrl_of(coords), ws.data_ptr(),
+                              (size_t)ws.numel(), stream_of(coords)),
         "keyspec_device");
-  layout->expect_bits(stream_of(coords));
+  layout->expect_bits(bits.written());
   return {layout, keys};
 }
 
@@ -328,17 +360,17 @@ mn_dtype dtype_code(at::ScalarType t) {
 // Blocking read of a small int64 tensor.
 std::vector<int64_t> read_back(const Tensor &t) {
   std::vector<int64_t> host((size_t)t.numel());
-  const size_t bytes = host.size() * sizeof(int64_t);
-  const cudaStream_t st = stream_of(t);
-  if (bytes > PinnedPool::kBytes) {
-    Tensor h = t.cpu();
-    std::copy_n(static_cast<int64_t *>(h.data_ptr()), host.size(), host.begin());
-    return host;
-  }
-  PinnedPool::Buffer b = pinned_pool().take(t.get_device());
-  cudaError_t e = cudaMemcpyAsync(b.host, t.data_ptr(), bytes, cudaMemcpyDeviceToHost, st);
-  if (e == cudaSuccess) e = cudaEventRecord(b.event, st);
-  if (e == cudaSuccess) e = cudaEventSynchronize(b.event);
+  Tensor h = t.cpu();
+  std::copy_n(static_cast<int64_t *>(h.data_ptr()), host.size(), host.begin());
+  return host;
+}
+
+// What `reply` holds, or where the values did not fit it what `t` holds on the device.
+std::vector<int64_t> read_reply(Reply &reply, const Tensor &t) {
+  if (!reply.used()) return read_back(t);
+  const PinnedPool::Buffer b = reply.written();
+  const cudaError_t e = cudaEventSynchronize(b.event);
+  std::vector<int64_t> host((size_t)t.numel());
   if (e == cudaSuccess) std::copy_n(static_cast<int64_t *>(b.host), host.size(), host.begin());
   pinned_pool().give(b);
   check_cuda(e, "device-to-host read");
@@ -360,12 +392,13 @@ std::tuple<Tensor, Tensor, Tensor, std::vector<int64_t>> downsample(const Tensor
   Tensor meta = empty_on(coords, {nb + 4}, at::kLong);   // count, cloud starts, status, key bits
   Tensor ws = workspace(coords, api.mn_map_workspace_bytes(n, n, 1));
   layout.look_for_bits();
+  Reply reply(coords, sizeof(int64_t) * (size_t)(nb + 4));
   check(api.mn_downsample_coordinates(raw<int32_t>(coords), n, (int)ndim, raw<int64_t>(batch_dims), nb,
                                       tstride.data(), &layout.spec, raw<int32_t>(unique), raw<uint64_t>(keys),
-                                      raw<int64_t>(meta), ctrl_of(coords), ws.data_ptr(), (size_t)ws.numel(),
-                                      stream_of(coords)),
+                                      raw<int64_t>(meta), reply.host<int64_t>(), ctrl_of(coords), ws.data_ptr(),
+                                      (size_t)ws.numel(), stream_of(coords)),
         "downsample_coordinates");
-  const std::vector<int64_t> host = read_back(meta);
+  const std::vector<int64_t> host = read_reply(reply, meta);
   if (host[(size_t)nb + 2] != 0) raise_device_status((int)host[(size_t)nb + 2], coords.get_device());
   layout.spec.total_bits = (int32_t)host[(size_t)nb + 3];   // later levels launch no digit too many
   const int64_t count = host[0];
@@ -396,13 +429,14 @@ std::optional<std::tuple<Tensor, Tensor, OptTensor, OptTensor>> voxelize(const T
   Tensor voxels = empty_on(points, {n, ndim}, at::kInt);
   Tensor meta = empty_on(points, {nb + 4}, at::kLong);
   Tensor ws = workspace(points, api.mn_voxelize_workspace_bytes(n));
+  Reply reply(points, sizeof(int64_t) * (size_t)(nb + 4));
   check(api.mn_voxelize(points.data_ptr(), points.scalar_type() == at::kDouble, n, (int)ndim, voxel_size.data(),
                         raw<int64_t>(batch_dims), nb, raw<void>(features), features.has_value() ? features->size(1) : 0,
                         features.has_value() ? dtype_code(features->scalar_type()) : MN_F32, raw<int32_t>(voxels),
-                        raw<int64_t>(inv), raw<void>(means), raw<int64_t>(meta), ctrl_of(points), ws.data_ptr(),
-                        (size_t)ws.numel(), stream_of(points)),
+                        raw<int64_t>(inv), raw<void>(means), raw<int64_t>(meta), reply.host<int64_t>(),
+                        reply.event(), ctrl_of(points), ws.data_ptr(), (size_t)ws.numel(), stream_of(points)),
         "voxelize");
-  const std::vector<int64_t> host = read_back(meta);
+  const std::vector<int64_t> host = read_reply(reply, meta);
   int index_bits = 1;
   while ((1ll << index_bits) < n) index_bits++;
   if (host[(size_t)nb + 3] + index_bits > 64) return std::nullopt;
@@ -510,6 +544,11 @@ struct Plan {
     }
     return sizes_;
   }
+  // the same, written by the kernel itself
+  void expect_sizes(PinnedPool::Buffer written) {
+    buffer_ = written;
+    pending_ = true;
+  }
   int64_t pairs() {
     sizes();
     return total_;
@@ -544,13 +583,15 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, PlanPtr> build_map(const Tensor &sour
   Tensor ws = workspace(source_keys, api.mn_map_workspace_bytes(S, T, O));
   const uint64_t *sk = raw<uint64_t>(source_keys);
   const uint64_t *tk = same ? sk : raw<uint64_t>(target_keys);
+  Reply reply(source_keys, sizeof(int32_t) * (size_t)(O + 1));
   check(api.mn_build_kernel_map(sk, S, tk, T, offsets.table.data(), O, &layout.spec, reorder ? 1 : 0,
                                 raw<int32_t>(sm), raw<int32_t>(tm), p, p + pad(O + 1),
                                 reinterpret_cast<uint32_t *>(p + base),
-                                reinterpret_cast<uint32_t *>(p + base + pad(S)), ctrl_of(source_keys),
-                                ws.data_ptr(), (size_t)ws.numel(), stream_of(source_keys)),
+                                reinterpret_cast<uint32_t *>(p + base + pad(S)), reply.host<int32_t>(),
+                                ctrl_of(source_keys), ws.data_ptr(), (size_t)ws.numel(), stream_of(source_keys)),
         "build_kernel_map");
-  plan->expect_sizes(small.narrow(0, pad(O + 1), O + 1));
+  if (reply.used()) plan->expect_sizes(reply.written());
+  else plan->expect_sizes(small.narrow(0, pad(O + 1), O + 1));
   return {sm, tm, small.narrow(0, 0, O), small.narrow(0, pad(O + 1), O), plan};
 }
 
@@ -1061,7 +1102,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   py::class_<Plan, PlanPtr>(m, "Plan")
       .def(py::init<int64_t, int64_t, int64_t>())
       .def("set_sizes", &Plan::set_sizes)
-      .def("expect_sizes", &Plan::expect_sizes)
+      .def("expect_sizes", py::overload_cast<const Tensor &>(&Plan::expect_sizes))
       .def("sizes", [](Plan &p) { return p.sizes(); }, NoGil())
       .def("pairs", &Plan::pairs, NoGil())
       .def_property_readonly("source_bits", [](Plan &p) { return optional(p.bits_s); })

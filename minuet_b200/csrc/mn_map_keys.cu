@@ -187,6 +187,7 @@ struct RootArgs {
   int32_t *partial;        // workspace [grid][8]
   mn_keyspec *spec_out;
   uint64_t *keys_out;      // may be NULL: layout only
+  int32_t *bits_host;      // may be NULL: total_bits, in host memory
   int32_t *ctrl;
 };
 
@@ -240,7 +241,10 @@ root_keys_kernel(const __grid_constant__ RootArgs a) {
     s_p.spec.dev = nullptr;
     s_p.has_stride = 0;
     for (int k = 0; k < 4; k++) s_p.tstride[k] = 1;
-    if (b == 0) *a.spec_out = s_p.spec.host;
+    if (b == 0) {
+      *a.spec_out = s_p.spec.host;
+      if (a.bits_host != nullptr) *a.bits_host = s_p.spec.host.total_bits;
+    }
   }
   __syncthreads();
   if (a.keys_out == nullptr) return;
@@ -311,8 +315,8 @@ extern "C" mn_status mn_keyspec_make(const int32_t *minmax_host, int ndim,
 extern "C" mn_status mn_keyspec_device(const int32_t *coords, int64_t n, int ndim,
                                        const int64_t *batch_dims, int64_t num_clouds,
                                        int32_t margin, void *spec_dev, mn_keyspec *spec,
-                                       uint64_t *keys_out, int32_t *ctrl, void *ws_ptr,
-                                       size_t ws_bytes, void *stream) {
+                                       uint64_t *keys_out, int32_t *bits_host, int32_t *ctrl,
+                                       void *ws_ptr, size_t ws_bytes, void *stream) {
   using namespace mn;
   MN_CHECK_ARG(ndim >= 1 && ndim <= MN_MAX_NDIM, "keyspec_device: ndim %d not in 1..4", ndim);
   MN_CHECK_ARG(n >= 0 && margin >= 0, "keyspec_device: bad arguments");
@@ -343,6 +347,7 @@ extern "C" mn_status mn_keyspec_device(const int32_t *coords, int64_t n, int ndi
   a.ndim = ndim; a.margin = margin;
   a.spec_out = static_cast<mn_keyspec *>(spec_dev);
   a.keys_out = n > 0 ? keys_out : nullptr;
+  a.bits_host = bits_host;
   a.ctrl = ctrl;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   void *params[] = {&a};

@@ -460,6 +460,7 @@ struct EmitArgs {
   int32_t *source_masks;     // [O, S]
   int32_t *order_out;        // [O] offset at mask row p
   int32_t *sizes_out;        // [O + 1] size of mask row p, then a copy of the status word
+  int32_t *sizes_host;       // the same in host memory, or NULL
   uint32_t *bits_t;          // optional [T]: bit p set when mask row p has an entry for the target
   uint32_t *bits_s;          // optional [S]: the same for the sources
   int32_t *agg;              // workspace [64 pairs][grid]: hit counts of every block's rows;
@@ -589,9 +590,14 @@ emit_masks_kernel(const __grid_constant__ EmitArgs e) {
     if (b == 0) {
       e.order_out[pos] = tid;
       e.sizes_out[pos] = s_size[tid];
+      if (e.sizes_host != nullptr) e.sizes_host[pos] = s_size[tid];
     }
   }
-  if (b == 0 && tid == 0) e.sizes_out[O] = e.ctrl[MN_CTRL_STATUS];
+  if (b == 0 && tid == 0) {
+    const int32_t status = e.ctrl[MN_CTRL_STATUS];
+    e.sizes_out[O] = status;
+    if (e.sizes_host != nullptr) e.sizes_host[O] = status;
+  }
   __syncthreads();
   // from here on lane p stands for mask row p
   const int ord = s_ord[lane];
@@ -652,11 +658,15 @@ emit_masks_kernel(const __grid_constant__ EmitArgs e) {
   MN_MARK(g_marks_emit, 6);
 }
 
-__global__ void identity_order_kernel(int O, int32_t *order_out, int32_t *sizes_out,
+__global__ void identity_order_kernel(int O, int32_t *order_out, int32_t *sizes_out, int32_t *sizes_host,
                                       const int32_t *ctrl) {
   const int o = blockIdx.x * blockDim.x + threadIdx.x;
-  if (o < O) { order_out[o] = o; sizes_out[o] = 0; }
-  if (o == O) sizes_out[O] = ctrl[MN_CTRL_STATUS];
+  if (o < O) order_out[o] = o;
+  if (o <= O) {
+    const int32_t v = o < O ? 0 : ctrl[MN_CTRL_STATUS];
+    sizes_out[o] = v;
+    if (sizes_host != nullptr) sizes_host[o] = v;
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -927,8 +937,8 @@ extern "C" mn_status mn_build_kernel_map(const uint64_t *source_keys, int64_t S,
                                          int32_t *source_masks_out, int32_t *target_masks_out,
                                          int32_t *order_out, int32_t *sizes_out,
                                          uint32_t *source_bits_out, uint32_t *target_bits_out,
-                                         int32_t *ctrl, void *ws_ptr, size_t ws_bytes,
-                                         void *stream) {
+                                         int32_t *sizes_host, int32_t *ctrl, void *ws_ptr,
+                                         size_t ws_bytes, void *stream) {
   MN_CHECK_ARG(S >= 0 && T >= 0, "build_kernel_map: negative size");
   MN_CHECK_ARG(spec != nullptr, "build_kernel_map: null key spec");
   MN_CHECK_ARG(S < (1ll << 31) && T < (1ll << 31), "build_kernel_map: more than 2^31-1 rows");
@@ -951,7 +961,7 @@ extern "C" mn_status mn_build_kernel_map(const uint64_t *source_keys, int64_t S,
     if (S > 0 && source_bits_out != nullptr) MN_CHECK_CUDA(cudaMemsetAsync(source_bits_out, 0, sizeof(uint32_t) * S, st));
     if (T > 0 && target_bits_out != nullptr) MN_CHECK_CUDA(cudaMemsetAsync(target_bits_out, 0, sizeof(uint32_t) * T, st));
     MN_LAUNCH("identity_order_kernel", st,
-              identity_order_kernel<<<1, MN_MAX_OFFSETS + 32, 0, st>>>((int)O, order_out, sizes_out, ctrl));
+              identity_order_kernel<<<1, MN_MAX_OFFSETS + 32, 0, st>>>((int)O, order_out, sizes_out, sizes_host, ctrl));
     return MN_OK;
   }
   MN_CHECK_ARG(source_keys != nullptr && target_keys != nullptr && source_masks_out != nullptr &&
@@ -1009,7 +1019,7 @@ extern "C" mn_status mn_build_kernel_map(const uint64_t *source_keys, int64_t S,
   EmitArgs e{};
   e.words_t = words_t; e.words_s = words_s;
   e.target_masks = target_masks_out; e.source_masks = source_masks_out;
-  e.order_out = order_out; e.sizes_out = sizes_out; e.agg = agg; e.ctrl = ctrl;
+  e.order_out = order_out; e.sizes_out = sizes_out; e.sizes_host = sizes_host; e.agg = agg; e.ctrl = ctrl;
   e.bits_t = target_bits_out; e.bits_s = source_bits_out;
   e.T = T; e.S = S; e.units_t = units_t; e.units_s = units_s;
   e.num_offsets = (int)O; e.reorder = reorder ? 1 : 0;

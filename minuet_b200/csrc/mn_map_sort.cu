@@ -184,6 +184,7 @@ struct UniqueKeysArgs {
   uint64_t *keys_out;                // [n]
   int32_t *rows_out;                 // [n, ndim]
   int64_t *meta;                     // [num_clouds + 4]: count, cloud starts [num_clouds + 1], status, key bits
+  int64_t *meta_host;                // the same in host memory, or NULL
   int32_t num_clouds;
   uint32_t *block_counts;            // workspace [grid]
   int32_t *ctrl;
@@ -250,6 +251,10 @@ unique_keys_kernel(const __grid_constant__ UniqueKeysArgs a) {
   __syncthreads();
   uint32_t run = s_before;
   const uint32_t total = s_total;
+  auto put_meta = [&](int64_t i, int64_t v) {
+    a.meta[i] = v;
+    if (a.meta_host != nullptr) a.meta_host[i] = v;   // a posted write; it lands before the launch has ended
+  };
 
   // ---- compact, unpack, cloud starts ----------------------------------------------
   for (int64_t s0 = c0; s0 < c1; s0 += kUkStep) {
@@ -305,17 +310,17 @@ unique_keys_kernel(const __grid_constant__ UniqueKeysArgs a) {
         // first key of cloud c: every cloud after the previous key's cloud starts here
         const int64_t c_here = (int64_t)(key >> spec.cloud_shift);
         const int64_t c_prev = i == 0 ? -1 : (int64_t)(pk[j] >> ib >> spec.cloud_shift);
-        for (int64_t g = c_prev + 1; g <= c_here && g <= a.num_clouds; g++) a.meta[1 + g] = pos;
+        for (int64_t g = c_prev + 1; g <= c_here && g <= a.num_clouds; g++) put_meta(1 + g, pos);
       }
     }
     run += s_step_total;
   }
   if (b == 0 && tid == 0) {
-    a.meta[0] = total;
+    put_meta(0, total);
     const int64_t c_last = a.n > 0 ? (int64_t)(__ldcg(keys + a.n - 1) >> ib >> spec.cloud_shift) : -1;
-    for (int64_t g = c_last + 1; g <= a.num_clouds; g++) a.meta[1 + g] = total;
-    a.meta[a.num_clouds + 2] = a.ctrl[MN_CTRL_STATUS];
-    a.meta[a.num_clouds + 3] = spec.total_bits;
+    for (int64_t g = c_last + 1; g <= a.num_clouds; g++) put_meta(1 + g, total);
+    put_meta(a.num_clouds + 2, a.ctrl[MN_CTRL_STATUS]);
+    put_meta(a.num_clouds + 3, spec.total_bits);
   }
 }
 
@@ -513,7 +518,7 @@ extern "C" mn_status mn_unique_coordinates(const int32_t *coords, int64_t n, int
 extern "C" mn_status mn_downsample_coordinates(
     const int32_t *coords, int64_t n, int ndim, const int64_t *batch_dims, int64_t num_clouds,
     const int32_t *tstride, const mn_keyspec *spec, int32_t *unique_out, uint64_t *keys_out,
-    int64_t *meta_out, int32_t *ctrl, void *ws_ptr, size_t ws_bytes, void *stream) {
+    int64_t *meta_out, int64_t *meta_host, int32_t *ctrl, void *ws_ptr, size_t ws_bytes, void *stream) {
   MN_CHECK_ARG(n >= 0 && ndim >= 1 && ndim <= MN_MAX_NDIM, "downsample: bad n/ndim");
   MN_CHECK_ARG(spec != nullptr && spec->ndim == ndim, "downsample: key spec missing or of another ndim");
   MN_CHECK_ARG(tstride != nullptr && meta_out != nullptr && ctrl != nullptr, "downsample: null pointer");
@@ -551,6 +556,7 @@ extern "C" mn_status mn_downsample_coordinates(
   a.keys_out = keys_out;
   a.rows_out = unique_out;
   a.meta = meta_out;
+  a.meta_host = meta_host;
   a.num_clouds = (int)num_clouds;
   a.block_counts = block_counts;
   a.ctrl = ctrl;
@@ -699,8 +705,8 @@ mn_status run_mean(const void *features, int64_t channels, const Runs &r, void *
 template <typename F>
 mn_status run_voxelize(const F *points, int64_t n, int ndim, const double *voxel_size, const int64_t *batch_dims,
                        int64_t num_clouds, const void *features, int64_t channels, mn_dtype dtype,
-                       int32_t *voxels_out, int64_t *inverse_out, void *means_out, int64_t *meta_out, int32_t *ctrl,
-                       Workspace &ws, cudaStream_t st) {
+                       int32_t *voxels_out, int64_t *inverse_out, void *means_out, int64_t *meta_out,
+                       int64_t *meta_host, cudaEvent_t meta_event, int32_t *ctrl, Workspace &ws, cudaStream_t st) {
   Runs r{};
   r.keys = ws.take<uint64_t>(n);
   r.keys_tmp = ws.take<uint64_t>(n);
@@ -747,6 +753,7 @@ mn_status run_voxelize(const F *points, int64_t n, int ndim, const double *voxel
   u.spec = sort.spec;
   u.rows_out = voxels_out;
   u.meta = meta_out;
+  u.meta_host = meta_host;
   u.num_clouds = (int)num_clouds;
   u.block_counts = block_counts;
   u.ctrl = ctrl;
@@ -754,6 +761,8 @@ mn_status run_voxelize(const F *points, int64_t n, int ndim, const double *voxel
   u.run_start = r.run_start;
   u.inverse = inverse_out;
   MN_RETURN_IF(launch_unique_keys(u, st));
+  // the host goes on with the number of voxels while their means are still made
+  if (meta_event != nullptr) MN_CHECK_CUDA(cudaEventRecord(meta_event, st));
   if (features == nullptr) return MN_OK;
   switch (dtype) {
     case MN_F32: return run_mean<float>(features, channels, r, means_out, st);
@@ -774,8 +783,8 @@ extern "C" size_t mn_voxelize_workspace_bytes(int64_t n) {
 extern "C" mn_status mn_voxelize(const void *points, int points_are_double, int64_t n, int ndim,
                                  const double *voxel_size, const int64_t *batch_dims, int64_t num_clouds,
                                  const void *features, int64_t channels, mn_dtype dtype, int32_t *voxels_out,
-                                 int64_t *inverse_out, void *means_out, int64_t *meta_out, int32_t *ctrl,
-                                 void *ws_ptr, size_t ws_bytes, void *stream) {
+                                 int64_t *inverse_out, void *means_out, int64_t *meta_out, int64_t *meta_host,
+                                 void *meta_event, int32_t *ctrl, void *ws_ptr, size_t ws_bytes, void *stream) {
   MN_CHECK_ARG(n >= 1 && n < (1ll << 31) - 1 && ndim >= 1 && ndim <= MN_MAX_NDIM, "voxelize: bad n/ndim");
   if (batch_dims == nullptr) num_clouds = 1;
   MN_CHECK_ARG(num_clouds >= 1 && num_clouds < (1ll << 31), "voxelize: bad num_clouds");
@@ -788,9 +797,11 @@ extern "C" mn_status mn_voxelize(const void *points, int points_are_double, int6
   Workspace ws(ws_ptr, ws_bytes);
   if (points_are_double)
     return run_voxelize(static_cast<const double *>(points), n, ndim, voxel_size, batch_dims, num_clouds, features,
-                        channels, dtype, voxels_out, inverse_out, means_out, meta_out, ctrl, ws, st);
+                        channels, dtype, voxels_out, inverse_out, means_out, meta_out, meta_host,
+                        static_cast<cudaEvent_t>(meta_event), ctrl, ws, st);
   return run_voxelize(static_cast<const float *>(points), n, ndim, voxel_size, batch_dims, num_clouds, features,
-                      channels, dtype, voxels_out, inverse_out, means_out, meta_out, ctrl, ws, st);
+                      channels, dtype, voxels_out, inverse_out, means_out, meta_out, meta_host,
+                      static_cast<cudaEvent_t>(meta_event), ctrl, ws, st);
 }
 
 // ---------------------------------------------------------------------------

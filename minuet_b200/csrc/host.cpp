@@ -740,6 +740,8 @@ Tensor run_forward(Plan &plan, bool swapped, Tensor x, Tensor w, const Tensor &s
   const auto &sizes = plan.sizes();
   const int choice = pick_algorithm(plan, swapped, c_in, c_out, code, o);
   plan.last_algorithm = choice;
+  // weights that only their transpose is read of may stay a view (an input gradient's)
+  if (choice != kImplicit || code == MN_F32 || !w_t.has_value()) w = w.contiguous();
   Tensor out = empty_on(x, {T, c_out}, w.scalar_type());
   if (T == 0) return out;
   const cudaStream_t st = stream_of(x);
@@ -990,7 +992,7 @@ struct Convolution : torch::autograd::Function<Convolution> {
     const Tensor g = grads[0].to(w.scalar_type()).contiguous();
     if (ctx->needs_input_grad(0)) {
       // [O, c_out, c_in] weights; their transpose, which the tensor-core kernels read, is w
-      grad_x = run_forward(plan, !m.swapped, g, w.transpose(1, 2).contiguous(), m.tm, m.sm, m.order,
+      grad_x = run_forward(plan, !m.swapped, g, w.transpose(1, 2), m.tm, m.sm, m.order,
                            w.scalar_type() == at::kFloat ? OptTensor() : OptTensor(w), std::nullopt, std::nullopt,
                            std::nullopt, flipped(m.holder)->options);
     }

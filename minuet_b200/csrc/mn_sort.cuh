@@ -6,7 +6,7 @@
 // A digit pass moves every key once: a block takes the next tile of keys, ranks them in
 // registers (equal digits of a warp find each other with match.any), learns how many keys of
 // each digit the tiles before it hold by looking back over their published counts (every thread
-// follows two digits; a tile publishes its own count at once and the running total as soon as it
+// follows one or two digits; a tile publishes its own count at once and the running total as soon as it
 // knows it), reorders the tile in shared memory and writes it out in runs.  Tiles are numbered
 // in the order in which blocks start, so a block only ever waits for blocks that already run;
 // the waits are bounded all the same (status bit 4).  An index that travels with the keys sits
@@ -23,14 +23,14 @@
 #include "mn_pack.cuh"
 
 #include <algorithm>
+#include <type_traits>
 
 namespace mn {
 namespace rsort {
 
-constexpr int kThreads = 256;
-constexpr int kWarps = kThreads / 32;
+constexpr int kThreads = 256;                 // of the key kernel
 constexpr int kBits = 9;
-constexpr int kDigits = 1 << kBits;           // == 2 * kThreads: a thread per pair of digits
+constexpr int kDigits = 1 << kBits;
 constexpr int kMaxPasses = 8;                 // more than 64 / kBits
 constexpr uint32_t kSpinLimit = 1u << 22;
 
@@ -128,7 +128,7 @@ sort_keys_kernel(const __grid_constant__ Args a, const __grid_constant__ Source 
   }
 }
 
-// exclusive prefix of one value per thread over the block; s_part: [kWarps]
+// exclusive prefix of one value per thread over the block; s_part: [warps]
 __device__ __forceinline__ uint32_t block_exclusive(uint32_t v, uint32_t *s_part, int lane, int warp) {
   uint32_t inc = v;
 #pragma unroll
@@ -144,14 +144,18 @@ __device__ __forceinline__ uint32_t block_exclusive(uint32_t v, uint32_t *s_part
   return before + inc - v;
 }
 
-template <int kItems, bool kVals>
-__global__ void __launch_bounds__(kThreads)
+// A thread looks after kPer consecutive digits: two of them with 256 threads, one with 512.
+template <int kThr, int kItems, bool kVals>
+__global__ void __launch_bounds__(kThr, kItems == 16 ? 3 : kThr == 512 ? 2 : 4)
 sort_pass_kernel(const __grid_constant__ Args a, int pass) {
   begin_early();
-  constexpr int kTile = kThreads * kItems;
-  __shared__ uint64_t s_key[kTile];
-  // counts, then first positions inside the tile's digit, per warp and digit (at most kTile)
-  __shared__ __align__(8) uint16_t s_cnt[kWarps][kDigits];
+  constexpr int kTile = kThr * kItems, kWarps = kThr / 32, kPer = kDigits / kThr;
+  // the tile's keys; before that, the warps' counts per digit, then their first positions inside the
+  // tile's digit (at most kTile)
+  constexpr int kShared = kTile * 8 > kWarps * kDigits * 2 ? kTile * 8 : kWarps * kDigits * 2;
+  __shared__ __align__(16) unsigned char s_raw[kShared];
+  uint64_t *s_key = reinterpret_cast<uint64_t *>(s_raw);
+  uint16_t (*s_cnt)[kDigits] = reinterpret_cast<uint16_t (*)[kDigits]>(s_raw);
   __shared__ uint32_t s_local[kDigits];              // first position of a digit inside the tile
   __shared__ uint32_t s_dest[kDigits];               // its first position in the output, minus s_local
   __shared__ uint32_t s_part[kWarps];
@@ -162,11 +166,15 @@ sort_pass_kernel(const __grid_constant__ Args a, int pass) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const unsigned lt = lanes_below();
   if (tid == 0) s_tile = (int)atomicAdd(a.next_tile + pass, 1u);
+  for (int i = tid; i < kWarps * kDigits / 2; i += kThr) reinterpret_cast<uint32_t *>(&s_cnt[0][0])[i] = 0u;
+  // where this thread's digits start in the output (every block adds up the totals itself)
+  uint32_t totals[kPer], all = 0u;
 #pragma unroll
-  for (int w = 0; w < kWarps; w++) reinterpret_cast<uint32_t *>(s_cnt[w])[tid] = 0u;
-  // where this thread's two digits start in the output (every block adds up the totals itself)
-  const uint2 totals = __ldcg(reinterpret_cast<const uint2 *>(a.hist + pass * kDigits) + tid);
-  const uint32_t digit_start = block_exclusive(totals.x + totals.y, s_part, lane, warp);
+  for (int i = 0; i < kPer; i++) {
+    totals[i] = __ldcg(a.hist + pass * kDigits + kPer * tid + i);
+    all += totals[i];
+  }
+  const uint32_t digit_start = block_exclusive(all, s_part, lane, warp);
   const int tile = s_tile;
   if (tile >= a.tiles) return;
   if (tile == 0 && tid == 0 && last_pass && a.result_in_second != nullptr) *a.result_in_second = passes & 1;
@@ -194,57 +202,76 @@ sort_pass_kernel(const __grid_constant__ Args a, int pass) {
   }
   __syncthreads();
   // ---- per digit: the warps' first positions, the tile's count ---------------------------------
-  uint2 count = make_uint2(0u, 0u);
+  uint32_t count[kPer] = {};
 #pragma unroll
   for (int w = 0; w < kWarps; w++) {
-    uint32_t *at = reinterpret_cast<uint32_t *>(s_cnt[w]) + tid;    // two digits
-    const uint32_t c = *at;
-    *at = count.x | (count.y << 16);
-    count.x += c & 0xffffu;
-    count.y += c >> 16;
+    if constexpr (kPer == 2) {
+      uint32_t *at = reinterpret_cast<uint32_t *>(s_cnt[w]) + tid;    // two digits
+      const uint32_t c = *at;
+      *at = count[0] | (count[1] << 16);
+      count[0] += c & 0xffffu;
+      count[1] += c >> 16;
+    } else {
+      const uint32_t c = s_cnt[w][tid];
+      s_cnt[w][tid] = (uint16_t)count[0];
+      count[0] += c;
+    }
   }
-  // a published word: 2 * value + (running total ? 1 : 0) + 1; 0: nothing yet.  A thread's two
-  // words are one 8-byte access, so both say the same about what they hold.
-  volatile uint64_t *state = reinterpret_cast<uint64_t *>(a.state + ((size_t)pass * a.tiles) * kDigits) + tid;
-  constexpr int kPairs = kDigits / 2;
-  auto publish = [&](uint32_t x, uint32_t y, uint32_t mark) {
-    state[(size_t)tile * kPairs] = (uint64_t)(2u * x + mark) | ((uint64_t)(2u * y + mark) << 32);
+  // A published word: 2 * value + (running total ? 1 : 0) + 1; 0: nothing yet.  A thread's words are
+  // one access, so two of them say the same about what they hold.
+  using Word = std::conditional_t<kPer == 2, uint64_t, uint32_t>;
+  constexpr int kWords = kDigits / kPer;
+  volatile Word *state = reinterpret_cast<Word *>(a.state + ((size_t)pass * a.tiles) * kDigits) + tid;
+  auto publish = [&](const uint32_t (&v)[kPer], uint32_t mark) {
+    Word w = (Word)(2u * v[0] + mark);
+    if constexpr (kPer == 2) w |= (Word)(2u * v[1] + mark) << 32;
+    state[(size_t)tile * kWords] = w;
   };
-  publish(count.x, count.y, tile == 0 ? 2u : 1u);
-  const uint32_t local = block_exclusive(count.x + count.y, s_part, lane, warp);
+  publish(count, tile == 0 ? 2u : 1u);
+  uint32_t sum = 0u;
+#pragma unroll
+  for (int i = 0; i < kPer; i++) sum += count[i];
+  uint32_t local = block_exclusive(sum, s_part, lane, warp);
   // ---- look back: keys of these digits in the tiles before --------------------------------------
-  uint2 before = make_uint2(0u, 0u);
+  uint32_t before[kPer] = {};
   if (tile > 0) {
     uint32_t spins = 0;
     for (int prev = tile - 1; prev >= 0;) {
-      const uint64_t v = state[(size_t)prev * kPairs];
-      const uint32_t x = (uint32_t)v, y = (uint32_t)(v >> 32);
+      const Word v = state[(size_t)prev * kWords];
+      const uint32_t x = (uint32_t)v;
       if (x == 0u) {
         if (++spins > a.wait_limit) { atomicOr(a.status, MN_STATUS_GRID_TIMEOUT); break; }
         continue;
       }
-      before.x += (x - 1u) >> 1;
-      before.y += (y - 1u) >> 1;
+      before[0] += (x - 1u) >> 1;
+      if constexpr (kPer == 2) before[1] += ((uint32_t)(v >> 32) - 1u) >> 1;
       if (((x - 1u) & 1u) != 0u) break;
       prev--;
     }
-    publish(before.x + count.x, before.y + count.y, 2u);
+    uint32_t upto[kPer];
+#pragma unroll
+    for (int i = 0; i < kPer; i++) upto[i] = before[i] + count[i];
+    publish(upto, 2u);
   }
-  s_local[2 * tid] = local;
-  s_local[2 * tid + 1] = local + count.x;
-  s_dest[2 * tid] = digit_start + before.x - local;
-  s_dest[2 * tid + 1] = digit_start + totals.x + before.y - (local + count.x);
+  uint32_t start = digit_start;
+#pragma unroll
+  for (int i = 0; i < kPer; i++) {
+    s_local[kPer * tid + i] = local;
+    s_dest[kPer * tid + i] = start + before[i] - local;
+    local += count[i];
+    start += totals[i];
+  }
   __syncthreads();
   // ---- reorder in shared memory, write in runs -------------------------------------------------
 #pragma unroll
   for (int j = 0; j < kItems; j++) {
-    if (base + j * 32 < a.n) {
-      const unsigned d = (unsigned)(key[j] >> shift) & (kDigits - 1);
-      const uint32_t pos = s_local[d] + s_cnt[warp][d] + rank[j];
-      rank[j] = (uint16_t)pos;
-      s_key[pos] = key[j];
-    }
+    const unsigned d = (unsigned)(key[j] >> shift) & (kDigits - 1);
+    if (base + j * 32 < a.n) rank[j] = (uint16_t)(s_local[d] + s_cnt[warp][d] + rank[j]);
   }
+  __syncthreads();                                    // the counts have been read: keys take their place
+#pragma unroll
+  for (int j = 0; j < kItems; j++)
+    if (base + j * 32 < a.n) s_key[rank[j]] = key[j];
   __syncthreads();
   const int in_tile = (int)min((int64_t)kTile, a.n - (int64_t)tile * kTile);
   const bool write_index = last_pass && (a.index32 != nullptr || a.index64 != nullptr);
@@ -253,7 +280,7 @@ sort_pass_kernel(const __grid_constant__ Args a, int pass) {
   uint32_t dest[kItems];
 #pragma unroll
   for (int j = 0; j < kItems; j++) {
-    const int i = j * kThreads + tid;
+    const int i = j * kThr + tid;
     if (i < in_tile) {
       const uint64_t k = s_key[i];
       // After a look-back that timed out (status bit 4) keys may land on one another and leave
@@ -280,7 +307,7 @@ sort_pass_kernel(const __grid_constant__ Args a, int pass) {
     int32_t *vout = a.vals[(pass & 1) ^ 1];
 #pragma unroll
     for (int j = 0; j < kItems; j++) {
-      const int i = j * kThreads + tid;
+      const int i = j * kThr + tid;
       if (i < in_tile) {
         const int32_t v = (int32_t)min((uint32_t)s_val[i], (uint32_t)a.n - 1u);
         if (!write_index) vout[dest[j]] = v;
@@ -291,10 +318,21 @@ sort_pass_kernel(const __grid_constant__ Args a, int pass) {
   }
 }
 
-// 4096 keys per tile; 1024 where those would leave SMs without a tile (a pass is then a chain of
-// latencies, and smaller tiles shorten every link).
-inline int items_of(int64_t n) { return n < 4096ll * kNumSMs ? 4 : 16; }
-inline int64_t tiles_of(int64_t n) { return div_up(std::max<int64_t>(n, 1), (int64_t)kThreads * items_of(n)); }
+// Threads and keys per thread of a tile.  Every tile that runs at the same time lengthens the look-back, so
+// tiles are large: 4096 keys, with 512 threads up to two tiles per SM and with 256 beyond (three
+// blocks of 80 registers share an SM: at 128 registers and two, 7.3 M keys took 7 % longer); 1024
+// keys where larger ones would leave SMs without a tile.  Measured, all passes, us for 256 x 4 / 512 x 8 /
+// 256 x 16: 30k keys 29 / 37 / 39; 120k 45 / 51 / 53; 250k 64 / 59 / 62; 464k 80 / 74 / 78; 900k 115 / 94 /
+// 100; 1.9 M 184 / 141 / 127; 7.3 M 755 / 491 / 445.
+struct TileShape { int threads, items; };
+inline TileShape tile_shape(int64_t n) {
+  if (n < 1024ll * kNumSMs) return TileShape{256, 4};
+  return n < 2 * 4096ll * kNumSMs ? TileShape{512, 8} : TileShape{256, 16};
+}
+inline int64_t tiles_of(int64_t n) {
+  const TileShape s = tile_shape(n);
+  return div_up(std::max<int64_t>(n, 1), (int64_t)s.threads * s.items);
+}
 inline size_t control_words(int64_t n, int passes) {
   return (size_t)kMaxPasses * kDigits + 64 + (size_t)passes * tiles_of(n) * kDigits;
 }
@@ -306,13 +344,13 @@ inline int bits_for(int64_t values) {    // bits that tell `values` different va
   return b;
 }
 
-template <int kItems>
+template <int kThr, int kItems>
 mn_status launch_passes(const Args &a, int launches, cudaStream_t st) {
   for (int p = 0; p < launches; p++) {
     if (a.vals[0] != nullptr) {
-      MN_LAUNCH("sort_pass_kernel", st, launch_early(sort_pass_kernel<kItems, true>, a.tiles, kThreads, 0, st, a, p));
+      MN_LAUNCH("sort_pass_kernel", st, launch_early(sort_pass_kernel<kThr, kItems, true>, a.tiles, kThr, 0, st, a, p));
     } else {
-      MN_LAUNCH("sort_pass_kernel", st, launch_early(sort_pass_kernel<kItems, false>, a.tiles, kThreads, 0, st, a, p));
+      MN_LAUNCH("sort_pass_kernel", st, launch_early(sort_pass_kernel<kThr, kItems, false>, a.tiles, kThr, 0, st, a, p));
     }
   }
   return MN_OK;
@@ -336,7 +374,9 @@ mn_status run(Args a, const Source &source, Workspace &ws, cudaStream_t st) {
   MN_CHECK_CUDA(cudaMemsetAsync(control, 0, control_words(a.n, launches) * sizeof(uint32_t), st));
   const int blocks = (int)std::min<int64_t>(kNumSMs * 8, div_up(a.n, kThreads));
   MN_LAUNCH("sort_keys_kernel", st, launch_early(sort_keys_kernel<Source>, blocks, kThreads, 0, st, a, source));
-  return items_of(a.n) == 4 ? launch_passes<4>(a, launches, st) : launch_passes<16>(a, launches, st);
+  const TileShape shape = tile_shape(a.n);
+  if (shape.threads == 512) return launch_passes<512, 8>(a, launches, st);
+  return shape.items == 4 ? launch_passes<256, 4>(a, launches, st) : launch_passes<256, 16>(a, launches, st);
 }
 
 }  // namespace rsort

@@ -5,7 +5,7 @@
 // Python side loaded is the one that runs.
 //
 // A layer on a small cloud is bound by host time: one launch of a few microseconds took 55 us
-// of interpreter and ctypes work, a kernel map 98; from here 14 and 48.
+// of interpreter and ctypes work, a kernel map 98; from here 14 and 38.
 #include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDACachingAllocator.h>

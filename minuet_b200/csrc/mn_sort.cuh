@@ -325,8 +325,9 @@ sort_pass_kernel(const __grid_constant__ Args a, int pass) {
 // 256 x 16: 30k keys 29 / 37 / 39; 120k 45 / 51 / 53; 250k 64 / 59 / 62; 464k 80 / 74 / 78; 900k 115 / 94 /
 // 100; 1.9 M 184 / 141 / 127; 7.3 M 755 / 491 / 445.
 struct TileShape { int threads, items; };
+constexpr int64_t kFewKeys = 1024ll * kNumSMs;
 inline TileShape tile_shape(int64_t n) {
-  if (n < 1024ll * kNumSMs) return TileShape{256, 4};
+  if (n < kFewKeys) return TileShape{256, 4};
   return n < 2 * 4096ll * kNumSMs ? TileShape{512, 8} : TileShape{256, 16};
 }
 inline int64_t tiles_of(int64_t n) {
@@ -336,7 +337,12 @@ inline int64_t tiles_of(int64_t n) {
 inline size_t control_words(int64_t n, int passes) {
   return (size_t)kMaxPasses * kDigits + 64 + (size_t)passes * tiles_of(n) * kDigits;
 }
-inline size_t workspace_bytes(int64_t n) { return align_up(control_words(n, kMaxPasses) * sizeof(uint32_t), 256) + 256; }
+// Enough for any number of keys up to n: the most of the small tiles are more than the large ones of up to
+// four times as many keys.
+inline size_t workspace_bytes(int64_t n) {
+  const size_t words = std::max(control_words(n, kMaxPasses), control_words(std::min(n, kFewKeys - 1), kMaxPasses));
+  return align_up(words * sizeof(uint32_t), 256) + 256;
+}
 
 inline int bits_for(int64_t values) {    // bits that tell `values` different values apart, at least 1
   int b = 1;

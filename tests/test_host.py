@@ -76,6 +76,20 @@ def test_plan_buckets_matches_oracle(mn_lib, oracle_lib):
             assert cumsum.tolist() == want_c.tolist()
 
 
+def test_workspace_for_some_rows_holds_fewer_rows(mn_lib):
+    # a caller sizes its buffer once, for the most rows it expects: at the row counts around which the
+    # sort's tiles change size (1024 and 2 * 4096 keys per SM of 148), and between them
+    rows = sorted({0, 1, 1023, 1024, 4096, 10 ** 7} | {
+        max(0, edge + d) for edge in (1024 * 148, 4096 * 148, 2 * 4096 * 148) for d in (-4097, -1, 0, 1, 48_448)})
+    none = np.zeros(1, dtype=np.int32).ctypes.data_as(ctypes.c_void_p)
+    for name, nbytes in (("map", lambda n: mn_lib.mn_map_workspace_bytes(n, n, 1)),
+                         ("map, sources", lambda n: mn_lib.mn_map_workspace_bytes(n, 5, 27)),
+                         ("voxelize", mn_lib.mn_voxelize_workspace_bytes),
+                         ("table", lambda n: mn_lib.mn_neighbor_table_workspace_bytes(none, 1, n))):
+        sizes = [nbytes(n) for n in rows]
+        assert sizes == sorted(sizes), (name, list(zip(rows, sizes)))
+
+
 def test_keyspec_layout(mn_lib):
     mm = np.array([-5, 0, 10, 0, 100, 7, 10, 0], np.int32)
     spec = _lib.KeySpec()

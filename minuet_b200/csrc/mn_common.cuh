@@ -92,20 +92,30 @@ __device__ __forceinline__ void begin_early() {
   release_successor();
 }
 
+// The same in clusters of `cluster` blocks along x (grid.x a multiple of it).
 template <typename... Params, typename... Args>
-inline void launch_early(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
-                         Args &&...args) {
+inline void launch_early_clusters(void (*kernel)(Params...), unsigned cluster, dim3 grid, dim3 block, size_t smem,
+                                  cudaStream_t st, Args &&...args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
+  cudaLaunchAttribute attr[2]{};
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
   (void)cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);   // errors: MN_CHECK_LAUNCH
+}
+
+template <typename... Params, typename... Args>
+inline void launch_early(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                         Args &&...args) {
+  launch_early_clusters(kernel, 1u, grid, block, smem, st, std::forward<Args>(args)...);
 }
 
 // Optional phase timing of a kernel (builds with -DMN_PHASE_TIMING only): thread 0

@@ -16,13 +16,17 @@
 // that have the offset, picked from anywhere in the block, so that next to no zeros are multiplied.  A
 // block lists these items offset by offset and deals them out to its warps in turn; each warp
 // runs its own ring of copies and waits for no other, except that products enter the sums in the
-// order of the list, handed from warp to warp.  So the offsets of a tile are worked on side by side: a
-// tile with 27 of them is no longer a chain of 27 steps that the whole chip waits for, and few
-// rows (the coarse levels of a network) fill the chip without products in global memory and a
-// second launch that adds them.
+// order of the list, handed from warp to warp.  So the offsets of a tile are worked on side by side, and a
+// tile with 27 of them is no chain of 27 steps that the whole chip waits for.
+//
+// Few rows (the coarse levels of a network) leave SMs without a block, and a block of eight warps with 27
+// items runs four products one after the other: there a cluster of eight blocks shares a tile's
+// list.  Every product stays in the shared memory of the block that made it, and after a barrier of the
+// cluster each block adds the products of some of the rows, in the same order.
 #include "mn_common.cuh"
 
 #include <algorithm>
+#include <type_traits>
 
 namespace mn {
 
@@ -57,17 +61,17 @@ __device__ __forceinline__ void cs_copy_4(void *dst, const void *src, uint32_t s
                : "memory");
 }
 
+__device__ __forceinline__ float cs_epilogue(float f, const CsArgs &a, int64_t row, int c) {
+  if (a.scale != nullptr) f *= __ldg(a.scale + c);
+  if (a.shift != nullptr) f += __ldg(a.shift + c);
+  if (a.residual != nullptr) f += __ldg(a.residual + row * a.N + c);
+  return a.relu ? fmaxf(f, 0.f) : f;
+}
 __device__ __forceinline__ float4 cs_epilogue(float4 v, const CsArgs &a, int64_t row, int c) {
   float f[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-  for (int j = 0; j < 4; j++) {
-    if (c + j < a.N) {
-      if (a.scale != nullptr) f[j] *= __ldg(a.scale + c + j);
-      if (a.shift != nullptr) f[j] += __ldg(a.shift + c + j);
-      if (a.residual != nullptr) f[j] += __ldg(a.residual + row * a.N + c + j);
-      if (a.relu) f[j] = fmaxf(f[j], 0.f);
-    }
-  }
+  for (int j = 0; j < 4; j++)
+    if (c + j < a.N) f[j] = cs_epilogue(f[j], a, row, c + j);
   return make_float4(f[0], f[1], f[2], f[3]);
 }
 
@@ -82,10 +86,31 @@ __device__ __forceinline__ void cs_turn_pass(int id) {
   asm volatile("bar.arrive %0, 64;" ::"r"(id) : "memory");
 }
 
-// BM x (32 kCols) sums per block of W warps, a product of 32 x 32 per warp, 8 x 4 of it per thread.
-// Blocks take the tiles from the last to the first: the rows with rare offsets sort to the end, and
-// their tiles take longest.  At most cs_cap(BM) offsets are looked at at a time (index blocks in
-// shared memory).  kVec: rows of the features and of the weights can be copied 16 bytes at a time.
+// Blocks of a cluster: what every block wrote before its arrival can be read by the others after their wait.
+__device__ __forceinline__ void cs_cluster_arrive() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cs_cluster_wait() {
+  __syncwarp();
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// the value at `at` in the shared memory of another block of the cluster
+__device__ __forceinline__ float cs_load_from(const float *at, int block) {
+  uint32_t addr;
+  float v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+               : "=r"(addr) : "r"((uint32_t)__cvta_generic_to_shared(at)), "r"(block));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+  return v;
+}
+
+// BM x (32 kCols) sums per block of W warps or per cluster of kCluster of them, a product of 32 x 32 per warp,
+// 8 x 4 of it per thread.  Blocks take the tiles from the last to the first: the rows with rare
+// offsets sort to the end, and their tiles take longest.  At most cs_cap offsets are looked at at a
+// time (index blocks in shared memory).  kVec: rows of the features and of the weights can be copied 16
+// bytes at a time.  kFew: an item of up to 16 rows costs half as much (maps of 3.5 pairs a row: 32-row tiles
+// take 15 % less time); not for the tall blocks of large maps, whose full items the second loop body costs 10 %.
 //
 // What bounds it: instruction issue.  Of 56 M warp instructions of a layer of 3.6k rows 128->128 with 14.5
 // pairs 38 M run on the FMA pipe, 27 M of them useful products, and a scheduler issues in 61 % of
@@ -95,30 +120,43 @@ __device__ __forceinline__ void cs_turn_pass(int id) {
 // Against a block of 64 x 64 (or 32 x 32) sums in registers that walked its tile's offsets one after
 // the other, and a second launch for maps of few rows (us): 59k rows 32->32, 3 pairs 67 -> 34; 42k
 // 64->32, 7.5 pairs 146 -> 78; 16k 64->64, 12.5 pairs 137 -> 85; 16k 128->64 262 -> 150; 3.6k 128->128,
-// 14.5 pairs 108 -> 95; 700 256->256 131 -> 122; 196k 64->64, 3 pairs 228 -> 213; 50k 32->32, 1.1
-// pairs 30 -> 17; 59k 3->32 98 -> 21.
-constexpr int cs_cap(int bm) { return bm == 32 ? kCsMaxOffsets : 16; }
-constexpr size_t cs_smem(int bm, int cols, int warps, int stages) {
-  return (size_t)warps * stages * kCsStageFloats * 4 + (size_t)bm * cols * kCsRows * 4 + (size_t)cs_cap(bm) * bm * 5;
+// 14.5 pairs 108 -> 95; 196k 64->64, 3 pairs 228 -> 213; 50k 32->32, 1.1 pairs 29 -> 15; 59k 3->32 98 -> 21.
+// Clusters against that second launch, 8 to 21 pairs: 13 rows 256->256 25 -> 15, 64->64 16 -> 8; 130 rows 128->128 23
+// -> 16; 325 rows 256->64 37 -> 28; 700 rows 256->256 137 -> 128 (3.5 pairs 79 -> 63).
+constexpr int cs_cap(int bm, int cluster) { return bm == 32 || cluster > 1 ? kCsMaxOffsets : 16; }
+// items of one block of a cluster at most
+constexpr int cs_share(int bm, int cluster) { return kCsMaxOffsets * (bm / kCsRows) / cluster; }
+constexpr size_t cs_smem(int bm, int cols, int warps, int stages, int cluster) {
+  return (size_t)warps * stages * kCsStageFloats * 4 + (size_t)cs_cap(bm, cluster) * bm * 5 +
+         (size_t)(cluster > 1 ? cs_share(bm, cluster) * kCsRows : bm * cols) * kCsRows * 4;
 }
 
-template <int BM, int kCols, int W, int kStages, bool kVec>
-__global__ void __launch_bounds__(W * 32, W == 4 ? (cs_smem(BM, kCols, W, kStages) <= 55 * 1024 ? 4 : 3) : 2)
+template <int BM, int kCols, int W, int kStages, int kCluster, bool kVec>
+__global__ void __launch_bounds__(W * 32, W == 4 ? (cs_smem(BM, kCols, W, kStages, kCluster) <= 55 * 1024 ? 4 : 3) : 2)
 conv_simt_kernel(const __grid_constant__ CsArgs a) {
   begin_early();
-  constexpr int kThreads = W * 32, kSubs = BM / 32, kCap = cs_cap(BM), kSumCols = kCols * kCsRows;
-  constexpr bool kDirect = BM > 32;
+  constexpr int kThreads = W * 32, kSubs = BM / 32, kCap = cs_cap(BM, kCluster), kSumCols = kCols * kCsRows;
+  constexpr int kTeam = W * kCluster;                // warps of a tile
+  constexpr bool kDirect = BM > 32 && kCluster == 1;
+  constexpr bool kFew = BM == 32 || kCluster > 1;
+  static_assert(kCluster == 1 || (kCols == 1 && kCap == kCsMaxOffsets), "clusters: one list of items per tile");
   extern __shared__ __align__(16) float s_mem[];
   __shared__ int32_t s_active[kCsMaxOffsets], s_weight[kCsMaxOffsets];
   __shared__ uint8_t s_have[kCap];                // rows that have the offset
   __shared__ uint16_t s_items[kCap * kSubs * kCols];   // offset of the chunk | 32 of its rows << 5 | 32 columns << 8
+  __shared__ uint8_t s_first[kCap];               // an offset's first item
+  __shared__ uint32_t s_present;                  // offsets that have items
   __shared__ int32_t s_count, s_perm[BM];
-  float *s_sum = s_mem + W * kStages * kCsStageFloats;                  // [BM][kSumCols]
-  int32_t *s_idx = reinterpret_cast<int32_t *>(s_sum + BM * kSumCols);   // [kCap][BM]: source rows, then those that exist
-  uint8_t *s_row = reinterpret_cast<uint8_t *>(s_idx + kCap * BM);      // [kCap][BM]: the block's rows they feed
+  // the sums [BM][kSumCols]; in a cluster the products of this block's items [item][32][32]
+  float *s_sum = s_mem + W * kStages * kCsStageFloats;
+  constexpr int kSums = kCluster > 1 ? cs_share(BM, kCluster) * kCsRows * kCsRows : BM * kSumCols;
+  int32_t *s_idx = reinterpret_cast<int32_t *>(s_sum + kSums);          // [kCap][BM]: source rows, then those that exist
+  // [kCap][BM]: the block's rows they feed; in a cluster the other way round, a row's place among them (none: 0xff)
+  uint8_t *s_row = reinterpret_cast<uint8_t *>(s_idx + kCap * BM);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int tx = lane % 8, ty = lane / 8;
-  const int64_t r0 = (int64_t)(gridDim.x - 1 - blockIdx.x) * BM;
+  const int rank = (int)(blockIdx.x % kCluster);                         // of this block in its cluster
+  const int64_t r0 = (int64_t)((gridDim.x - 1 - blockIdx.x) / kCluster) * BM;
   const int n0 = blockIdx.y * kSumCols;
   float *ring = s_mem + warp * kStages * kCsStageFloats;
 
@@ -151,7 +189,8 @@ conv_simt_kernel(const __grid_constant__ CsArgs a) {
   };
   // One offset, and every row has it (most blocks of a sparse map): the products are the sums.
   bool direct = false;
-  if (n_bits == 0) clear_sums();
+  int n_items = 0;
+  if (kCluster == 1 && n_bits == 0) clear_sums();
 
   for (int chunk = 0; chunk < n_bits; chunk += kCap) {
     __syncthreads();
@@ -175,7 +214,10 @@ conv_simt_kernel(const __grid_constant__ CsArgs a) {
         if (source[sub] >= 0) {
           const int at = n + __popc(hit & ((1u << lane) - 1u));
           s_idx[j * BM + at] = source[sub];
-          s_row[j * BM + at] = (uint8_t)(sub * 32 + lane);
+          if (kCluster == 1) s_row[j * BM + at] = (uint8_t)(sub * 32 + lane);
+          else s_row[j * BM + sub * 32 + lane] = (uint8_t)at;
+        } else if (kCluster > 1) {
+          s_row[j * BM + sub * 32 + lane] = (uint8_t)0xff;
         }
         n += __popc(hit);
       }
@@ -184,7 +226,7 @@ conv_simt_kernel(const __grid_constant__ CsArgs a) {
     }
     __syncthreads();
     direct = kDirect && n_bits == 1 && s_have[0] == (int)min((int64_t)BM, a.T - r0);
-    if (chunk == 0 && !direct) clear_sums();
+    if (kCluster == 1 && chunk == 0 && !direct) clear_sums();
     if (warp == 0) {
       const int mine = lane < n_chunk ? (s_have[lane % kCap] + 31) / 32 * tiles : 0;
       int end = mine;
@@ -193,17 +235,25 @@ conv_simt_kernel(const __grid_constant__ CsArgs a) {
         const int t = __shfl_up_sync(0xffffffffu, end, d);
         if (lane >= d) end += t;
       }
+      if (kCluster > 1 && lane < n_chunk) s_first[lane % kCap] = (uint8_t)(end - mine);
       for (int g = 0; g < mine; g++) s_items[end - mine + g] = (uint16_t)(lane | ((g / tiles) << 5) | ((g % tiles) << 8));
       if (lane == 31) s_count = end;
+      const uint32_t present = __ballot_sync(0xffffffffu, mine > 0);
+      if (kCluster > 1 && lane == 0) s_present = present;
     }
     __syncthreads();
-    const int n_items = s_count;
-    const int n_step = (n_items > warp ? (n_items - warp + W - 1) / W : 0) * a.k_steps;
+    n_items = s_count;
+    // item i is worked on by block i % kCluster, so that a tile with few items has them on as many SMs
+    const int first_item = warp * kCluster + rank;
+    const int n_step = (n_items > first_item ? (n_items - first_item + kTeam - 1) / kTeam : 0) * a.k_steps;
 
+    // kFew: rows 16 to 31 of an item of up to 16 are neither copied nor multiplied (rare offsets: a few rows each)
+    auto few_rows = [&](int entry) { return kFew && (int)s_have[entry & 31] - ((entry >> 5) & 7) * kCsRows <= kCsRows / 2; };
     // the cursor of the copies: item, first channel, ring stage; the item's rows and weights
-    int l_item = warp, l_k = 0, l_stage = 0;
+    int l_item = first_item, l_k = 0, l_stage = 0;
     const float *l_src[kCsRows / 8], *l_w = nullptr;
     uint32_t l_valid = 0u;
+    bool l_few = false;
     auto load_step = [&]() {
       float *sa = ring + l_stage * kCsStageFloats, *sb = sa + kCsK * kCsRows;
       const int item = s_items[l_item], j = item & 31;
@@ -212,6 +262,7 @@ conv_simt_kernel(const __grid_constant__ CsArgs a) {
       if constexpr (kVec) {
         const int c = (lane & 3) * 4;
         if (l_k == 0) {
+          if (kFew) l_few = few_rows(item);
           l_w = a.weights + ((int64_t)s_weight[chunk + j] * a.K + ty) * a.N + c0 + tx * 4;
           l_valid = 0u;
 #pragma unroll
@@ -225,7 +276,7 @@ conv_simt_kernel(const __grid_constant__ CsArgs a) {
         const int place = (((lane & 3) ^ ((lane >> 3) & 3)) << 2);   // pieces of row r: position ^ (r >> 1) & 3
 #pragma unroll
         for (int i = 0; i < kCsRows / 8; i++)
-          cs_copy_16(sa + (i * 8 + (lane >> 2)) * kCsK + place, (valid >> i) & 1u ? l_src[i] + l_k : a.in,
+          if (i < kCsRows / 16 || !kFew || !l_few) cs_copy_16(sa + (i * 8 + (lane >> 2)) * kCsK + place, (valid >> i) & 1u ? l_src[i] + l_k : a.in,
                      (valid >> i) & 1u ? 16u : 0u);
         const bool col = c0 + tx * 4 < a.N;
 #pragma unroll
@@ -236,12 +287,13 @@ conv_simt_kernel(const __grid_constant__ CsArgs a) {
         l_w += kCsK * (int64_t)a.N;
       } else {
         const float *w = a.weights + ((int64_t)s_weight[chunk + j] * a.K + l_k) * a.N + c0 + lane;
-        const bool col = c0 + lane < a.N;
+        const bool col = c0 + lane < a.N, item_few = few_rows(item);
         for (int k = 0; k < kCsK && l_k + k < a.K; k += 4) {      // the channels that are multiplied
           const int c = k + (lane & 3);
           const int place = (((k >> 2) ^ ((lane >> 3) & 3)) << 2) | (lane & 3);
 #pragma unroll
           for (int i = 0; i < kCsRows / 8; i++) {
+            if (kFew && i >= kCsRows / 16 && item_few) break;
             const int r = i * 8 + (lane >> 2), row = idx[r];
             const bool valid = row >= 0 && l_k + c < a.K;
             cs_copy_4(sa + r * kCsK + place, valid ? a.in + (int64_t)row * a.K + l_k + c : a.in, valid ? 4u : 0u);
@@ -255,7 +307,7 @@ conv_simt_kernel(const __grid_constant__ CsArgs a) {
       }
       asm volatile("cp.async.commit_group;" ::: "memory");
       l_k += kCsK;
-      if (l_k >= a.K) { l_k = 0; l_item += W; }
+      if (l_k >= a.K) { l_k = 0; l_item += kTeam; }
       if (++l_stage == kStages) l_stage = 0;
     };
     for (int s = 0; s < kStages - 1; s++) {
@@ -271,7 +323,13 @@ conv_simt_kernel(const __grid_constant__ CsArgs a) {
     int place[4];                                  // of the four-channel pieces of this lane's rows
 #pragma unroll
     for (int k = 0; k < 4; k++) place[k] = ty * kCsK + ((k ^ (ty >> 1)) << 2);
-    int item = warp, k0 = 0, stage = 0;
+    int item = first_item, k0 = 0, stage = 0;
+    bool few = n_step > 0 && few_rows(s_items[item]);
+    auto next_item = [&]() {
+      item += kTeam;
+      k0 = 0;
+      if (kFew && item < n_items) few = few_rows(s_items[item]);
+    };
     for (int step = 0; step < n_step; step++) {
       asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
       __syncwarp();
@@ -281,33 +339,49 @@ conv_simt_kernel(const __grid_constant__ CsArgs a) {
       const int kmax = min(kCsK, a.K - k0);        // zeros up to a multiple of 4
       if (++stage == kStages) stage = 0;
       k0 += kCsK;
+      auto multiply = [&](auto n) {
+        constexpr int kRows = decltype(n)::value;                  // of a lane
 #pragma unroll
-      for (int k = 0; k < kCsK; k += 4) {
-        if (k < kmax) {
-          float4 av[8], bv[4];
+        for (int k = 0; k < kCsK; k += 4) {
+          if (k < kmax) {
+            float4 av[kRows], bv[4];
 #pragma unroll
-          for (int i = 0; i < 8; i++)
-            av[i] = *reinterpret_cast<const float4 *>(sa + i * 4 * kCsK + place[(k / 4) ^ (2 * (i & 1))]);
+            for (int i = 0; i < kRows; i++)
+              av[i] = *reinterpret_cast<const float4 *>(sa + i * 4 * kCsK + place[(k / 4) ^ (2 * (i & 1))]);
 #pragma unroll
-          for (int j = 0; j < 4; j++) bv[j] = *reinterpret_cast<const float4 *>(sb + (k + j) * kCsRows);
+            for (int j = 0; j < 4; j++) bv[j] = *reinterpret_cast<const float4 *>(sb + (k + j) * kCsRows);
 #pragma unroll
-          for (int i = 0; i < 8; i++) {
-            const float ak[4] = {av[i].x, av[i].y, av[i].z, av[i].w};
+            for (int i = 0; i < kRows; i++) {
+              const float ak[4] = {av[i].x, av[i].y, av[i].z, av[i].w};
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-              acc[i][0] = fmaf(ak[j], bv[j].x, acc[i][0]);
-              acc[i][1] = fmaf(ak[j], bv[j].y, acc[i][1]);
-              acc[i][2] = fmaf(ak[j], bv[j].z, acc[i][2]);
-              acc[i][3] = fmaf(ak[j], bv[j].w, acc[i][3]);
+              for (int j = 0; j < 4; j++) {
+                acc[i][0] = fmaf(ak[j], bv[j].x, acc[i][0]);
+                acc[i][1] = fmaf(ak[j], bv[j].y, acc[i][1]);
+                acc[i][2] = fmaf(ak[j], bv[j].z, acc[i][2]);
+                acc[i][3] = fmaf(ak[j], bv[j].w, acc[i][3]);
+              }
             }
           }
         }
-      }
+      };
+      if (kFew && few) multiply(std::integral_constant<int, 4>());
+      else multiply(std::integral_constant<int, 8>());
       if (k0 < a.K) continue;
       // the product is complete: it is added when the items before it have been
       const int entry = s_items[item], j0 = entry & 31, first = ((entry >> 5) & 7) * 32 + ty;
       const int left = s_have[j0] - first;
       const uint8_t *rows = s_row + j0 * BM + first;
+      if constexpr (kCluster > 1) {
+        float4 *product = reinterpret_cast<float4 *>(s_sum + (item / kCluster * kCsRows + ty) * kCsRows) + tx;
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+          if (4 * i < left) product[i * 4 * (kCsRows / 4)] = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+#pragma unroll
+          for (int j = 0; j < 4; j++) acc[i][j] = 0.f;
+        }
+        next_item();
+        continue;
+      }
       if (kDirect && direct) {
 #pragma unroll
         for (int i = 0; i < 8; i++) {
@@ -317,8 +391,7 @@ conv_simt_kernel(const __grid_constant__ CsArgs a) {
 #pragma unroll
           for (int j = 0; j < 4; j++) acc[i][j] = 0.f;
         }
-        item += W;
-        k0 = 0;
+        next_item();
         continue;
       }
       if (W > 1 && item > 0) cs_turn_wait(1 + warp);
@@ -336,9 +409,42 @@ conv_simt_kernel(const __grid_constant__ CsArgs a) {
       if (W > 1 && item + 1 < n_items) {
         cs_turn_pass(1 + (warp + 1) % W);
       }
-      item += W;
-      k0 = 0;
+      next_item();
     }
+  }
+  if constexpr (kCluster > 1) {
+    // every block adds the products of some rows, read from where they are, in the order of the list
+    constexpr int kRows = BM / kCluster, kBatch = 8;
+    asm volatile("cp.async.wait_all;" ::: "memory");      // (s_perm of a tile without offsets)
+    cs_cluster_arrive();
+    cs_cluster_wait();
+    const uint32_t present = n_bits > 0 ? s_present : 0u;
+    const int c = n0 + lane;
+    for (int r = rank * kRows + warp; r < (rank + 1) * kRows; r += W) {
+      float sum = 0.f;
+      for (uint32_t left = present; left != 0u;) {
+        float v[kBatch];
+#pragma unroll
+        for (int q = 0; q < kBatch; q++) {
+          const int j = left != 0u ? __ffs(left) - 1 : 0;
+          const int at = left != 0u ? s_row[j * BM + r] : 0xff;
+          left &= left - 1u;
+          v[q] = 0.f;
+          if (at == 0xff) continue;
+          const int item = s_first[j] + at / kCsRows;
+          v[q] = cs_load_from(s_sum + (item / kCluster * kCsRows + at % kCsRows) * kCsRows + lane, item % kCluster);
+        }
+#pragma unroll
+        for (int q = 0; q < kBatch; q++) sum += v[q];     // (a zero for a row without the offset changes no bit)
+      }
+      if (r0 + r < a.T && c < a.N) {
+        const int64_t t = a.perm != nullptr ? (int64_t)s_perm[r] : r0 + r;
+        a.out[t * a.N + c] = cs_epilogue(sum, a, t, c);
+      }
+    }
+    cs_cluster_arrive();
+    cs_cluster_wait();                                    // the others have read this block's products
+    return;
   }
   if (kDirect && direct) return;
   asm volatile("cp.async.wait_all;" ::: "memory");
@@ -350,28 +456,24 @@ conv_simt_kernel(const __grid_constant__ CsArgs a) {
   }
 }
 
-template <int BM, int kCols, int W, int kStages>
+template <int BM, int kCols, int W, int kStages, int kCluster = 1>
 mn_status launch_cs(const CsArgs &a, cudaStream_t st) {
   const bool vec = a.K % 4 == 0 && a.N % 4 == 0 &&
                    ((reinterpret_cast<uintptr_t>(a.in) | reinterpret_cast<uintptr_t>(a.weights)) & 15) == 0;
-  constexpr size_t smem = cs_smem(BM, kCols, W, kStages);
-  const dim3 grid((unsigned)div_up(a.T, BM), (unsigned)div_up(a.N, kCols * kCsRows));
+  constexpr size_t smem = cs_smem(BM, kCols, W, kStages, kCluster);
+  const dim3 grid((unsigned)(div_up(a.T, BM) * kCluster), (unsigned)div_up(a.N, kCols * kCsRows));
   static thread_local bool sized[kMaxDevices] = {false};
   int device = 0;
   MN_CHECK_CUDA(cudaGetDevice(&device));
   MN_CHECK_ARG(device >= 0 && device < kMaxDevices, "fp32 forward: device index %d out of range", device);
+  const auto with_vec = conv_simt_kernel<BM, kCols, W, kStages, kCluster, true>;
+  const auto by_element = conv_simt_kernel<BM, kCols, W, kStages, kCluster, false>;
   if (!sized[device]) {
-    MN_CHECK_CUDA(cudaFuncSetAttribute(conv_simt_kernel<BM, kCols, W, kStages, true>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    MN_CHECK_CUDA(cudaFuncSetAttribute(conv_simt_kernel<BM, kCols, W, kStages, false>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    MN_CHECK_CUDA(cudaFuncSetAttribute(with_vec, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    MN_CHECK_CUDA(cudaFuncSetAttribute(by_element, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     sized[device] = true;
   }
-  if (vec) {
-    MN_LAUNCH("conv_simt_kernel", st, launch_early(conv_simt_kernel<BM, kCols, W, kStages, true>, grid, W * 32, smem, st, a));
-  } else {
-    MN_LAUNCH("conv_simt_kernel", st, launch_early(conv_simt_kernel<BM, kCols, W, kStages, false>, grid, W * 32, smem, st, a));
-  }
+  MN_LAUNCH("conv_simt_kernel", st, launch_early_clusters(vec ? with_vec : by_element, kCluster, grid, W * 32, smem, st, a));
   return MN_OK;
 }
 
@@ -415,9 +517,18 @@ extern "C" mn_status mn_sparse_convolution_forward_implicit_fp32(
   // 59k 32->32 42 / 40 / 34 / 43; 16k 64->64 156 / 130 / 95 / 84; 3.6k 128->128 185 / 190 / 140 / 95.  Eight
   // warps instead of four where blocks of 32 rows leave half the chip idle: 700 rows 256->256 136 -> 121,
   // 5k rows 256->64 60 -> 50.
+  // Clusters as long as their blocks run in one wave (three per SM): of 32 rows up to 48 tiles, of 64 rows (half
+  // the items where offsets are rare) up to 55.  us for clusters of 32 rows / of 64 rows / eight warps: 325
+  // rows 256->64, 19 pairs, 22 tiles 28 / 36 / 79; 325 rows 256->256, 88 tiles 69 / 67 / 80, with 3.2 pairs 49 / 34
+  // / 56; 1.5k 128->128, 188 tiles 83 / 78 / 65.  A second wave of them pays for deep products where the
+  // blocks of eight warps are a few more than the SMs: 700 rows 256->256, 88 tiles of 64 rows, 21 pairs 133 /
+  // 128 / 122, 3.5 pairs 93 / 63 / 85.
   const int64_t columns = div_up(c_out, kCsRows);
-  if (div_up(T, 128) * columns >= 8 * kNumSMs) return columns > 1 ? launch_cs<64, 2, 4, 2>(a, st) : launch_cs<128, 1, 4, 2>(a, st);
-  if (div_up(T, 64) * columns >= 4 * kNumSMs) return launch_cs<64, 1, 4, 3>(a, st);
-  if (2 * div_up(T, 32) * columns >= 5 * kNumSMs) return launch_cs<32, 1, 4, 3>(a, st);
+  const int64_t tall = div_up(T, 128) * columns, mid = div_up(T, 64) * columns, low = div_up(T, 32) * columns;
+  if (low <= 48) return launch_cs<32, 1, 4, 3, 8>(a, st);
+  if (mid <= 55 || (c_in >= 256 && 2 * mid >= kNumSMs && 3 * mid <= 2 * kNumSMs)) return launch_cs<64, 1, 4, 2, 8>(a, st);
+  if (tall >= 8 * kNumSMs) return columns > 1 ? launch_cs<64, 2, 4, 2>(a, st) : launch_cs<128, 1, 4, 2>(a, st);
+  if (mid >= 4 * kNumSMs) return launch_cs<64, 1, 4, 3>(a, st);
+  if (2 * low >= 5 * kNumSMs) return launch_cs<32, 1, 4, 3>(a, st);
   return launch_cs<32, 1, 8, 2>(a, st);
 }

@@ -131,7 +131,8 @@ constexpr int kMaxSmemClouds = 2048;
 
 // Keys of rows [r_begin, r_end) (r_begin a multiple of 4), the work split over
 // `nthreads` threads of which this one is `thread`.  ndim == 3 fast path: 4 rows
-// (48 bytes) per thread as three 128-bit loads and two 128-bit stores.
+// (48 bytes) per thread as three 128-bit loads and two 128-bit stores, kUnroll of those in flight.
+template <int kUnroll>
 __device__ __forceinline__ void pack_rows(const int32_t *__restrict__ coords, int64_t r_begin,
                                           int64_t r_end, int ndim, const int64_t *bd,
                                           int num_clouds, const mn_keyspec &spec,
@@ -143,7 +144,7 @@ __device__ __forceinline__ void pack_rows(const int32_t *__restrict__ coords, in
     const int64_t q_begin = r_begin >> 2;
     const int64_t q_end = aligned ? (r_end >> 2) : q_begin;
     const int4 *cv = reinterpret_cast<const int4 *>(coords);
-#pragma unroll 2
+#pragma unroll kUnroll
     for (int64_t q = q_begin + thread; q < q_end; q += nthreads) {
       int4 v0 = __ldg(cv + 3 * q), v1 = __ldg(cv + 3 * q + 1), v2 = __ldg(cv + 3 * q + 2);
       int c0[4] = {v0.x, v0.y, v0.z, 0}, c1[4] = {v0.w, v1.x, v1.y, 0};
@@ -198,7 +199,7 @@ pack_kernel(const int32_t *__restrict__ coords, int64_t n, int ndim,
   __shared__ int64_t s_bd[kMaxSmemClouds + 1];
   const int64_t *bd = stage_batch_dims(batch_dims, num_clouds, s_bd);
   bool bad = false;
-  pack_rows(coords, 0, n, ndim, bd, num_clouds, spec, p, keys,
+  pack_rows<1>(coords, 0, n, ndim, bd, num_clouds, spec, p, keys,
             (int64_t)blockIdx.x * blockDim.x + threadIdx.x, (int64_t)gridDim.x * blockDim.x, bad);
   if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicOr(status, MN_STATUS_KEY_BOX);
 }
@@ -220,7 +221,12 @@ struct RootArgs {
   int32_t *ctrl;
 };
 
-__global__ void __launch_bounds__(kBBoxThreads)
+// kRows3: three dimensions, on a 16-byte boundary.  Its loops keep twelve 128-bit loads in flight, which takes 128
+// registers and so two blocks per SM; the other scan has one load in flight and wants the warps instead:
+// with the 128 registers of one kernel for both, 7.3 M rows of 1 / 2 / 4 dimensions took 78 / 113 / 180 us for
+// 65 / 82 / 115, of 3 off a 16-byte boundary 226 for 133.
+template <bool kRows3>
+__global__ void __launch_bounds__(kBBoxThreads, kRows3 ? 2 : 4)
 root_keys_kernel(const __grid_constant__ RootArgs a) {
   release_successor();
   __shared__ int s[kBBoxThreads / 32][8];
@@ -234,7 +240,7 @@ root_keys_kernel(const __grid_constant__ RootArgs a) {
   const int64_t r0 = min(a.n, (int64_t)b * per_block), r1 = min(a.n, r0 + per_block);
   int mn_[4] = {INT_MAX, INT_MAX, INT_MAX, INT_MAX};
   int mx_[4] = {INT_MIN, INT_MIN, INT_MIN, INT_MIN};
-  if (a.ndim == 3 && (reinterpret_cast<uintptr_t>(a.coords) & 15) == 0) scan_rows3(a.coords, r0, r1, mn_, mx_);
+  if constexpr (kRows3) scan_rows3(a.coords, r0, r1, mn_, mx_);
   else if (r1 > r0) scan_flat(a.coords, r0 * a.ndim, (r1 - r0) * a.ndim, a.ndim, threadIdx.x, blockDim.x, mn_, mx_);
 #pragma unroll
   for (int k = 0; k < 4; k++) {
@@ -281,8 +287,8 @@ root_keys_kernel(const __grid_constant__ RootArgs a) {
   const int nc = a.batch_dims != nullptr ? (int)a.num_clouds : 1;
   const int64_t *bd = stage_batch_dims(a.batch_dims, nc, s_bd);
   bool bad = false;
-  pack_rows(a.coords, r0, r1, a.ndim, bd, nc, s_p.spec.host, s_p, a.keys_out, threadIdx.x,
-            blockDim.x, bad);
+  pack_rows<kRows3 ? 2 : 1>(a.coords, r0, r1, kRows3 ? 3 : a.ndim, bd, nc, s_p.spec.host, s_p, a.keys_out,
+                            threadIdx.x, blockDim.x, bad);
   if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(a.ctrl + MN_CTRL_STATUS, MN_STATUS_KEY_BOX);
 }
 
@@ -355,19 +361,26 @@ extern "C" mn_status mn_keyspec_device(const int32_t *coords, int64_t n, int ndi
   MN_CHECK_ARG(spec_dev != nullptr && spec != nullptr && ctrl != nullptr && (n == 0 || coords != nullptr),
                "keyspec_device: null pointer");
   MN_CHECK_ARG((reinterpret_cast<uintptr_t>(spec_dev) & 15) == 0, "keyspec_device: spec_dev must be 16-byte aligned");
-  static thread_local int grid_cache[kMaxDevices] = {0};
+  const bool rows3 = ndim == 3 && (reinterpret_cast<uintptr_t>(coords) & 15) == 0;
+  const auto kernel = rows3 ? root_keys_kernel<true> : root_keys_kernel<false>;
+  static thread_local int grid_cache[2][kMaxDevices] = {{0}};
   int device = 0;
   MN_CHECK_CUDA(cudaGetDevice(&device));
   MN_CHECK_ARG(device >= 0 && device < kMaxDevices, "keyspec_device: device index %d out of range", device);
-  if (grid_cache[device] == 0) {
-    grid_cache[device] = std::min(kBBoxMaxBlocks, max_coresident_blocks(root_keys_kernel, kBBoxThreads, 0));
-    if (grid_cache[device] <= 0) {
-      grid_cache[device] = 0;
+  int &most = grid_cache[rows3][device];
+  if (most == 0) {
+    most = std::min(kBBoxMaxBlocks, max_coresident_blocks(kernel, kBBoxThreads, 0));
+    if (most <= 0) {
+      most = 0;
       set_error("keyspec_device: cannot size the cooperative grid");
       return MN_ERR_CUDA;
     }
   }
-  const int grid = (int)std::min<int64_t>(grid_cache[device],
+  // Up to 600k rows the barrier of more blocks than two per SM costs more than their loads in flight give, up to 3 M
+  // that of more than three.  Two / three / four per SM, us: 464k rows of one dimension 12.2 / 13.8 / 15.0, of
+  // four 15.5 / 15.8 / 17.5; 1.9 M 24.8 / 23.5 / 25.8 and 35.9 / 31.9 / 33.2; 7.3 M 75 / 67 / 66 and 180 / 134 / 115.
+  const int per_sm = n < 4096ll * kNumSMs ? 2 : n < 5 * 4096ll * kNumSMs ? 3 : 4;
+  const int grid = (int)std::min<int64_t>(std::min(most, per_sm * kNumSMs),
                                           std::max<int64_t>(1, div_up(n, kBBoxThreads * 4)));
   Workspace ws(ws_ptr, ws_bytes);
   RootArgs a{};
@@ -383,7 +396,7 @@ extern "C" mn_status mn_keyspec_device(const int32_t *coords, int64_t n, int ndi
   void *params[] = {&a};
   {
     LaunchScope scope("root_keys_kernel", st);
-    MN_CHECK_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void *>(root_keys_kernel), dim3(grid),
+    MN_CHECK_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void *>(kernel), dim3(grid),
                                               dim3(kBBoxThreads), params, 0, st));
   }
   MN_CHECK_LAUNCH();

@@ -517,8 +517,12 @@ struct Plan {
     for (int32_t n : sizes_) total_ += n;
     known_ = true;
   }
-  // the sizes and the status word behind them come with a copy that is already in flight
+  // The sizes and the status word behind them come with a copy that is already in flight.  Inside a stream
+  // capture they do not: every replay makes the map anew, with the sizes of the coordinates that it finds, and
+  // would write them to a buffer that may have been given back.
   void expect_sizes(const Tensor &sizes_and_status) {
+    captured_ = capturing();
+    if (captured_) return;
     const cudaStream_t st = stream_of(sizes_and_status);
     buffer_ = pinned_pool().take(sizes_and_status.get_device());
     pending_ = true;
@@ -529,6 +533,9 @@ struct Plan {
   const std::vector<int32_t> &sizes() {
     Lock lock(mutex);
     if (!known_) {
+      if (captured_)
+        throw std::runtime_error("the pair counts of a kernel map that was built inside a stream capture are not known "
+                                 "to the host: build the map outside, or pass copies of its masks and sizes");
       if (!pending_) throw std::runtime_error("the sizes of this kernel map are not known");
       const cudaError_t e = cudaEventSynchronize(buffer_.event);
       const int32_t *host = static_cast<const int32_t *>(buffer_.host);
@@ -557,7 +564,7 @@ struct Plan {
  private:
   std::vector<int32_t> sizes_;
   int64_t total_ = 0;
-  bool known_ = false, pending_ = false;
+  bool known_ = false, pending_ = false, captured_ = false;
   PinnedPool::Buffer buffer_;
 };
 using PlanPtr = std::shared_ptr<Plan>;

@@ -1,10 +1,12 @@
-"""The row counts and cloud starts that a strided level and a voxelisation bring back: written to host
-memory by the kernel where they fit the buffer (1024 values: 1020 clouds), copied beyond."""
+"""The counts that the host reads: of a strided level and a voxelisation (row counts and cloud starts, written to
+host memory by the kernel where they fit the buffer (1024 values: 1020 clouds), copied beyond) and of kernel
+maps, several of them on their way at once and inside stream captures."""
 import numpy as np
 import pytest
 import torch
 
 import minuet_b200 as minuet
+from minuet_b200 import engine
 from minuet_b200.nn import functional as F
 
 pytestmark = pytest.mark.gpu
@@ -36,3 +38,58 @@ def test_counts_and_cloud_starts(clouds):
     ref = torch.zeros(len(voxels), 5, device=DEV, dtype=torch.float64).index_add_(0, inverse, features.double())
     ref /= torch.bincount(inverse, minlength=len(voxels))[:, None]
     assert float((means - ref).abs().max()) < 8 * 2.0 ** -23   # at most eight values below one
+
+
+def _map_of(coords, kernel):
+    cache = minuet.nn.KernelMapCache(ndim=3, dtype=torch.int32, device=DEV)
+    return cache, cache.get_kernel_map(coords, 1, None, coords, 1, None, kernel, 1)
+
+
+def test_many_counts_on_their_way_at_once():
+    """Buffers of maps that are gone before the GPU has written them are not handed out again too early."""
+    rng = np.random.default_rng(0)
+    clouds = [torch.as_tensor(np.unique(rng.integers(0, 30, (200 * (k + 1), 3)), axis=0), dtype=torch.int32, device=DEV)
+              for k in range(24)]
+    for _ in range(2):                                # (the second time with buffers that were given back)
+        torch.cuda.synchronize()
+        torch.cuda._sleep(20_000_000)                 # some 10 ms in front of the maps
+        kept = []
+        for k, c in enumerate(clouds):
+            cache, result = _map_of(c, 3 if k % 3 else 2)
+            if k % 2:
+                kept.append((cache, result))
+            del cache, result
+        for _, (_, tm, _, sizes) in kept:
+            assert engine.host_copy(sizes).tolist() == (tm >= 0).sum(1).tolist()
+
+
+@pytest.mark.parametrize("kernel", [3, 5])            # 27 offsets, and more than the fused build takes
+@pytest.mark.parametrize("mode", ["global", "thread_local", "relaxed"])
+def test_a_map_built_inside_a_capture(kernel, mode):
+    rng = np.random.default_rng(kernel)
+    first, second = (torch.as_tensor(np.unique(rng.integers(0, 20, (4000, 3)), axis=0)[:2500], dtype=torch.int32,
+                                     device=DEV) for _ in range(2))
+    coords = first.clone()
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        _map_of(coords, kernel)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream, capture_error_mode=mode):
+        cache, (sm, tm, order, sizes) = _map_of(coords, kernel)
+    for points in (first, second):
+        coords.copy_(points)
+        graph.replay()
+        want = _map_of(points.clone(), kernel)[1]
+        for got, expected in zip((sm, tm, order, sizes), want):
+            assert torch.equal(got, expected)
+    # what every replay writes anew is not read as if it were fixed, and nothing is left behind
+    conv = minuet.nn.SparseConv3d(4, 4, kernel, device=DEV)
+    minuet.set_kernel_map_cache(conv, cache)
+    with pytest.raises(RuntimeError, match="stream capture"):
+        conv(minuet.SparseTensor(torch.ones(len(coords), 4, device=DEV), coords))
+    del conv, cache, sm, tm, order, sizes, graph
+    for _ in range(3):
+        _, (_, tm, _, sizes) = _map_of(first, kernel)
+        assert engine.host_copy(sizes).tolist() == (tm >= 0).sum(1).tolist()

@@ -121,6 +121,10 @@ __device__ __forceinline__ float cs_load_from(const float *at, int block) {
 // the other, and a second launch for maps of few rows (us): 59k rows 32->32, 3 pairs 67 -> 34; 42k
 // 64->32, 7.5 pairs 146 -> 78; 16k 64->64, 12.5 pairs 137 -> 85; 16k 128->64 262 -> 150; 3.6k 128->128,
 // 14.5 pairs 108 -> 95; 196k 64->64, 3 pairs 228 -> 213; 50k 32->32, 1.1 pairs 29 -> 15; 59k 3->32 98 -> 21.
+// Where every row of a 64 x 64 or 128 x 32 block has every offset, a warp's items are all those of its own rows and
+// columns and nothing is handed over.  Maps of 20 and more pairs a row in blocks like that are what the block with
+// sums in registers was better at, whose warps shared the copies of the weights: 250k rows 64->64, 23.9 pairs 1370
+// -> 1545 us, 16->16 308 -> 338, 60k 256->256 5030 -> 5185; with 11 pairs 0.55 to 0.8 of its time.
 // Clusters against that second launch, 8 to 21 pairs: 13 rows 256->256 25 -> 15, 64->64 16 -> 8; 130 rows 128->128 23
 // -> 16; 325 rows 256->64 37 -> 28; 700 rows 256->256 137 -> 128 (3.5 pairs 79 -> 63).
 constexpr int cs_cap(int bm, int cluster) { return bm == 32 || cluster > 1 ? kCsMaxOffsets : 16; }
@@ -146,6 +150,7 @@ conv_simt_kernel(const __grid_constant__ CsArgs a) {
   __shared__ uint16_t s_items[kCap * kSubs * kCols];   // offset of the chunk | 32 of its rows << 5 | 32 columns << 8
   __shared__ uint8_t s_first[kCap];               // an offset's first item
   __shared__ uint32_t s_present;                  // offsets that have items
+  __shared__ bool s_own;
   __shared__ int32_t s_count, s_perm[BM];
   // the sums [BM][kSumCols]; in a cluster the products of this block's items [item][32][32]
   float *s_sum = s_mem + W * kStages * kCsStageFloats;
@@ -225,7 +230,8 @@ conv_simt_kernel(const __grid_constant__ CsArgs a) {
       if (lane == 0) s_have[j] = (uint8_t)n;
     }
     __syncthreads();
-    direct = kDirect && n_bits == 1 && s_have[0] == (int)min((int64_t)BM, a.T - r0);
+    const int n_rows = (int)min((int64_t)BM, a.T - r0);
+    direct = kDirect && n_bits == 1 && s_have[0] == n_rows;
     if (kCluster == 1 && chunk == 0 && !direct) clear_sums();
     if (warp == 0) {
       const int mine = lane < n_chunk ? (s_have[lane % kCap] + 31) / 32 * tiles : 0;
@@ -240,9 +246,13 @@ conv_simt_kernel(const __grid_constant__ CsArgs a) {
       if (lane == 31) s_count = end;
       const uint32_t present = __ballot_sync(0xffffffffu, mine > 0);
       if (kCluster > 1 && lane == 0) s_present = present;
+      // every row has every offset: item i is that of the 32 rows and columns of warp i % W, and of no other
+      const bool whole = __all_sync(0xffffffffu, lane >= n_chunk || s_have[lane % kCap] == n_rows);
+      if (lane == 0) s_own = whole && kSubs * tiles == W && n_rows > BM - 32;
     }
     __syncthreads();
     n_items = s_count;
+    const bool own = kDirect && s_own;
     // item i is worked on by block i % kCluster, so that a tile with few items has them on as many SMs
     const int first_item = warp * kCluster + rank;
     const int n_step = (n_items > first_item ? (n_items - first_item + kTeam - 1) / kTeam : 0) * a.k_steps;
@@ -394,7 +404,7 @@ conv_simt_kernel(const __grid_constant__ CsArgs a) {
         next_item();
         continue;
       }
-      if (W > 1 && item > 0) cs_turn_wait(1 + warp);
+      if (W > 1 && !own && item > 0) cs_turn_wait(1 + warp);
 #pragma unroll
       for (int i = 0; i < 8; i++) {
         if (4 * i < left) {
@@ -406,7 +416,7 @@ conv_simt_kernel(const __grid_constant__ CsArgs a) {
 #pragma unroll
         for (int j = 0; j < 4; j++) acc[i][j] = 0.f;
       }
-      if (W > 1 && item + 1 < n_items) {
+      if (W > 1 && !own && item + 1 < n_items) {
         cs_turn_pass(1 + (warp + 1) % W);
       }
       next_item();

@@ -373,7 +373,7 @@ mn_status mn_sparse_convolution_forward_implicit(
 
 /* The same function in fp32 on FFMA units (sums in fp32, any channel counts, at most 32
  * offsets), every offset's product by itself and the products added in mask-row order, by one
- * output-stationary kernel over the neighbour table.  (It keeps nothing in the workspace.) */
+ * output-stationary kernel over the neighbour table.  Needs no workspace (0 bytes; ws may be NULL). */
 size_t mn_implicit_fp32_workspace_bytes(int64_t T, int64_t O, int64_t c_out);
 mn_status mn_sparse_convolution_forward_implicit_fp32(
     int64_t S, int64_t T, int64_t O, int64_t c_in, int64_t c_out, const float *sources,

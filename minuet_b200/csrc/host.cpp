@@ -43,7 +43,7 @@ namespace {
   X(mn_last_error) X(mn_keyspec_device) X(mn_pack_keys) X(mn_downsample_coordinates)              \
   X(mn_map_workspace_bytes) X(mn_build_kernel_map) X(mn_implicit_supported)                       \
   X(mn_neighbor_table_workspace_bytes) X(mn_build_neighbor_table) X(mn_implicit_workspace_bytes)  \
-  X(mn_sparse_convolution_forward_implicit) X(mn_implicit_fp32_workspace_bytes)                   \
+  X(mn_sparse_convolution_forward_implicit)                                                       \
   X(mn_sparse_convolution_forward_implicit_fp32) X(mn_pairs_supported) X(mn_pair_rows)            \
   X(mn_build_pair_list) X(mn_pairs_workspace_bytes) X(mn_sparse_convolution_forward_pairs)        \
   X(mn_conv_workspace_bytes) X(mn_sparse_convolution_forward) X(mn_apply_epilogue)                \
@@ -760,18 +760,18 @@ Tensor run_forward(Plan &plan, bool swapped, Tensor x, Tensor w, const Tensor &s
     const int32_t *perm = raw<int32_t>(n.perm), *nbr = raw<int32_t>(n.nbr);
     const uint32_t *tiles = raw<uint32_t>(n.tile_bits);
     if (code == MN_F32) {
-      Tensor ws = workspace(x, api.mn_implicit_fp32_workspace_bytes(T, O, c_out));
       check(api.mn_sparse_convolution_forward_implicit_fp32(
                 S, T, O, c_in, c_out, raw<float>(x), raw<float>(w), nbr, tiles, perm, ord, sc, sh,
-                static_cast<const float *>(res), o.relu, raw<float>(out), ws.data_ptr(), (size_t)ws.numel(), st),
+                static_cast<const float *>(res), o.relu, raw<float>(out), nullptr, 0, st),
             "sparse_convolution_forward_implicit_fp32");
       return out;
     }
-    Tensor ws = workspace(x, w_t.has_value() ? 0 : api.mn_implicit_workspace_bytes(O, c_in, c_out));
+    Tensor ws;                             // for the transposed weights, where the call makes them itself
+    if (!w_t.has_value()) ws = workspace(x, api.mn_implicit_workspace_bytes(O, c_in, c_out));
     check(api.mn_sparse_convolution_forward_implicit(
               S, T, O, c_in, c_out, code, x.data_ptr(), w.data_ptr(), raw<void>(w_t), nbr, tiles, perm, ord, sc,
               sh, res, o.relu, (double)plan.pairs() / (double)std::max<int64_t>(T, 1), o.sub_tiles, out.data_ptr(),
-              ctrl_of(x), ws.data_ptr(), (size_t)ws.numel(), st),
+              ctrl_of(x), raw<void>(ws), ws.defined() ? (size_t)ws.numel() : 0, st),
           "sparse_convolution_forward_implicit");
     return out;
   }

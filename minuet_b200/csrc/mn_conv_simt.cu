@@ -492,8 +492,7 @@ mn_status launch_cs(const CsArgs &a, cudaStream_t st) {
 
 using namespace mn;
 
-// (Nothing is kept in the workspace any more.)
-extern "C" size_t mn_implicit_fp32_workspace_bytes(int64_t, int64_t, int64_t) { return 256; }
+extern "C" size_t mn_implicit_fp32_workspace_bytes(int64_t, int64_t, int64_t) { return 0; }
 
 extern "C" mn_status mn_sparse_convolution_forward_implicit_fp32(
     int64_t S, int64_t T, int64_t O, int64_t c_in, int64_t c_out, const float *sources,
@@ -516,7 +515,7 @@ extern "C" mn_status mn_sparse_convolution_forward_implicit_fp32(
   a.K = (int)c_in; a.N = (int)c_out;
   a.k_steps = (int)div_up(c_in, kCsK);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  (void)ws_ptr;
+  (void)ws_ptr;             // products and sums stay on the chip
   (void)ws_bytes;
   MN_CHECK_ARG((reinterpret_cast<uintptr_t>(nbr) & 15) == 0 &&
                    (c_out % 4 != 0 || (reinterpret_cast<uintptr_t>(targets_out) & 15) == 0),

@@ -316,9 +316,10 @@ constexpr int kWsIdxAhead = kWsStages;
 // What bounds it: FFMA issue and the copies' latency.  With 8 x 4 sums a thread, and the list entries read
 // from memory before every copy, 586k pairs 64 x 64 took 230 us (products at the FFMA rate: 65 us), now
 // 124; 196k pairs 128 x 64 122 -> 96; 52k pairs 256 x 128 141 -> 115 (both with the host's part).  Small tiles
-// keep 8 x 4: their copies need the warps that 128 registers a thread would cost.
+// keep 8 x 4: their copies need the warps that 128 registers a thread would cost.  The ring of a 64 x 64 tile
+// (48 KB) lets four blocks share an SM, so its registers are limited for four (for six they spilled).
 template <typename T, int BM, int BN, int TN, bool kVec>
-__global__ void __launch_bounds__(kWsThreads, TN == 8 ? 4 : 6)
+__global__ void __launch_bounds__(kWsThreads, TN == 8 || BM + BN == 128 ? 4 : 6)
 wgrad_simt_kernel(const __grid_constant__ WgradArgs a, const __grid_constant__ WgradPlan plan, int n_tiles) {
   begin_early();
   constexpr int kHalves = TN / 4, kTileThreads = BM * BN / (8 * TN);

@@ -1,4 +1,5 @@
-"""The radix sort at the row counts where its tiles change shape, and one row to either side of a tile."""
+"""The radix sort at the row counts where its tiles change shape, and one row to either side of a tile, with
+the index below the key and (63 key bits) in an array of its own."""
 import pytest
 import torch
 
@@ -16,3 +17,17 @@ def test_permutation_is_stable(n, extent):
     key = ((c[:, 0].long() + extent) * 2 * extent + c[:, 1] + extent) * 2 * extent + c[:, 2] + extent
     got = F.arg_sort_coordinates(c, dtype=torch.int64)
     assert torch.equal(got, torch.sort(key, stable=True).indices)
+
+
+@pytest.mark.parametrize("n", [151_551, 151_552, 155_649, 1_212_415, 1_212_417])
+def test_index_beside_a_full_key(n):
+    extent = 2 ** 20
+    gen = torch.Generator(device=DEV).manual_seed(n)
+    c = torch.randint(-extent, extent, (n, 3), generator=gen, device=DEV, dtype=torch.int32)
+    c[n // 2:] = c[:n - n // 2].clone()                    # equal keys far apart
+    c[0], c[1] = -extent, extent - 1                       # 21 bits a dimension, whatever was drawn
+    got = F.arg_sort_coordinates(c, dtype=torch.int64)
+    want = torch.arange(n, device=DEV)
+    for d in (2, 1, 0):                                    # least significant first, each stable
+        want = want[torch.sort(c[want, d], stable=True).indices]
+    assert torch.equal(got, want)

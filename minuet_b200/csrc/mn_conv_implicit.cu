@@ -24,7 +24,7 @@
 // What bounds it.  Maps with three or more pairs a row: a 128 x 64 stage at 128 output columns
 // takes 795 cycles, of which shared memory explains 520 (256 of operand reads by the MMAs, 200 of
 // gathered rows, 64 of weights and the rest); what the other 275 are is not known.  Sparser
-// maps: the epilogue's chain of instructions (see there).  A warp needs five cycles per dependent
+// maps: the epilogue (see there).  A warp needs five cycles per dependent
 // instruction, so every role's loop is kept short: the issuing warps stay converged and elect
 // one lane only around the instruction itself (issued from a divergent lane-0 branch every MMA
 // took about 150 cycles of register moves), the index blocks arrive eight steps ahead and a lane
@@ -467,8 +467,11 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
     // quarter of the rows where there are eight: they take alternate pieces.  No shared-memory
     // staging: its barriers and index shuffles cost more than the wider stores gave, and the
     // 32 KB are worth more as ring stages.
-    // This role bounds the levels with few pairs a row, and what it costs is instruction
-    // latency: every piece is a chain of some 100 dependent instructions.  It must not spill:
+    // This role bounds the levels with few pairs a row (of 54 us for 480k rows 64->64 with 1.15 pairs a CTA
+    // spends 8 before its first tile is in flight, then 2.6 a tile).  Not by the latency of its instructions,
+    // although every piece is a chain of some 100: two groups of epilogue warps with a tile each, and
+    // residuals asked for a tile earlier, took the same time.  In the rows' own order (dense mode) it runs at
+    // the copy rate; what is left is that pieces of rows go to scattered places.  It must not spill:
     // next to 200 KB of shared memory L1 keeps no local memory, and each reload of a spilled
     // register was a trip to L2 (with 32 bytes of spills 918k rows 32->32 took 66 us, without
     // 52; the pieces' registers are therefore single, not double, buffered).

@@ -320,8 +320,9 @@ sort_pass_kernel(const __grid_constant__ Args a, int pass) {
 
 // Threads and keys per thread of a tile.  Every tile that runs at the same time lengthens the look-back, so
 // tiles are large: 4096 keys, with 512 threads up to two tiles per SM and with 256 beyond (three
-// blocks of 80 registers share an SM: at 128 registers and two, 7.3 M keys took 7 % longer); 1024
-// keys where larger ones would leave SMs without a tile.  Measured, all passes, us for 256 x 4 / 512 x 8 /
+// blocks of 80 registers share an SM: at 128 registers and two, 7.3 M keys took 7 % longer).  Up to one
+// tile of 1024 keys per SM a pass is shorter with those; beyond, up to 606k keys, the large ones
+// leave SMs without a tile and are faster all the same.  Measured, all passes, us for 256 x 4 / 512 x 8 /
 // 256 x 16: 30k keys 29 / 37 / 39; 120k 45 / 51 / 53; 250k 64 / 59 / 62; 464k 80 / 74 / 78; 900k 115 / 94 /
 // 100; 1.9 M 184 / 141 / 127; 7.3 M 755 / 491 / 445.
 struct TileShape { int threads, items; };

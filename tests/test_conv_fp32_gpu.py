@@ -1,6 +1,6 @@
 """The fused fp32 forward against gather - FFMA GEMM - scatter of the same library, which sums in
 the same order: the same bits, at remainders of the row, channel and offset blocks, with the
-offsets of a tile in one block and spread over blocks."""
+offsets of a tile in one block and spread over the blocks of a cluster."""
 import ctypes
 
 import numpy as np

@@ -134,20 +134,32 @@ inline T *raw(const Tensor &t) {
 
 // The MN_CTRL_WORDS control block of (device, current stream): word 0 is the status word.
 // One per stream, because kernels of different streams may overlap; never freed, as a stream
-// of torch's pool is not either.
+// of torch's pool is not either.  A stream that is first used inside a capture gets one per capture: it
+// comes from the graph's memory and is zeroed by the graph, so nothing outside may count on it.
+struct ControlBlock {
+  Tensor words;
+  unsigned long long capture = 0;      // of the capture that made it, 0: none
+};
 std::mutex ctrl_mutex;
-std::map<std::pair<int, cudaStream_t>, Tensor> &ctrl_blocks() {
-  static auto *blocks = new std::map<std::pair<int, cudaStream_t>, Tensor>;   // outlives the CUDA context
+std::map<std::pair<int, cudaStream_t>, ControlBlock> &ctrl_blocks() {
+  static auto *blocks = new std::map<std::pair<int, cudaStream_t>, ControlBlock>;   // outlives the CUDA context
   return *blocks;
 }
 
 Tensor control_block(int device) {
   const cudaStream_t st = c10::cuda::getCurrentCUDAStream(device).stream();
   std::lock_guard<std::mutex> lock(ctrl_mutex);
-  Tensor &t = ctrl_blocks()[{device, st}];
-  if (!t.defined())
-    t = at::zeros({MN_CTRL_WORDS}, at::TensorOptions().dtype(at::kInt).device(at::kCUDA, device));
-  return t;
+  ControlBlock &b = ctrl_blocks()[{device, st}];
+  if (b.words.defined() && b.capture == 0) return b.words;
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  check_cuda(cudaStreamGetCaptureInfo(st, &status, &id), "control block");
+  if (status != cudaStreamCaptureStatusActive) id = 0;
+  if (!b.words.defined() || b.capture != id) {
+    b.words = at::zeros({MN_CTRL_WORDS}, at::TensorOptions().dtype(at::kInt).device(at::kCUDA, device));
+    b.capture = id;
+  }
+  return b.words;
 }
 inline int32_t *ctrl_of(const Tensor &t) { return static_cast<int32_t *>(control_block(t.get_device()).data_ptr()); }
 

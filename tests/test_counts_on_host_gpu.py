@@ -93,3 +93,27 @@ def test_a_map_built_inside_a_capture(kernel, mode):
     for _ in range(3):
         _, (_, tm, _, sizes) = _map_of(first, kernel)
         assert engine.host_copy(sizes).tolist() == (tm >= 0).sum(1).tolist()
+
+
+def test_a_stream_that_is_first_used_inside_captures():
+    """Two graphs captured on one new stream, the second replayed first, then work outside a capture there."""
+    coords = [torch.as_tensor(np.unique(np.random.default_rng(k).integers(0, 20, (4000, 3)), axis=0), dtype=torch.int32,
+                              device=DEV) for k in range(2)]
+    want = [_map_of(c, 3)[1] for c in coords]
+    stream, graphs, maps = torch.cuda.Stream(), [], []
+    for c in coords:
+        torch.cuda.synchronize()
+        graphs.append(torch.cuda.CUDAGraph())
+        with torch.cuda.graph(graphs[-1], stream=stream):
+            maps.append(_map_of(c, 3))
+    for k in (1, 1, 0, 1):
+        for t in maps[k][1]:
+            t.fill_(-7)
+        graphs[k].replay()
+        assert all(torch.equal(got, expected) for got, expected in zip(maps[k][1], want[k]))
+    del graphs, maps
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        got = _map_of(coords[0], 3)[1]
+        assert engine.host_copy(got[3]).tolist() == engine.host_copy(want[0][3]).tolist()
+        assert all(torch.equal(a, b) for a, b in zip(got, want[0]))

@@ -26,7 +26,6 @@
 #include "mn_common.cuh"
 
 #include <algorithm>
-#include <type_traits>
 
 namespace mn {
 
@@ -110,7 +109,7 @@ __device__ __forceinline__ float cs_load_from(const float *at, int block) {
 // offsets sort to the end, and their tiles take longest.  At most cs_cap offsets are looked at at a
 // time (index blocks in shared memory).  kVec: rows of the features and of the weights can be copied 16
 // bytes at a time.  kFew: an item of up to 16 rows costs half as much (maps of 3.5 pairs a row: 32-row tiles
-// take 15 % less time); not for the tall blocks of large maps, whose full items the second loop body costs 10 %.
+// take 15 % less time, at 20 pairs 3 % more); not for the tall blocks of large maps, whose items are full.
 //
 // What bounds it: instruction issue.  Of 56 M warp instructions of a layer of 3.6k rows 128->128 with 14.5
 // pairs 38 M run on the FMA pipe, 27 M of them useful products, and a scheduler issues in 61 % of
@@ -124,9 +123,9 @@ __device__ __forceinline__ float cs_load_from(const float *at, int block) {
 // Where every row of a 64 x 64 or 128 x 32 block has every offset, a warp's items are all those of its own rows and
 // columns and nothing is handed over.  Maps of 20 and more pairs a row in blocks like that are what the block with
 // sums in registers was better at, whose warps shared the copies of the weights: 250k rows 64->64, 23.9 pairs 1370
-// -> 1545 us, 16->16 308 -> 338, 60k 256->256 5030 -> 5185; with 11 pairs 0.55 to 0.8 of its time.
+// -> 1579 us, 16->16 308 -> 329, 60k 256->256 5030 -> 5300; with 11 pairs 0.53 to 0.8 of its time.
 // Clusters against that second launch, 8 to 21 pairs: 13 rows 256->256 25 -> 15, 64->64 16 -> 8; 130 rows 128->128 23
-// -> 16; 325 rows 256->64 37 -> 28; 700 rows 256->256 137 -> 128 (3.5 pairs 79 -> 63).
+// -> 15; 325 rows 256->64 37 -> 26; 700 rows 256->256 137 -> 120 (3.5 pairs 79 -> 60).
 constexpr int cs_cap(int bm, int cluster) { return bm == 32 || cluster > 1 ? kCsMaxOffsets : 16; }
 // items of one block of a cluster at most
 constexpr int cs_share(int bm, int cluster) { return kCsMaxOffsets * (bm / kCsRows) / cluster; }
@@ -142,6 +141,7 @@ conv_simt_kernel(const __grid_constant__ CsArgs a) {
   constexpr int kThreads = W * 32, kSubs = BM / 32, kCap = cs_cap(BM, kCluster), kSumCols = kCols * kCsRows;
   constexpr int kTeam = W * kCluster;                // warps of a tile
   constexpr bool kDirect = BM > 32 && kCluster == 1;
+  constexpr bool kOwn = kDirect && kSubs * kCols == W;
   constexpr bool kFew = BM == 32 || kCluster > 1;
   static_assert(kCluster == 1 || (kCols == 1 && kCap == kCsMaxOffsets), "clusters: one list of items per tile");
   extern __shared__ __align__(16) float s_mem[];
@@ -244,15 +244,19 @@ conv_simt_kernel(const __grid_constant__ CsArgs a) {
       if (kCluster > 1 && lane < n_chunk) s_first[lane % kCap] = (uint8_t)(end - mine);
       for (int g = 0; g < mine; g++) s_items[end - mine + g] = (uint16_t)(lane | ((g / tiles) << 5) | ((g % tiles) << 8));
       if (lane == 31) s_count = end;
-      const uint32_t present = __ballot_sync(0xffffffffu, mine > 0);
-      if (kCluster > 1 && lane == 0) s_present = present;
+      if constexpr (kCluster > 1) {
+        const uint32_t present = __ballot_sync(0xffffffffu, mine > 0);
+        if (lane == 0) s_present = present;
+      }
       // every row has every offset: item i is that of the 32 rows and columns of warp i % W, and of no other
-      const bool whole = __all_sync(0xffffffffu, lane >= n_chunk || s_have[lane % kCap] == n_rows);
-      if (lane == 0) s_own = whole && kSubs * tiles == W && n_rows > BM - 32;
+      if constexpr (kOwn) {
+        const bool whole = __all_sync(0xffffffffu, lane >= n_chunk || s_have[lane % kCap] == n_rows);
+        if (lane == 0) s_own = whole && tiles == kCols && n_rows > BM - 32;
+      }
     }
     __syncthreads();
     n_items = s_count;
-    const bool own = kDirect && s_own;
+    const bool own = kOwn && s_own;
     // item i is worked on by block i % kCluster, so that a tile with few items has them on as many SMs
     const int first_item = warp * kCluster + rank;
     const int n_step = (n_items > first_item ? (n_items - first_item + kTeam - 1) / kTeam : 0) * a.k_steps;
@@ -349,33 +353,30 @@ conv_simt_kernel(const __grid_constant__ CsArgs a) {
       const int kmax = min(kCsK, a.K - k0);        // zeros up to a multiple of 4
       if (++stage == kStages) stage = 0;
       k0 += kCsK;
-      auto multiply = [&](auto n) {
-        constexpr int kRows = decltype(n)::value;                  // of a lane
 #pragma unroll
-        for (int k = 0; k < kCsK; k += 4) {
-          if (k < kmax) {
-            float4 av[kRows], bv[4];
+      for (int k = 0; k < kCsK; k += 4) {
+        if (k < kmax) {
+          float4 av[8], bv[4];
 #pragma unroll
-            for (int i = 0; i < kRows; i++)
+          for (int i = 0; i < 8; i++)
+            if (i < 4 || !kFew || !few)
               av[i] = *reinterpret_cast<const float4 *>(sa + i * 4 * kCsK + place[(k / 4) ^ (2 * (i & 1))]);
 #pragma unroll
-            for (int j = 0; j < 4; j++) bv[j] = *reinterpret_cast<const float4 *>(sb + (k + j) * kCsRows);
+          for (int j = 0; j < 4; j++) bv[j] = *reinterpret_cast<const float4 *>(sb + (k + j) * kCsRows);
 #pragma unroll
-            for (int i = 0; i < kRows; i++) {
-              const float ak[4] = {av[i].x, av[i].y, av[i].z, av[i].w};
+          for (int i = 0; i < 8; i++) {
+            if (kFew && i >= 4 && few) continue;
+            const float ak[4] = {av[i].x, av[i].y, av[i].z, av[i].w};
 #pragma unroll
-              for (int j = 0; j < 4; j++) {
-                acc[i][0] = fmaf(ak[j], bv[j].x, acc[i][0]);
-                acc[i][1] = fmaf(ak[j], bv[j].y, acc[i][1]);
-                acc[i][2] = fmaf(ak[j], bv[j].z, acc[i][2]);
-                acc[i][3] = fmaf(ak[j], bv[j].w, acc[i][3]);
-              }
+            for (int j = 0; j < 4; j++) {
+              acc[i][0] = fmaf(ak[j], bv[j].x, acc[i][0]);
+              acc[i][1] = fmaf(ak[j], bv[j].y, acc[i][1]);
+              acc[i][2] = fmaf(ak[j], bv[j].z, acc[i][2]);
+              acc[i][3] = fmaf(ak[j], bv[j].w, acc[i][3]);
             }
           }
         }
-      };
-      if (kFew && few) multiply(std::integral_constant<int, 4>());
-      else multiply(std::integral_constant<int, 8>());
+      }
       if (k0 < a.K) continue;
       // the product is complete: it is added when the items before it have been
       const int entry = s_items[item], j0 = entry & 31, first = ((entry >> 5) & 7) * 32 + ty;
@@ -527,7 +528,8 @@ extern "C" mn_status mn_sparse_convolution_forward_implicit_fp32(
   // warps instead of four where blocks of 32 rows leave half the chip idle: 700 rows 256->256 136 -> 121,
   // 5k rows 256->64 60 -> 50.
   // Clusters as long as their blocks run in one wave (three per SM): of 32 rows up to 48 tiles, of 64 rows (half
-  // the items where offsets are rare) up to 55.  us for clusters of 32 rows / of 64 rows / eight warps: 325
+  // the items where offsets are rare) up to 55.  us for clusters of 32 rows / of 64 rows / eight warps (with a
+  // loop body of its own for items of up to 16 rows, some 5 % slower in the clusters than now): 325
   // rows 256->64, 19 pairs, 22 tiles 28 / 36 / 79; 325 rows 256->256, 88 tiles 69 / 67 / 80, with 3.2 pairs 49 / 34
   // / 56; 1.5k 128->128, 188 tiles 83 / 78 / 65.  A second wave of them pays for deep products where the
   // blocks of eight warps are a few more than the SMs: 700 rows 256->256, 88 tiles of 64 rows, 21 pairs 133 /

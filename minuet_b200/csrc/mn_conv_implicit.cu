@@ -11,8 +11,8 @@
 //               (cp.async straight into the 128-byte-swizzled A tile, zeros where the
 //               kernel map has no entry)
 //   MMA warp    allocates TMEM and issues tcgen05.mma over (offset, k-block)
-//   TMA warp    starts the copy of every step's index block and the TMA load of every
-//               stage's transposed weight tile
+//   weight warp starts the TMA load of every stage's weight tile
+//   index warp  copies every step's index block, eight steps ahead
 //   epilogue    (8 or 4 warps): TMEM -> registers -> optional per-channel scale/shift
 //               (folded BatchNorm or bias), residual add, ReLU -> the output rows
 // so that features are read once per pair (mostly from L2), outputs are written
@@ -21,15 +21,18 @@
 // of target t under mask row p, or -1) is derived once per kernel map from the
 // masks by mn_build_neighbor_table.  Every barrier wait is bounded (status bit 2).
 //
-// What bounds it.  Maps with three or more pairs a row: a 128 x 64 stage at 128 output columns
-// takes 795 cycles, of which shared memory explains 520 (256 of operand reads by the MMAs, 200 of
-// gathered rows, 64 of weights and the rest); what the other 275 are is not known.  Sparser
+// What bounds it.  The memory does not, on maps with three or more pairs a row: indices that are all -1
+// take the same time.  Up to 64 columns a CTA's step of some 1000 cycles (2 CTAs per SM) is the chain of
+// one producer warp (wait, eight indices a lane, eight copies), before that it was the one warp that
+// sent index blocks and weights both.  At 128 columns shared memory: an M = N = 128 MMA reads 128 bytes of
+// operands per cycle, and the gathered rows and weights have to be written beside it.  At 256
+// columns the MMAs take 72 % of the cycles, at clocks that the power limit sets.  Sparser
 // maps: the epilogue (see there).  A warp needs five cycles per dependent
 // instruction, so every role's loop is kept short: the issuing warps stay converged and elect
 // one lane only around the instruction itself (issued from a divergent lane-0 branch every MMA
 // took about 150 cycles of register moves), the index blocks arrive eight steps ahead and a lane
 // reads the indices of all its rows with one load, and the next stage's barrier is probed before
-// the current stage is worked on.
+// the current stage is worked on (a wait that finds its phase complete costs 200 cycles, a probe 60).
 #include "mn_sort.cuh"
 #include "mn_tc.cuh"
 
@@ -42,7 +45,7 @@ namespace {
 using namespace tc;
 
 constexpr int kGatherWarps = 12;       // producer and epilogue warps together: 8 + 4 or 4 + 8
-constexpr int kImThreads = (kGatherWarps + 2) * 32;
+constexpr int kImThreads = (kGatherWarps + 3) * 32;
 constexpr int kImCtas = 2;             // CTAs per SM the register file allows
 constexpr int kBM = 128;
 constexpr int kBK = 64;
@@ -136,14 +139,6 @@ __device__ __forceinline__ int32_t load_ahead_1(const void *src) {
   return v;
 }
 
-// 16-byte aligned block of global memory -> shared memory
-__device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-          smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar))
-      : "memory");
-}
-
 // Offset bits of the sub-tiles of a CTA tile, in two steps: the request (unconditional, from a
 // clamped index: a load under a condition is waited for where the branch joins, a thousand cycles
 // per tile) and, a tile later, the value (pair mode: one offset each).
@@ -180,7 +175,7 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
                      const __grid_constant__ CUtensorMap map_b) {   // weights^T [O, N, K]; kMapNMajor: weights [O, K, N]
   constexpr bool kPairs = kMode == kPairRows, kNMajor = kMode == kMapNMajor;
   constexpr int kProdRows = 128 / kProdWarps;               // rows of a sub-tile per producer warp
-  constexpr int kMmaWarp = kProdWarps, kTmaWarp = kProdWarps + 1, kEpiWarp = kProdWarps + 2;
+  constexpr int kMmaWarp = kProdWarps, kTmaWarp = kProdWarps + 1, kIdxWarp = kProdWarps + 2, kEpiWarp = kProdWarps + 3;
   constexpr int kEpiCols = (kGatherWarps - kProdWarps) / 4;   // epilogue warps per quarter of the rows
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   __shared__ uint64_t bar_full[kMaxStages], bar_empty[kMaxStages];
@@ -205,7 +200,7 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
       mbar_init(&bar_empty[s], 1);
     }
     for (int a = 0; a < 2; a++) { mbar_init(&bar_acc_full[a], 1); mbar_init(&bar_acc_empty[a], 4 * kEpiCols); }
-    for (int i = 0; i < kIdxSlots; i++) { mbar_init(&bar_idx_full[i], 1); mbar_init(&bar_idx_empty[i], kProdWarps * 32); }
+    for (int i = 0; i < kIdxSlots; i++) { mbar_init(&bar_idx_full[i], 33); mbar_init(&bar_idx_empty[i], kProdWarps * 32); }
     s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -248,11 +243,10 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
     int stage = 0, slot = 0;
     uint32_t phase = 0, slot_phase = 0;
     bool alive = true;
-    bool ready = mbar_test(&bar_empty[0], 1u);
+    bool ready = mbar_test(&bar_empty[0], 1u), indices = false;
     while (kMode != kDense && alive) {
-      if (!mbar_wait(&bar_idx_full[slot], slot_phase, abort_flag, args.status)) break;
+      if (!indices && !mbar_wait(&bar_idx_full[slot], slot_phase, abort_flag, args.status)) break;
       const uint32_t has = s_idx_has[slot];        // sub-tiles that have this offset; 0: no more steps
-      if (has == 0u) break;
       int32_t q[kSub][kRpl];
 #pragma unroll
       for (int h = 0; h < kSub; h++) {
@@ -268,6 +262,7 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
           }
         }
       }
+      if (has == 0u) break;
       // The slot may be refilled only once the loads above have RETURNED, not when they have been
       // issued: behind a queue of copies they were overtaken by the arrival and read the block of
       // eight steps later (one launch in a hundred on freshly built tables).  So every lane arrives for
@@ -283,6 +278,7 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
         for (int i = 0; i < kRpl; i++) seen |= (uint32_t)q[h][i];
       mbar_arrive(&bar_idx_empty[slot] + (seen & (uint32_t)args.zero));
       if (++slot == kIdxSlots) { slot = 0; slot_phase ^= 1u; }
+      indices = mbar_test(&bar_idx_full[slot], slot_phase);   // of the next step
       for (int kb = 0; kb < args.k_blocks; kb++) {
         if (!ready && !mbar_wait(&bar_empty[stage], phase ^ 1u, abort_flag, args.status)) {
           alive = false;
@@ -297,11 +293,11 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
         ready = mbar_test(&bar_empty[stage], phase ^ 1u);   // of the next stage
 #pragma unroll
         for (int h = 0; h < kSub; h++) {
-          // a sub-tile without this offset has no index block: its rows are zero rows
-          const bool use = inside && (kSub == 1 || ((has >> h) & 1u) != 0u);
+          // a sub-tile without this offset has no index block, and no MMA reads its rows
+          if (kSub > 1 && ((has >> h) & 1u) == 0u) continue;
 #pragma unroll
           for (int i = 0; i < kRpl; i++) {
-            const bool valid = q[h][i] >= 0 && use;
+            const bool valid = q[h][i] >= 0 && inside;
             cp_async_16(sa + (uint32_t)(h * kBM * 128) + dst0[i],
                         valid ? src + (uint64_t)(uint32_t)q[h][i] * row_bytes : args.in, valid ? 16u : 0u);
           }
@@ -334,13 +330,14 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
     for (int tile = blockIdx.x; alive && tile < args.num_tiles; tile += gridDim.x) {
       uint32_t hb[kSub];
       take_bits<kSub>(args, tile, raw, hb);
-      const int n_offsets = __popc(union_of<kSub>(hb));
+      uint32_t rest = union_of<kSub>(hb);
       request_bits<kSub, kMode>(args, tile + (int)gridDim.x, raw);
       if (!mbar_wait_warp(false, &bar_acc_empty[acc], acc_phase ^ 1u, abort_flag, args.status)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t tmem_d = tmem_base + (uint32_t)(acc * kSub * args.n_pad);
-      uint32_t accumulate = 0u;
-      for (int o = 0; alive && o < n_offsets; o++) {
+      uint32_t begun = 0u;                                   // sub-tiles that have products already
+      for (; alive && rest != 0u; rest &= rest - 1u) {
+        const int p = __ffs(rest) - 1;
         for (int kb = 0; kb < args.k_blocks; kb++) {
           if (!mbar_wait_warp(ready, &bar_full[stage], phase, abort_flag, args.status)) { alive = false; break; }
           if (kMode != kDense) fence_generic_to_async();
@@ -356,73 +353,28 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
               if (k < nk) {
                 const uint64_t db = umma_desc_at(b_hi, lo_b + k * b_next);
 #pragma unroll
-                for (int h = 0; h < kSub; h++)                 // one weight tile, all sub-tiles
-                  umma_f16(tmem_d + (uint32_t)(h * args.n_pad),
-                           umma_desc_at(desc_hi, lo + h * (kBM * 128 / 16) + k * (kUmmaK * 2 / 16)), db,
-                           idesc, k == 0 ? accumulate : 1u);
+                for (int h = 0; h < kSub; h++)                 // one weight tile, the sub-tiles that need it
+                  if (kSub == 1 || ((hb[h] >> p) & 1u) != 0u)
+                    umma_f16(tmem_d + (uint32_t)(h * args.n_pad),
+                             umma_desc_at(desc_hi, lo + h * (kBM * 128 / 16) + k * (kUmmaK * 2 / 16)), db,
+                             idesc, k == 0 && kb == 0 ? (begun >> h) & 1u : 1u);
               }
             }
             umma_commit(empty);
           }
-          accumulate = 1u;
         }
+#pragma unroll
+        for (int h = 0; h < kSub; h++) begun |= ((hb[h] >> p) & 1u) << h;
       }
       if (!alive) break;
       if (elect_one()) umma_commit(&bar_acc_full[acc]);
       if (++acc == args.acc_bufs) { acc = 0; acc_phase ^= 1u; }
     }
   } else if (warp == kTmaWarp) {
-    // ------------------- index blocks and weight tiles --------------------------
-    // Two cursors over the same stream of (tile, offset) steps: the index blocks (128 entries
-    // of the neighbour table per sub-tile, one bulk copy each) run kIdxSlots steps ahead of
-    // the weight tiles, so that the producers never wait for an index from memory (loaded by
-    // the producers themselves, even two steps ahead, they cost a quarter of the time).
+    // ------------------------------ weight tiles -------------------------------
     const uint32_t b_bytes = (uint32_t)(args.stage_bytes - args.a_bytes);
     const int my_order = lane < args.num_offsets && args.order != nullptr ? __ldg(args.order + lane) : lane;
     bool alive = true;
-    int itile = (int)blockIdx.x - (int)gridDim.x, slot = 0;
-    uint32_t irest = 0u, slot_phase = 0, ihb[kSub], iraw[kSub];
-    request_bits<kSub, kMode>(args, (int)blockIdx.x, iraw);
-    bool more = kMode != kDense;   // false once the end mark is out
-    auto send_indices = [&]() {
-      while (irest == 0u && itile < args.num_tiles) {
-        itile += (int)gridDim.x;
-        take_bits<kSub>(args, itile, iraw, ihb);
-        irest = union_of<kSub>(ihb);
-        request_bits<kSub, kMode>(args, itile + (int)gridDim.x, iraw);
-      }
-      if (!mbar_wait_warp(false, &bar_idx_empty[slot], slot_phase ^ 1u, abort_flag, args.status)) {
-        alive = false;
-        return;
-      }
-      uint32_t has = 0u;
-      int p = 0;
-      if (irest != 0u) {
-        p = __ffs(irest) - 1;
-        irest &= irest - 1u;
-#pragma unroll
-        for (int h = 0; h < kSub; h++) has |= ((ihb[h] >> p) & 1u) << h;
-      } else {
-        more = false;
-      }
-      if (elect_one()) {
-        s_idx_has[slot] = has;
-        if (has == 0u) {
-          mbar_arrive(&bar_idx_full[slot]);
-        } else {
-          mbar_expect_tx(&bar_idx_full[slot], (uint32_t)__popc(has) * (kBM * 4u));
-          const int32_t *src = args.nbr + (int64_t)p * args.pitch + (int64_t)itile * (kSub * kBM);
-#pragma unroll
-          for (int h = 0; h < kSub; h++)
-            if ((has >> h) & 1u)
-              bulk_load(idx_ring + (slot * kSub + h) * kBM, src + h * kBM, kBM * 4u, &bar_idx_full[slot]);
-        }
-      }
-      __syncwarp();
-      if (++slot == kIdxSlots) { slot = 0; slot_phase ^= 1u; }
-    };
-    for (int i = 0; i < kIdxSlots && alive && more; i++) send_indices();
-
     int stage = 0;
     uint32_t phase = 0;
     uint32_t raw[kSub];
@@ -456,9 +408,55 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
           }
           __syncwarp();
         }
-        if (alive && more) send_indices();
       }
     }
+  } else if (warp == kIdxWarp) {
+    // ------------------------------ index blocks -------------------------------
+    // 128 entries of the neighbour table per step and sub-tile, up to kIdxSlots steps ahead of the
+    // producers, so that they never wait for an index from memory (loaded by the producers
+    // themselves, even two steps ahead, they cost a quarter of the time).  A lane copies 16 bytes of
+    // a block: no lane has to be elected, no byte count announced.  In one warp with the weight tiles a
+    // step took that warp 1000 cycles and bound the layers of up to 64 channels (us, before / now: 464k rows
+    // 32->32, 1.15 pairs a row, 37.7 / 32.8; 64->64 45 / 42; 406k 64->64, 3.4 pairs, 74.6 / 68; 123k 64->64,
+    // 16.7 pairs, 70 / 62; 406k 64->128 90 / 86).
+    const uint32_t ring = smem_u32(idx_ring) + (uint32_t)lane * 16u;
+    uint32_t raw[kSub], phase = 0;
+    request_bits<kSub, kMode>(args, (int)blockIdx.x, raw);
+    int slot = 0;
+    bool ready = true;
+    // one step of the tile at `src`: offsets p of the sub-tiles in `has`; 0 marks the end
+    auto send = [&](const int32_t *src, uint32_t has) {
+      if (!mbar_wait_warp(ready, &bar_idx_empty[slot], phase ^ 1u, abort_flag, args.status)) return false;
+      const uint32_t dst = ring + (uint32_t)(slot * kSub) * (kBM * 4);
+#pragma unroll
+      for (int h = 0; h < kSub; h++)
+        if ((has >> h) & 1u) cp_async_16(dst + h * (kBM * 4), src + h * kBM, 16u);
+      uint64_t *full = &bar_idx_full[slot];
+      asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(full)) : "memory");
+      if (lane == 0) {
+        s_idx_has[slot] = has;
+        mbar_arrive(full);
+      }
+      if (++slot == kIdxSlots) { slot = 0; phase ^= 1u; }
+      ready = mbar_test(&bar_idx_empty[slot], phase ^ 1u);
+      return true;
+    };
+    bool alive = kMode != kDense;
+    for (int tile = blockIdx.x; alive && tile < args.num_tiles; tile += gridDim.x) {
+      uint32_t hb[kSub];
+      take_bits<kSub>(args, tile, raw, hb);
+      request_bits<kSub, kMode>(args, tile + (int)gridDim.x, raw);
+      const int32_t *blocks = args.nbr + (int64_t)tile * (kSub * kBM) + lane * 4;
+      for (uint32_t rest = union_of<kSub>(hb); alive && rest != 0u; rest &= rest - 1u) {
+        const int p = __ffs(rest) - 1;
+        uint32_t has = 0u;
+#pragma unroll
+        for (int h = 0; h < kSub; h++) has |= ((hb[h] >> p) & 1u) << h;
+        alive = send(blocks + (int64_t)p * args.pitch, has);
+      }
+    }
+    if (alive) send(args.nbr, 0u);
+    asm volatile("cp.async.wait_all;" ::: "memory");   // nothing of this lane is in flight at exit
   } else {
     // ------------------------------ epilogue ----------------------------------
     // A lane owns one accumulator row and takes it 16 columns at a time: one 32-byte store
@@ -475,6 +473,7 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
     // next to 200 KB of shared memory L1 keeps no local memory, and each reload of a spilled
     // register was a trip to L2 (with 32 bytes of spills 918k rows 32->32 took 66 us, without
     // 52; the pieces' registers are therefore single, not double, buffered).
+    // tcgen05.ld reads the quarter of the tensor memory that the warp's number names
     const int quarter = warp & 3, first_piece = (warp - kEpiWarp) >> 2;
     const int n = args.N, pieces = args.n_pad / 16;
     const bool affine = args.scale != nullptr || args.shift != nullptr;
@@ -502,7 +501,6 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
     for (int tile = blockIdx.x; tile < args.num_tiles; tile += gridDim.x) {
       uint32_t hb[kSub];
       take_bits<kSub>(args, tile, raw, hb);
-      const bool empty_tile = union_of<kSub>(hb) == 0u;   // no MMA ran: the rows are zero
       request_bits<kSub, kMode>(args, tile + (int)gridDim.x, raw);
 #pragma unroll
       for (int h = 0; h < kSub; h++) { grow[h] = take_row(tile, h, rows_1[h]); rows_1[h] = rows_2[h]; }
@@ -577,7 +575,7 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
           // the branches inside the loop over the values a piece took 1300 cycles of latencies
           float f[16];
 #pragma unroll
-          for (int i = 0; i < 16; i++) f[i] = empty_tile ? 0.f : __uint_as_float(cur[i]);
+          for (int i = 0; i < 16; i++) f[i] = hb[h] == 0u ? 0.f : __uint_as_float(cur[i]);
           if (affine) {
 #pragma unroll
             for (int i = 0; i < 4; i++) {
@@ -1003,22 +1001,26 @@ extern "C" mn_status mn_sparse_convolution_forward_implicit(
   a.k_blocks = (int)div_up(c_in, kBK);
   a.n_tiles128 = (int)div_up(T, kBM);
   // One sub-tile: four producer and eight epilogue warps (918k rows 32->32 52 -> 50 us against
-  // eight and four, 243k rows 128->256 with stride 2 90 -> 78 us, 64->64 with 3.5 pairs a row
-  // 164 -> 158 us, 256->256 the same); two sub-tiles: twice the rows to fetch per step, eight
-  // producers (128->128 with 9.4 pairs a row 387 against 395 us).
-  // Sub-tiles per CTA tile.  The two sub-tiles of a CTA tile share the weight tile of a
-  // stage, at the price of a shallower ring; at 256 columns they also leave no room for a
-  // second accumulator set (the epilogue then no longer overlaps the next tile's MMAs).
-  // Measured on maps with 3.5 to 17 pairs per row (1 / 2 sub-tiles): 64 columns 155 / 191 us,
-  // 128 columns 399 / 366 us, 256 columns 535 / 593 us.  Callers that have timed the layer
-  // pass their own choice.
+  // eight and four, 243k rows 128->256 with stride 2 90 -> 78 us, 464k rows 64->64 45 -> 42 us); two
+  // sub-tiles: twice the rows to fetch per step, eight producers (128->128 with 9.4 pairs a row 387
+  // against 395 us).
+  // Sub-tiles per CTA tile.  The two sub-tiles of a CTA tile share the steps' bookkeeping and the weight
+  // tile of a stage, at the price of a shallower ring, fewer epilogue warps and tiles twice as large; a sub-tile
+  // is skipped in the steps of offsets that only the other one has.  It pays where the bookkeeping
+  // bounds a step and every CTA has several tiles (us, 1 / 2 sub-tiles).  32->32: 21.4k tiles of 1.15 pairs a
+  // row 145 / 110, 3.5k of 1.6 39 / 38, 0.9k 19 / 23.  64->64: 13.9k tiles of 9.3 pairs 570 / 541, 2.6k of 7
+  // 78 / 74, 3.2k of 3.4 70 / 72, 21.4k of 1.15 152 / 161.  More channels: 128->64 821 / 834, 64->128 472 /
+  // 512 (18.8k tiles), 128->128 1059 / 1100, 136 / 147 (3.2k), 57 / 62 (0.8k), 176 / 171 (2.3k of 9.3 pairs),
+  // 256->256 336 / 404.  Callers that have timed the layer pass their own choice.
   int sub = sub_hint;
   if (sub <= 0) {
+    const double tiles = a.n_tiles128;
     sub = 1;
-    if (pairs_per_row >= 2.0 && a.n_pad > 64 && a.n_pad <= 128) sub = 2;
-    while (sub > 1 && (sub * a.n_pad > 512 || a.n_tiles128 < 2 * sub * kNumSMs ||
-                       2 * (sub * kBM * kBK * 2 + a.n_pad * kBK * 2) + 2048 > 227 * 1024))
-      sub--;
+    if (c_in <= 32 && a.n_pad <= 32) {
+      if (tiles >= 32 * kNumSMs) sub = 2;
+    } else if (c_in <= 64 && a.n_pad <= 64) {
+      if (pairs_per_row >= 3.0 && tiles >= 16 * kNumSMs && tiles * pairs_per_row >= 16384) sub = 2;
+    }
   }
   MN_CHECK_ARG(sub_hint <= 4 && (sub_hint <= 0 || sub_hint * a.n_pad <= 512),
                "implicit forward: %d sub-tiles of %d columns do not fit TMEM", sub_hint, a.n_pad);

@@ -666,6 +666,10 @@ struct CumSizes {
   int64_t cum[MN_MAX_OFFSETS + 1];
 };
 
+// Rows of a block of rank_to_source_kernel, four loads a thread in flight: with one, the launch was the
+// rate at which 11 000 blocks start (105k rows, 27 offsets: 14.6 us).
+constexpr int kRankRows = 1024;
+
 // src_of_rank[cum[p] + source_masks[p, s]] = s.  Masks without hit words are a caller's own: a rank
 // that their sizes have no place for, or that only one side has, makes no pair (the ranks start
 // as -1).
@@ -674,10 +678,16 @@ rank_to_source_kernel(const int32_t *__restrict__ source_masks, int64_t S, int O
                       const __grid_constant__ CumSizes cs, int32_t *__restrict__ src_of_rank) {
   begin_early();
   const int p = blockIdx.y;
-  const int64_t gsz = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < S; s += gsz) {
-    const int m = __ldg(source_masks + (int64_t)p * S + s);
-    if (m >= 0 && m < cs.cum[p + 1] - cs.cum[p]) src_of_rank[cs.cum[p] + m] = (int32_t)s;
+  const int32_t *mask = source_masks + (int64_t)p * S;
+  const int64_t size = cs.cum[p + 1] - cs.cum[p];
+  int32_t *out = src_of_rank + cs.cum[p];
+  for (int64_t s0 = (int64_t)blockIdx.x * kRankRows + threadIdx.x; s0 < S; s0 += (int64_t)gridDim.x * kRankRows) {
+    int m[kRankRows / 256];
+#pragma unroll
+    for (int i = 0; i < kRankRows / 256; i++) m[i] = s0 + i * 256 < S ? __ldg(mask + s0 + i * 256) : -1;
+#pragma unroll
+    for (int i = 0; i < kRankRows / 256; i++)
+      if (m[i] >= 0 && m[i] < size) out[m[i]] = (int32_t)(s0 + i * 256);
   }
 }
 
@@ -705,6 +715,10 @@ rank_to_source_bits_kernel(const int32_t *__restrict__ source_masks,
 // of the table is never read by the forward pass, which checks tile_bits first.  The rows of
 // the table are `pitch` (T rounded up to 128) entries apart and -1 past T, so that the forward
 // pass reads whole tiles with vector loads.
+// What bounds it: a chain of dependent loads per thread.  With the offsets one after the other it was two trips
+// to L2 for each of them (105k rows, 27 offsets: 19.5 us); the loads of kTableBatch offsets are in flight together.
+constexpr int kTableBatch = 9;
+
 __global__ void __launch_bounds__(128)
 neighbor_table_kernel(const int32_t *__restrict__ target_masks, int64_t T, int64_t pitch, int O,
                       const __grid_constant__ CumSizes cs,
@@ -724,26 +738,42 @@ neighbor_table_kernel(const int32_t *__restrict__ target_masks, int64_t T, int64
     __syncthreads();
     const uint32_t tile = s_bits;
     if (threadIdx.x == 0) tile_bits[blockIdx.x] = tile;
-    for (uint32_t rest = tile; rest != 0u; rest &= rest - 1u) {
-      const int p = __ffs(rest) - 1;
-      int v = -1;
-      if ((mine >> p) & 1u) {
-        const int m = __ldg(target_masks + (int64_t)p * T + t);
-        if (m >= 0) v = __ldg(src_of_rank + cs.cum[p] + m);
+    for (uint32_t rest = tile; rest != 0u;) {
+      int p[kTableBatch], v[kTableBatch];
+#pragma unroll
+      for (int i = 0; i < kTableBatch; i++) {
+        p[i] = rest != 0u ? __ffs(rest) - 1 : -1;
+        rest &= rest - 1u;
+        v[i] = p[i] >= 0 && ((mine >> p[i]) & 1u) ? __ldg(target_masks + (int64_t)p[i] * T + t) : -1;
       }
-      nbr[(int64_t)p * pitch + r] = v;
+#pragma unroll
+      for (int i = 0; i < kTableBatch; i++)
+        if (v[i] >= 0) v[i] = __ldg(src_of_rank + cs.cum[p[i]] + v[i]);
+#pragma unroll
+      for (int i = 0; i < kTableBatch; i++)
+        if (p[i] >= 0) nbr[(int64_t)p[i] * pitch + r] = v[i];
     }
     return;
   }
   uint32_t mine = 0u;
-  for (int p = 0; p < O; p++) {
-    int v = -1;
-    if (r < T) {
-      const int m = __ldg(target_masks + (int64_t)p * T + t);
-      if (m >= 0 && m < cs.cum[p + 1] - cs.cum[p]) v = __ldg(src_of_rank + cs.cum[p] + m);
+  for (int p0 = 0; p0 < O; p0 += kTableBatch) {
+    int v[kTableBatch];
+#pragma unroll
+    for (int i = 0; i < kTableBatch; i++)
+      v[i] = r < T && p0 + i < O ? __ldg(target_masks + (int64_t)(p0 + i) * T + t) : -1;
+#pragma unroll
+    for (int i = 0; i < kTableBatch; i++) {
+      const int p = p0 + i;
+      if (p >= O) break;
+      const bool pair = v[i] >= 0 && v[i] < cs.cum[p + 1] - cs.cum[p];
+      v[i] = pair ? __ldg(src_of_rank + cs.cum[p] + v[i]) : -1;
     }
-    nbr[(int64_t)p * pitch + r] = v;
-    mine |= (v >= 0 ? 1u : 0u) << p;
+#pragma unroll
+    for (int i = 0; i < kTableBatch; i++) {
+      if (p0 + i >= O) break;
+      nbr[(int64_t)(p0 + i) * pitch + r] = v[i];
+      mine |= (v[i] >= 0 ? 1u : 0u) << (p0 + i);
+    }
   }
   mine = __reduce_or_sync(0xffffffffu, mine);
   if ((threadIdx.x & 31) == 0 && mine != 0u) atomicOr(&s_bits, mine);
@@ -924,7 +954,7 @@ extern "C" mn_status mn_build_neighbor_table(const int32_t *source_masks,
               launch_early(rank_to_source_bits_kernel, blocks, 256, 0, st, source_masks, source_bits, S, cs,
                                                                   src_of_rank));
   } else if (S > 0) {
-    const dim3 grid((unsigned)std::min<int64_t>(kNumSMs * 4, div_up(S, 256)), (unsigned)O);
+    const dim3 grid((unsigned)std::min<int64_t>(kNumSMs * 4, div_up(S, kRankRows)), (unsigned)O);
     MN_LAUNCH("rank_to_source_kernel", st,
               launch_early(rank_to_source_kernel, grid, 256, 0, st, source_masks, S, (int)O, cs, src_of_rank));
   }

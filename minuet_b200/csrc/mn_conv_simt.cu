@@ -111,9 +111,12 @@ __device__ __forceinline__ float cs_load_from(const float *at, int block) {
 // bytes at a time.  kFew: an item of up to 16 rows costs half as much (maps of 3.5 pairs a row: 32-row tiles
 // take 15 % less time, at 20 pairs 3 % more); not for the tall blocks of large maps, whose items are full.
 //
-// What bounds it: instruction issue.  Of 56 M warp instructions of a layer of 3.6k rows 128->128 with 14.5
-// pairs 38 M run on the FMA pipe, 27 M of them useful products, and a scheduler issues in 61 % of
-// the cycles (12 to 16 warps per SM; registers and shared memory allow no more).  Sparse maps: the
+// What bounds it: issue and latency at 12 to 16 warps per SM (registers and shared memory allow no more).
+// With one product per instruction, of 56 M warp instructions of a layer of 3.6k rows 128->128 with 14.5
+// pairs 38 M ran on the FMA pipe, and a scheduler issued in 61 % of the cycles; with two (the same rate of
+// products, half the issue slots) layers of 15k rows 64->64 with 12.3 pairs take 75 instead of 85 us, 41k 32->32
+// with 7.7 45 instead of 48.5, 3.4k 128->128 79 instead of 89, 700 rows 256->256 103 instead of 113.  The weight
+// gradients, whose tiles are 8 x 8, gain nothing by it.  Sparse maps: the
 // chain tile bits -> index blocks -> rows before a block's first product.
 //
 // Against a block of 64 x 64 (or 32 x 32) sums in registers that walked its tile's offsets one after
@@ -329,11 +332,9 @@ conv_simt_kernel(const __grid_constant__ CsArgs a) {
       else asm volatile("cp.async.commit_group;" ::: "memory");
     }
 
-    float acc[8][4];
+    f32_pair acc[8][2];                            // 8 rows x 4 columns
 #pragma unroll
-    for (int i = 0; i < 8; i++)
-#pragma unroll
-      for (int j = 0; j < 4; j++) acc[i][j] = 0.f;
+    for (int i = 0; i < 8; i++) acc[i][0] = acc[i][1] = 0u;
     int place[4];                                  // of the four-channel pieces of this lane's rows
 #pragma unroll
     for (int k = 0; k < 4; k++) place[k] = ty * kCsK + ((k ^ (ty >> 1)) << 2);
@@ -369,10 +370,9 @@ conv_simt_kernel(const __grid_constant__ CsArgs a) {
             const float ak[4] = {av[i].x, av[i].y, av[i].z, av[i].w};
 #pragma unroll
             for (int j = 0; j < 4; j++) {
-              acc[i][0] = fmaf(ak[j], bv[j].x, acc[i][0]);
-              acc[i][1] = fmaf(ak[j], bv[j].y, acc[i][1]);
-              acc[i][2] = fmaf(ak[j], bv[j].z, acc[i][2]);
-              acc[i][3] = fmaf(ak[j], bv[j].w, acc[i][3]);
+              const f32_pair a2 = make_pair_f32(ak[j], ak[j]);
+              fma_pair_f32(a2, make_pair_f32(bv[j].x, bv[j].y), acc[i][0]);
+              fma_pair_f32(a2, make_pair_f32(bv[j].z, bv[j].w), acc[i][1]);
             }
           }
         }
@@ -386,9 +386,8 @@ conv_simt_kernel(const __grid_constant__ CsArgs a) {
         float4 *product = reinterpret_cast<float4 *>(s_sum + (item / kCluster * kCsRows + ty) * kCsRows) + tx;
 #pragma unroll
         for (int i = 0; i < 8; i++) {
-          if (4 * i < left) product[i * 4 * (kCsRows / 4)] = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
-#pragma unroll
-          for (int j = 0; j < 4; j++) acc[i][j] = 0.f;
+          if (4 * i < left) product[i * 4 * (kCsRows / 4)] = split_pairs_f32(acc[i][0], acc[i][1]);
+          acc[i][0] = acc[i][1] = 0u;
         }
         next_item();
         continue;
@@ -398,9 +397,8 @@ conv_simt_kernel(const __grid_constant__ CsArgs a) {
         for (int i = 0; i < 8; i++) {
           const int c = n0 + (entry >> 8) * kCsRows + tx * 4;
           if (4 * i < left && c < a.N)
-            store_row(make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]), r0 + first + 4 * i, c);
-#pragma unroll
-          for (int j = 0; j < 4; j++) acc[i][j] = 0.f;
+            store_row(split_pairs_f32(acc[i][0], acc[i][1]), r0 + first + 4 * i, c);
+          acc[i][0] = acc[i][1] = 0u;
         }
         next_item();
         continue;
@@ -410,12 +408,12 @@ conv_simt_kernel(const __grid_constant__ CsArgs a) {
       for (int i = 0; i < 8; i++) {
         if (4 * i < left) {
           float4 *sum = reinterpret_cast<float4 *>(s_sum + rows[4 * i] * kSumCols + (entry >> 8) * kCsRows) + tx;
+          const float4 mine = split_pairs_f32(acc[i][0], acc[i][1]);
           float4 v = *sum;
-          v.x += acc[i][0]; v.y += acc[i][1]; v.z += acc[i][2]; v.w += acc[i][3];
+          v.x += mine.x; v.y += mine.y; v.z += mine.z; v.w += mine.w;
           *sum = v;
         }
-#pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j] = 0.f;
+        acc[i][0] = acc[i][1] = 0u;
       }
       if (W > 1 && !own && item + 1 < n_items) {
         cs_turn_pass(1 + (warp + 1) % W);

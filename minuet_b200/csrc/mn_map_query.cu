@@ -16,10 +16,13 @@
 // shared memory as a hash set of CELLS (32 consecutive values of the last
 // dimension -> {cell id, 32-bit occupancy}, 8-byte slots, linear probing): the
 // offsets that differ only in the last dimension (a "group", split so that its
-// span is at most 16) are answered by ONE lookup per row, plus a second one for
-// the few rows whose strip crosses a cell boundary; shared-memory bandwidth, not
-// instruction issue, is what bounds this kernel, hence the 64-bit single-slot
-// lookups.  Tiles whose window does not fit the hash are
+// span is at most 14) are answered by ONE lookup per row, of 16 bytes, i.e. two slots at once.
+// What bounds it: instructions and their latency, at five blocks per SM.  A tile of 7.3 million rows and
+// 27 offsets took 35 000 cycles, 12 000 of them before its window was known and 19 400 in lookups;
+// now 7 500 (layout, keys and tile ends in one trip, the hash cleared before the wait for the kernel
+// before, bounds looked for near the tile where the rows are the table) and 13 000 (strips that lie in one cell,
+// keys of 32 bits, the few longer probes of a warp in one loop at the end).  464k rows, four
+// maps: 138 -> 99 us of searches; 7.3 million, two maps: 634 -> 534 us.  Tiles whose window does not fit the hash are
 // processed group range by group range, and ranges that still do not fit fall
 // back to binary search in global memory.  The kernel writes kernel-map rows
 // or, for the fused build, one 32-bit word of per-offset hit bits per row.
@@ -48,11 +51,13 @@ constexpr int kQWarps = kQThreads / 32;
 constexpr int kQRows = 2;                    // rows per thread
 constexpr int kQTile = kQThreads * kQRows;   // 512 rows per block
 constexpr int kQSlots = 4096;                // hash slots of 8 bytes: {cell, occupancy}
-constexpr int kQMaxWindow = 1280;            // table keys per hashed stage (load factor <= 0.31)
-constexpr int kQMaxSpan = 16;                // last-dimension span of one group
+constexpr int kQMaxWindow = 1280;            // table keys per hashed stage (load factor <= 0.31, with a key in two cells 0.33 for 3 x 3 x 3)
+constexpr int kQMaxSpan = 14;                // last-dimension span of one group
 constexpr uint32_t kQPad = 64;               // relative keys start at kQPad
 constexpr uint32_t kHashEmpty = 0xffffffffu;
 constexpr uint64_t kRelLimit = 0xffffffffull - 4ull * kQPad;
+constexpr uint64_t kNarrow = 1ull << 29;
+constexpr uint32_t kQNowhere = 0xffffffe0u;  // relative key in a cell past every window's (below kRelLimit)
 
 __device__ __forceinline__ unsigned lanemask_lt() {
   unsigned m;
@@ -86,6 +91,24 @@ __device__ __forceinline__ int64_t warp_bound(const uint64_t *__restrict__ t, in
   return lo;
 }
 
+// The same for a bound that is probably near a known place (the tile's own rows, where the rows are
+// the table): one round of probes at doubling distances, then the search between two of them.
+// Lower bound of q <= t[at] (upper false), upper bound of q >= t[at] (upper true), at inside [0, n).
+__device__ __forceinline__ int64_t warp_bound_near(const uint64_t *__restrict__ t, int64_t n, int64_t at, uint64_t q,
+                                                   bool upper, int lane) {
+  constexpr int64_t kFirst = 16;
+  const int64_t idx = upper ? at + (kFirst << lane) : at - (kFirst << lane);
+  bool inside = false;                       // the bound lies beyond this probe
+  if (idx >= 0 && idx < n) {
+    const uint64_t v = __ldg(t + idx);
+    inside = upper ? v <= q : v >= q;
+  }
+  const int c = __popc(__ballot_sync(0xffffffffu, inside));
+  const int64_t near = c > 0 ? kFirst << (c - 1) : 0, far = kFirst << min(c, 31);
+  if (upper) return warp_bound(t, at + near + 1, min(at + far, n), q, true, lane);
+  return warp_bound(t, max(at - far + 1, (int64_t)0), at - near, q, false, lane);
+}
+
 struct SearchArgs {
   const uint64_t *rows;
   const uint64_t *table;
@@ -97,11 +120,29 @@ struct SearchArgs {
   int32_t n_tiles;
 };
 
+// Cells overlap: cell c holds the keys from c * step to c * step + 31, step = 32 - (largest span of a group),
+// rounded down to even, so that the strip that a group asks for lies in one cell, and a key near the start of a
+// cell is in the one before too.  (In cells side by side one strip in sixteen crossed into the next, i.e. one in
+// almost every warp.)  The quotient is exact: k / 2 < 2^31, magic = ceil(2^35 / (step / 2)), step / 2 in 9..16.
+struct CellStep {
+  uint32_t step, magic;
+  __device__ __forceinline__ uint32_t cell(uint32_t k) const { return (uint32_t)(((uint64_t)(k >> 1) * magic) >> 35); }
+};
+inline CellStep cell_step(const OffsetTable &t) {
+  int span = 0;
+  for (int g = 0; g < t.num_groups; g++)
+    span = std::max(span, t.off[t.member[t.group_begin[g + 1] - 1]][t.ndim - 1] -
+                              t.off[t.member[t.group_begin[g]]][t.ndim - 1]);
+  const uint32_t half = (uint32_t)(32 - span) / 2;
+  return CellStep{2 * half, (uint32_t)(((1ull << 35) + half - 1) / half)};
+}
+
 // One launch can serve two searches (e.g. targets->sources and sources->targets).
 struct SearchPair {
   SearchArgs a[2];
   OffsetTable tab[2];
   SpecRef spec;
+  CellStep cells[2];
   int32_t tiles0;   // blocks of the first search
 };
 
@@ -113,23 +154,9 @@ enum SearchMode { kMap = 0, kBits = 1, kBitsRev = 2 };
 MN_MARKS_DECL(g_marks_search);
 MN_MARKS_DECL(g_marks_emit);
 
+// First of the two slots that a lookup reads at once.
 __device__ __forceinline__ uint32_t hash_slot(uint32_t c) {
-  return (c * 0x9E3779B1u) >> 20;  // top 12 bits: 4096 slots
-}
-
-// Occupancy mask of cell c (0 when absent) and the slot that holds it: linear
-// probing over 8-byte {cell, mask} slots, one 64-bit shared-memory load per step.
-// At the load factors used (<= 0.31) most lookups end at the first slot.
-__device__ __forceinline__ uint32_t find_cell(const uint2 *slots, uint32_t c, uint32_t *slot) {
-  uint32_t h = hash_slot(c);
-  for (int probe = 0; probe < kQSlots; probe++) {
-    const uint2 v = slots[h];
-    if (v.x == c) { *slot = h; return v.y; }
-    if (v.x == kHashEmpty) break;
-    h = (h + 1) & (kQSlots - 1);
-  }
-  *slot = 0;
-  return 0u;
+  return (c * 0x9E3779B1u) >> 20 & ~1u;  // top 12 bits: 4096 slots
 }
 
 __device__ __forceinline__ uint32_t insert_cell(uint2 *slots, uint32_t c, uint32_t bit) {
@@ -146,19 +173,18 @@ __device__ __forceinline__ uint32_t insert_cell(uint2 *slots, uint32_t c, uint32
 template <int kMode>
 __global__ void __launch_bounds__(kQThreads, kMode == kBits ? 5 : 4)
 search_kernel(const __grid_constant__ SearchPair sp) {
-  begin_early();
   constexpr bool kPos = kMode != kBits;   // table positions are needed
   // blocks [0, tiles0) serve direction 0, the rest direction 1 (rows and table swapped)
   const int dir = (int)blockIdx.x >= sp.tiles0 ? 1 : 0;
   const int bid = (int)blockIdx.x - dir * sp.tiles0;
   const SearchArgs &a = sp.a[dir];
   const OffsetTable &tab = sp.tab[dir];
-  const mn_keyspec &spec = spec_of(sp.spec);
+  const CellStep cells = sp.cells[dir];
   __shared__ __align__(16) uint2 s_slots[kQSlots];
   __shared__ uint16_t s_hpos[kPos ? kQSlots : 2];   // first position of a cell
   __shared__ int64_t s_delta[MN_MAX_OFFSETS];
   __shared__ int64_t s_gdelta[MN_MAX_OFFSETS];       // per group: delta of its first member
-  __shared__ uint32_t s_gmeta[MN_MAX_OFFSETS];       // span | first offset << 8 | members << 16 | compact << 24
+  __shared__ uint32_t s_gmeta[MN_MAX_OFFSETS];       // first offset | members << 8 | compact << 16
   __shared__ int64_t s_glo[MN_MAX_OFFSETS], s_ghi[MN_MAX_OFFSETS];
   __shared__ int64_t s_slo[MN_MAX_OFFSETS], s_shi[MN_MAX_OFFSETS];
   __shared__ uint8_t s_stage_gbeg[MN_MAX_OFFSETS + 1];
@@ -171,29 +197,27 @@ search_kernel(const __grid_constant__ SearchPair sp) {
   const int64_t tile0 = (int64_t)bid * kQTile;
   const int tile_rows = (int)min((int64_t)kQTile, a.n_rows - tile0);
   const int64_t row0 = tile0 + tid * kQRows;
-  MN_MARK(g_marks_search, 0);
-
-  for (int o = tid; o < O; o += kQThreads) {
-    int64_t d = 0;
-    for (int k = 0; k < tab.ndim; k++) d += (int64_t)tab.off[o][k] * ((int64_t)1 << spec.shift[k]);
-    s_delta[o] = d;
-  }
+  auto clear_slots = [&]() {
+    uint4 *clear = reinterpret_cast<uint4 *>(s_slots);
+    for (int i = tid; i < kQSlots / 2; i += kQThreads)
+      clear[i] = make_uint4(kHashEmpty, 0u, kHashEmpty, 0u);   // two {cell, mask} slots
+  };
+  // what needs no memory of the GPU, while the kernel before this one drains
+  clear_slots();
   for (int g = tid; g < G; g += kQThreads) {
     const int mb = tab.group_begin[g], me = tab.group_begin[g + 1];
     const int o_first = tab.member[mb];
-    int64_t d = 0;
-    for (int k = 0; k < tab.ndim; k++) d += (int64_t)tab.off[o_first][k] * ((int64_t)1 << spec.shift[k]);
-    s_gdelta[g] = d;
     // compact: member i is offset o_first + i and sits i values further along the last dimension
     bool compact = true;
     for (int m = mb; m < me; m++)
       compact &= tab.member[m] == o_first + (m - mb) &&
                  tab.off[tab.member[m]][last] - tab.off[o_first][last] == m - mb;
-    const int span = tab.off[tab.member[me - 1]][last] - tab.off[o_first][last];
-    s_gmeta[g] = (uint32_t)span | ((uint32_t)o_first << 8) | ((uint32_t)(me - mb) << 16) |
-                 ((compact ? 1u : 0u) << 24);
+    s_gmeta[g] = (uint32_t)o_first | ((uint32_t)(me - mb) << 8) | ((compact ? 1u : 0u) << 16);
   }
+  begin_early();
+  MN_MARK(g_marks_search, 0);
 
+  // one trip to memory: the rows' keys, the tile's ends and the key layout together
   uint64_t key[kQRows];
   bool live[kQRows];
   if (tid * kQRows + kQRows <= tile_rows && (reinterpret_cast<uintptr_t>(a.rows) & 15) == 0) {
@@ -209,14 +233,31 @@ search_kernel(const __grid_constant__ SearchPair sp) {
   }
   const uint64_t kfirst = __ldg(a.rows + tile0);
   const uint64_t klast = __ldg(a.rows + tile0 + tile_rows - 1);
+  {
+    const mn_keyspec &spec = spec_of(sp.spec);
+    int shift[MN_MAX_NDIM];
+#pragma unroll
+    for (int k = 0; k < MN_MAX_NDIM; k++) shift[k] = k < tab.ndim ? spec.shift[k] : 0;
+    for (int o = tid; o < O; o += kQThreads) {
+      int64_t d = 0;
+#pragma unroll
+      for (int k = 0; k < MN_MAX_NDIM; k++)
+        if (k < tab.ndim) d += (int64_t)tab.off[o][k] * ((int64_t)1 << shift[k]);
+      s_delta[o] = d;
+    }
+  }
   __syncthreads();
+  for (int g = tid; g < G; g += kQThreads) s_gdelta[g] = s_delta[tab.member[tab.group_begin[g]]];
   MN_MARK(g_marks_search, 1);
 
   // window of the table over all offsets: members are ordered by delta
   if (warp < 2) {
     const uint64_t q = warp == 0 ? kfirst + (uint64_t)s_delta[tab.member[0]]
                                  : klast + (uint64_t)s_delta[tab.member[O - 1]];
-    const int64_t r = warp_bound(a.table, 0, a.n_table, q, warp == 1, lane);
+    // rows that are the table: the window surrounds the tile
+    const bool own = a.rows == a.table && a.n_rows == a.n_table && (warp == 0 ? q <= kfirst : q >= klast);
+    const int64_t r = own ? warp_bound_near(a.table, a.n_table, warp == 0 ? tile0 : tile0 + tile_rows - 1, q, warp == 1, lane)
+                          : warp_bound(a.table, 0, a.n_table, q, warp == 1, lane);
     if (lane == 0) s_union[warp] = r;
   }
   __syncthreads();
@@ -271,9 +312,8 @@ search_kernel(const __grid_constant__ SearchPair sp) {
   MN_MARK(g_marks_search, 2);
 
   uint32_t bits[kQRows] = {0u, 0u};
-  const bool vec_ok = kMode == kMap && (a.n_rows & 1) == 0 &&
-                      (reinterpret_cast<uintptr_t>(a.kernel_map) & 7) == 0 && live[kQRows - 1];
   const int num_stages = s_num_stages;
+  bool clean = true;                          // no keys in the hash yet
   for (int st = 0; st < num_stages; st++) {
     const int gb = s_stage_gbeg[st], ge = s_stage_gbeg[st + 1];
     const int64_t lo = s_slo[st], hi = s_shi[st];
@@ -285,22 +325,24 @@ search_kernel(const __grid_constant__ SearchPair sp) {
       hashed = __ldg(a.table + hi - 1) - base < kRelLimit;
     }
     if (hashed) {
-      {
-        uint4 *clear = reinterpret_cast<uint4 *>(s_slots);
-        for (int i = tid; i < kQSlots / 2; i += kQThreads)
-          clear[i] = make_uint4(kHashEmpty, 0u, kHashEmpty, 0u);   // two {cell, mask} slots
+      if (!clean) {
+        clear_slots();
+        __syncthreads();
       }
-      __syncthreads();
+      clean = false;
       MN_MARK(g_marks_search, 3);
       // relative keys start at kQPad, so that a query below the window stays non-negative
       for (int w = tid; w < wn; w += kQThreads) {
         const uint32_t k = (uint32_t)(__ldg(a.table + lo + w) - base) + kQPad;
-        const uint32_t h = insert_cell(s_slots, k >> 5, k & 31u);
-        if (kPos) {
-          // the table is sorted: exactly one key of a cell has a predecessor in another cell
-          uint32_t pk = 0;
-          if (w > 0) pk = (uint32_t)(__ldg(a.table + lo + w - 1) - base) + kQPad;
-          if (w == 0 || (pk >> 5) != (k >> 5)) s_hpos[h] = (uint16_t)w;
+        // the table is sorted: a cell's keys follow one another, and all but the first have a predecessor in it
+        uint32_t pk = 0;
+        if (kPos && w > 0) pk = (uint32_t)(__ldg(a.table + lo + w - 1) - base) + kQPad;
+        const uint32_t c = cells.cell(k), at = k - c * cells.step;
+        const uint32_t h = insert_cell(s_slots, c, at);
+        if (kPos && (w == 0 || pk < k - at)) s_hpos[h] = (uint16_t)w;
+        if (at + cells.step < 32u) {
+          const uint32_t h1 = insert_cell(s_slots, c - 1u, at + cells.step);
+          if (kPos && (w == 0 || pk < k - at - cells.step)) s_hpos[h1] = (uint16_t)w;
         }
       }
       __syncthreads();
@@ -309,76 +351,77 @@ search_kernel(const __grid_constant__ SearchPair sp) {
 #pragma unroll
       for (int j = 0; j < kQRows; j++)   // a dead row gets a value that no window can reach
         rel[j] = live[j] ? (int64_t)(key[j] - base) + kQPad : (int64_t)1 << 62;
-      for (int g = gb; g < ge; g++) {
-        const int64_t dg = s_gdelta[g];
-        const uint32_t meta = s_gmeta[g];
-        const uint32_t e_span = meta & 0xffu, o_first = (meta >> 8) & 0xffu,
-                       members = (meta >> 16) & 0xffu;
-        // per row: the strip of last-dimension values [q0, q0 + 31] as one 32-bit mask, from
-        // the cell of q0 and, when the group reaches past its end, the next cell
-        uint32_t sh[kQRows], mlo[kQRows], mhi[kQRows], slo[kQRows], shi[kQRows];
-#pragma unroll
-        for (int j = 0; j < kQRows; j++) {
-          const uint64_t t0 = (uint64_t)(rel[j] + dg);
-          const uint32_t q0 = (uint32_t)t0;
-          const bool ok = t0 < kRelLimit;
-          sh[j] = q0 & 31u;
-          slo[j] = shi[j] = 0u;
-          mlo[j] = mhi[j] = 0u;
-          if (ok) {
-            mlo[j] = find_cell(s_slots, q0 >> 5, &slo[j]);
-            if (sh[j] + e_span > 31u) mhi[j] = find_cell(s_slots, (q0 >> 5) + 1u, &shi[j]);
+      // Where window, rows and offsets span less than 2^29 the relative keys are sums of 32 bits: what
+      // falls outside the window is in no cell of it (a dead row's sums are off by 2^31).
+      const int64_t first_delta = s_delta[tab.member[0]], last_delta = s_delta[tab.member[O - 1]];
+      const bool narrow = __ldg(a.table + hi - 1) - base < kNarrow && (int64_t)(kfirst - base) > -(int64_t)kNarrow &&
+                          (int64_t)(klast - base) < (int64_t)kNarrow && first_delta > -(int64_t)kNarrow &&
+                          last_delta < (int64_t)kNarrow;
+      auto relative = [&](int j, int g) {
+        if (narrow) return (uint32_t)rel[j] + (uint32_t)s_gdelta[g] + (live[j] ? 0u : 0x80000000u);
+        const uint64_t t0 = (uint64_t)(rel[j] + s_gdelta[g]);
+        return t0 < kRelLimit ? (uint32_t)t0 : kQNowhere;
+      };
+      // what the offsets of group g find for row j: the strip of its cell from `sh` on
+      auto found = [&](int j, int g, uint32_t mask, uint32_t sh, uint32_t slot) {
+        const uint32_t meta = s_gmeta[g], o_first = meta & 0xffu, members = (meta >> 8) & 0xffu;
+        if (kMode != kMap && (meta >> 16) != 0u) {
+          const uint32_t strip = (mask >> sh) & ((1u << members) - 1u);
+          bits[j] |= strip << o_first;
+          if (kMode == kBitsRev && strip != 0u) {
+            // entries of a cell follow one another
+            uint32_t *at = a.table_words + lo + s_hpos[slot] + __popc(mask & ((1u << sh) - 1u));
+            for (uint32_t rest = strip; rest != 0u; rest &= rest - 1u, at++)
+              atomicOr(at, (rest & (0u - rest)) << o_first);
+          }
+          return;
+        }
+        const int mb = tab.group_begin[g], e_first = tab.off[o_first][last];
+        for (int m = mb; m < mb + (int)members; m++) {
+          const int o = tab.member[m];
+          const uint32_t b = sh + (uint32_t)(tab.off[o][last] - e_first);   // < 32
+          const bool hit = (mask >> b) & 1u;
+          int32_t idx = -1;
+          if (kPos && hit) idx = (int32_t)(lo + s_hpos[slot] + __popc(mask & ((1u << b) - 1u)));
+          if (kMode == kMap) {
+            if (live[j]) a.kernel_map[(int64_t)o * a.n_rows + row0 + j] = idx;
+          } else if (hit) {
+            bits[j] |= 1u << o;
+            if (kMode == kBitsRev) atomicOr(a.table_words + idx, 1u << o);
           }
         }
-        if (kMode == kBits && (meta >> 24) != 0u) {
+      };
+      // Linear probing over {cell, mask} slots.  The first two slots are one load and hold nearly all answers;
+      // a lookup that has to go on is put off (its offsets have found nothing so far) until the others are
+      // through, so that a warp goes round the probing loop for its few of them together.
+      for (int g0 = gb; g0 < ge; g0 += 32) {
+        const int g1 = min(ge, g0 + 32);
+        uint32_t open[kQRows] = {0u, 0u};
+#pragma unroll 3
+        for (int g = g0; g < g1; g++) {
 #pragma unroll
           for (int j = 0; j < kQRows; j++) {
-            const uint32_t strip = (uint32_t)((((uint64_t)mhi[j] << 32) | mlo[j]) >> sh[j]);
-            bits[j] |= (strip & ((1u << members) - 1u)) << o_first;
+            const uint32_t q = relative(j, g), c = cells.cell(q), sh = q - c * cells.step, slot = hash_slot(c);
+            const uint4 v = *reinterpret_cast<const uint4 *>(s_slots + slot);
+            const bool second = v.z == c;
+            const uint32_t mask = v.x == c ? v.y : second ? v.w : 0u;
+            if (v.x != c && !second && v.z != kHashEmpty) open[j] |= 1u << (g - g0);
+            found(j, g, mask, sh, slot + (second ? 1u : 0u));
           }
-          continue;
         }
-        const int mb = tab.group_begin[g], me = mb + (int)members;
-        const int e_first = tab.off[o_first][last];
-        for (int m = mb; m < me; m++) {
-          const int o = tab.member[m];
-          const int de = tab.off[o][last] - e_first;
-          if (kMode == kBits) {
 #pragma unroll
-            for (int j = 0; j < kQRows; j++) {
-              const uint64_t both = ((uint64_t)mhi[j] << 32) | mlo[j];
-              bits[j] |= ((uint32_t)(both >> (sh[j] + de)) & 1u) << o;
-            }
-          } else {
-            int32_t idx[kQRows];
-#pragma unroll
-            for (int j = 0; j < kQRows; j++) {
-              const uint32_t b = sh[j] + (uint32_t)de;   // < 48
-              idx[j] = -1;
-              if (b < 32u) {
-                if ((mlo[j] >> b) & 1u)
-                  idx[j] = (int32_t)(lo + s_hpos[slo[j]] + __popc(mlo[j] & ((1u << b) - 1u)));
-              } else if ((mhi[j] >> (b - 32u)) & 1u) {
-                idx[j] = (int32_t)(lo + s_hpos[shi[j]] + __popc(mhi[j] & ((1u << (b - 32u)) - 1u)));
-              }
-            }
-            if (kMode == kBitsRev) {
-#pragma unroll
-              for (int j = 0; j < kQRows; j++) {
-                if (idx[j] >= 0) {
-                  bits[j] |= 1u << o;
-                  atomicOr(a.table_words + idx[j], 1u << o);
-                }
-              }
-            } else {
-              int32_t *dst = a.kernel_map + (int64_t)o * a.n_rows + row0;
-              if (vec_ok) {
-                *reinterpret_cast<int2 *>(dst) = make_int2(idx[0], idx[1]);
-              } else {
-#pragma unroll
-                for (int j = 0; j < kQRows; j++) if (live[j]) dst[j] = idx[j];
-              }
-            }
+        for (int j = 0; j < kQRows; j++) {
+          for (; open[j] != 0u; open[j] &= open[j] - 1u) {
+            const int g = g0 + __ffs(open[j]) - 1;
+            const uint32_t q = relative(j, g), c = cells.cell(q);
+            uint32_t slot = hash_slot(c) + 1u;
+            uint2 v;
+            int probe = 0;
+            do {
+              slot = (slot + 1u) & (kQSlots - 1);
+              v = s_slots[slot];
+            } while (v.x != c && v.x != kHashEmpty && ++probe < kQSlots);
+            if (v.x == c) found(j, g, v.y, q - c * cells.step, slot);
           }
         }
       }
@@ -781,12 +824,14 @@ mn_status run_search(int mode, const mn_keyspec &spec, const SearchArgs &first,
   thread_local static SearchPair sp;   // ~5 KB: kept off the stack; passed by value per launch
   sp.a[0] = first;
   sp.tab[0] = tab_first;
+  sp.cells[0] = cell_step(tab_first);
   sp.spec = make_spec_ref(spec);
   sp.tiles0 = first.n_tiles;
   int blocks = first.n_tiles;
   if (second != nullptr) {
     sp.a[1] = *second;
     sp.tab[1] = *tab_second;
+    sp.cells[1] = cell_step(*tab_second);
     blocks += second->n_tiles;
   }
   if (blocks == 0) return MN_OK;

@@ -54,6 +54,7 @@ constexpr int kMaxStages = 8;
 constexpr int kMaxN = 256;
 constexpr int kIdxSlots = 8;           // steps the index blocks run ahead
 constexpr int kMaxSub = 2;             // 128-row sub-tiles per CTA tile
+constexpr int kResSlot = 32 * 64;      // bytes of 32 columns of 32 rows of the residual
 constexpr int kNBlock = kBK * 128;     // kMapNMajor: bytes of one block of 64 columns of a weight tile
 
 // What feeds the kernel: a kernel map; the same with weights as they are, [O, K, N], as N-major
@@ -119,6 +120,11 @@ __device__ __forceinline__ void ld_global_16(const void *src, uint32_t *r) {
   r[0] = v.x; r[1] = v.y; r[2] = v.z; r[3] = v.w;
 }
 
+__device__ __forceinline__ void ld_shared_16(uint32_t src, uint32_t *r) {
+  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(src) : "memory");
+}
+
 __device__ __forceinline__ void st_global_32(void *dst, const uint32_t *r) {
   asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(r[0]),
                "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
@@ -167,8 +173,9 @@ __device__ __forceinline__ uint32_t union_of(const uint32_t (&hb)[kSub]) {
 
 // kSub: sub-tiles per CTA tile (they share every weight tile); kLpr: lanes that copy one
 // 128-byte slice (4 where a source row has at most 64 bytes: half the copies, twice the rows
-// per copy); kProdWarps: 4 producer and 8 epilogue warps or 8 and 4.
-template <int kSub, int kLpr, int kProdWarps, int kMode>
+// per copy); kProdWarps: 4 producer and 8 epilogue warps or 8 and 4; kStaged: the epilogue's
+// residual comes through shared memory.
+template <int kSub, int kLpr, int kProdWarps, int kMode, bool kStaged>
 __global__ void __launch_bounds__(kImThreads, kImCtas)
 conv_implicit_kernel(const __grid_constant__ ImArgs args,
                      const __grid_constant__ CUtensorMap map_a,     // kDense: features [S, K]
@@ -462,28 +469,31 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
     // A lane owns one accumulator row and takes it 16 columns at a time: one 32-byte store
     // (a whole sector of the output row, wherever perm puts it) and, with a residual, one
     // 32-byte load requested while the piece before is rounded and stored.  Two warps share a
-    // quarter of the rows where there are eight: they take alternate pieces.  No shared-memory
-    // staging: its barriers and index shuffles cost more than the wider stores gave, and the
-    // 32 KB are worth more as ring stages.
-    // This role bounds the levels with few pairs a row (of 54 us for 480k rows 64->64 with 1.15 pairs a CTA
-    // spends 8 before its first tile is in flight, then 2.6 a tile).  Not by the latency of its instructions,
-    // although every piece is a chain of some 100: two groups of epilogue warps with a tile each, and
-    // residuals asked for a tile earlier, took the same time.  In the rows' own order (dense mode) it runs at
-    // the copy rate; what is left is that pieces of rows go to scattered places.  It must not spill:
+    // quarter of the rows where there are eight: they take alternate pieces.  Stores stay 32 bytes a lane: rows
+    // written by four lanes together (an exchange between lanes or through shared memory before) took the
+    // same time or longer.
+    // This role bounds the levels with few pairs a row (64->64, 1.15 pairs a row: the first tile of a CTA is in
+    // flight after 8 us, then 2.3 a tile).  Not by the latency of its instructions, although every piece is a chain
+    // of some 100: two groups of epilogue warps with a tile each took the same time.  What it spends is
+    // the issue of scattered accesses: 32 lanes that each touch a line of their own.  It must not spill:
     // next to 200 KB of shared memory L1 keeps no local memory, and each reload of a spilled
     // register was a trip to L2 (with 32 bytes of spills 918k rows 32->32 took 66 us, without
     // 52; the pieces' registers are therefore single, not double, buffered).
     // tcgen05.ld reads the quarter of the tensor memory that the warp's number names
-    const int quarter = warp & 3, first_piece = (warp - kEpiWarp) >> 2;
-    const int n = args.N, pieces = args.n_pad / 16;
+    const int quarter = warp & 3, group = (warp - kEpiWarp) >> 2;
+    // two warps of a quarter take alternate pieces, or neighbouring ones where they copy residuals
+    constexpr int kStep = kStaged ? 1 : kEpiCols;
+    const int n = args.N, pieces = args.n_pad / 16, share = (pieces + kEpiCols - 1) / kEpiCols;
+    const int first_piece = kStaged ? group * share : group;
+    const int last_piece = kStaged ? min(pieces, first_piece + share) : pieces;
     const bool affine = args.scale != nullptr || args.shift != nullptr;
     int acc = 0;
     uint32_t acc_phase = 0;
     uint32_t raw[kSub];
     request_bits<kSub, kMode>(args, (int)blockIdx.x, raw);
     // Row of the output (and of the residual) that this lane's accumulator row belongs to, per
-    // sub-tile (-1: none): requested two tiles ahead, so that the residual rows of the next tile
-    // can be on their way to L2 while this one is worked on.
+    // sub-tile (-1: none): requested two tiles ahead (one where residuals are copied ahead), so that the residual
+    // rows of the next tile can be on their way to L2 while this one is worked on.
     const bool permuted = kMode <= kMapNMajor && args.perm != nullptr;
     auto table_row = [&](int tile, int h) { return ((int64_t)tile * kSub + h) * kBM + quarter * 32 + lane; };
     auto request_rows = [&](int tile, int32_t (&rows)[kSub]) {
@@ -497,15 +507,42 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
     };
     int32_t grow[kSub], rows_1[kSub] = {}, rows_2[kSub] = {};
     request_rows((int)blockIdx.x, rows_1);
-    request_rows((int)(blockIdx.x + gridDim.x), rows_2);
+    if (!kStaged) request_rows((int)(blockIdx.x + gridDim.x), rows_2);
+    // Residuals of 33 to 64 columns come through a ring of this warp's own, one use of it (two pieces) ahead:
+    // four lanes copy 64 bytes of a row, where a lane that reads its own row's pieces makes every load
+    // 32 lines of 128 bytes.  64->64, us: 464k rows of 1.15 pairs 55.3 -> 48.5, 406k of 3.4 81 -> 76, 298k of 9.3
+    // 94 -> 92, 2.7M of 1.15 229 -> 186.
+    const uint32_t res_ring = smem_u32(idx_ring + kIdxSlots * kSub * kBM) + (uint32_t)((warp - kEpiWarp) * 2 * kResSlot);
+    uint32_t res_turn = 0;                                    // the slot that is read next
+    // copies the residual's pieces q and q + 1 of the quarter's rows (`row`: this lane's, -1: none)
+    auto stage_residual = [&](uint32_t turn, int32_t row, int q) {
+      const int k = lane & 3, c = q * 16 + k * 8;
+      const bool inside = c < min(n, last_piece * 16);
+      const uint32_t slot = res_ring + turn * kResSlot + (uint32_t)(lane >> 2) * 64u;
+#pragma unroll
+      for (int i = 0; i < 4; i++) {                           // rows 8 i + lane / 4
+        const int32_t from = __shfl_sync(0xffffffffu, row, (lane >> 2) + 8 * i);
+        if (from >= 0 && inside)
+          cp_async_16(slot + (uint32_t)(i * 512) + ((uint32_t)(k ^ ((lane >> 3) & 3)) << 4),
+                      args.residual + ((int64_t)from * n + c) * 2, 16u);
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    if (kStaged && first_piece < last_piece) stage_residual(0u, take_row((int)blockIdx.x, 0, rows_1[0]), first_piece);
     for (int tile = blockIdx.x; tile < args.num_tiles; tile += gridDim.x) {
       uint32_t hb[kSub];
       take_bits<kSub>(args, tile, raw, hb);
       request_bits<kSub, kMode>(args, tile + (int)gridDim.x, raw);
 #pragma unroll
-      for (int h = 0; h < kSub; h++) { grow[h] = take_row(tile, h, rows_1[h]); rows_1[h] = rows_2[h]; }
-      request_rows(tile + 2 * (int)gridDim.x, rows_2);
-      if (!kPairs && args.residual != nullptr) {
+      for (int h = 0; h < kSub; h++) grow[h] = take_row(tile, h, rows_1[h]);
+      if (kStaged) {
+        request_rows(tile + (int)gridDim.x, rows_1);
+      } else {
+#pragma unroll
+        for (int h = 0; h < kSub; h++) rows_1[h] = rows_2[h];
+        request_rows(tile + 2 * (int)gridDim.x, rows_2);
+      }
+      if (!kPairs && args.residual != nullptr && !kStaged) {
 #pragma unroll
         for (int h = 0; h < kSub; h++) {
           const int32_t next = take_row(tile + (int)gridDim.x, h, rows_1[h]);
@@ -540,18 +577,27 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
           load_narrow(src, c);
         }
       };
-      if (!kPairs) load_residual(0, first_piece * 16);
+      if (!kPairs && !kStaged) load_residual(0, first_piece * 16);
       if (!mbar_wait_warp(false, &bar_acc_full[acc], acc_phase, abort_flag, args.status)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll
+#pragma unroll (kStaged ? 1 : kSub)
       for (int h = 0; h < kSub; h++) {
+        // (kStaged: one body for both sub-tiles, two of them spill; no index into registers then)
+        auto row_now = [&]() {
+          if constexpr (kStaged) return h == 0 ? grow[0] : grow[kSub - 1];
+          else return grow[h];
+        };
+        auto bits_now = [&]() {
+          if constexpr (kStaged) return h == 0 ? hb[0] : hb[kSub - 1];
+          else return hb[h];
+        };
         const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) +
                                (uint32_t)((acc * kSub + h) * args.n_pad);
         auto piece = [&](int q) {
           uint32_t cur[16];
           __syncwarp();
           tmem_ld_32x16(taddr + (uint32_t)q * 16, cur);
-          const bool more = q + kEpiCols < pieces;
+          const bool more = q + kStep < last_piece;
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
           if (!more && h + 1 == kSub) {
             // the last read of this accumulator set: the next tile's MMAs may have it
@@ -560,9 +606,9 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
           }
           const int c = q * 16;
           if (kPairs) {
-            if (grow[h] < 0) return;
+            if (row_now() < 0) return;
             // pair mode: the fp32 accumulators of this row go out as they are
-            float *dst = args.out_f32 + (int64_t)grow[h] * n + c;
+            float *dst = args.out_f32 + (int64_t)row_now() * n + c;
 #pragma unroll
             for (int i = 0; i < 4; i++)
               if (c + 4 * i < n)
@@ -575,7 +621,7 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
           // the branches inside the loop over the values a piece took 1300 cycles of latencies
           float f[16];
 #pragma unroll
-          for (int i = 0; i < 16; i++) f[i] = hb[h] == 0u ? 0.f : __uint_as_float(cur[i]);
+          for (int i = 0; i < 16; i++) f[i] = bits_now() == 0u ? 0.f : __uint_as_float(cur[i]);
           if (affine) {
 #pragma unroll
             for (int i = 0; i < 4; i++) {
@@ -587,7 +633,13 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
               f[4 * i + 3] = f[4 * i + 3] * sc.w + sh.w;
             }
           }
-          if (args.residual != nullptr) {
+          if (kStaged || args.residual != nullptr) {
+            if (kStaged) {
+              const uint32_t row = res_ring + res_turn * kResSlot + (uint32_t)lane * 64u;
+              const uint32_t k = (uint32_t)((q - first_piece) & 1) * 2u ^ ((uint32_t)lane >> 1 & 3u);
+              ld_shared_16(row + (k << 4), res);
+              ld_shared_16(row + ((k ^ 1u) << 4), res + 4);
+            }
             if (args.elem_is_bf16) {
 #pragma unroll
               for (int i = 0; i < 8; i++) {
@@ -602,13 +654,14 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
               }
             }
           }
-          if (more) load_residual(h, (q + kEpiCols) * 16);
+          if (kStaged) {
+          } else if (more) load_residual(h, (q + kStep) * 16);
           else if (h + 1 < kSub) load_residual(h + 1, first_piece * 16);
           if (args.relu) {
 #pragma unroll
             for (int i = 0; i < 16; i++) f[i] = fmaxf(f[i], 0.f);
           }
-          if (grow[h] < 0) return;
+          if (row_now() < 0) return;
           uint32_t out[8];
           if (args.elem_is_bf16) {
 #pragma unroll
@@ -623,7 +676,7 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
               out[i] = *reinterpret_cast<uint32_t *>(&pk);
             }
           }
-          uint8_t *dst = args.out16 + ((int64_t)grow[h] * n + c) * 2;
+          uint8_t *dst = args.out16 + ((int64_t)row_now() * n + c) * 2;
           if (args.wide && c + 16 <= n) {
             st_global_32(dst, out);
           } else if (kMode == kDense && (n & 7) != 0) {
@@ -635,15 +688,28 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
             if (c + 8 < n) *reinterpret_cast<uint4 *>(dst + 16) = make_uint4(out[4], out[5], out[6], out[7]);
           }
         };
-        int q = first_piece;
-        if (kEpiCols > 1 && q >= pieces && h + 1 == kSub) {   // no columns for this warp
+        if (kEpiCols > 1 && first_piece >= last_piece && h + 1 == kSub) {   // no columns for this warp
           asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
           if (lane == 0) mbar_arrive(&bar_acc_empty[acc]);
         }
-        for (; q < pieces; q += kEpiCols) piece(q);
+        if constexpr (kStaged) {
+          for (int q0 = first_piece; q0 < last_piece; q0 += 2) {
+            __syncwarp();                                     // every lane has read the slot that is filled now
+            const bool same = q0 + 2 < last_piece;
+            const int32_t row = same ? row_now() : h + 1 < kSub ? grow[kSub - 1] : take_row(tile + (int)gridDim.x, 0, rows_1[0]);
+            stage_residual(res_turn ^ 1u, row, same ? q0 + 2 : first_piece);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+            __syncwarp();
+            for (int q = q0; q < min(q0 + 2, last_piece); q++) piece(q);
+            res_turn ^= 1u;
+          }
+        } else {
+          for (int q = first_piece; q < last_piece; q += kStep) piece(q);
+        }
       }
       if (++acc == args.acc_bufs) { acc = 0; acc_phase ^= 1u; }
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");   // nothing of this lane is in flight at exit
   }
 
   // ------------------------------ teardown ------------------------------------
@@ -801,16 +867,25 @@ inline int row_chunk_shift(int64_t T, int64_t pairs, int64_t O) {
 
 namespace {
 
-template <int kSub, int kLpr, int kProdWarps, int kMode>
+template <int kSub, int kLpr, int kProdWarps, int kMode, bool kStaged = false>
 mn_status launch_implicit(const ImArgs &a, const TcSizing &sizing, const CUtensorMap &map_a,
                           const CUtensorMap &map_b, cudaStream_t st) {
-  auto kernel = conv_implicit_kernel<kSub, kLpr, kProdWarps, kMode>;
+  auto kernel = conv_implicit_kernel<kSub, kLpr, kProdWarps, kMode, kStaged>;
   MN_RETURN_IF(allow_max_shared_memory(reinterpret_cast<const void *>(kernel)));
   const int grid = std::min(a.num_tiles, kNumSMs * sizing.ctas_per_sm);
   MN_LAUNCH(kMode == kPairRows ? "conv_implicit_kernel<pairs>" : kMode == kDense ? "conv_implicit_kernel<dense>"
                                                                                  : "conv_implicit_kernel", st,
             launch_early(kernel, grid, kImThreads, sizing.smem_bytes, st, a, map_a, map_b));
   return MN_OK;
+}
+
+template <int kMode, bool kStaged>
+mn_status launch_map(const ImArgs &a, int sub, const TcSizing &sizing, const CUtensorMap &map_b, cudaStream_t st) {
+  if (sub == 1)
+    return a.K <= 32 ? launch_implicit<1, 4, 4, kMode, kStaged>(a, sizing, map_b, map_b, st)
+                     : launch_implicit<1, 8, 4, kMode, kStaged>(a, sizing, map_b, map_b, st);
+  return a.K <= 32 ? launch_implicit<2, 4, 8, kMode, kStaged>(a, sizing, map_b, map_b, st)
+                   : launch_implicit<2, 8, 8, kMode, kStaged>(a, sizing, map_b, map_b, st);
 }
 
 }  // namespace
@@ -1041,7 +1116,10 @@ extern "C" mn_status mn_sparse_convolution_forward_implicit(
   // row 145 / 110, 3.5k of 1.6 39 / 38, 0.9k 19 / 23.  64->64: 13.9k tiles of 9.3 pairs 570 / 541, 2.6k of 7
   // 78 / 74, 3.2k of 3.4 70 / 72, 21.4k of 1.15 152 / 161.  More channels: 128->64 821 / 834, 64->128 472 /
   // 512 (18.8k tiles), 128->128 1059 / 1100, 136 / 147 (3.2k), 57 / 62 (0.8k), 176 / 171 (2.3k of 9.3 pairs),
-  // 256->256 336 / 404.  Callers that have timed the layer pass their own choice.
+  // 256->256 336 / 404.  All that is one layer at a time on a GPU that keeps its clocks.  A network on a large
+  // batch runs at the power limit, and weights read and written once for both sub-tiles are energy saved:
+  // with two at 128 columns a forward pass of 64 clouds takes 76.4 instead of 78.5 ms.  Callers that have timed
+  // the layer pass their own choice.
   int sub = sub_hint;
   if (sub <= 0) {
     const double tiles = a.n_tiles128;
@@ -1050,6 +1128,8 @@ extern "C" mn_status mn_sparse_convolution_forward_implicit(
       if (tiles >= 32 * kNumSMs) sub = 2;
     } else if (c_in <= 64 && a.n_pad <= 64) {
       if (pairs_per_row >= 3.0 && tiles >= 16 * kNumSMs && tiles * pairs_per_row >= 16384) sub = 2;
+    } else if (a.n_pad > 64 && a.n_pad <= 128) {
+      if (pairs_per_row >= 2.0 && tiles >= 32 * kNumSMs) sub = 2;
     }
   }
   MN_CHECK_ARG(sub_hint <= 4 && (sub_hint <= 0 || sub_hint * a.n_pad <= 512),
@@ -1059,7 +1139,12 @@ extern "C" mn_status mn_sparse_convolution_forward_implicit(
   a.acc_bufs = 2 * sub * a.n_pad <= 512 ? 2 : 1;
   a.a_bytes = sub * kBM * kBK * 2;
   a.stage_bytes = a.a_bytes + (n_major ? (int)div_up(a.n_pad, 64) * kNBlock : a.n_pad * kBK * 2);
-  const TcSizing sizing = size_tc_kernel(a.stage_bytes, a.acc_bufs * sub * a.n_pad, kMaxStages, kImCtas, kIdxSlots * kMaxSub * kBM * 4, kMaxStages);
+  // The residual's ring: two slots of 32 rows per epilogue warp.  At 32 columns rows of 64 bytes are two sectors for
+  // two lanes either way (464k rows, 1.15 pairs: 37.9 / 39.8 us, 336k, 7 pairs 61.4 / 63.5), and beyond 64 the
+  // 32 KB are a stage or two of the ring.
+  const bool staged = residual != nullptr && a.n_pad > 32 && a.n_pad <= 64;
+  const int rings = kIdxSlots * sub * kBM * 4 + (staged ? (sub == 1 ? 8 : 4) * 2 * kResSlot : 0);
+  const TcSizing sizing = size_tc_kernel(a.stage_bytes, a.acc_bufs * sub * a.n_pad, kMaxStages, kImCtas, rings, kMaxStages);
   a.stages = sizing.stages;
   a.tmem_cols = sizing.tmem_cols;
   a.num_offsets = (int)O;
@@ -1072,16 +1157,8 @@ extern "C" mn_status mn_sparse_convolution_forward_implicit(
   CUtensorMap map_b;
   MN_RETURN_IF(n_major ? make_kmajor_map(&map_b, weights_t, bf16, c_out, c_in, O, kBK)
                        : make_kmajor_map(&map_b, weights_t, bf16, c_in, c_out, O, a.n_pad));
-  if (n_major) {
-    if (sub == 1)
-      return c_in <= 32 ? launch_implicit<1, 4, 4, kMapNMajor>(a, sizing, map_b, map_b, st)
-                        : launch_implicit<1, 8, 4, kMapNMajor>(a, sizing, map_b, map_b, st);
-    return c_in <= 32 ? launch_implicit<2, 4, 8, kMapNMajor>(a, sizing, map_b, map_b, st)
-                      : launch_implicit<2, 8, 8, kMapNMajor>(a, sizing, map_b, map_b, st);
-  }
-  if (sub == 1)
-    return c_in <= 32 ? launch_implicit<1, 4, 4, kMap>(a, sizing, map_b, map_b, st)
-                      : launch_implicit<1, 8, 4, kMap>(a, sizing, map_b, map_b, st);
-  return c_in <= 32 ? launch_implicit<2, 4, 8, kMap>(a, sizing, map_b, map_b, st)
-                    : launch_implicit<2, 8, 8, kMap>(a, sizing, map_b, map_b, st);
+  if (n_major)
+    return staged ? launch_map<kMapNMajor, true>(a, sub, sizing, map_b, st)
+                           : launch_map<kMapNMajor, false>(a, sub, sizing, map_b, st);
+  return staged ? launch_map<kMap, true>(a, sub, sizing, map_b, st) : launch_map<kMap, false>(a, sub, sizing, map_b, st);
 }

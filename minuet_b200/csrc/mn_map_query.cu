@@ -352,9 +352,10 @@ search_kernel(const __grid_constant__ SearchPair sp) {
       for (int j = 0; j < kQRows; j++)   // a dead row gets a value that no window can reach
         rel[j] = live[j] ? (int64_t)(key[j] - base) + kQPad : (int64_t)1 << 62;
       // Where window, rows and offsets span less than 2^29 the relative keys are sums of 32 bits: what
-      // falls outside the window is in no cell of it (a dead row's sums are off by 2^31).
+      // falls outside the window is in no cell of it (a dead row's sums are off by 2^31).  A window without
+      // keys has no last one.
       const int64_t first_delta = s_delta[tab.member[0]], last_delta = s_delta[tab.member[O - 1]];
-      const bool narrow = __ldg(a.table + hi - 1) - base < kNarrow && (int64_t)(kfirst - base) > -(int64_t)kNarrow &&
+      const bool narrow = wn > 0 && __ldg(a.table + hi - 1) - base < kNarrow && (int64_t)(kfirst - base) > -(int64_t)kNarrow &&
                           (int64_t)(klast - base) < (int64_t)kNarrow && first_delta > -(int64_t)kNarrow &&
                           last_delta < (int64_t)kNarrow;
       auto relative = [&](int j, int g) {

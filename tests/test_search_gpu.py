@@ -47,3 +47,16 @@ def test_offsets_on_one_side_of_the_rows_own_place(oracle_lib, sign):
     d = torch.as_tensor(src, device=DEV)
     got = F.query_sorted_index_with_offsets(d, d, torch.as_tensor(off, device=DEV))
     assert np.array_equal(got.cpu().numpy(), oracle_lib.query(src, src, off))
+
+
+@pytest.mark.parametrize("shift", [-1000, 1000])
+@pytest.mark.parametrize("n", [1, 700])
+def test_windows_without_a_key(oracle_lib, shift, n):
+    """Targets that all lie before, or behind, every source: no tile has anything to look through."""
+    rng = np.random.default_rng(n)
+    src = _cloud(rng, (40, 40, 70), 2000)
+    tgt = (src[:n] + np.array([shift, 0, 0])).astype(np.int32)
+    off = generate_kernel_offsets(3, 3, 1, 1).astype(np.int32)
+    d_src, d_tgt = (torch.as_tensor(c, device=DEV) for c in (src, tgt))
+    got = F.query_sorted_index_with_offsets(d_src, d_tgt, torch.as_tensor(off, device=DEV))
+    assert (got == -1).all()

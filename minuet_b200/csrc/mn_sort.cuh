@@ -145,8 +145,8 @@ __device__ __forceinline__ uint32_t block_exclusive(uint32_t v, uint32_t *s_part
 }
 
 // A thread looks after kPer consecutive digits: two of them with 256 threads, one with 512.
-template <int kThr, int kItems, bool kVals>
-__global__ void __launch_bounds__(kThr, kItems == 16 ? 3 : kThr == 512 ? 2 : 4)
+template <int kThr, int kItems, int kBlocks, bool kVals>
+__global__ void __launch_bounds__(kThr, kBlocks)
 sort_pass_kernel(const __grid_constant__ Args a, int pass) {
   begin_early();
   constexpr int kTile = kThr * kItems, kWarps = kThr / 32, kPer = kDigits / kThr;
@@ -331,18 +331,24 @@ sort_pass_kernel(const __grid_constant__ Args a, int pass) {
   }
 }
 
-// Threads and keys per thread of a tile.  Every tile that runs at the same time lengthens the look-back, so
-// tiles are large: 4096 keys, with 512 threads up to two tiles per SM and with 256 beyond (three
-// blocks of 80 registers share an SM: at 128 registers and two, 7.3 M keys took 7 % longer).  Up to one
-// tile of 1024 keys per SM a pass is shorter with those; beyond, up to 606k keys, the large ones
-// leave SMs without a tile and are faster all the same.  Measured, all passes, us for 256 x 4 / 512 x 8 /
-// 256 x 16: 30k keys 29 / 37 / 39; 120k 45 / 51 / 53; 250k 64 / 59 / 62; 464k 80 / 74 / 78; 900k 115 / 94 /
-// 100; 1.9 M 184 / 141 / 127; 7.3 M 755 / 491 / 445.
-struct TileShape { int threads, items; };
+// Threads and keys per thread of a tile, and its blocks per SM.  Every tile that runs at the same time lengthens
+// the look-back, so tiles are large: 4096 keys, with 512 threads up to two tiles per SM and with 256 beyond,
+// three to an SM (80 registers; at 128 registers and two, 7.3 M keys took 7 % longer) while that is one wave.  Four
+// to an SM (64 registers, 8 bytes spilled) pay once there are more tiles than one wave, and tiles of 3072
+// keys where the second wave would be small.  Up to one tile of 1024 keys per SM a pass is shorter with
+// those; beyond, up to 606k keys, the large ones leave SMs without a tile and are faster all the same.  Measured,
+// all passes, us for 256 x 4 / 512 x 8 / 256 x 16: 30k keys 29 / 37 / 39; 120k 45 / 51 / 53; 250k 64 / 59 / 62;
+// 464k 80 / 74 / 78; 900k 115 / 94 / 100; 1.9 M 184 / 141 / 127; 7.3 M 755 / 491 / 445.  36 bits, 256 x 16 with three
+// / with four blocks / 256 x 12 with four: 1.5 M 129 / 150 / 132; 1.9 M 147 / 157 / 140; 2.1 M 165 / 159 / 156;
+// 2.4 M 188 / 164 / 182; 7.3 M 417 / 390 / 406.
+struct TileShape { int threads, items, blocks; };
 constexpr int64_t kFewKeys = 1024ll * kNumSMs;
+constexpr int64_t kOneWave = 3 * 4096ll * kNumSMs, kSmallSecondWave = kOneWave + kOneWave / 5;
 inline TileShape tile_shape(int64_t n) {
-  if (n < kFewKeys) return TileShape{256, 4};
-  return n < 2 * 4096ll * kNumSMs ? TileShape{512, 8} : TileShape{256, 16};
+  if (n < kFewKeys) return TileShape{256, 4, 4};
+  if (n < 2 * 4096ll * kNumSMs) return TileShape{512, 8, 2};
+  if (n <= kOneWave) return TileShape{256, 16, 3};
+  return n <= kSmallSecondWave ? TileShape{256, 12, 4} : TileShape{256, 16, 4};
 }
 inline int64_t tiles_of(int64_t n) {
   const TileShape s = tile_shape(n);
@@ -351,10 +357,11 @@ inline int64_t tiles_of(int64_t n) {
 inline size_t control_words(int64_t n, int passes) {
   return (size_t)kMaxPasses * kDigits + 64 + (size_t)passes * tiles_of(n) * kDigits;
 }
-// Enough for any number of keys up to n: the most of the small tiles are more than the large ones of up to
-// four times as many keys.
+// Enough for any number of keys up to n: small tiles are more than the large ones of a larger number of keys.
 inline size_t workspace_bytes(int64_t n) {
-  const size_t words = std::max(control_words(n, kMaxPasses), control_words(std::min(n, kFewKeys - 1), kMaxPasses));
+  size_t words = 0;
+  for (int64_t keys : {n, kFewKeys - 1, kSmallSecondWave})
+    words = std::max(words, control_words(std::min(n, keys), kMaxPasses));
   return align_up(words * sizeof(uint32_t), 256) + 256;
 }
 
@@ -364,13 +371,13 @@ inline int bits_for(int64_t values) {    // bits that tell `values` different va
   return b;
 }
 
-template <int kThr, int kItems>
+template <int kThr, int kItems, int kBlocks>
 mn_status launch_passes(const Args &a, int launches, cudaStream_t st) {
   for (int p = 0; p < launches; p++) {
     if (a.vals[0] != nullptr) {
-      MN_LAUNCH("sort_pass_kernel", st, launch_early(sort_pass_kernel<kThr, kItems, true>, a.tiles, kThr, 0, st, a, p));
+      MN_LAUNCH("sort_pass_kernel", st, launch_early(sort_pass_kernel<kThr, kItems, kBlocks, true>, a.tiles, kThr, 0, st, a, p));
     } else {
-      MN_LAUNCH("sort_pass_kernel", st, launch_early(sort_pass_kernel<kThr, kItems, false>, a.tiles, kThr, 0, st, a, p));
+      MN_LAUNCH("sort_pass_kernel", st, launch_early(sort_pass_kernel<kThr, kItems, kBlocks, false>, a.tiles, kThr, 0, st, a, p));
     }
   }
   return MN_OK;
@@ -392,11 +399,15 @@ mn_status run(Args a, const Source &source, Workspace &ws, cudaStream_t st) {
   a.next_tile = control + kMaxPasses * kDigits;
   a.state = a.next_tile + 64;
   MN_CHECK_CUDA(cudaMemsetAsync(control, 0, control_words(a.n, launches) * sizeof(uint32_t), st));
-  const int blocks = (int)std::min<int64_t>(kNumSMs * 8, div_up(a.n, kThreads));
+  // Every block adds its counts to the digits' totals: no more blocks than run at once, two keys a thread at least
+  // (1184 blocks of one key a thread: 120k points 12.5 -> 10.9 us, 464k rows 20.5 -> 16.9, 1.9 M points 32.8 -> 29)
+  const int blocks = (int)std::min<int64_t>(kNumSMs * 4, div_up(a.n, 2 * kThreads));
   MN_LAUNCH("sort_keys_kernel", st, launch_early(sort_keys_kernel<Source>, blocks, kThreads, 0, st, a, source));
   const TileShape shape = tile_shape(a.n);
-  if (shape.threads == 512) return launch_passes<512, 8>(a, launches, st);
-  return shape.items == 4 ? launch_passes<256, 4>(a, launches, st) : launch_passes<256, 16>(a, launches, st);
+  if (shape.threads == 512) return launch_passes<512, 8, 2>(a, launches, st);
+  if (shape.items == 4) return launch_passes<256, 4, 4>(a, launches, st);
+  if (shape.items == 12) return launch_passes<256, 12, 4>(a, launches, st);
+  return shape.blocks == 3 ? launch_passes<256, 16, 3>(a, launches, st) : launch_passes<256, 16, 4>(a, launches, st);
 }
 
 }  // namespace rsort

@@ -31,3 +31,9 @@ def test_index_beside_a_full_key(n):
     for d in (2, 1, 0):                                    # least significant first, each stable
         want = want[torch.sort(c[want, d], stable=True).indices]
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("n", [1_818_623, 1_818_624, 1_818_625, 2_182_348, 2_182_349])
+@pytest.mark.parametrize("extent", [2, 700])
+def test_permutation_is_stable_where_one_wave_ends(n, extent):
+    test_permutation_is_stable(n, extent)

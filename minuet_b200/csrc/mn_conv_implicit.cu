@@ -53,6 +53,7 @@ constexpr int kUmmaK = 16;
 constexpr int kMaxStages = 8;
 constexpr int kMaxN = 256;
 constexpr int kIdxSlots = 8;           // steps the index blocks run ahead
+constexpr int kTileSlots = 4;          // tiles that a CTA holds at most
 constexpr int kMaxSub = 2;             // 128-row sub-tiles per CTA tile
 constexpr int kResSlot = 32 * 64;      // bytes of 32 columns of 32 rows of the residual
 constexpr int kNBlock = kBK * 128;     // kMapNMajor: bytes of one block of 64 columns of a weight tile
@@ -145,14 +146,34 @@ __device__ __forceinline__ int32_t load_ahead_1(const void *src) {
   return v;
 }
 
-// Offset bits of the sub-tiles of a CTA tile, in two steps: the request (unconditional, from a
-// clamped index: a load under a condition is waited for where the branch joins, a thousand cycles
-// per tile) and, a tile later, the value (pair mode: one offset each).
+// Asks for the next block of this grid that has not started, which will then not start: its number comes to
+// `answer` (16 bytes) and completes `bar`.  Not to be called again once the answer was "none".
+__device__ __forceinline__ void claim_block(void *answer, uint64_t *bar) {
+  mbar_expect_tx(bar, 16u);
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(
+                   smem_u32(answer)), "r"(smem_u32(bar))
+               : "memory");
+}
+__device__ __forceinline__ int claimed_block(const void *answer) {      // -1: none
+  uint32_t got, x = 0u;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b128 v;\n\t"
+      "ld.shared.b128 v, [%2];\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, v;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t"
+      "mov.u32 %1, 0;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid.v4.b32.b128 {%1, _, _, _}, v;\n\t}"
+      : "=r"(got), "=r"(x) : "r"(smem_u32(answer)) : "memory");
+  return got != 0u ? (int)x : -1;
+}
+
+// Offset bits of the sub-tiles of a CTA tile (pair and dense mode: one offset each): the request and, later, the
+// value.  A request under a condition would be waited for where the branch joins.
 template <int kSub, int kMode>
 __device__ __forceinline__ void request_bits(const ImArgs &args, int tile, uint32_t (&raw)[kSub]) {
 #pragma unroll
   for (int h = 0; h < kSub; h++)
-    raw[h] = kMode > kMapNMajor ? 1u : (uint32_t)load_ahead_1(args.tile_bits + min(tile * kSub + h, args.n_tiles128 - 1));
+    raw[h] = kMode > kMapNMajor ? 1u : (uint32_t)load_ahead_1(args.tile_bits + min(max(tile, 0) * kSub + h, args.n_tiles128 - 1));
 }
 
 template <int kSub>
@@ -160,7 +181,7 @@ __device__ __forceinline__ void take_bits(const ImArgs &args, int tile, const ui
                                           uint32_t (&hb)[kSub]) {
 #pragma unroll
   for (int h = 0; h < kSub; h++)
-    hb[h] = tile < args.num_tiles && tile * kSub + h < args.n_tiles128 ? raw[h] : 0u;
+    hb[h] = tile >= 0 && tile * kSub + h < args.n_tiles128 ? raw[h] : 0u;
 }
 
 template <int kSub>
@@ -188,6 +209,10 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
   __shared__ uint64_t bar_full[kMaxStages], bar_empty[kMaxStages];
   __shared__ uint64_t bar_acc_full[2], bar_acc_empty[2];
   __shared__ uint64_t bar_idx_full[kIdxSlots], bar_idx_empty[kIdxSlots];
+  __shared__ uint64_t bar_tile_full[kTileSlots], bar_tile_empty[kTileSlots], bar_claim;
+  __shared__ __align__(16) uint4 s_claim;
+  __shared__ int32_t s_tile[kTileSlots];
+  __shared__ uint32_t s_tile_bits[kTileSlots][kSub];
   __shared__ uint32_t s_idx_has[kIdxSlots];
   __shared__ uint32_t s_tmem_base;
   __shared__ int s_abort;
@@ -208,6 +233,9 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
     }
     for (int a = 0; a < 2; a++) { mbar_init(&bar_acc_full[a], 1); mbar_init(&bar_acc_empty[a], 4 * kEpiCols); }
     for (int i = 0; i < kIdxSlots; i++) { mbar_init(&bar_idx_full[i], 33); mbar_init(&bar_idx_empty[i], kProdWarps * 32); }
+    // read by the weight warp, the MMA warp and the epilogue warps
+    for (int i = 0; i < kTileSlots; i++) { mbar_init(&bar_tile_full[i], 1); mbar_init(&bar_tile_empty[i], 2 + 4 * kEpiCols); }
+    mbar_init(&bar_claim, 1);
     s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -230,6 +258,21 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
   release_successor();   // every block has its tensor memory before another kernel's block can ask for some
   const uint32_t tmem_base = s_tmem_base;
   volatile int *abort_flag = &s_abort;
+  // The next of this CTA's tiles and its offset bits, for the warps of the roles that follow them (-1: no more).
+  int tile_slot = 0;
+  uint32_t tile_phase = 0;
+  auto next_tile = [&](int &tile, uint32_t (&hb)[kSub]) {
+    if (!mbar_wait_warp(false, &bar_tile_full[tile_slot], tile_phase, abort_flag, args.status)) return false;
+    tile = s_tile[tile_slot];
+    uint32_t seen = (uint32_t)tile;
+#pragma unroll
+    for (int h = 0; h < kSub; h++) { hb[h] = s_tile_bits[tile_slot][h]; seen |= hb[h]; }
+    __syncwarp();
+    // (the loads have returned: the arrival's address depends on them, see the producers)
+    if (lane == 0) mbar_arrive(&bar_tile_empty[tile_slot] + (seen & (uint32_t)args.zero));
+    if (++tile_slot == kTileSlots) { tile_slot = 0; tile_phase ^= 1u; }
+    return true;
+  };
 
   if (warp < kProdWarps) {
     // ------------------------------ producers ---------------------------------
@@ -331,14 +374,11 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
     int stage = 0, acc = 0;
     uint32_t phase = 0, acc_phase = 0;
     bool alive = true;
-    uint32_t raw[kSub];
-    request_bits<kSub, kMode>(args, (int)blockIdx.x, raw);
     bool ready = mbar_test(&bar_full[0], 0u);
-    for (int tile = blockIdx.x; alive && tile < args.num_tiles; tile += gridDim.x) {
-      uint32_t hb[kSub];
-      take_bits<kSub>(args, tile, raw, hb);
+    int tile;
+    uint32_t hb[kSub];
+    while (alive && next_tile(tile, hb) && tile >= 0) {
       uint32_t rest = union_of<kSub>(hb);
-      request_bits<kSub, kMode>(args, tile + (int)gridDim.x, raw);
       if (!mbar_wait_warp(false, &bar_acc_empty[acc], acc_phase ^ 1u, abort_flag, args.status)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t tmem_d = tmem_base + (uint32_t)(acc * kSub * args.n_pad);
@@ -384,14 +424,11 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
     bool alive = true;
     int stage = 0;
     uint32_t phase = 0;
-    uint32_t raw[kSub];
-    request_bits<kSub, kMode>(args, (int)blockIdx.x, raw);
     bool ready = mbar_test(&bar_empty[0], 1u);
-    for (int tile = blockIdx.x; alive && tile < args.num_tiles; tile += gridDim.x) {
-      uint32_t hb[kSub];
-      take_bits<kSub>(args, tile, raw, hb);
+    int tile;
+    uint32_t hb[kSub];
+    while (alive && next_tile(tile, hb) && tile >= 0) {
       uint32_t rest = union_of<kSub>(hb);
-      request_bits<kSub, kMode>(args, tile + (int)gridDim.x, raw);
       const int pair_row = kPairs ? pair_row_of_tile(args, tile) : 0;
       while (alive && rest != 0u) {
         const int p = kPairs ? pair_row : __ffs(rest) - 1;
@@ -418,7 +455,13 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
       }
     }
   } else if (warp == kIdxWarp) {
-    // ------------------------------ index blocks -------------------------------
+    // ------------------------------ tiles and index blocks ---------------------
+    // Tiles are handed out while the kernel runs: a CTA starts with the tile of its own number, counted from the last,
+    // and takes over the tiles of blocks that have not started (cluster launch control) as it needs them, at most
+    // kTileSlots before its epilogue.  Rows with many and rare offsets sort to the end, so the dear tiles go first.
+    // With every gridDim-th tile for a CTA the busiest had 1.2 to 1.7 times the average of steps (one to
+    // four clouds; FIGURES).
+    //
     // 128 entries of the neighbour table per step and sub-tile, up to kIdxSlots steps ahead of the
     // producers, so that they never wait for an index from memory (loaded by the producers
     // themselves, even two steps ahead, they cost a quarter of the time).  A lane copies 16 bytes of
@@ -428,7 +471,23 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
     // 16.7 pairs, 70 / 62; 406k 64->128 90 / 86).
     const uint32_t ring = smem_u32(idx_ring) + (uint32_t)lane * 16u;
     uint32_t raw[kSub], phase = 0;
-    request_bits<kSub, kMode>(args, (int)blockIdx.x, raw);
+    int tile = args.num_tiles - 1 - (int)blockIdx.x;
+    request_bits<kSub, kMode>(args, tile, raw);
+    uint32_t claim_phase = 0, publish_phase = 0;
+    int publish_slot = 0;
+    bool claim_open = false;                       // an answer is on its way
+    auto publish = [&](const uint32_t (&hb)[kSub]) {
+      if (!mbar_wait_warp(false, &bar_tile_empty[publish_slot], publish_phase ^ 1u, abort_flag, args.status)) return false;
+      if (lane == 0) {
+        s_tile[publish_slot] = tile;
+#pragma unroll
+        for (int h = 0; h < kSub; h++) s_tile_bits[publish_slot][h] = hb[h];
+        mbar_arrive(&bar_tile_full[publish_slot]);
+      }
+      __syncwarp();
+      if (++publish_slot == kTileSlots) { publish_slot = 0; publish_phase ^= 1u; }
+      return true;
+    };
     int slot = 0;
     bool ready = true;
     // one step of the tile at `src`: offsets p of the sub-tiles in `has`; 0 marks the end
@@ -448,21 +507,41 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
       ready = mbar_test(&bar_idx_empty[slot], phase ^ 1u);
       return true;
     };
-    bool alive = kMode != kDense;
-    for (int tile = blockIdx.x; alive && tile < args.num_tiles; tile += gridDim.x) {
+    bool alive = true;
+    while (alive) {
       uint32_t hb[kSub];
       take_bits<kSub>(args, tile, raw, hb);
-      request_bits<kSub, kMode>(args, tile + (int)gridDim.x, raw);
+      alive = publish(hb);
+      if (!alive || tile < 0) break;
       const int32_t *blocks = args.nbr + (int64_t)tile * (kSub * kBM) + lane * 4;
-      for (uint32_t rest = union_of<kSub>(hb); alive && rest != 0u; rest &= rest - 1u) {
+      for (uint32_t rest = kMode == kDense ? 0u : union_of<kSub>(hb); alive && rest != 0u; rest &= rest - 1u) {
         const int p = __ffs(rest) - 1;
         uint32_t has = 0u;
 #pragma unroll
         for (int h = 0; h < kSub; h++) has |= ((hb[h] >> p) & 1u) << h;
         alive = send(blocks + (int64_t)p * args.pitch, has);
       }
+      if (!alive) break;
+      // the next tile, no earlier: a CTA that holds tiles it has not begun keeps them from one that is done
+      if (lane == 0) {
+        fence_generic_to_async();                  // the answer before has been read
+        claim_block(&s_claim, &bar_claim);
+      }
+      claim_open = true;
+      __syncwarp();
+      if (!mbar_wait_warp(false, &bar_claim, claim_phase, abort_flag, args.status)) break;
+      claim_open = false;
+      claim_phase ^= 1u;
+      const int block = claimed_block(&s_claim);
+      __syncwarp();
+      tile = block >= 0 ? args.num_tiles - 1 - block : -1;
+      request_bits<kSub, kMode>(args, tile, raw);
     }
-    if (alive) send(args.nbr, 0u);
+    if (alive && tile < 0 && kMode != kDense) send(args.nbr, 0u);
+    // an answer that is still on its way lands before this block's shared memory goes
+    if (claim_open) {
+      for (uint32_t spin = 0; spin < 4096u && !mbar_try_wait(&bar_claim, claim_phase); spin++) {}
+    }
     asm volatile("cp.async.wait_all;" ::: "memory");   // nothing of this lane is in flight at exit
   } else {
     // ------------------------------ epilogue ----------------------------------
@@ -489,25 +568,25 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
     const bool affine = args.scale != nullptr || args.shift != nullptr;
     int acc = 0;
     uint32_t acc_phase = 0;
-    uint32_t raw[kSub];
-    request_bits<kSub, kMode>(args, (int)blockIdx.x, raw);
-    // Row of the output (and of the residual) that this lane's accumulator row belongs to, per
-    // sub-tile (-1: none): requested two tiles ahead (one where residuals are copied ahead), so that the residual
-    // rows of the next tile can be on their way to L2 while this one is worked on.
+    // Row of the output (and of the residual) that this lane's accumulator row belongs to, per sub-tile (-1: none):
+    // requested a tile ahead, so that the residual rows of the next tile can be on their way while this one is
+    // worked on.
     const bool permuted = kMode <= kMapNMajor && args.perm != nullptr;
     auto table_row = [&](int tile, int h) { return ((int64_t)tile * kSub + h) * kBM + quarter * 32 + lane; };
     auto request_rows = [&](int tile, int32_t (&rows)[kSub]) {
 #pragma unroll
       for (int h = 0; h < kSub; h++)
-        if (permuted) rows[h] = load_ahead_1(args.perm + min(table_row(tile, h), args.T - 1));
+        if (permuted) rows[h] = load_ahead_1(args.perm + min(table_row(max(tile, 0), h), args.T - 1));
     };
     auto take_row = [&](int tile, int h, int32_t raw_row) {
       const int64_t row = table_row(tile, h);
-      return tile < args.num_tiles && row < args.T ? (permuted ? raw_row : (int32_t)row) : -1;
+      return tile >= 0 && row < args.T ? (permuted ? raw_row : (int32_t)row) : -1;
     };
-    int32_t grow[kSub], rows_1[kSub] = {}, rows_2[kSub] = {};
-    request_rows((int)blockIdx.x, rows_1);
-    if (!kStaged) request_rows((int)(blockIdx.x + gridDim.x), rows_2);
+    int32_t grow[kSub], next_rows[kSub] = {};
+    int tile, next = -1;
+    uint32_t hb[kSub], next_hb[kSub];
+    if (!next_tile(tile, hb)) tile = -1;
+    request_rows(tile, next_rows);
     // Residuals of 33 to 64 columns come through a ring of this warp's own, one use of it (two pieces) ahead:
     // four lanes copy 64 bytes of a row, where a lane that reads its own row's pieces makes every load
     // 32 lines of 128 bytes.  64->64, us: 464k rows of 1.15 pairs 55.3 -> 48.5, 406k of 3.4 81 -> 76, 298k of 9.3
@@ -528,29 +607,12 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
       }
       asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    if (kStaged && first_piece < last_piece) stage_residual(0u, take_row((int)blockIdx.x, 0, rows_1[0]), first_piece);
-    for (int tile = blockIdx.x; tile < args.num_tiles; tile += gridDim.x) {
-      uint32_t hb[kSub];
-      take_bits<kSub>(args, tile, raw, hb);
-      request_bits<kSub, kMode>(args, tile + (int)gridDim.x, raw);
+    if (kStaged && first_piece < last_piece) stage_residual(0u, take_row(tile, 0, next_rows[0]), first_piece);
+    while (tile >= 0) {
 #pragma unroll
-      for (int h = 0; h < kSub; h++) grow[h] = take_row(tile, h, rows_1[h]);
-      if (kStaged) {
-        request_rows(tile + (int)gridDim.x, rows_1);
-      } else {
-#pragma unroll
-        for (int h = 0; h < kSub; h++) rows_1[h] = rows_2[h];
-        request_rows(tile + 2 * (int)gridDim.x, rows_2);
-      }
-      if (!kPairs && args.residual != nullptr && !kStaged) {
-#pragma unroll
-        for (int h = 0; h < kSub; h++) {
-          const int32_t next = take_row(tile + (int)gridDim.x, h, rows_1[h]);
-          if (next < 0) continue;
-          const uint8_t *row = args.residual + (int64_t)next * n * 2;
-          for (int off = 0; off < n * 2; off += 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(row + off));
-        }
-      }
+      for (int h = 0; h < kSub; h++) grow[h] = take_row(tile, h, next_rows[h]);
+      if (!next_tile(next, next_hb)) break;
+      request_rows(next, next_rows);
       uint32_t res[8];
       // rows that are no whole number of 16-byte pieces (kDense): 8-byte pieces
       auto load_narrow = [&](const uint8_t *src, int c) {
@@ -580,6 +642,15 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
       if (!kPairs && !kStaged) load_residual(0, first_piece * 16);
       if (!mbar_wait_warp(false, &bar_acc_full[acc], acc_phase, abort_flag, args.status)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      if (!kPairs && !kStaged && args.residual != nullptr) {
+#pragma unroll
+        for (int h = 0; h < kSub; h++) {
+          const int32_t ahead = take_row(next, h, next_rows[h]);
+          if (ahead < 0) continue;
+          const uint8_t *row = args.residual + (int64_t)ahead * n * 2;
+          for (int off = 0; off < n * 2; off += 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(row + off));
+        }
+      }
 #pragma unroll (kStaged ? 1 : kSub)
       for (int h = 0; h < kSub; h++) {
         // (kStaged: one body for both sub-tiles, two of them spill; no index into registers then)
@@ -696,7 +767,7 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
           for (int q0 = first_piece; q0 < last_piece; q0 += 2) {
             __syncwarp();                                     // every lane has read the slot that is filled now
             const bool same = q0 + 2 < last_piece;
-            const int32_t row = same ? row_now() : h + 1 < kSub ? grow[kSub - 1] : take_row(tile + (int)gridDim.x, 0, rows_1[0]);
+            const int32_t row = same ? row_now() : h + 1 < kSub ? grow[kSub - 1] : take_row(next, 0, next_rows[0]);
             stage_residual(res_turn ^ 1u, row, same ? q0 + 2 : first_piece);
             asm volatile("cp.async.wait_group 1;" ::: "memory");
             __syncwarp();
@@ -708,6 +779,9 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
         }
       }
       if (++acc == args.acc_bufs) { acc = 0; acc_phase ^= 1u; }
+      tile = next;
+#pragma unroll
+      for (int h = 0; h < kSub; h++) hb[h] = next_hb[h];
     }
     asm volatile("cp.async.wait_all;" ::: "memory");   // nothing of this lane is in flight at exit
   }
@@ -872,10 +946,9 @@ mn_status launch_implicit(const ImArgs &a, const TcSizing &sizing, const CUtenso
                           const CUtensorMap &map_b, cudaStream_t st) {
   auto kernel = conv_implicit_kernel<kSub, kLpr, kProdWarps, kMode, kStaged>;
   MN_RETURN_IF(allow_max_shared_memory(reinterpret_cast<const void *>(kernel)));
-  const int grid = std::min(a.num_tiles, kNumSMs * sizing.ctas_per_sm);
   MN_LAUNCH(kMode == kPairRows ? "conv_implicit_kernel<pairs>" : kMode == kDense ? "conv_implicit_kernel<dense>"
                                                                                  : "conv_implicit_kernel", st,
-            launch_early(kernel, grid, kImThreads, sizing.smem_bytes, st, a, map_a, map_b));
+            launch_early(kernel, (unsigned)a.num_tiles, kImThreads, sizing.smem_bytes, st, a, map_a, map_b));
   return MN_OK;
 }
 

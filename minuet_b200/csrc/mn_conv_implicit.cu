@@ -240,6 +240,9 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   wait_for_predecessor();
+  // the first tile's offset bits, on their way while the rest is set up
+  uint32_t raw[kSub];
+  if (warp == kIdxWarp) request_bits<kSub, kMode>(args, args.num_tiles - 1 - (int)blockIdx.x, raw);
   if (!kPairs && (args.scale != nullptr || args.shift != nullptr)) {
     for (int c = threadIdx.x; c < args.n_pad; c += kImThreads) {
       s_scale[c] = args.scale != nullptr && c < args.N ? __ldg(args.scale + c) : 1.f;
@@ -460,7 +463,8 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
     // and takes over the tiles of blocks that have not started (cluster launch control) as it needs them, at most
     // kTileSlots before its epilogue.  Rows with many and rare offsets sort to the end, so the dear tiles go first.
     // With every gridDim-th tile for a CTA the busiest had 1.2 to 1.7 times the average of steps (one to
-    // four clouds; FIGURES).
+    // four clouds).  us, before / now: 406k rows of 3.4 pairs 64->64 70 / 59, 128->128 137 / 110, 256->256 328 /
+    // 271; 1.8M of 9.3 256->256 3090 / 2810; 31k of 16.7 84 / 79; a single tile per CTA 0.1 to 0.3 more.
     //
     // 128 entries of the neighbour table per step and sub-tile, up to kIdxSlots steps ahead of the
     // producers, so that they never wait for an index from memory (loaded by the producers
@@ -470,10 +474,8 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
     // 32->32, 1.15 pairs a row, 37.7 / 32.8; 64->64 45 / 42; 406k 64->64, 3.4 pairs, 74.6 / 68; 123k 64->64,
     // 16.7 pairs, 70 / 62; 406k 64->128 90 / 86).
     const uint32_t ring = smem_u32(idx_ring) + (uint32_t)lane * 16u;
-    uint32_t raw[kSub], phase = 0;
     int tile = args.num_tiles - 1 - (int)blockIdx.x;
-    request_bits<kSub, kMode>(args, tile, raw);
-    uint32_t claim_phase = 0, publish_phase = 0;
+    uint32_t phase = 0, claim_phase = 0, publish_phase = 0;
     int publish_slot = 0;
     bool claim_open = false;                       // an answer is on its way
     auto publish = [&](const uint32_t (&hb)[kSub]) {

@@ -63,6 +63,10 @@ __device__ __forceinline__ int row_of_item(const WgradPlan &plan, int item) {
 
 // list[row_begin[p] + masks[p, r]] = r for every entry of the masks; with `bits` (hit words)
 // only the entries that exist are looked at.
+// What bounds it: a row's loads, when they follow one another (the stores between them keep the order).  With
+// kPairBatch of them in flight: 27 offsets of 58 800 rows 7.7 us -> 5.5, of 15 700 rows 12.5 -> 7 (more pairs a row).
+constexpr int kPairBatch = 9;
+
 __global__ void __launch_bounds__(256)
 pair_side_kernel(const int32_t *__restrict__ masks, const uint32_t *__restrict__ bits, int64_t rows,
                  const __grid_constant__ WgradPlan plan, int32_t *__restrict__ list) {
@@ -70,10 +74,17 @@ pair_side_kernel(const int32_t *__restrict__ masks, const uint32_t *__restrict__
   const int64_t gsz = (int64_t)gridDim.x * blockDim.x;
   for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < rows; r += gsz) {
     if (bits != nullptr) {
-      for (uint32_t w = __ldg(bits + r); w != 0u; w &= w - 1u) {
-        const int p = __ffs(w) - 1;
-        const int m = __ldg(masks + (int64_t)p * rows + r);
-        if (m >= 0) list[plan.row_begin[p] + m] = (int32_t)r;
+      for (uint32_t w = __ldg(bits + r); w != 0u;) {
+        int p[kPairBatch], m[kPairBatch];
+#pragma unroll
+        for (int i = 0; i < kPairBatch; i++) {
+          p[i] = w != 0u ? __ffs(w) - 1 : 0;
+          m[i] = w != 0u ? __ldg(masks + (int64_t)p[i] * rows + r) : -1;
+          w &= w - 1u;
+        }
+#pragma unroll
+        for (int i = 0; i < kPairBatch; i++)
+          if (m[i] >= 0) list[plan.row_begin[p[i]] + m[i]] = (int32_t)r;
       }
     } else {
       const int p = blockIdx.y;

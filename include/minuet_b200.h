@@ -401,6 +401,11 @@ mn_status mn_sparse_convolution_weight_gradient(
     const void *grad_targets, const int32_t *pair_src, const int32_t *pair_dst, const int32_t *order,
     const int32_t *sizes_host, void *grad_weights_out, int32_t *status_dev, void *ws,
     size_t ws_bytes, void *stream);
+/* The weight gradient of a 1x1x1 convolution: grad_weight_out = x^T g, [c_in, c_out], of two fp32 matrices of
+ * `rows` rows; sums in fp32 in a fixed order. */
+size_t mn_dense_weight_gradient_workspace_bytes(int64_t rows, int64_t c_in, int64_t c_out);
+mn_status mn_dense_weight_gradient(int64_t rows, int64_t c_in, int64_t c_out, const float *x, const float *g,
+                                   float *grad_weight_out, void *ws, size_t ws_bytes, void *stream);
 
 /* weights_t_out[o, n, k] = weights[o, k, n]: the K-major weight layout the tensor-core
  * kernels read.  The three 16-bit forward entry points (implicit, pairs, dense) take

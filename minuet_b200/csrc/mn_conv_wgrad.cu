@@ -38,10 +38,11 @@ struct WgradPlan {
 struct WgradArgs {
   const void *x;             // [S, c_in]
   const void *g;             // [T, c_out]
-  const int32_t *pair_src;   // source row of every pair, -1 in the padding
+  const int32_t *pair_src;   // source row of every pair, -1 in the padding; null: row i of both arrays is pair i (FFMA)
   const int32_t *pair_dst;   // target row of every pair, -1 in the padding
   float *partial;            // [items, c_in, c_out]
   int32_t *status;
+  int64_t rows;              // of both arrays, where there are no lists
   int32_t c_in, c_out, n_pad;
   int32_t a_blocks, b_blocks;   // 64-channel blocks of one stage
   int32_t m_tiles;              // 128-channel accumulator tiles of this block
@@ -352,6 +353,11 @@ wgrad_simt_kernel(const __grid_constant__ WgradArgs a, const __grid_constant__ W
   auto load_pairs = [&](int st) {
     if (tid < 2 * kWsRows && st < n_stage) {
       const int side = tid / kWsRows, r = tid % kWsRows;
+      if (a.pair_src == nullptr) {
+        const int64_t row = first + (int64_t)st * kWsRows + r;
+        s_pair[st % kWsIdxSlots][side][r] = row < a.rows ? (int)row : -1;
+        return;
+      }
       asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(&s_pair[st % kWsIdxSlots][side][r])),
                    "l"((side ? a.pair_dst : a.pair_src) + first + (int64_t)st * kWsRows + r)
                    : "memory");
@@ -732,4 +738,40 @@ extern "C" mn_status mn_sparse_convolution_weight_gradient(
     case MN_F16: return run_wgrad_reduce<__half>(partial, plan, order, O, matrix, grad_weights_out, st);
     default: return run_wgrad_reduce<__nv_bfloat16>(partial, plan, order, O, matrix, grad_weights_out, st);
   }
+}
+
+// ---------------------------------------------------------------------------
+// x^T g: the weight gradient of a 1x1x1 convolution, fp32
+// ---------------------------------------------------------------------------
+// One offset whose pair i is row i of both arrays, so no lists.  A library GEMM sees a small matrix and a long
+// contraction and gives it
+// few blocks (58 800 rows x 96 x 20: 26); here the rows are cut into items for a wave of them: 157 us -> 24, 32 x 20 148 ->
+// 17, 192 x 128 151 -> 81, and a smaller error against fp64 (2.1e-8 -> 7e-9 of the terms' sum).
+extern "C" size_t mn_dense_weight_gradient_workspace_bytes(int64_t rows, int64_t c_in, int64_t c_out) {
+  if (rows < 0 || rows > INT32_MAX - kPairRows) return 0;
+  const int32_t size = (int32_t)rows;
+  return mn_weight_gradient_workspace_bytes(&size, 1, c_in, c_out, MN_F32);
+}
+
+extern "C" mn_status mn_dense_weight_gradient(int64_t rows, int64_t c_in, int64_t c_out, const float *x, const float *g,
+                                              float *grad_weight_out, void *ws_ptr, size_t ws_bytes, void *stream) {
+  MN_CHECK_ARG(rows >= 0 && rows <= INT32_MAX - kPairRows, "dense weight gradient: bad number of rows");
+  MN_CHECK_ARG(c_in >= 1 && c_out >= 1 && c_in < (1 << 20) && c_out < (1 << 20) && c_in * c_out < (1ll << 31),
+               "dense weight gradient: bad channels");
+  MN_CHECK_ARG(grad_weight_out != nullptr && (rows == 0 || (x != nullptr && g != nullptr)),
+               "dense weight gradient: null pointer");
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const int32_t size = (int32_t)rows;
+  const WgradPlan plan = make_wgrad_plan(&size, 1, c_in, c_out, MN_F32);
+  const int items = plan.item_prefix[MN_MAX_OFFSETS];
+  Workspace ws(ws_ptr, ws_bytes);
+  float *partial = ws.take<float>((size_t)std::max(items, 1) * c_in * c_out);
+  MN_CHECK_WS(ws);
+  if (items > 0) {
+    WgradArgs a{};
+    a.x = x; a.g = g; a.partial = partial; a.rows = rows;
+    a.c_in = (int)c_in; a.c_out = (int)c_out;
+    MN_RETURN_IF(run_wgrad_simt_t<float>(a, plan, items, st));
+  }
+  return run_wgrad_reduce<float>(partial, plan, nullptr, 1, c_in * c_out, grad_weight_out, st);
 }

@@ -9,6 +9,7 @@ from typing import Any, Dict, Optional, Union
 
 import numpy as np
 import torch
+from torch.autograd import forward_ad
 from torch.nn import Module
 
 from minuet_b200 import _lib, engine
@@ -16,6 +17,16 @@ from minuet_b200.nn import functional as F
 from minuet_b200.nn.functional import convolution as conv_functional
 from minuet_b200.tensors import SparseTensor
 from minuet_b200.utils.helpers import as_tuple, generate_kernel_offsets
+
+
+def _plain(*tensors) -> bool:
+    """Nothing that watches or rewrites torch's own operations sees these calls: no subclasses, tracing,
+    compilation, functorch transforms, dispatch or function modes, autocast or forward-mode differentiation."""
+    return (all(type(t) in (torch.Tensor, torch.nn.Parameter) for t in tensors) and
+            not torch._C._are_functorch_transforms_active() and
+            torch._C._get_tracing_state() is None and not torch.compiler.is_compiling() and
+            torch._C._len_torch_dispatch_stack() == 0 and torch._C._len_torch_function_stack() == 0 and
+            not torch.is_autocast_enabled("cuda") and forward_ad._current_level < 0)
 
 
 class KernelMapCache(object):
@@ -540,8 +551,14 @@ class SparseConv(Module):
         trivial = self._shape()[4]
         if trivial and torch.is_grad_enabled() and (
                 features.requires_grad or self.kernel.requires_grad):
-            # training: the plain product, differentiated by autograd
-            out = features @ self.kernel.view(self.in_channels, self.out_channels)
+            # training: the plain product, differentiated by autograd (the weight's gradient of many rows by a
+            # kernel of this library)
+            weight = self.kernel.view(self.in_channels, self.out_channels)
+            if _plain(features, self.kernel) and features.is_cuda and \
+                    _lib.host().dense_product_takes(features, weight):
+                out = _lib.host().dense_product(features, weight)
+            else:
+                out = features @ weight
             if self.bias is not None:
                 out = out + self.bias
             return SparseTensor(out, inputs.C, stride=inputs.stride, batch_dims=inputs.batch_dims)

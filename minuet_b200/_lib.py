@@ -103,6 +103,8 @@ PROTOTYPES = {
     "mn_sparse_convolution_weight_gradient": (c_int, [c_i64, c_i64, c_i64, c_i64, c_i64, c_int, c_ptr,
                                                       c_ptr, c_ptr, c_ptr, c_ptr, c_ptr, c_ptr, c_ptr,
                                                       c_ptr, c_size, c_ptr]),
+    "mn_dense_weight_gradient_workspace_bytes": (c_size, [c_i64, c_i64, c_i64]),
+    "mn_dense_weight_gradient": (c_int, [c_i64, c_i64, c_i64, c_ptr, c_ptr, c_ptr, c_ptr, c_size, c_ptr]),
     "mn_transpose_weights": (c_int, [c_ptr, c_i64, c_i64, c_i64, c_int, c_ptr, c_ptr]),
     "mn_pairs_supported": (c_int, [c_i64, c_i64, c_i64, c_int]),
     "mn_pair_rows": (c_i64, [c_ptr, c_i64, c_i64, c_i64, c_int]),

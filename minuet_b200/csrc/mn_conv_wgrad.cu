@@ -744,9 +744,10 @@ extern "C" mn_status mn_sparse_convolution_weight_gradient(
 // x^T g: the weight gradient of a 1x1x1 convolution, fp32
 // ---------------------------------------------------------------------------
 // One offset whose pair i is row i of both arrays, so no lists.  A library GEMM sees a small matrix and a long
-// contraction and gives it
-// few blocks (58 800 rows x 96 x 20: 26); here the rows are cut into items for a wave of them: 157 us -> 24, 32 x 20 148 ->
-// 17, 192 x 128 151 -> 81, and a smaller error against fp64 (2.1e-8 -> 7e-9 of the terms' sum).
+// contraction and gives it few blocks (58 800 rows x 96 x 20: 26); here the rows are cut into items for a wave of
+// them.  60 000 rows 32 x 20: 148 us -> 17, 96 x 20 157 -> 24, 192 x 128 151 -> 81, and a smaller error against
+// fp64 (96 x 20: 2.1e-8 -> 7e-9 of the terms' sum).  What bounds it: the chain of an item and of the sums over
+// the items up to some 20 000 rows, FFMA issue beyond.
 extern "C" size_t mn_dense_weight_gradient_workspace_bytes(int64_t rows, int64_t c_in, int64_t c_out) {
   if (rows < 0 || rows > INT32_MAX - kPairRows) return 0;
   const int32_t size = (int32_t)rows;

@@ -57,7 +57,7 @@ constexpr uint32_t kQPad = 64;               // relative keys start at kQPad
 constexpr uint32_t kHashEmpty = 0xffffffffu;
 constexpr uint64_t kRelLimit = 0xffffffffull - 4ull * kQPad;
 constexpr uint64_t kNarrow = 1ull << 29;
-constexpr uint32_t kQNowhere = 0xffffffe0u;  // relative key in a cell past every window's (below kRelLimit)
+constexpr uint32_t kQNowhere = 0xffffffe0u;  // relative key in a cell past every window's (below kRelLimit + kQPad)
 
 __device__ __forceinline__ unsigned lanemask_lt() {
   unsigned m;
@@ -361,7 +361,7 @@ search_kernel(const __grid_constant__ SearchPair sp) {
       auto relative = [&](int j, int g) {
         if (narrow) return (uint32_t)rel[j] + (uint32_t)s_gdelta[g] + (live[j] ? 0u : 0x80000000u);
         const uint64_t t0 = (uint64_t)(rel[j] + s_gdelta[g]);
-        return t0 < kRelLimit ? (uint32_t)t0 : kQNowhere;
+        return t0 < kRelLimit + kQPad ? (uint32_t)t0 : kQNowhere;   // the window's last key may be kQPad past the limit
       };
       // what the offsets of group g find for row j: the strip of its cell from `sh` on
       auto found = [&](int j, int g, uint32_t mask, uint32_t sh, uint32_t slot) {

@@ -60,3 +60,19 @@ def test_windows_without_a_key(oracle_lib, shift, n):
     d_src, d_tgt = (torch.as_tensor(c, device=DEV) for c in (src, tgt))
     got = F.query_sorted_index_with_offsets(d_src, d_tgt, torch.as_tensor(off, device=DEV))
     assert (got == -1).all()
+
+
+@pytest.mark.parametrize("z", [255, 256, 257, 258, 259, 300, 319, 320, 321, 322, 323, 400])
+def test_windows_as_wide_as_relative_keys_go(oracle_lib, z):
+    """Two voxels whose keys are 2^32 - z apart (nine bits of the last dimension): a window is searched by 32-bit
+    relative keys up to 2^32 - 258, and its last voxel is found there as beyond."""
+    src = np.array([[0, 0, z], [0, 1 << 23, 0]], np.int32)
+    off = generate_kernel_offsets(3, 3, 1, 1).astype(np.int32)
+    d = torch.as_tensor(src, device=DEV)
+    want = oracle_lib.query(src, src, off)
+    assert (want >= 0).sum() == 2
+    got = F.query_sorted_index_with_offsets(d, d, torch.as_tensor(off, device=DEV))
+    assert np.array_equal(got.cpu().numpy(), want)
+    cache = minuet.nn.KernelMapCache(ndim=3, dtype=torch.int32, device=DEV)
+    sm, tm, _, sizes = cache.get_kernel_map(d, 1, None, d, 1, None, 3, 1)
+    assert sizes.cpu().tolist() == [0] * 26 + [2] and sm[26].cpu().tolist() == tm[26].cpu().tolist() == [0, 1]

@@ -974,6 +974,9 @@ struct MapRef {
   }
 };
 
+// A gradient that torch knows to be zero (sgn's) comes without memory.
+Tensor with_memory(const Tensor &grad) { return grad._is_zerotensor() ? grad.clone() : grad; }
+
 struct WeightGradient : torch::autograd::Function<WeightGradient> {
   static Tensor forward(torch::autograd::AutogradContext *ctx, const Tensor &x, const Tensor &g, const Tensor &sm,
                         const Tensor &tm, const OptTensor &order, bool swapped, Holder holder);
@@ -999,7 +1002,7 @@ struct Convolution : torch::autograd::Function<Convolution> {
     const MapRef m = MapRef::load(ctx);
     Tensor grad_x, grad_w;
     if (at::GradMode::is_enabled()) {
-      const Tensor g = grads[0].to(w.scalar_type()).contiguous();
+      const Tensor g = with_memory(grads[0]).to(w.scalar_type()).contiguous();
       if (ctx->needs_input_grad(0))
         grad_x = Convolution::apply(g, w.transpose(1, 2).contiguous(), m.tm, m.sm, m.order, !m.swapped,
                                     flipped(m.holder));
@@ -1009,7 +1012,7 @@ struct Convolution : torch::autograd::Function<Convolution> {
     }
     at::AutoDispatchBelowADInplaceOrView below;
     Plan &plan = *m.holder->plan;
-    const Tensor g = grads[0].to(w.scalar_type()).contiguous();
+    const Tensor g = with_memory(grads[0]).to(w.scalar_type()).contiguous();
     if (ctx->needs_input_grad(0)) {
       // [O, c_out, c_in] weights; their transpose, which the tensor-core kernels read, is w
       grad_x = run_forward(plan, !m.swapped, g, w.transpose(1, 2), m.tm, m.sm, m.order,
@@ -1037,7 +1040,7 @@ torch::autograd::variable_list WeightGradient::backward(torch::autograd::Autogra
   const Tensor &x = saved[0], &g = saved[1];
   c10::cuda::CUDAGuard guard(x.get_device());
   const MapRef m = MapRef::load(ctx);
-  const Tensor u = grads[0].to(x.scalar_type()).contiguous();
+  const Tensor u = with_memory(grads[0]).to(x.scalar_type()).contiguous();
   Tensor grad_x, grad_g;
   if (ctx->needs_input_grad(0))
     grad_x = Convolution::apply(g, u.transpose(1, 2).contiguous(), m.tm, m.sm, m.order, !m.swapped, flipped(m.holder));
@@ -1121,7 +1124,7 @@ bool dense_product_takes(const Tensor &x, const Tensor &w) {
 bool plain_values(const Tensor &t) {
   for (const auto key : {c10::DispatchKey::FuncTorchBatched, c10::DispatchKey::FuncTorchGradWrapper,
                          c10::DispatchKey::FuncTorchVmapMode, c10::DispatchKey::Batched, c10::DispatchKey::Functionalize,
-                         c10::DispatchKey::Python, c10::DispatchKey::Negative})
+                         c10::DispatchKey::Python, c10::DispatchKey::Negative, c10::DispatchKey::ZeroTensor})
     if (t.key_set().has(key)) return false;
   return t.is_cuda() && t.layout() == at::kStrided && t.scalar_type() == at::kFloat && !t._fw_grad(0).defined() &&
          !c10::impl::TorchDispatchModeTLS::any_modes_set();

@@ -42,3 +42,24 @@ def test_weight_gradient(oracle_lib, n, c_in, c_out, dtype, kernel):
     (again,) = torch.autograd.grad(conv(minuet.SparseTensor(x, torch.as_tensor(src, device=DEV))).F,
                                    (conv.kernel,), g)
     assert torch.equal(dw, again)
+
+
+@pytest.mark.parametrize("kernel", [1, 3])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+@pytest.mark.parametrize("create_graph", [False, True])
+def test_a_gradient_that_torch_keeps_without_memory(kernel, dtype, create_graph):
+    """The gradient of sgn is zero, and a tensor that has no memory."""
+    rng = np.random.default_rng(3)
+    src, _ = synth.random_small_batch(rng, 1, 3000, 24)
+    assert len(src) >= 1024
+    conv = minuet.nn.SparseConv3d(16, 24, kernel, dtype=dtype, device=DEV)
+    cache = minuet.nn.KernelMapCache(ndim=3, dtype=torch.int32, device=DEV)
+    minuet.set_kernel_map_cache(conv, cache)
+    x = torch.ones(len(src), 16, device=DEV, dtype=dtype, requires_grad=True)
+    seen = []
+    out = conv(minuet.SparseTensor(x, torch.as_tensor(src, device=DEV))).F
+    out.register_hook(lambda g: seen.append(g._is_zerotensor()))
+    grads = torch.autograd.grad(torch.sgn(out).sum(), (x, conv.kernel), create_graph=create_graph)
+    assert seen == [True]
+    for grad, of in zip(grads, (x, conv.kernel)):
+        assert grad.shape == of.shape and grad.dtype == dtype and bool((grad == 0).all())

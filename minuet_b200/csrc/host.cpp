@@ -1104,11 +1104,8 @@ std::pair<Tensor, bool> dense_forward(const Tensor &features_in, const Tensor &w
   return {out, tensor_core};
 }
 
-// x w in training, differentiated as torch does, except that x^T g is a kernel of its own.
-//
-// The line between them, x^T g in a library GEMM and here, us: 1000 rows 128 x 64 10.3, 8.8; 192 x 128 10.5, 9.0 (512
-// rows: 7.6, 9.4); 60 000 rows 32 x 20 148, 17; 96 x 20 157, 24; 192 x 128 151, 81.  A matrix of many tiles keeps
-// the library busy too: 256 x 256 60 000 rows 292, 187, but 240 000 rows 708, 738; 512 x 512 16 000 rows 197, 201.
+// x w in training, differentiated as torch does, except that x^T g may be a kernel of its own (own_gradient_pays; with
+// fewer rows, or more weights, it never is: 512 rows 192 x 128 7.6 us in torch, 9.4 here).
 bool dense_product_takes(const Tensor &x, const Tensor &w) {
   if (x.dim() != 2 || w.dim() != 2 || x.size(0) < 1024 || w.numel() > (1 << 16) ||
       (w.numel() > (1 << 15) && x.size(0) > (1 << 17)))
@@ -1130,6 +1127,28 @@ bool plain_values(const Tensor &t) {
          !c10::impl::TorchDispatchModeTLS::any_modes_set();
 }
 
+// Where x^T g is faster in the library's kernel than in torch's GEMM, us, torch / here.  One channel is a matrix times a
+// vector there: 400k rows 96 x 1 46 / 163.  Channels in fours: 1000 rows 128 x 64 10.3 / 8.8; 60k rows 32 x 20 148 / 18, 96 x
+// 20 156 / 25, 192 x 128 152 / 83.  Channels that are not are copied one by one here, and torch is good at few of them into
+// many: 1024 rows 32 x 13 18.8 / 8.6, 65 x 65 11.1 / 14.7, 8000 rows 7 x 64 10.1 / 13.2, 30k rows 42 / 17, 400k 88 / 99.  Matrices
+// of many tiles keep torch's GEMM busy too: 256 x 256 131k rows 444 / 391, 240k 708 / 738; 160 x 200 400k rows 899 / 878, 1 M
+// 2144 / 2178; 65 x 65 131k rows 224 / 165, 400k 414 / 490; 4 x 4096 100k rows 708 / 677, 131k 785 / 887.
+// A caller who allows TF32 has a faster GEMM there: 60k rows 32 x 20 64 / 18, 64 x 64 66 / 26, 128 x 64 68 / 37, 192 x 128 77 /
+// 83; 131k rows 256 x 256 137 / 391; 4000 rows 64 x 64 9.1 / 11.1, 16k 17.8 / 12.6; 400k rows 128 x 64 171 / 169, 1 M 269 / 387.
+bool own_gradient_pays(int64_t rows, int64_t c_in, int64_t c_out) {
+  if (c_in == 1 || c_out == 1) return false;
+  const bool fours = c_in % 4 == 0 && c_out % 4 == 0;
+  if (!fours && c_out > 32 && rows < (c_in < 32 ? 1 << 14 : 1 << 11)) return false;
+  auto tiled = [](int64_t c) { return c <= 32 ? 32 : (c + 63) / 64 * 64; };
+  const int64_t tiles = tiled(c_in) * tiled(c_out), cost = fours ? tiles : 3 * tiles;
+  if ((cost > (1 << 15) || (!fours && c_out > 32)) &&
+      (double)rows * (double)std::max<int64_t>(cost, 1 << 15) > 1.3e10)
+    return false;
+  const auto precision = at::globalContext().float32Precision(at::Float32Backend::CUDA, at::Float32Op::MATMUL);
+  if (precision == at::Float32Precision::IEEE || precision == at::Float32Precision::NONE) return true;
+  return tiles <= 32 * 32 || (tiles <= 128 * 64 && rows >= 8192 && (double)rows * (double)tiles <= 3.3e9);
+}
+
 struct DenseProduct : torch::autograd::Function<DenseProduct> {
   static Tensor forward(torch::autograd::AutogradContext *ctx, const Tensor &x, const Tensor &w) {
     at::AutoDispatchBelowADInplaceOrView below;
@@ -1144,7 +1163,8 @@ struct DenseProduct : torch::autograd::Function<DenseProduct> {
     Tensor grad_x, grad_w;
     if (ctx->needs_input_grad(0)) grad_x = at::mm(grads[0], w.t());
     if (ctx->needs_input_grad(1)) {
-      if (at::GradMode::is_enabled() || !plain_values(grads[0]) || !plain_values(x) || !x.is_contiguous()) {
+      if (at::GradMode::is_enabled() || !plain_values(grads[0]) || !plain_values(x) || !x.is_contiguous() ||
+          !own_gradient_pays(x.size(0), w.size(0), w.size(1))) {
         grad_w = at::mm(x.t(), grads[0]);
       } else {
         at::AutoDispatchBelowADInplaceOrView below;

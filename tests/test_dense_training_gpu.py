@@ -47,6 +47,38 @@ def test_gradients(rows, c_in, c_out):
     assert torch.equal(gw.view(c_in, c_out), (whole[0].double().t() @ whole[1].double()).float())
 
 
+@pytest.mark.parametrize("rows,c_in,c_out,tf32", [
+    (4097, 1, 48, False), (4097, 96, 1, False), (16_383, 7, 64, False), (2047, 33, 36, False), (400_000, 13, 40, False),
+    (131_072, 4, 4096, False), (20_000, 192, 128, True), (8191, 64, 64, True), (500_000, 64, 80, True)])
+def test_weight_gradients_that_are_left_to_torch(rows, c_in, c_out, tf32):
+    """One channel, channels not in fours into many, many tiles, a faster GEMM that the caller allows: its bits."""
+    gen = torch.Generator(device=DEV).manual_seed(rows + c_in)
+    conv, run = _layer(c_in, c_out)
+    x, g = (torch.randn(rows, c, generator=gen, device=DEV) for c in (c_in, c_out))
+    before = torch.backends.cuda.matmul.allow_tf32
+    torch.backends.cuda.matmul.allow_tf32 = tf32
+    try:
+        got, want = (torch.autograd.grad(out, conv.kernel, g)[0] for out in (run(x), x @ _matrix(conv)))
+    finally:
+        torch.backends.cuda.matmul.allow_tf32 = before
+    assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("rows,c_in,c_out", [(1024, 32, 20), (8192, 64, 64), (8192, 128, 64)])
+def test_weight_gradients_in_fp32_where_tf32_is_allowed(rows, c_in, c_out):
+    gen = torch.Generator(device=DEV).manual_seed(rows + c_in)
+    conv, run = _layer(c_in, c_out)
+    x, g = (torch.randn(rows, c, generator=gen, device=DEV) for c in (c_in, c_out))
+    want, = torch.autograd.grad(run(x), conv.kernel, g)
+    before = torch.backends.cuda.matmul.allow_tf32
+    torch.backends.cuda.matmul.allow_tf32 = True
+    try:
+        got, = torch.autograd.grad(run(x), conv.kernel, g)
+    finally:
+        torch.backends.cuda.matmul.allow_tf32 = before
+    assert torch.equal(got, want)
+
+
 @pytest.mark.parametrize("case", ["few rows", "half", "strided", "frozen", "autocast", "wide", "no rows", "function mode"])
 def test_calls_that_stay_a_plain_product(case):
     gen = torch.Generator(device=DEV).manual_seed(1)

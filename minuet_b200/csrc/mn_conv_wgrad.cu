@@ -38,7 +38,7 @@ struct WgradPlan {
 struct WgradArgs {
   const void *x;             // [S, c_in]
   const void *g;             // [T, c_out]
-  const int32_t *pair_src;   // source row of every pair, -1 in the padding; null: row i of both arrays is pair i (FFMA)
+  const int32_t *pair_src;   // source row of every pair, -1 in the padding; null: row i of both arrays is pair i (FFMA only)
   const int32_t *pair_dst;   // target row of every pair, -1 in the padding
   float *partial;            // [items, c_in, c_out]
   int32_t *status;
@@ -323,14 +323,16 @@ constexpr int kWsIdxAhead = kWsStages;
 // A block owns a BM x BN tile of one item's matrix; a thread 8 x TN of it, 4 rows in each half (and 4
 // columns in each half, TN == 8).  The threads form kGroups groups that take every kGroups-th
 // pair of a stage and are added up at the end, two by two.  kVec: rows of both arrays can be
-// copied 16 bytes at a time (fp32, channels a multiple of 4, aligned).
+// copied 16 bytes at a time (fp32, channels a multiple of 4, aligned).  kLists: pairs are named by the lists, otherwise
+// pair i is row i of both arrays (an instance of its own: as a branch it cost the layers with lists 3 to 5 %, 200k rows
+// 32 x 32 with 13.5 pairs 180.5 -> 190.4 us).
 //
 // What bounds it: FFMA issue and the copies' latency.  With 8 x 4 sums a thread, and the list entries read
 // from memory before every copy, 586k pairs 64 x 64 took 230 us (products at the FFMA rate: 65 us), now
 // 124; 196k pairs 128 x 64 122 -> 96; 52k pairs 256 x 128 141 -> 115 (both with the host's part).  Small tiles
 // keep 8 x 4: their copies need the warps that 128 registers a thread would cost.  The ring of a 64 x 64 tile
 // (48 KB) lets four blocks share an SM, so its registers are limited for four (for six they spilled).
-template <typename T, int BM, int BN, int TN, bool kVec>
+template <typename T, int BM, int BN, int TN, bool kVec, bool kLists>
 __global__ void __launch_bounds__(kWsThreads, TN == 8 || BM + BN == 128 ? 4 : 6)
 wgrad_simt_kernel(const __grid_constant__ WgradArgs a, const __grid_constant__ WgradPlan plan, int n_tiles) {
   begin_early();
@@ -353,14 +355,14 @@ wgrad_simt_kernel(const __grid_constant__ WgradArgs a, const __grid_constant__ W
   auto load_pairs = [&](int st) {
     if (tid < 2 * kWsRows && st < n_stage) {
       const int side = tid / kWsRows, r = tid % kWsRows;
-      if (a.pair_src == nullptr) {
+      if constexpr (!kLists) {
         const int64_t row = first + (int64_t)st * kWsRows + r;
         s_pair[st % kWsIdxSlots][side][r] = row < a.rows ? (int)row : -1;
-        return;
+      } else {
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(&s_pair[st % kWsIdxSlots][side][r])),
+                     "l"((side ? a.pair_dst : a.pair_src) + first + (int64_t)st * kWsRows + r)
+                     : "memory");
       }
-      asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(&s_pair[st % kWsIdxSlots][side][r])),
-                   "l"((side ? a.pair_dst : a.pair_src) + first + (int64_t)st * kWsRows + r)
-                   : "memory");
     }
   };
   auto load_stage = [&](int st) {
@@ -591,7 +593,10 @@ WgradPlan make_wgrad_plan(const int32_t *sizes, int64_t O, int64_t c_in, int64_t
 
 template <typename T, int BM, int BN, int TN, bool kVec>
 mn_status launch_wgrad_simt(const WgradArgs &a, const WgradPlan &plan, int items, cudaStream_t st) {
-  const auto kernel = wgrad_simt_kernel<T, BM, BN, TN, kVec>;
+  auto kernel = wgrad_simt_kernel<T, BM, BN, TN, kVec, true>;
+  if constexpr (sizeof(T) == 4) {
+    if (a.pair_src == nullptr) kernel = wgrad_simt_kernel<T, BM, BN, TN, kVec, false>;
+  }
   const int n_tiles = (int)div_up(a.c_out, BN);
   const dim3 grid((unsigned)items, (unsigned)(div_up(a.c_in, BM) * n_tiles));
   const size_t smem = (size_t)kWsStages * kWsRows * (BM + BN) * sizeof(float);

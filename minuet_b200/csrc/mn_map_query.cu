@@ -312,6 +312,8 @@ search_kernel(const __grid_constant__ SearchPair sp) {
   MN_MARK(g_marks_search, 2);
 
   uint32_t bits[kQRows] = {0u, 0u};
+  const bool in_pairs = kMode == kMap && (a.n_rows & 1) == 0 &&
+                        (reinterpret_cast<uintptr_t>(a.kernel_map) & 7) == 0 && live[kQRows - 1];
   const int num_stages = s_num_stages;
   bool clean = true;                          // no keys in the hash yet
   for (int st = 0; st < num_stages; st++) {
@@ -392,6 +394,40 @@ search_kernel(const __grid_constant__ SearchPair sp) {
           }
         }
       };
+      // The same for the thread's rows together, where a member at a time is looked at: the layout of the members is
+      // read once, and a map's entries of two rows are one store.
+      auto found_by_member = [&](int g, const uint32_t (&mask)[kQRows], const uint32_t (&sh)[kQRows],
+                                 const uint32_t (&slot)[kQRows]) {
+        const uint32_t meta = s_gmeta[g], o_first = meta & 0xffu;
+        const int members = (int)((meta >> 8) & 0xffu), mb = tab.group_begin[g], e_first = tab.off[o_first][last];
+        int32_t first[kQRows];
+#pragma unroll
+        for (int j = 0; j < kQRows; j++) first[j] = kPos ? (int32_t)(lo + s_hpos[slot[j]]) : 0;
+        for (int m = 0; m < members; m++) {
+          const bool compact = (meta >> 16) != 0u;
+          const int o = compact ? (int)o_first + m : tab.member[mb + m];
+          const uint32_t de = (uint32_t)(compact ? m : tab.off[o][last] - e_first);
+          int32_t idx[kQRows];
+#pragma unroll
+          for (int j = 0; j < kQRows; j++) {
+            const uint32_t below = mask[j] & ((1u << (sh[j] + de)) - 1u), hit = mask[j] >> (sh[j] + de) & 1u;
+            idx[j] = hit != 0u ? first[j] + __popc(below) : -1;
+            if (kMode != kMap) {
+              bits[j] |= hit << o;
+              if (kMode == kBitsRev && hit != 0u) atomicOr(a.table_words + idx[j], 1u << o);
+            }
+          }
+          if (kMode == kMap) {
+            int32_t *dst = a.kernel_map + (int64_t)o * a.n_rows + row0;
+            if (in_pairs) {
+              *reinterpret_cast<int2 *>(dst) = make_int2(idx[0], idx[1]);
+            } else {
+#pragma unroll
+              for (int j = 0; j < kQRows; j++) if (live[j]) dst[j] = idx[j];
+            }
+          }
+        }
+      };
       // Linear probing over {cell, mask} slots.  The first two slots are one load and hold nearly all answers;
       // a lookup that has to go on is put off (its offsets have found nothing so far) until the others are
       // through, so that a warp goes round the probing loop for its few of them together.
@@ -400,14 +436,23 @@ search_kernel(const __grid_constant__ SearchPair sp) {
         uint32_t open[kQRows] = {0u, 0u};
 #pragma unroll 3
         for (int g = g0; g < g1; g++) {
+          uint32_t mask[kQRows], sh[kQRows], slot[kQRows];
 #pragma unroll
           for (int j = 0; j < kQRows; j++) {
-            const uint32_t q = relative(j, g), c = cells.cell(q), sh = q - c * cells.step, slot = hash_slot(c);
-            const uint4 v = *reinterpret_cast<const uint4 *>(s_slots + slot);
+            const uint32_t q = relative(j, g), c = cells.cell(q);
+            sh[j] = q - c * cells.step;
+            slot[j] = hash_slot(c);
+            const uint4 v = *reinterpret_cast<const uint4 *>(s_slots + slot[j]);
             const bool second = v.z == c;
-            const uint32_t mask = v.x == c ? v.y : second ? v.w : 0u;
+            mask[j] = v.x == c ? v.y : second ? v.w : 0u;
             if (v.x != c && !second && v.z != kHashEmpty) open[j] |= 1u << (g - g0);
-            found(j, g, mask, sh, slot + (second ? 1u : 0u));
+            slot[j] += second ? 1u : 0u;
+          }
+          if (kMode == kMap || (s_gmeta[g] >> 16) == 0u) {
+            found_by_member(g, mask, sh, slot);
+          } else {
+#pragma unroll
+            for (int j = 0; j < kQRows; j++) found(j, g, mask[j], sh[j], slot[j]);
           }
         }
 #pragma unroll

@@ -22,7 +22,10 @@
 // now 7 500 (layout, keys and tile ends in one trip, the hash cleared before the wait for the kernel
 // before, bounds looked for near the tile where the rows are the table) and 13 000 (strips that lie in one cell,
 // keys of 32 bits, the few longer probes of a warp in one loop at the end).  464k rows, four
-// maps: 138 -> 99 us of searches; 7.3 million, two maps: 634 -> 534 us.  Tiles whose window does not fit the hash are
+// maps: 138 -> 99 us of searches; 7.3 million, two maps: 634 -> 534 us.  Keys in two cells cost what they save where few and
+// long groups ask (build of 1 x 1 x 5 dilated by 7, 464k rows: 31 -> 33 us; 3 x 3 x 3 dilated by 4 77 -> 75, 50k uniform rows
+// 10 % more).  Lanes that add up their bits of a cell before one inserts it: 0.9 of the time on full grids,
+// 1.04 on scans, not kept.  Tiles whose window does not fit the hash are
 // processed group range by group range, and ranges that still do not fit fall
 // back to binary search in global memory.  The kernel writes kernel-map rows
 // or, for the fused build, one 32-bit word of per-offset hit bits per row.
@@ -51,7 +54,9 @@ constexpr int kQWarps = kQThreads / 32;
 constexpr int kQRows = 2;                    // rows per thread
 constexpr int kQTile = kQThreads * kQRows;   // 512 rows per block
 constexpr int kQSlots = 4096;                // hash slots of 8 bytes: {cell, occupancy}
-constexpr int kQMaxWindow = 1280;            // table keys per hashed stage (load factor <= 0.31, with a key in two cells 0.33 for 3 x 3 x 3)
+// Table keys per hashed stage.  A key near a cell's start is in two cells: the load factor is at most
+// (1 + span / step) * 1280 / 4096, 0.33 for 3 x 3 x 3 and 0.56 for the longest groups (span 14, step 18).
+constexpr int kQMaxWindow = 1280;
 constexpr int kQMaxSpan = 14;                // last-dimension span of one group
 constexpr uint32_t kQPad = 64;               // relative keys start at kQPad
 constexpr uint32_t kHashEmpty = 0xffffffffu;
@@ -184,7 +189,7 @@ search_kernel(const __grid_constant__ SearchPair sp) {
   __shared__ uint16_t s_hpos[kPos ? kQSlots : 2];   // first position of a cell
   __shared__ int64_t s_delta[MN_MAX_OFFSETS];
   __shared__ int64_t s_gdelta[MN_MAX_OFFSETS];       // per group: delta of its first member
-  __shared__ uint32_t s_gmeta[MN_MAX_OFFSETS];       // first offset | members << 8 | compact << 16
+  __shared__ uint32_t s_gmeta[MN_MAX_OFFSETS];       // first offset | members << 8 | stride << 16
   __shared__ int64_t s_glo[MN_MAX_OFFSETS], s_ghi[MN_MAX_OFFSETS];
   __shared__ int64_t s_slo[MN_MAX_OFFSETS], s_shi[MN_MAX_OFFSETS];
   __shared__ uint8_t s_stage_gbeg[MN_MAX_OFFSETS + 1];
@@ -207,12 +212,14 @@ search_kernel(const __grid_constant__ SearchPair sp) {
   for (int g = tid; g < G; g += kQThreads) {
     const int mb = tab.group_begin[g], me = tab.group_begin[g + 1];
     const int o_first = tab.member[mb];
-    // compact: member i is offset o_first + i and sits i values further along the last dimension
-    bool compact = true;
+    // stride: member i is offset o_first + i and sits i * stride values further along the last dimension; 0: no such
+    // order (a dilated kernel's members were looked up one by one in the parameters, two dependent reads each)
+    const int stride = me - mb > 1 ? tab.off[tab.member[mb + 1]][last] - tab.off[o_first][last] : 1;
+    bool regular = true;
     for (int m = mb; m < me; m++)
-      compact &= tab.member[m] == o_first + (m - mb) &&
-                 tab.off[tab.member[m]][last] - tab.off[o_first][last] == m - mb;
-    s_gmeta[g] = (uint32_t)o_first | ((uint32_t)(me - mb) << 8) | ((compact ? 1u : 0u) << 16);
+      regular &= tab.member[m] == o_first + (m - mb) &&
+                 tab.off[tab.member[m]][last] - tab.off[o_first][last] == (m - mb) * stride;
+    s_gmeta[g] = (uint32_t)o_first | ((uint32_t)(me - mb) << 8) | ((regular ? (uint32_t)stride : 0u) << 16);
   }
   begin_early();
   MN_MARK(g_marks_search, 0);
@@ -366,47 +373,35 @@ search_kernel(const __grid_constant__ SearchPair sp) {
         return t0 < kRelLimit + kQPad ? (uint32_t)t0 : kQNowhere;   // the window's last key may be kQPad past the limit
       };
       // what the offsets of group g find for row j: the strip of its cell from `sh` on
-      auto found = [&](int j, int g, uint32_t mask, uint32_t sh, uint32_t slot) {
-        const uint32_t meta = s_gmeta[g], o_first = meta & 0xffu, members = (meta >> 8) & 0xffu;
-        if (kMode != kMap && (meta >> 16) != 0u) {
-          const uint32_t strip = (mask >> sh) & ((1u << members) - 1u);
-          bits[j] |= strip << o_first;
-          if (kMode == kBitsRev && strip != 0u) {
-            // entries of a cell follow one another
-            uint32_t *at = a.table_words + lo + s_hpos[slot] + __popc(mask & ((1u << sh) - 1u));
-            for (uint32_t rest = strip; rest != 0u; rest &= rest - 1u, at++)
-              atomicOr(at, (rest & (0u - rest)) << o_first);
-          }
-          return;
-        }
-        const int mb = tab.group_begin[g], e_first = tab.off[o_first][last];
-        for (int m = mb; m < mb + (int)members; m++) {
-          const int o = tab.member[m];
-          const uint32_t b = sh + (uint32_t)(tab.off[o][last] - e_first);   // < 32
-          const bool hit = (mask >> b) & 1u;
-          int32_t idx = -1;
-          if (kPos && hit) idx = (int32_t)(lo + s_hpos[slot] + __popc(mask & ((1u << b) - 1u)));
-          if (kMode == kMap) {
-            if (live[j]) a.kernel_map[(int64_t)o * a.n_rows + row0 + j] = idx;
-          } else if (hit) {
-            bits[j] |= 1u << o;
-            if (kMode == kBitsRev) atomicOr(a.table_words + idx, 1u << o);
-          }
+      auto found_strip = [&](int j, uint32_t meta, uint32_t mask, uint32_t sh, uint32_t slot) {
+        const uint32_t o_first = meta & 0xffu, members = (meta >> 8) & 0xffu;
+        const uint32_t strip = (mask >> sh) & ((1u << members) - 1u);
+        bits[j] |= strip << o_first;
+        if (kMode == kBitsRev && strip != 0u) {
+          // entries of a cell follow one another
+          uint32_t *at = a.table_words + lo + s_hpos[slot] + __popc(mask & ((1u << sh) - 1u));
+          for (uint32_t rest = strip; rest != 0u; rest &= rest - 1u, at++)
+            atomicOr(at, (rest & (0u - rest)) << o_first);
         }
       };
-      // The same for the thread's rows together, where a member at a time is looked at: the layout of the members is
-      // read once, and a map's entries of two rows are one store.
-      auto found_by_member = [&](int g, const uint32_t (&mask)[kQRows], const uint32_t (&sh)[kQRows],
+      auto member_of = [&](int g, uint32_t meta, int m, int &o, uint32_t &de) {
+        const int o_first = (int)(meta & 0xffu);
+        const uint32_t stride = meta >> 16;
+        o = stride != 0u ? o_first + m : tab.member[tab.group_begin[g] + m];
+        de = stride != 0u ? (uint32_t)m * stride : (uint32_t)(tab.off[o][last] - tab.off[o_first][last]);   // sh + de < 32
+      };
+      // The same for the thread's rows together, where a member at a time is looked at: a map's entries of two rows
+      // are one store.
+      auto found_by_member = [&](int g, uint32_t meta, const uint32_t (&mask)[kQRows], const uint32_t (&sh)[kQRows],
                                  const uint32_t (&slot)[kQRows]) {
-        const uint32_t meta = s_gmeta[g], o_first = meta & 0xffu;
-        const int members = (int)((meta >> 8) & 0xffu), mb = tab.group_begin[g], e_first = tab.off[o_first][last];
+        const int members = (int)((meta >> 8) & 0xffu);
         int32_t first[kQRows];
 #pragma unroll
         for (int j = 0; j < kQRows; j++) first[j] = kPos ? (int32_t)(lo + s_hpos[slot[j]]) : 0;
         for (int m = 0; m < members; m++) {
-          const bool compact = (meta >> 16) != 0u;
-          const int o = compact ? (int)o_first + m : tab.member[mb + m];
-          const uint32_t de = (uint32_t)(compact ? m : tab.off[o][last] - e_first);
+          int o;
+          uint32_t de;
+          member_of(g, meta, m, o, de);
           int32_t idx[kQRows];
 #pragma unroll
           for (int j = 0; j < kQRows; j++) {
@@ -425,6 +420,28 @@ search_kernel(const __grid_constant__ SearchPair sp) {
 #pragma unroll
               for (int j = 0; j < kQRows; j++) if (live[j]) dst[j] = idx[j];
             }
+          }
+        }
+      };
+      // and for one row whose lookup was put off: its offsets have found nothing so far
+      auto found_late = [&](int j, int g, uint32_t mask, uint32_t sh, uint32_t slot) {
+        const uint32_t meta = s_gmeta[g];
+        if (kMode != kMap && (meta >> 16) == 1u) {
+          found_strip(j, meta, mask, sh, slot);
+          return;
+        }
+        const int members = (int)((meta >> 8) & 0xffu);
+        for (int m = 0; m < members; m++) {
+          int o;
+          uint32_t de;
+          member_of(g, meta, m, o, de);
+          if ((mask >> (sh + de) & 1u) == 0u) continue;
+          const int32_t idx = kPos ? (int32_t)(lo + s_hpos[slot] + __popc(mask & ((1u << (sh + de)) - 1u))) : 0;
+          if (kMode == kMap) {
+            if (live[j]) a.kernel_map[(int64_t)o * a.n_rows + row0 + j] = idx;
+          } else {
+            bits[j] |= 1u << o;
+            if (kMode == kBitsRev) atomicOr(a.table_words + idx, 1u << o);
           }
         }
       };
@@ -448,11 +465,12 @@ search_kernel(const __grid_constant__ SearchPair sp) {
             if (v.x != c && !second && v.z != kHashEmpty) open[j] |= 1u << (g - g0);
             slot[j] += second ? 1u : 0u;
           }
-          if (kMode == kMap || (s_gmeta[g] >> 16) == 0u) {
-            found_by_member(g, mask, sh, slot);
+          const uint32_t meta = s_gmeta[g];
+          if (kMode == kMap || (meta >> 16) != 1u) {
+            found_by_member(g, meta, mask, sh, slot);
           } else {
 #pragma unroll
-            for (int j = 0; j < kQRows; j++) found(j, g, mask[j], sh[j], slot[j]);
+            for (int j = 0; j < kQRows; j++) found_strip(j, meta, mask[j], sh[j], slot[j]);
           }
         }
 #pragma unroll
@@ -467,7 +485,7 @@ search_kernel(const __grid_constant__ SearchPair sp) {
               slot = (slot + 1u) & (kQSlots - 1);
               v = s_slots[slot];
             } while (v.x != c && v.x != kHashEmpty && ++probe < kQSlots);
-            if (v.x == c) found(j, g, v.y, q - c * cells.step, slot);
+            if (v.x == c) found_late(j, g, v.y, q - c * cells.step, slot);
           }
         }
       }

@@ -75,6 +75,7 @@ struct ImArgs {
   int64_t T;
   int64_t pitch;              // of the neighbour table: T rounded up to 128
   int32_t K, N, n_pad, k_blocks, stages, a_bytes, stage_bytes, elem_is_bf16, num_tiles, relu;
+  int32_t claims;                               // more tiles than CTAs that run at once: they are handed out
   int32_t wide;        // rows of the output and the residual start on 32-byte boundaries
   int32_t acc_bufs;    // accumulator sets in TMEM (2 when 2 * sub * n_pad <= 512, else 1)
   int32_t n_tiles128;  // entries of tile_bits
@@ -241,8 +242,9 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
   }
   wait_for_predecessor();
   // the first tile's offset bits, on their way while the rest is set up
+  const int own_tile = args.num_tiles - 1 - (int)blockIdx.x;
   uint32_t raw[kSub];
-  if (warp == kIdxWarp) request_bits<kSub, kMode>(args, args.num_tiles - 1 - (int)blockIdx.x, raw);
+  if (warp == kIdxWarp) request_bits<kSub, kMode>(args, own_tile, raw);
   if (!kPairs && (args.scale != nullptr || args.shift != nullptr)) {
     for (int c = threadIdx.x; c < args.n_pad; c += kImThreads) {
       s_scale[c] = args.scale != nullptr && c < args.N ? __ldg(args.scale + c) : 1.f;
@@ -262,18 +264,25 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
   const uint32_t tmem_base = s_tmem_base;
   volatile int *abort_flag = &s_abort;
   // The next of this CTA's tiles and its offset bits, for the warps of the roles that follow them (-1: no more).
-  int tile_slot = 0;
-  uint32_t tile_phase = 0;
+  // The first is the block's own, which every role knows by itself; `turn` counts the others.
+  uint32_t turn = 0;
   auto next_tile = [&](int &tile, uint32_t (&hb)[kSub]) {
-    if (!mbar_wait_warp(false, &bar_tile_full[tile_slot], tile_phase, abort_flag, args.status)) return false;
-    tile = s_tile[tile_slot];
+    const uint32_t slot = turn % kTileSlots, phase = turn / kTileSlots & 1u;
+    turn++;
+    if (args.claims == 0) {
+      tile = -1;
+#pragma unroll
+      for (int h = 0; h < kSub; h++) hb[h] = 0u;
+      return true;
+    }
+    if (!mbar_wait_warp(false, &bar_tile_full[slot], phase, abort_flag, args.status)) return false;
+    tile = s_tile[slot];
     uint32_t seen = (uint32_t)tile;
 #pragma unroll
-    for (int h = 0; h < kSub; h++) { hb[h] = s_tile_bits[tile_slot][h]; seen |= hb[h]; }
+    for (int h = 0; h < kSub; h++) { hb[h] = s_tile_bits[slot][h]; seen |= hb[h]; }
     __syncwarp();
     // (the loads have returned: the arrival's address depends on them, see the producers)
-    if (lane == 0) mbar_arrive(&bar_tile_empty[tile_slot] + (seen & (uint32_t)args.zero));
-    if (++tile_slot == kTileSlots) { tile_slot = 0; tile_phase ^= 1u; }
+    if (lane == 0) mbar_arrive(&bar_tile_empty[slot] + (seen & (uint32_t)args.zero));
     return true;
   };
 
@@ -378,9 +387,11 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
     uint32_t phase = 0, acc_phase = 0;
     bool alive = true;
     bool ready = mbar_test(&bar_full[0], 0u);
-    int tile;
+    int tile = own_tile;
     uint32_t hb[kSub];
-    while (alive && next_tile(tile, hb) && tile >= 0) {
+    request_bits<kSub, kMode>(args, tile, hb);
+    take_bits<kSub>(args, tile, hb, hb);
+    while (alive && tile >= 0) {
       uint32_t rest = union_of<kSub>(hb);
       if (!mbar_wait_warp(false, &bar_acc_empty[acc], acc_phase ^ 1u, abort_flag, args.status)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -419,6 +430,7 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
       if (!alive) break;
       if (elect_one()) umma_commit(&bar_acc_full[acc]);
       if (++acc == args.acc_bufs) { acc = 0; acc_phase ^= 1u; }
+      alive = next_tile(tile, hb);
     }
   } else if (warp == kTmaWarp) {
     // ------------------------------ weight tiles -------------------------------
@@ -428,9 +440,11 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
     int stage = 0;
     uint32_t phase = 0;
     bool ready = mbar_test(&bar_empty[0], 1u);
-    int tile;
+    int tile = own_tile;
     uint32_t hb[kSub];
-    while (alive && next_tile(tile, hb) && tile >= 0) {
+    request_bits<kSub, kMode>(args, tile, hb);
+    take_bits<kSub>(args, tile, hb, hb);
+    while (alive && tile >= 0) {
       uint32_t rest = union_of<kSub>(hb);
       const int pair_row = kPairs ? pair_row_of_tile(args, tile) : 0;
       while (alive && rest != 0u) {
@@ -456,6 +470,7 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
           __syncwarp();
         }
       }
+      if (alive) alive = next_tile(tile, hb);
     }
   } else if (warp == kIdxWarp) {
     // ------------------------------ tiles and index blocks ---------------------
@@ -464,7 +479,9 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
     // kTileSlots before its epilogue.  Rows with many and rare offsets sort to the end, so the dear tiles go first.
     // With every gridDim-th tile for a CTA the busiest had 1.2 to 1.7 times the average of steps (one to
     // four clouds).  us, before / now: 406k rows of 3.4 pairs 64->64 70 / 59, 128->128 137 / 110, 256->256 328 /
-    // 271; 1.8M of 9.3 256->256 3090 / 2810; 31k of 16.7 84 / 79; a single tile per CTA 0.1 to 0.3 more.
+    // 271; 1.8M of 9.3 256->256 3090 / 2810; 31k of 16.7 84 / 79.  The block's own tile is nobody's news, and where no
+    // block waits for a place nothing is asked for: small layers had lost 0.2 us to that (20k rows 64->64, one offset, 5.30
+    // dealt out, 5.50 asked for, 5.00 now; 128->128 6.32 / 6.63 / 6.12).
     //
     // 128 entries of the neighbour table per step and sub-tile, up to kIdxSlots steps ahead of the
     // producers, so that they never wait for an index from memory (loaded by the producers
@@ -474,7 +491,7 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
     // 32->32, 1.15 pairs a row, 37.7 / 32.8; 64->64 45 / 42; 406k 64->64, 3.4 pairs, 74.6 / 68; 123k 64->64,
     // 16.7 pairs, 70 / 62; 406k 64->128 90 / 86).
     const uint32_t ring = smem_u32(idx_ring) + (uint32_t)lane * 16u;
-    int tile = args.num_tiles - 1 - (int)blockIdx.x;
+    int tile = own_tile;
     uint32_t phase = 0, claim_phase = 0, publish_phase = 0;
     int publish_slot = 0;
     bool claim_open = false;                       // an answer is on its way
@@ -513,7 +530,7 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
     while (alive) {
       uint32_t hb[kSub];
       take_bits<kSub>(args, tile, raw, hb);
-      alive = publish(hb);
+      if (tile != own_tile) alive = publish(hb);
       if (!alive || tile < 0) break;
       const int32_t *blocks = args.nbr + (int64_t)tile * (kSub * kBM) + lane * 4;
       for (uint32_t rest = kMode == kDense ? 0u : union_of<kSub>(hb); alive && rest != 0u; rest &= rest - 1u) {
@@ -524,6 +541,10 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
         alive = send(blocks + (int64_t)p * args.pitch, has);
       }
       if (!alive) break;
+      if (args.claims == 0) {
+        tile = -1;
+        break;
+      }
       // the next tile, no earlier: a CTA that holds tiles it has not begun keeps them from one that is done
       if (lane == 0) {
         fence_generic_to_async();                  // the answer before has been read
@@ -564,7 +585,8 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
     const int quarter = warp & 3, group = (warp - kEpiWarp) >> 2;
     // two warps of a quarter take alternate pieces, or neighbouring ones where they copy residuals
     constexpr int kStep = kStaged ? 1 : kEpiCols;
-    const int n = args.N, pieces = args.n_pad / 16, share = (pieces + kEpiCols - 1) / kEpiCols;
+    // (residuals are copied at three or four pieces)
+    const int n = args.N, pieces = args.n_pad / 16, share = kStaged && kEpiCols == 2 ? 2 : (pieces + kEpiCols - 1) / kEpiCols;
     const int first_piece = kStaged ? group * share : group;
     const int last_piece = kStaged ? min(pieces, first_piece + share) : pieces;
     const bool affine = args.scale != nullptr || args.shift != nullptr;
@@ -585,10 +607,11 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
       return tile >= 0 && row < args.T ? (permuted ? raw_row : (int32_t)row) : -1;
     };
     int32_t grow[kSub], next_rows[kSub] = {};
-    int tile, next = -1;
+    int tile = own_tile, next = -1;
     uint32_t hb[kSub], next_hb[kSub];
-    if (!next_tile(tile, hb)) tile = -1;
     request_rows(tile, next_rows);
+    request_bits<kSub, kMode>(args, tile, hb);
+    take_bits<kSub>(args, tile, hb, hb);
     // Residuals of 33 to 64 columns come through a ring of this warp's own, one use of it (two pieces) ahead:
     // four lanes copy 64 bytes of a row, where a lane that reads its own row's pieces makes every load
     // 32 lines of 128 bytes.  64->64, us: 464k rows of 1.15 pairs 55.3 -> 48.5, 406k of 3.4 81 -> 76, 298k of 9.3
@@ -768,13 +791,14 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
         if constexpr (kStaged) {
           for (int q0 = first_piece; q0 < last_piece; q0 += 2) {
             __syncwarp();                                     // every lane has read the slot that is filled now
-            const bool same = q0 + 2 < last_piece;
+            const bool same = kEpiCols == 1 && q0 + 2 < last_piece;
             const int32_t row = same ? row_now() : h + 1 < kSub ? grow[kSub - 1] : take_row(next, 0, next_rows[0]);
             stage_residual(res_turn ^ 1u, row, same ? q0 + 2 : first_piece);
             asm volatile("cp.async.wait_group 1;" ::: "memory");
             __syncwarp();
             for (int q = q0; q < min(q0 + 2, last_piece); q++) piece(q);
             res_turn ^= 1u;
+            if (kEpiCols == 2) break;
           }
         } else {
           for (int q = first_piece; q < last_piece; q += kStep) piece(q);
@@ -948,9 +972,11 @@ mn_status launch_implicit(const ImArgs &a, const TcSizing &sizing, const CUtenso
                           const CUtensorMap &map_b, cudaStream_t st) {
   auto kernel = conv_implicit_kernel<kSub, kLpr, kProdWarps, kMode, kStaged>;
   MN_RETURN_IF(allow_max_shared_memory(reinterpret_cast<const void *>(kernel)));
+  ImArgs args = a;
+  args.claims = a.num_tiles > kNumSMs * sizing.ctas_per_sm ? 1 : 0;
   MN_LAUNCH(kMode == kPairRows ? "conv_implicit_kernel<pairs>" : kMode == kDense ? "conv_implicit_kernel<dense>"
                                                                                  : "conv_implicit_kernel", st,
-            launch_early(kernel, (unsigned)a.num_tiles, kImThreads, sizing.smem_bytes, st, a, map_a, map_b));
+            launch_early(kernel, (unsigned)a.num_tiles, kImThreads, sizing.smem_bytes, st, args, map_a, map_b));
   return MN_OK;
 }
 

@@ -45,7 +45,6 @@ namespace {
 using namespace tc;
 
 constexpr int kGatherWarps = 12;       // producer and epilogue warps together: 8 + 4 or 4 + 8
-constexpr int kImThreads = (kGatherWarps + 3) * 32;
 constexpr int kImCtas = 2;             // CTAs per SM the register file allows
 constexpr int kBM = 128;
 constexpr int kBK = 64;
@@ -53,7 +52,7 @@ constexpr int kUmmaK = 16;
 constexpr int kMaxStages = 8;
 constexpr int kMaxN = 256;
 constexpr int kIdxSlots = 8;           // steps the index blocks run ahead
-constexpr int kTileSlots = 4;          // tiles that a CTA holds at most
+constexpr int kTileSlots = 4;          // tiles that a CTA holds at most beside its own (a dense product's two)
 constexpr int kMaxSub = 2;             // 128-row sub-tiles per CTA tile
 constexpr int kResSlot = 32 * 64;      // bytes of 32 columns of 32 rows of the residual
 constexpr int kNBlock = kBK * 128;     // kMapNMajor: bytes of one block of 64 columns of a weight tile
@@ -62,6 +61,8 @@ constexpr int kNBlock = kBK * 128;     // kMapNMajor: bytes of one block of 64 c
 // tiles; the product rows of a pair list; the rows of one dense product (the 1x1x1 convolution),
 // whose tiles TMA fetches whole.
 enum ImMode { kMap = 0, kMapNMajor = 1, kPairRows = 2, kDense = 3 };
+// (one dense product: no rows to gather and no index blocks, so that a producer's place does for the tiles' warp)
+constexpr int threads_of(int mode) { return (kGatherWarps + (mode == kDense ? 2 : 3)) * 32; }
 
 struct ImArgs {
   const uint8_t *in;          // [S, K] 16-bit
@@ -75,7 +76,7 @@ struct ImArgs {
   int64_t T;
   int64_t pitch;              // of the neighbour table: T rounded up to 128
   int32_t K, N, n_pad, k_blocks, stages, a_bytes, stage_bytes, elem_is_bf16, num_tiles, relu;
-  int32_t claims;                               // more tiles than CTAs that run at once: they are handed out
+  int32_t claims;             // tiles are handed out; 0: every gridDim-th is a CTA's
   int32_t wide;        // rows of the output and the residual start on 32-byte boundaries
   int32_t acc_bufs;    // accumulator sets in TMEM (2 when 2 * sub * n_pad <= 512, else 1)
   int32_t n_tiles128;  // entries of tile_bits
@@ -198,13 +199,14 @@ __device__ __forceinline__ uint32_t union_of(const uint32_t (&hb)[kSub]) {
 // per copy); kProdWarps: 4 producer and 8 epilogue warps or 8 and 4; kStaged: the epilogue's
 // residual comes through shared memory.
 template <int kSub, int kLpr, int kProdWarps, int kMode, bool kStaged>
-__global__ void __launch_bounds__(kImThreads, kImCtas)
+__global__ void __launch_bounds__(threads_of(kMode), kImCtas)
 conv_implicit_kernel(const __grid_constant__ ImArgs args,
                      const __grid_constant__ CUtensorMap map_a,     // kDense: features [S, K]
                      const __grid_constant__ CUtensorMap map_b) {   // weights^T [O, N, K]; kMapNMajor: weights [O, K, N]
   constexpr bool kPairs = kMode == kPairRows, kNMajor = kMode == kMapNMajor;
   constexpr int kProdRows = 128 / kProdWarps;               // rows of a sub-tile per producer warp
-  constexpr int kMmaWarp = kProdWarps, kTmaWarp = kProdWarps + 1, kIdxWarp = kProdWarps + 2, kEpiWarp = kProdWarps + 3;
+  constexpr int kMmaWarp = kProdWarps, kTmaWarp = kProdWarps + 1, kIdxWarp = kMode == kDense ? 0 : kProdWarps + 2;
+  constexpr int kEpiWarp = threads_of(kMode) / 32 - (kGatherWarps - kProdWarps), kSlots = kMode == kDense ? 2 : kTileSlots;
   constexpr int kEpiCols = (kGatherWarps - kProdWarps) / 4;   // epilogue warps per quarter of the rows
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   __shared__ uint64_t bar_full[kMaxStages], bar_empty[kMaxStages];
@@ -233,20 +235,23 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
       mbar_init(&bar_empty[s], 1);
     }
     for (int a = 0; a < 2; a++) { mbar_init(&bar_acc_full[a], 1); mbar_init(&bar_acc_empty[a], 4 * kEpiCols); }
-    for (int i = 0; i < kIdxSlots; i++) { mbar_init(&bar_idx_full[i], 33); mbar_init(&bar_idx_empty[i], kProdWarps * 32); }
-    // read by the weight warp, the MMA warp and the epilogue warps
-    for (int i = 0; i < kTileSlots; i++) { mbar_init(&bar_tile_full[i], 1); mbar_init(&bar_tile_empty[i], 2 + 4 * kEpiCols); }
-    mbar_init(&bar_claim, 1);
+    if (kMode != kDense)
+      for (int i = 0; i < kIdxSlots; i++) { mbar_init(&bar_idx_full[i], 33); mbar_init(&bar_idx_empty[i], kProdWarps * 32); }
+    if (args.claims != 0) {
+      // read by the weight warp, the MMA warp and the epilogue warps
+      for (int i = 0; i < kTileSlots; i++) { mbar_init(&bar_tile_full[i], 1); mbar_init(&bar_tile_empty[i], 2 + 4 * kEpiCols); }
+      mbar_init(&bar_claim, 1);
+    }
     s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   wait_for_predecessor();
   // the first tile's offset bits, on their way while the rest is set up
-  const int own_tile = args.num_tiles - 1 - (int)blockIdx.x;
+  const int own_tile = args.num_tiles - 1 - (int)blockIdx.x;      // (the grid has no more blocks than tiles)
   uint32_t raw[kSub];
   if (warp == kIdxWarp) request_bits<kSub, kMode>(args, own_tile, raw);
   if (!kPairs && (args.scale != nullptr || args.shift != nullptr)) {
-    for (int c = threadIdx.x; c < args.n_pad; c += kImThreads) {
+    for (int c = threadIdx.x; c < args.n_pad; c += threads_of(kMode)) {
       s_scale[c] = args.scale != nullptr && c < args.N ? __ldg(args.scale + c) : 1.f;
       s_shift[c] = args.shift != nullptr && c < args.N ? __ldg(args.shift + c) : 0.f;
     }
@@ -263,16 +268,16 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
   release_successor();   // every block has its tensor memory before another kernel's block can ask for some
   const uint32_t tmem_base = s_tmem_base;
   volatile int *abort_flag = &s_abort;
-  // The next of this CTA's tiles and its offset bits, for the warps of the roles that follow them (-1: no more).
+  // This CTA's tile after `tile` and its offset bits, for the warps of the roles that follow them (-1: no more).
   // The first is the block's own, which every role knows by itself; `turn` counts the others.
   uint32_t turn = 0;
   auto next_tile = [&](int &tile, uint32_t (&hb)[kSub]) {
-    const uint32_t slot = turn % kTileSlots, phase = turn / kTileSlots & 1u;
+    const uint32_t slot = turn % kSlots, phase = turn / kSlots & 1u;
     turn++;
     if (args.claims == 0) {
-      tile = -1;
+      tile = kMode > kMapNMajor ? max(tile - (int)gridDim.x, -1) : -1;   // (a map's grid has all its tiles then)
 #pragma unroll
-      for (int h = 0; h < kSub; h++) hb[h] = 0u;
+      for (int h = 0; h < kSub; h++) hb[h] = kMode > kMapNMajor ? 1u : 0u;
       return true;
     }
     if (!mbar_wait_warp(false, &bar_tile_full[slot], phase, abort_flag, args.status)) return false;
@@ -286,7 +291,7 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
     return true;
   };
 
-  if (warp < kProdWarps) {
+  if (kMode != kDense && warp < kProdWarps) {
     // ------------------------------ producers ---------------------------------
     // Lane l of warp w copies 16-byte piece l % kLpr of rows r0 .. r0 + kRpl - 1 of every
     // sub-tile, r0 = 16 w + kRpl (l / kLpr): the lane's indices are consecutive in the index
@@ -306,7 +311,7 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
     uint32_t phase = 0, slot_phase = 0;
     bool alive = true;
     bool ready = mbar_test(&bar_empty[0], 1u), indices = false;
-    while (kMode != kDense && alive) {
+    while (alive) {
       if (!indices && !mbar_wait(&bar_idx_full[slot], slot_phase, abort_flag, args.status)) break;
       const uint32_t has = s_idx_has[slot];        // sub-tiles that have this offset; 0: no more steps
       int32_t q[kSub][kRpl];
@@ -476,7 +481,7 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
     // ------------------------------ tiles and index blocks ---------------------
     // Tiles are handed out while the kernel runs: a CTA starts with the tile of its own number, counted from the last,
     // and takes over the tiles of blocks that have not started (cluster launch control) as it needs them, at most
-    // kTileSlots before its epilogue.  Rows with many and rare offsets sort to the end, so the dear tiles go first.
+    // kSlots before its epilogue.  Rows with many and rare offsets sort to the end, so the dear tiles go first.
     // With every gridDim-th tile for a CTA the busiest had 1.2 to 1.7 times the average of steps (one to
     // four clouds).  us, before / now: 406k rows of 3.4 pairs 64->64 70 / 59, 128->128 137 / 110, 256->256 328 /
     // 271; 1.8M of 9.3 256->256 3090 / 2810; 31k of 16.7 84 / 79.  The block's own tile is nobody's news, and where no
@@ -504,7 +509,7 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
         mbar_arrive(&bar_tile_full[publish_slot]);
       }
       __syncwarp();
-      if (++publish_slot == kTileSlots) { publish_slot = 0; publish_phase ^= 1u; }
+      if (++publish_slot == kSlots) { publish_slot = 0; publish_phase ^= 1u; }
       return true;
     };
     int slot = 0;
@@ -530,7 +535,7 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
     while (alive) {
       uint32_t hb[kSub];
       take_bits<kSub>(args, tile, raw, hb);
-      if (tile != own_tile) alive = publish(hb);
+      if (args.claims != 0 && tile != own_tile) alive = publish(hb);
       if (!alive || tile < 0) break;
       const int32_t *blocks = args.nbr + (int64_t)tile * (kSub * kBM) + lane * 4;
       for (uint32_t rest = kMode == kDense ? 0u : union_of<kSub>(hb); alive && rest != 0u; rest &= rest - 1u) {
@@ -542,8 +547,9 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
       }
       if (!alive) break;
       if (args.claims == 0) {
-        tile = -1;
-        break;
+        tile = kPairs ? max(tile - (int)gridDim.x, -1) : -1;
+        if (tile < 0) break;
+        continue;
       }
       // the next tile, no earlier: a CTA that holds tiles it has not begun keeps them from one that is done
       if (lane == 0) {
@@ -566,7 +572,7 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
       for (uint32_t spin = 0; spin < 4096u && !mbar_try_wait(&bar_claim, claim_phase); spin++) {}
     }
     asm volatile("cp.async.wait_all;" ::: "memory");   // nothing of this lane is in flight at exit
-  } else {
+  } else if (warp >= kEpiWarp) {
     // ------------------------------ epilogue ----------------------------------
     // A lane owns one accumulator row and takes it 16 columns at a time: one 32-byte store
     // (a whole sector of the output row, wherever perm puts it) and, with a residual, one
@@ -607,7 +613,7 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
       return tile >= 0 && row < args.T ? (permuted ? raw_row : (int32_t)row) : -1;
     };
     int32_t grow[kSub], next_rows[kSub] = {};
-    int tile = own_tile, next = -1;
+    int tile = own_tile, next = own_tile;
     uint32_t hb[kSub], next_hb[kSub];
     request_rows(tile, next_rows);
     request_bits<kSub, kMode>(args, tile, hb);
@@ -973,10 +979,20 @@ mn_status launch_implicit(const ImArgs &a, const TcSizing &sizing, const CUtenso
   auto kernel = conv_implicit_kernel<kSub, kLpr, kProdWarps, kMode, kStaged>;
   MN_RETURN_IF(allow_max_shared_memory(reinterpret_cast<const void *>(kernel)));
   ImArgs args = a;
-  args.claims = a.num_tiles > kNumSMs * sizing.ctas_per_sm ? 1 : 0;
+  const int at_once = kNumSMs * sizing.ctas_per_sm;
+  // Tiles of one offset cost the same and are dealt out up to some ten a CTA, with one CTA an SM always; narrow rows are
+  // handed out.  1x1x1 layers, us, dealt out / handed out: 64->64 120k rows 7.3 / 8.2, 320k 13.6 / 15.7, 460k 21.3 / 21.0,
+  // 1.5 M 70 / 58, with a residual 240k 19.0 / 19.5, 320k 28.0 / 26.6; 64->20 460k 13.5 / 14.8, with one 17.1 / 18.4, 700k
+  // 25.0 / 21.4; 256->256 700k 141 / 147; 32->32 120k 7.2 / 7.1, 460k 19.3 / 17.8.  Pair products 32->32 103 / 105 (2184
+  // tiles), 729 / 720 (30 754).
+  int64_t dealt = 1;
+  if (kMode > kMapNMajor && (kMode == kPairRows || a.K > 32))
+    dealt = sizing.ctas_per_sm == 1 ? a.num_tiles : a.residual == nullptr || a.n_pad <= 32 ? 13 : 8;
+  args.claims = a.num_tiles > dealt * at_once ? 1 : 0;
+  const int grid = args.claims != 0 ? a.num_tiles : std::min(a.num_tiles, at_once);
   MN_LAUNCH(kMode == kPairRows ? "conv_implicit_kernel<pairs>" : kMode == kDense ? "conv_implicit_kernel<dense>"
                                                                                  : "conv_implicit_kernel", st,
-            launch_early(kernel, (unsigned)a.num_tiles, kImThreads, sizing.smem_bytes, st, args, map_a, map_b));
+            launch_early(kernel, (unsigned)grid, threads_of(kMode), sizing.smem_bytes, st, args, map_a, map_b));
   return MN_OK;
 }
 

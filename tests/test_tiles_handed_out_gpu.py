@@ -45,14 +45,17 @@ def test_tiles_of_one_layer(c_in, c_out, sub_tiles, residual, per_cta):
     assert torch.equal(got.float(), want + skip.float() if residual else want)
 
 
-@pytest.mark.parametrize("rows", [100, 128, 37_888, 37_889, 75_776, 75_777, 400_001])
-def test_tiles_of_a_dense_layer(rows):
+@pytest.mark.parametrize("c_in,c_out", [(24, 64), (72, 64), (72, 20), (64, 256)])
+@pytest.mark.parametrize("rows", [100, 128, 18_945, 37_888, 37_889, 75_777, 303_104, 303_105, 600_001])
+def test_tiles_of_a_dense_layer(rows, c_in, c_out):
+    """1x1x1 layers: dealt out or handed out, by their tiles and widths."""
     gen = torch.Generator(device=DEV).manual_seed(rows)
-    x = torch.randint(-2, 3, (rows, 72), generator=gen, device=DEV).half()
-    w = torch.randint(-1, 2, (72, 64), generator=gen, device=DEV).half()
-    skip = torch.randint(-8, 9, (rows, 64), generator=gen, device=DEV).half()
-    got = F.dense_forward(x, w, residual=skip)
-    assert torch.equal(got.float(), x.float() @ w.float() + skip.float())
+    x = torch.randint(-2, 3, (rows, c_in), generator=gen, device=DEV).half()
+    w = torch.randint(-1, 2, (c_in, c_out), generator=gen, device=DEV).half()
+    skip = torch.randint(-8, 9, (rows, c_out), generator=gen, device=DEV).half()
+    want = x.float() @ w.float()
+    assert torch.equal(F.dense_forward(x, w).float(), want)
+    assert torch.equal(F.dense_forward(x, w, residual=skip).float(), want + skip.float())
 
 
 def test_two_layers_at_once():

@@ -1229,24 +1229,25 @@ extern "C" mn_status mn_sparse_convolution_forward_implicit(
   // Sub-tiles per CTA tile.  The two sub-tiles of a CTA tile share the steps' bookkeeping and the weight
   // tile of a stage, at the price of a shallower ring, fewer epilogue warps and tiles twice as large; a sub-tile
   // is skipped in the steps of offsets that only the other one has.  It pays where the bookkeeping
-  // bounds a step and every CTA has several tiles (us, 1 / 2 sub-tiles).  32->32: 21.4k tiles of 1.15 pairs a
-  // row 145 / 110, 3.5k of 1.6 39 / 38, 0.9k 19 / 23.  64->64: 13.9k tiles of 9.3 pairs 570 / 541, 2.6k of 7
-  // 78 / 74, 3.2k of 3.4 70 / 72, 21.4k of 1.15 152 / 161.  More channels: 128->64 821 / 834, 64->128 472 /
-  // 512 (18.8k tiles), 128->128 1059 / 1100, 136 / 147 (3.2k), 57 / 62 (0.8k), 176 / 171 (2.3k of 9.3 pairs),
-  // 256->256 336 / 404.  All that is one layer at a time on a GPU that keeps its clocks.  A network on a large
-  // batch runs at the power limit, and weights read and written once for both sub-tiles are energy saved:
-  // with two at 128 columns a forward pass of 64 clouds takes 76.4 instead of 78.5 ms.  Callers that have timed
-  // the layer pass their own choice.
+  // bounds a step and every CTA has several tiles.  us, 1 / 2 sub-tiles, of one layer at a time (14k tiles and more: at the
+  // power limit, near 1.5 GHz).  32->32: 938 tiles of 1.15 pairs a row 10.6 / 15.2, 2026 of 1.1 15.2 / 16.7, 1849 of 5.4
+  // 40.3 / 37.7, 3629 of 1.15 22.4 / 20.8, 57k of 1.15 279 / 226.  64->64: 3176 of 3.5 49.0 / 49.4, with a residual 54.6 /
+  // 57.7, 5456 of 5.4 153 / 145, 57k of 1.15 365 / 332, with one 447 / 462, 37k of 9.3 1077 / 982.  Beyond 64 columns few
+  // pairs leave the epilogue as the bound, which has half the warps with two.  64->128: 57k of 1.15 537 / 758, 50k of 3.4
+  // 1033 / 1111, 5456 of 5.4 189 / 182, 9257 of 9.3 345 / 327, 878 of 12.6 39.8 / 40.3, with a residual 49.5 / 53.8.  128->128:
+  // 12.6k of 3.5 416 / 415, with one 592 / 612, 10.1k of 7.5 541 / 527 and 683 / 638, 2331 of 9.3 153 / 148, 1083 of 7.2
+  // 58.7 / 59.3.  More input channels are more steps a tile: 256->128 12.6k of 3.5 775 / 723, 26.8k of 3.0 1225 / 1262.
+  // 128->64 0.96 to 1.04, 256->256 336 / 404.  Callers that have timed the layer pass their own choice.
   int sub = sub_hint;
   if (sub <= 0) {
     const double tiles = a.n_tiles128;
     sub = 1;
     if (c_in <= 32 && a.n_pad <= 32) {
-      if (tiles >= 32 * kNumSMs) sub = 2;
+      if (tiles >= 24 * kNumSMs) sub = 2;
     } else if (c_in <= 64 && a.n_pad <= 64) {
       if (pairs_per_row >= 3.0 && tiles >= 16 * kNumSMs && tiles * pairs_per_row >= 16384) sub = 2;
     } else if (a.n_pad > 64 && a.n_pad <= 128) {
-      if (pairs_per_row >= 2.0 && tiles >= 32 * kNumSMs) sub = 2;
+      if (pairs_per_row >= (c_in > 128 ? 3.2 : 5.0) && tiles >= 16 * kNumSMs) sub = 2;
     }
   }
   MN_CHECK_ARG(sub_hint <= 4 && (sub_hint <= 0 || sub_hint * a.n_pad <= 512),

@@ -333,21 +333,23 @@ sort_pass_kernel(const __grid_constant__ Args a, int pass) {
 
 // Threads and keys per thread of a tile, and its blocks per SM.  Every tile that runs at the same time lengthens
 // the look-back, so tiles are large: 4096 keys, with 512 threads up to two tiles per SM and with 256 beyond,
-// three to an SM (80 registers; at 128 registers and two, 7.3 M keys took 7 % longer) while that is one wave.  Four
-// to an SM (64 registers, 8 bytes spilled) pay once there are more tiles than one wave, and tiles of 3072
-// keys where the second wave would be small.  Up to one tile of 1024 keys per SM a pass is shorter with
+// three to an SM (80 registers; at 128 registers and two, 7.3 M keys took 7 % longer) while that is one wave and a hundredth
+// (the few tiles over start as soon as others end).  Four to an SM (64 registers, 8 bytes spilled, 28 with an index array)
+// pay beyond, and tiles of 3072 keys where the second wave would be small.  Up to one tile of 1024 keys per SM a pass is shorter with
 // those; beyond, up to 606k keys, the large ones leave SMs without a tile and are faster all the same.  Measured,
 // all passes, us for 256 x 4 / 512 x 8 / 256 x 16: 30k keys 29 / 37 / 39; 120k 45 / 51 / 53; 250k 64 / 59 / 62;
 // 464k 80 / 74 / 78; 900k 115 / 94 / 100; 1.9 M 184 / 141 / 127; 7.3 M 755 / 491 / 445.  36 bits, 256 x 16 with three
 // / with four blocks / 256 x 12 with four: 1.5 M 129 / 150 / 132; 1.9 M 147 / 157 / 140; 2.1 M 165 / 159 / 156;
-// 2.4 M 188 / 164 / 182; 7.3 M 417 / 390 / 406.
+// 2.4 M 188 / 164 / 182; 7.3 M 417 / 390 / 406.  At the line, 256 x 16 with three / 256 x 12 with four, 42 bits: 1.83 M 167 / 173,
+// 1.85 M 170 / 175, 1.87 M 175 / 173; 63 bits and an index array: 1.82 M 254 / 261, 1.85 M 266 / 259, 1.91 M 292 / 266; past the
+// small second wave 256 x 16 with three / with four, an index array: 2.4 M 373 / 317, 3.5 M 442 / 442, 7.3 M 826 / 782.
 struct TileShape { int threads, items, blocks; };
 constexpr int64_t kFewKeys = 1024ll * kNumSMs;
-constexpr int64_t kOneWave = 3 * 4096ll * kNumSMs, kSmallSecondWave = kOneWave + kOneWave / 5;
+constexpr int64_t kOneWave = 3 * 4096ll * kNumSMs, kHardlyTwo = kOneWave + kOneWave / 100, kSmallSecondWave = kOneWave + kOneWave / 5;
 inline TileShape tile_shape(int64_t n) {
   if (n < kFewKeys) return TileShape{256, 4, 4};
   if (n < 2 * 4096ll * kNumSMs) return TileShape{512, 8, 2};
-  if (n <= kOneWave) return TileShape{256, 16, 3};
+  if (n <= kHardlyTwo) return TileShape{256, 16, 3};
   return n <= kSmallSecondWave ? TileShape{256, 12, 4} : TileShape{256, 16, 4};
 }
 inline int64_t tiles_of(int64_t n) {

@@ -554,8 +554,9 @@ class SparseConv(Module):
             # training: the plain product, differentiated by autograd (the weight's gradient of many rows by a
             # kernel of this library)
             weight = self.kernel.view(self.in_channels, self.out_channels)
-            if _plain(features, self.kernel) and features.is_cuda and \
-                    _lib.host().dense_product_takes(features, weight):
+            # (the rows first: few of them are never taken, and the questions cost as much as the launch)
+            if features.dim() == 2 and features.size(0) >= 1024 and features.is_cuda and \
+                    _plain(features, self.kernel) and _lib.host().dense_product_takes(features, weight):
                 out = _lib.host().dense_product(features, weight)
             else:
                 out = features @ weight

@@ -23,8 +23,8 @@
 // before, bounds looked for near the tile where the rows are the table) and 13 000 (strips that lie in one cell,
 // keys of 32 bits, the few longer probes of a warp in one loop at the end).  464k rows, four
 // maps: 138 -> 99 us of searches; 7.3 million, two maps: 634 -> 534 us.  Keys in two cells cost what they save where few and
-// long groups ask (build of 1 x 1 x 5 dilated by 7, 464k rows: 31 -> 33 us; 3 x 3 x 3 dilated by 4 77 -> 75, 50k uniform rows
-// 10 % more).  Lanes that add up their bits of a cell before one inserts it: 0.9 of the time on full grids,
+// long groups ask (build of 1 x 1 x 5 dilated by 7, 464k rows: 31.0 -> 31.9 us; 3 x 3 x 3 dilated by 4 77 -> 72, 50k uniform
+// rows 6 % more).  Lanes that add up their bits of a cell before one inserts it: 0.9 of the time on full grids,
 // 1.04 on scans, not kept.  Tiles whose window does not fit the hash are
 // processed group range by group range, and ranges that still do not fit fall
 // back to binary search in global memory.  The kernel writes kernel-map rows
@@ -391,13 +391,15 @@ search_kernel(const __grid_constant__ SearchPair sp) {
         de = stride != 0u ? (uint32_t)m * stride : (uint32_t)(tab.off[o][last] - tab.off[o_first][last]);   // sh + de < 32
       };
       // The same for the thread's rows together, where a member at a time is looked at: a map's entries of two rows
-      // are one store.
+      // are one store.  (Not unrolled: beside it the strips, which most maps are made of, lost 3 %: 7.3 M rows 3 x 3 x 3, build,
+      // 636 -> 618 us; dilated by 4 841 -> 786.)
       auto found_by_member = [&](int g, uint32_t meta, const uint32_t (&mask)[kQRows], const uint32_t (&sh)[kQRows],
                                  const uint32_t (&slot)[kQRows]) {
         const int members = (int)((meta >> 8) & 0xffu);
         int32_t first[kQRows];
 #pragma unroll
         for (int j = 0; j < kQRows; j++) first[j] = kPos ? (int32_t)(lo + s_hpos[slot[j]]) : 0;
+#pragma unroll 1
         for (int m = 0; m < members; m++) {
           int o;
           uint32_t de;
@@ -431,6 +433,7 @@ search_kernel(const __grid_constant__ SearchPair sp) {
           return;
         }
         const int members = (int)((meta >> 8) & 0xffu);
+#pragma unroll 1
         for (int m = 0; m < members; m++) {
           int o;
           uint32_t de;

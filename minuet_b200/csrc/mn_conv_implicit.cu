@@ -52,7 +52,7 @@ constexpr int kUmmaK = 16;
 constexpr int kMaxStages = 8;
 constexpr int kMaxN = 256;
 constexpr int kIdxSlots = 8;           // steps the index blocks run ahead
-constexpr int kTileSlots = 4;          // tiles that a CTA holds at most beside its own (a dense product's two)
+constexpr int kTileSlots = 2;          // tiles that a CTA holds at most beside the one it works on (see the index warp)
 constexpr int kMaxSub = 2;             // 128-row sub-tiles per CTA tile
 constexpr int kResSlot = 32 * 64;      // bytes of 32 columns of 32 rows of the residual
 constexpr int kNBlock = kBK * 128;     // kMapNMajor: bytes of one block of 64 columns of a weight tile
@@ -206,7 +206,7 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
   constexpr bool kPairs = kMode == kPairRows, kNMajor = kMode == kMapNMajor;
   constexpr int kProdRows = 128 / kProdWarps;               // rows of a sub-tile per producer warp
   constexpr int kMmaWarp = kProdWarps, kTmaWarp = kProdWarps + 1, kIdxWarp = kMode == kDense ? 0 : kProdWarps + 2;
-  constexpr int kEpiWarp = threads_of(kMode) / 32 - (kGatherWarps - kProdWarps), kSlots = kMode == kDense ? 2 : kTileSlots;
+  constexpr int kEpiWarp = threads_of(kMode) / 32 - (kGatherWarps - kProdWarps);
   constexpr int kEpiCols = (kGatherWarps - kProdWarps) / 4;   // epilogue warps per quarter of the rows
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   __shared__ uint64_t bar_full[kMaxStages], bar_empty[kMaxStages];
@@ -272,7 +272,7 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
   // The first is the block's own, which every role knows by itself; `turn` counts the others.
   uint32_t turn = 0;
   auto next_tile = [&](int &tile, uint32_t (&hb)[kSub]) {
-    const uint32_t slot = turn % kSlots, phase = turn / kSlots & 1u;
+    const uint32_t slot = turn % kTileSlots, phase = turn / kTileSlots & 1u;
     turn++;
     if (args.claims == 0) {
       tile = kMode > kMapNMajor ? max(tile - (int)gridDim.x, -1) : -1;   // (a map's grid has all its tiles then)
@@ -481,7 +481,8 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
     // ------------------------------ tiles and index blocks ---------------------
     // Tiles are handed out while the kernel runs: a CTA starts with the tile of its own number, counted from the last,
     // and takes over the tiles of blocks that have not started (cluster launch control) as it needs them, at most
-    // kSlots before its epilogue.  Rows with many and rare offsets sort to the end, so the dear tiles go first.
+    // kTileSlots before its epilogue (with four the last CTAs had tiles left when others had none: 464k rows 64->64 of 1.15
+    // pairs with a residual 35.8 / 34.4, 406k 128->128 of 3.5 136 / 128).  Rows with many and rare offsets sort to the end, so the dear tiles go first.
     // With every gridDim-th tile for a CTA the busiest had 1.2 to 1.7 times the average of steps (one to
     // four clouds).  us, before / now: 406k rows of 3.4 pairs 64->64 70 / 59, 128->128 137 / 110, 256->256 328 /
     // 271; 1.8M of 9.3 256->256 3090 / 2810; 31k of 16.7 84 / 79.  The block's own tile is nobody's news, and where no
@@ -509,7 +510,7 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
         mbar_arrive(&bar_tile_full[publish_slot]);
       }
       __syncwarp();
-      if (++publish_slot == kSlots) { publish_slot = 0; publish_phase ^= 1u; }
+      if (++publish_slot == kTileSlots) { publish_slot = 0; publish_phase ^= 1u; }
       return true;
     };
     int slot = 0;

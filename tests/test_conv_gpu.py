@@ -413,12 +413,12 @@ def _dense_batch(seed, clouds=2, draws=50_000, extent=72):
     return synth.random_small_batch(rng, clouds, draws, extent)
 
 
-@pytest.mark.parametrize("algorithm,sub_tiles", [("implicit", 0), ("implicit", 1), ("implicit", 2), ("explicit", 0)])
+@pytest.mark.parametrize("algorithm", ["implicit", "explicit"])
 @pytest.mark.parametrize("c_in,c_out", [(64, 64), (128, 256), (32, 128)])
-def test_benchmark_size_tiles_with_full_epilogue(oracle_lib, algorithm, sub_tiles, c_in, c_out):
-    """More than 75 776 targets through the fused kernel with one and two 128-row
-    sub-tiles per CTA tile, whichever the rule picks, with two accumulator sets in TMEM (C_out = 64,
-    128) and with one (two sub-tiles of C_out = 256); scale + shift + residual + ReLU applied;
+def test_benchmark_size_tiles_with_full_epilogue(oracle_lib, algorithm, c_in, c_out):
+    """More than 75 776 targets, so that the fused kernel runs with two 128-row
+    sub-tiles per CTA tile, once with two accumulator sets in TMEM (C_out = 64,
+    128) and once with one (C_out = 256); scale + shift + residual + ReLU applied;
     the same inputs through gather - GEMM - scatter."""
     from minuet_b200.nn.functional import convolution as conv_mod
     coords, bd = _dense_batch(21)
@@ -435,13 +435,13 @@ def test_benchmark_size_tiles_with_full_epilogue(oracle_lib, algorithm, sub_tile
     minuet.set_kernel_map_cache(conv, cache)
     xt, rt = dev(x).half(), dev(res).half()
     inp = minuet.SparseTensor(xt, dev(coords), batch_dims=dev(bd))
-    old = conv_mod.ALGORITHM, conv_mod.IMPLICIT_SUB_TILES
-    conv_mod.ALGORITHM, conv_mod.IMPLICIT_SUB_TILES = algorithm, sub_tiles
+    old = conv_mod.ALGORITHM
+    conv_mod.ALGORITHM = algorithm
     try:
         out = conv.forward_fused(inp, scale=dev(scale), shift=dev(shift), residual=rt, relu=True)
         plain = conv(inp)
     finally:
-        conv_mod.ALGORITHM, conv_mod.IMPLICIT_SUB_TILES = old
+        conv_mod.ALGORITHM = old
     off = generate_kernel_offsets(3, 3, 1, 1).astype(np.int32)
     m = oracle_lib.build_kernel_map(coords, coords, off, bd, bd)
     ref = oracle_lib.conv_forward(xt.float().cpu().numpy(), conv.kernel.detach().float().cpu().numpy(),
@@ -449,6 +449,16 @@ def test_benchmark_size_tiles_with_full_epilogue(oracle_lib, algorithm, sub_tile
     assert_close(plain.F, ref, torch.float16)
     ref = np.maximum(ref * scale + shift + rt.float().cpu().numpy(), 0)
     assert_close(out.F, ref, torch.float16)
+
+
+@pytest.mark.parametrize("sub_tiles", [1, 2])
+@pytest.mark.parametrize("c_in,c_out", [(64, 64), (128, 256), (32, 128)])
+def test_benchmark_size_tiles_with_either_number_of_sub_tiles(oracle_lib, monkeypatch, sub_tiles, c_in, c_out):
+    """The same with one and with two 128-row sub-tiles per CTA tile, whichever the rule picks: two accumulator
+    sets in TMEM, and one (two sub-tiles of 256 columns)."""
+    from minuet_b200.nn.functional import convolution as conv_mod
+    monkeypatch.setattr(conv_mod, "IMPLICIT_SUB_TILES", sub_tiles)
+    test_benchmark_size_tiles_with_full_epilogue(oracle_lib, "implicit", c_in, c_out)
 
 
 @pytest.mark.parametrize("dtype,c_in,c_out,kernel", [(torch.float32, 12, 24, 5), (torch.float16, 12, 24, 5),

@@ -21,13 +21,14 @@
 // of target t under mask row p, or -1) is derived once per kernel map from the
 // masks by mn_build_neighbor_table.  Every barrier wait is bounded (status bit 2).
 //
-// What bounds it.  The memory does not, on maps with three or more pairs a row: indices that are all -1
-// take the same time.  Up to 64 columns a CTA's step of some 1000 cycles (2 CTAs per SM) is the chain of
+// What bounds it.  Up to 128 columns and with three or more pairs a row the memory does not: indices that are all -1,
+// sequential or random take the same time.  Up to 64 columns a CTA's step of some 1000 cycles (2 CTAs per SM) is the chain of
 // one producer warp (wait, eight indices a lane, eight copies), before that it was the one warp that
-// sent index blocks and weights both.  At 128 columns shared memory: an M = N = 128 MMA reads 128 bytes of
-// operands per cycle, and the gathered rows and weights have to be written beside it.  At 256
-// columns the MMAs take 72 % of the cycles, at clocks that the power limit sets.  Sparser
-// maps: the epilogue (see there).  A warp needs five cycles per dependent
+// sent index blocks and weights both.  From 128 columns on shared memory: per 64-channel step of 128 rows the gathered rows and
+// weights are written (16 KB and 128 bytes a column) and read again by the MMAs, at 128 bytes a cycle 512 cycles
+// for 256 of MMA at 128 columns (measured 595 to 650), 768 for 512 at 256 (726 to 804).  There the
+// gather shows too, behind a ring of four stages: 524k rows 256->256, nine offsets, 408 us with indices of -1, 473
+// sequential, 506 random.  Sparser maps: the epilogue (see there).  A warp needs five cycles per dependent
 // instruction, so every role's loop is kept short: the issuing warps stay converged and elect
 // one lane only around the instruction itself (issued from a divergent lane-0 branch every MMA
 // took about 150 cycles of register moves), the index blocks arrive eight steps ahead and a lane

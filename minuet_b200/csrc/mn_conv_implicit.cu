@@ -53,7 +53,7 @@ constexpr int kUmmaK = 16;
 constexpr int kMaxStages = 8;
 constexpr int kMaxN = 256;
 constexpr int kIdxSlots = 8;           // steps the index blocks run ahead
-constexpr int kTileSlots = 2;          // tiles that a CTA holds at most beside the one it works on (see the index warp)
+constexpr int kTileSlots = 3;          // tiles that a CTA holds at most beside the one it works on (see the index warp)
 constexpr int kMaxSub = 2;             // 128-row sub-tiles per CTA tile
 constexpr int kResSlot = 32 * 64;      // bytes of 32 columns of 32 rows of the residual
 constexpr int kNBlock = kBK * 128;     // kMapNMajor: bytes of one block of 64 columns of a weight tile
@@ -482,8 +482,10 @@ conv_implicit_kernel(const __grid_constant__ ImArgs args,
     // ------------------------------ tiles and index blocks ---------------------
     // Tiles are handed out while the kernel runs: a CTA starts with the tile of its own number, counted from the last,
     // and takes over the tiles of blocks that have not started (cluster launch control) as it needs them, at most
-    // kTileSlots before its epilogue (with four the last CTAs had tiles left when others had none: 464k rows 64->64 of 1.15
-    // pairs with a residual 35.8 / 34.4, 406k 128->128 of 3.5 136 / 128).  Rows with many and rare offsets sort to the end, so the dear tiles go first.
+    // kTileSlots before its epilogue.  With four the last CTAs had tiles left when others had none, with two the answer to a
+    // request shows between tiles of few steps.  us, two / three / four: 464k rows 32->32 of 1.15 pairs with a residual 28.5 /
+    // 28.7 / 29.5, 105k rows 128->128 of 3 with one 45.7 / 47.9 / 48.2, 420k 120.5 / 120.9 / 123.8; 290k rows 128->256 of 1.1
+    // 53.1 / 52.0 / 52.0, 464k 192->48 of 1.15 45.8 / 44.9 / 44.4, 879k rows to strided ones 64->16 35.1 / 34.4 / 34.4.  Rows with many and rare offsets sort to the end, so the dear tiles go first.
     // With every gridDim-th tile for a CTA the busiest had 1.2 to 1.7 times the average of steps (one to
     // four clouds).  us, before / now: 406k rows of 3.4 pairs 64->64 70 / 59, 128->128 137 / 110, 256->256 328 /
     // 271; 1.8M of 9.3 256->256 3090 / 2810; 31k of 16.7 84 / 79.  The block's own tile is nobody's news, and where no

@@ -456,8 +456,13 @@ def test_benchmark_size_tiles_with_full_epilogue(oracle_lib, algorithm, c_in, c_
 def test_benchmark_size_tiles_with_either_number_of_sub_tiles(oracle_lib, monkeypatch, sub_tiles, c_in, c_out):
     """The same with one and with two 128-row sub-tiles per CTA tile, whichever the rule picks: two accumulator
     sets in TMEM, and one (two sub-tiles of 256 columns)."""
-    from minuet_b200.nn.functional import convolution as conv_mod
-    monkeypatch.setattr(conv_mod, "IMPLICIT_SUB_TILES", sub_tiles)
+    made = minuet.nn.SparseConv3d
+
+    def with_sub_tiles(*args, **kwargs):
+        conv = made(*args, **kwargs)
+        conv.tunable_config.update(sub_tiles=sub_tiles)
+        return conv
+    monkeypatch.setattr(minuet.nn, "SparseConv3d", with_sub_tiles)
     test_benchmark_size_tiles_with_full_epilogue(oracle_lib, "implicit", c_in, c_out)
 
 

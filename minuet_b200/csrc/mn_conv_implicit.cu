@@ -1240,7 +1240,11 @@ extern "C" mn_status mn_sparse_convolution_forward_implicit(
   // pairs leave the epilogue as the bound, which has half the warps with two.  64->128: 57k of 1.15 537 / 758, 50k of 3.4
   // 1033 / 1111, 5456 of 5.4 189 / 182, 9257 of 9.3 345 / 327, 878 of 12.6 39.8 / 40.3, with a residual 49.5 / 53.8.  128->128:
   // 12.6k of 3.5 416 / 415, with one 592 / 612, 10.1k of 7.5 541 / 527 and 683 / 638, 2331 of 9.3 153 / 148, 1083 of 7.2
-  // 58.7 / 59.3.  More input channels are more steps a tile: 256->128 12.6k of 3.5 775 / 723, 26.8k of 3.0 1225 / 1262.
+  // 58.7 / 59.3.  More input channels are more steps a tile, and without a residual the epilogue has less to do.  Without / with
+  // one: 192->128, 3.0k tiles of 3.0 117 / 115, 145 / 154; 4.8k of 2.6 158 / 154, 199 / 215; 4.8k of 2.0 125 / 126, 168 / 193;
+  // 2.6k of 4.6 144 / 138, 167 / 171; 5.1k of 4.6 298 / 285, 341 / 339.  256->128, 4.8k of 2.6 203 / 195, 243 / 252; 10.4k of 3.0 484 /
+  // 460, 585 / 610; 5.1k of 4.6 387 / 375, 439 / 436.  128->128, 3.0k of 3.0 88.2 / 88.6, 117 / 130; 4.8k of 2.6 118 / 118,
+  // 161 / 184; 10.4k of 3.0 273 / 262, 364 / 408; 5.1k of 4.6 214 / 204, 256 / 262.  128->96 5.2k of 3.0 141 / 144, 10.4k 236 / 231.
   // 128->64 0.96 to 1.04, 256->256 336 / 404.  Callers that have timed the layer pass their own choice.
   int sub = sub_hint;
   if (sub <= 0) {
@@ -1251,7 +1255,9 @@ extern "C" mn_status mn_sparse_convolution_forward_implicit(
     } else if (c_in <= 64 && a.n_pad <= 64) {
       if (pairs_per_row >= 3.0 && tiles >= 16 * kNumSMs && tiles * pairs_per_row >= 16384) sub = 2;
     } else if (a.n_pad > 64 && a.n_pad <= 128) {
-      if (pairs_per_row >= (c_in > 128 ? 3.2 : 5.0) && tiles >= 16 * kNumSMs) sub = 2;
+      const bool many = tiles >= 32 * kNumSMs;
+      const double line = a.residual != nullptr ? (c_in > 128 && many ? 3.6 : 5.0) : c_in > 128 ? 2.5 : c_in > 64 && many ? 3.0 : 5.0;
+      if (pairs_per_row >= line && tiles >= 16 * kNumSMs) sub = 2;
     }
   }
   MN_CHECK_ARG(sub_hint <= 4 && (sub_hint <= 0 || sub_hint * a.n_pad <= 512),
